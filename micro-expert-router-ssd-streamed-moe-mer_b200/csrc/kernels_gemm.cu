@@ -689,7 +689,7 @@ GemmScratch gemm_scratch(void *scratch, size_t scratch_bytes, uint32_t max_token
 }  // namespace
 
 bool gemm_ffn_supported(int dtype, uint32_t D, uint32_t F) {
-  return (dtype == MER_DTYPE_Q4_0 || dtype == MER_DTYPE_Q8_0) && D % 256 == 0 && F % 256 == 0;
+  return (dtype == MER_DTYPE_Q4_0 || dtype == MER_DTYPE_Q8_0) && D % 128 == 0 && F % 128 == 0;  // whole 128-row tiles, whole groups of four blocks
 }
 
 // Activation images: rows padded to whole passes (at most 3 x max_pairs rows), 4 bytes per value plus the skew.

@@ -51,7 +51,7 @@ struct StreamParams {
   int phase;                 // 0 = gate/up (+SiLU*mul), 1 = down
   const float *act;          // activations, row-major fp32: x [n_tokens x D] (gate/up) or h [P x F] (down)
   uint32_t act_per_pair;     // 1: rows indexed by pair (down); 0: by token = pair / slots (gate/up)
-  uint32_t rows;             // output rows of the projection (F for gate/up, D for down)
+  uint32_t packed_tiles;     // 16-row tiles of the projection (F / 8 for gate/up, D / 16 for down)
   uint32_t kb_total;         // 32-weight blocks per row
   uint32_t kb_split;         // blocks per K split (kb_total when n_ksplit == 1)
   uint32_t n_ksplit;
@@ -140,10 +140,10 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 160);  // [TP] pair index of each token of the current pass
   float *s_un = reinterpret_cast<float *>(smem + 192);          // [TP] its 2^24 / scale
   uint32_t *s_amax = reinterpret_cast<uint32_t *>(smem + 224);  // [TP] max |activation| of its row, as float bits
-  // per-block accumulator seeds, [TP][kb_split + 2]: the four token rows a warp reads together (one per t) must not start
+  // per-block accumulator seeds, [TP][about kb_split + 2]: the four token rows a warp reads together (one per t) must not start
   // in the same bank (a stride of 32 blocks put every 64-bit read four-deep on one bank pair: 25 % more shared-memory
   // wavefronts in the whole gate/up phase)
-  const uint32_t seed_stride = p.kb_split + 2;
+  const uint32_t seed_stride = (p.kb_split + 3) & ~1u;  // even: seeds are read two at a time
   float *s_init = reinterpret_cast<float *>(smem + HEADER_BYTES);
   uint8_t *s_frag = reinterpret_cast<uint8_t *>(s_init + seed_stride * TP);  // [TP*2][frag_stride]
   s_frag = reinterpret_cast<uint8_t *>(((size_t)s_frag + 127) & ~(size_t)127);
@@ -160,7 +160,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   }
   __syncthreads();
 
-  const uint32_t n_tiles = p.rows / ((p.phase == 0 ? 8u : 16u) * CONSUMER_WARPS);  // items per (pass, K split)
+  const uint32_t n_tiles = (p.packed_tiles + CONSUMER_WARPS - 1) / CONSUMER_WARPS;  // items per (pass, K split); the last one may hold fewer tiles
   const uint32_t n_passes = *d.n_passes;
   const uint64_t n_items = (uint64_t)n_passes * p.n_ksplit * n_tiles;
   // the grouping kernel cut the item list into one contiguous range per CTA, balanced by the tokens of the passes
@@ -197,15 +197,18 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       if (!base) continue;  // consumers skip the same item
       // item -> packed tiles 16*tile .. 16*tile + 15 of the phase's region; lane m < 16 copies tile m's chunk
       const uint8_t *src = base + (p.phase == 0 ? 0 : 2 * proj_bytes) + (size_t)(CONSUMER_WARPS * tile + my_tile) * tile_bytes;
+      // tiles of this producer that exist (none: the stage's other half still completes the barrier's second arrival)
+      const uint32_t first = CONSUMER_WARPS * tile + (warp - CONSUMER_WARPS) * TILES_PER_PRODUCER;
+      const uint32_t live = first >= p.packed_tiles ? 0u : min(TILES_PER_PRODUCER, p.packed_tiles - first);
       for (uint32_t c0 = 0; c0 < kbn && ok; c0 += p.kc) {
         uint32_t nb = min(p.kc, kbn - c0);
         if (round > 0) ok = mbar_wait(&empty[stage], (round - 1) & 1);
         if (*(volatile uint32_t *)s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(&full[stage], TILES_PER_PRODUCER * nb * 16 * BB);
+        if (lane == 0) mbar_expect_tx(&full[stage], live * nb * 16 * BB);
         __syncwarp();
-        if (lane < TILES_PER_PRODUCER)
+        if (lane < live)
           bulk_g2s(s_stage + (size_t)stage * stage_bytes + my_tile * p.chunk_stride, src + (size_t)(kb0 + c0) * 16 * BB, nb * 16 * BB,
                    &full[stage]);
         if (++stage == p.n_stages) stage = 0, round++;
@@ -304,8 +307,9 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         float *seed_dst = s_init + (size_t)my_tok * seed_stride;
         // float4 groups of this K split: 8 per block; a warp converts 4 blocks per step
 #pragma unroll 1
-        for (uint32_t q = my_sub * 32 + lane; q < kbn * 8; q += wpt * 32) {
-          float4 v = __ldg(reinterpret_cast<const float4 *>(row + (size_t)kb0 * 32) + q);
+        for (uint32_t q = my_sub * 32 + lane; q < ((kbn + 3) & ~3u) * 8; q += wpt * 32) {  // whole warps, the shuffles below need them
+          const bool inside = q < kbn * 8;
+          float4 v = inside ? __ldg(reinterpret_cast<const float4 *>(row + (size_t)kb0 * 32) + q) : make_float4(0, 0, 0, 0);
           v.x *= sc, v.y *= sc, v.z *= sc, v.w *= sc;  // exact (power of two) unless it overflows
           const uint32_t kbl = q >> 3, j0 = (q & 7u) * 4;
           uint32_t pos;
@@ -319,12 +323,14 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
             hi[i] = __half_as_ushort(h);
             lo[i] = __half_as_ushort(__float2half_rn(vs[i] - __half2float(h)));
           }
-          *reinterpret_cast<uint2 *>(hi_dst + kbl * 64 + pos * 2) = make_uint2(hi[0] | hi[1] << 16, hi[2] | hi[3] << 16);
-          *reinterpret_cast<uint2 *>(lo_dst + kbl * 64 + pos * 2) = make_uint2(lo[0] | lo[1] << 16, lo[2] | lo[3] << 16);
+          if (inside) {
+            *reinterpret_cast<uint2 *>(hi_dst + kbl * 64 + pos * 2) = make_uint2(hi[0] | hi[1] << 16, hi[2] | hi[3] << 16);
+            *reinterpret_cast<uint2 *>(lo_dst + kbl * 64 + pos * 2) = make_uint2(lo[0] | lo[1] << 16, lo[2] | lo[3] << 16);
+          }
           float sum = (v.x + v.y) + (v.z + v.w);  // eight consecutive lanes hold one block
 #pragma unroll
           for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          if ((lane & 7) == 0) seed_dst[kbl] = -zp * sum * (1.0f / POW2_24);
+          if (inside && (lane & 7) == 0) seed_dst[kbl] = -zp * sum * (1.0f / POW2_24);
         }
       }
       consumer_sync();  // fragments, seeds, s_pair, s_un visible to every warp
@@ -337,6 +343,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       const uint32_t rows_here = (p.phase == 0 ? 8u : 16u) * CONSUMER_WARPS;
       for (uint32_t i = threadIdx.x; i < rows_here * pcount; i += CONSUMER_WARPS * 32) {
         const uint32_t pair = d.perm[pstart + i / rows_here], row = tile * rows_here + i % rows_here;
+        if (row >= p.packed_tiles * (p.phase == 0 ? 8u : 16u)) continue;
         if (split_gate_up) {
           float *gp = p.out + ((size_t)ks * n_pairs + pair) * 2 * d.F;
           gp[row] = 0.0f, gp[d.F + row] = 0.0f;
@@ -399,11 +406,40 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       }
     };
 
+    // the last block of an odd K, alone: a single record (Q4_0: half a pair record)
+    auto do_last = [&](uint32_t rec, uint32_t kb) {
+      uint32_t a[4], ah[4];
+      float2 ds;
+      if (DT == MER_DTYPE_Q4_0) {
+        const uint2 w = lds64(rec + (piece16 >> 1));
+        ds = h2_to_f2(lds32(rec + 256 + g * 4));
+        unpack_q4(w.x, a), unpack_q4(w.y, ah);
+      } else {
+        const uint4 w = lds128(rec + piece16);
+        ds = h2_to_f2(lds32(rec + 512 + g * 4));
+        unpack_q8(w.x, w.y, a), unpack_q8(w.z, w.w, ah);
+      }
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        if (n > 0 && (uint32_t)n >= n_live) break;  // uniform
+        const uint4 bf = lds128(fa[n] + kb * 64);
+        const float seed = __uint_as_float(lds32(ia[n] + kb * 4));
+        float c1[4], c2[4];
+        mma_f16(c1, a[0], ah[0], a[1], ah[1], bf.x, bf.y, seed, 0.0f, seed, 0.0f);
+        mma_f16(c2, a[2], ah[2], a[3], ah[3], bf.z, bf.w, c1[0], c1[1], c1[2], c1[3]);
+        acc[n][0] = fmaf(ds.x, c2[0], acc[n][0]);
+        acc[n][1] = fmaf(ds.x, c2[1], acc[n][1]);
+        acc[n][2] = fmaf(ds.y, c2[2], acc[n][2]);
+        acc[n][3] = fmaf(ds.y, c2[3], acc[n][3]);
+      }
+    };
+
+    const bool my_tile_exists = CONSUMER_WARPS * tile + warp < p.packed_tiles;
     for (uint32_t c0 = 0; c0 < kbn; c0 += p.kc) {
       const uint32_t nb = min(p.kc, kbn - c0);
       if (!dead && !mbar_wait(&full[stage], round & 1)) dead = true;
       dead = __any_sync(0xffffffffu, dead);
-      if (!dead) {
+      if (!dead && my_tile_exists) {
         constexpr uint32_t PAIR_BYTES = 2 * 16 * BB;  // 576 (Q4_0) / 1088 (Q8_0)
         const uint32_t np = nb >> 1;                  // block pairs in this chunk
         uint32_t rec = stage0 + stage * stage_bytes;
@@ -414,6 +450,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
           do_pair(rec, kb);
           if (pr + 1 < np) do_pair(rec + PAIR_BYTES, kb + 2);
         }
+        if (nb & 1) do_last(stage0 + stage * stage_bytes + np * PAIR_BYTES, c0 + nb - 1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[stage]);
@@ -421,7 +458,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     }
 
     // ---- item epilogue: this warp's tile is complete over the item's K range; write it out
-    if (!dead) {
+    if (!dead && my_tile_exists) {
       const uint32_t ptile = CONSUMER_WARPS * tile + warp;  // packed tile index within the phase's region
 #pragma unroll
       for (int n = 0; n < NT; n++) {
@@ -649,8 +686,8 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   const uint32_t bb = dtype == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
   const uint32_t tp = 4 * nt;
   Plan pl{};
-  if (packed_tiles % CONSUMER_WARPS) return pl;
-  const uint64_t items_per_split = (uint64_t)active_groups * (packed_tiles / CONSUMER_WARPS);
+  const uint32_t tile_groups = (packed_tiles + CONSUMER_WARPS - 1) / CONSUMER_WARPS;
+  const uint64_t items_per_split = (uint64_t)active_groups * tile_groups;
   uint32_t n_ksplit = 1, kb_split = kb_total;
   if (max_ksplit > MAX_KSPLIT) max_ksplit = MAX_KSPLIT;
   // Pick the K split that minimises the busiest CTA's estimated time, in units of one block step (16 tiles x one
@@ -659,7 +696,6 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   // measures about 4 us, i.e. ~10 block steps of Q8_0 or ~20 of Q4_0 at the rate one SM streams.
   {
     const double rebuild = dtype == MER_DTYPE_Q4_0 ? 20.0 : 10.0, per_item = 2.0;
-    const uint32_t tile_groups = packed_tiles / CONSUMER_WARPS;
     double best = 1e30;
     uint32_t seen_split = 0;
     for (uint32_t n = 1; n <= max_ksplit; n++) {
@@ -681,7 +717,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   for (;;) {
     const uint32_t frag_cols = 2 * (max_group_tokens < tp ? max_group_tokens : tp);
     const uint32_t frag_stride = kb_split * 64 + 64;
-    const size_t fixed = HEADER_BYTES + (size_t)(kb_split + 2) * tp * 4 + 128 + (size_t)frag_cols * frag_stride;
+    const size_t fixed = HEADER_BYTES + (size_t)(kb_split + 3) * tp * 4 + 128 + (size_t)frag_cols * frag_stride;
     if (fixed < SMEM_LIMIT) {
       const size_t avail = SMEM_LIMIT - fixed;
       for (uint32_t ppw = 4; ppw >= 1; ppw >>= 1) {
@@ -758,7 +794,7 @@ cudaError_t launch_phase(const StreamParams &p, uint32_t nt, size_t smem, int gr
 
 bool stream_ffn_supported(int dtype, uint32_t D, uint32_t F) {
   if (dtype != MER_DTYPE_Q4_0 && dtype != MER_DTYPE_Q8_0) return false;
-  if (D == 0 || F == 0 || D % 256 != 0 || F % 256 != 0) return false;  // 16-byte aligned rows, whole 16-tile groups
+  if (D == 0 || F == 0 || D % 32 != 0 || F % 32 != 0) return false;  // rows of whole blocks: every tile chunk is a multiple of 16 bytes
   Plan a = make_plan(dtype, D / 32, F / 8, 1, 4, 1, 148, MAX_KSPLIT), b = make_plan(dtype, F / 32, D / 16, 1, 4, 1, 148, MAX_KSPLIT);
   return a.n_stages >= 2 && b.n_stages >= 2;
 }
@@ -803,8 +839,8 @@ void stream_bind(MoeDispatch &d, void *scratch, int sm_count) {
   const Plans pl = plan_dispatch(d, sm_count);
   d.tokens_per_pass = 4 * pl.nt;
   d.item_bounds = reinterpret_cast<uint32_t *>(base + L.bounds);
-  d.items_per_pass[0] = pl.gate_up.n_ksplit * (d.F / 8 / CONSUMER_WARPS);
-  d.items_per_pass[1] = pl.down.n_ksplit * (d.D / 16 / CONSUMER_WARPS);
+  d.items_per_pass[0] = pl.gate_up.n_ksplit * ((d.F / 8 + CONSUMER_WARPS - 1) / CONSUMER_WARPS);
+  d.items_per_pass[1] = pl.down.n_ksplit * ((d.D / 16 + CONSUMER_WARPS - 1) / CONSUMER_WARPS);
   d.n_ctas = (uint32_t)sm_count;
 }
 
@@ -824,7 +860,7 @@ cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaS
   p.d = d;
   // phase 0: gate/up, activations = x by token
   p.phase = 0, p.act = d.x, p.act_per_pair = 0;
-  p.rows = d.F, p.kb_total = d.D / 32, p.kb_split = pg.kb_split, p.n_ksplit = pg.n_ksplit, p.kc = pg.kc;
+  p.packed_tiles = d.F / 8, p.kb_total = d.D / 32, p.kb_split = pg.kb_split, p.n_ksplit = pg.n_ksplit, p.kc = pg.kc;
   p.n_stages = pg.n_stages, p.chunk_stride = pg.chunk_stride, p.frag_stride = pg.frag_stride, p.frag_cols = pg.frag_cols;
   p.out = pg.n_ksplit > 1 ? parts : d.h;
   auto launch = [&](size_t smem) {
@@ -850,7 +886,7 @@ cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaS
   if (ev_mid) cudaEventRecord(ev_mid, s);
   // phase 1: down, activations = h by pair, scaled by the row maxima collected above
   p.phase = 1, p.act = d.h, p.act_per_pair = 1;
-  p.rows = d.D, p.kb_total = d.F / 32, p.kb_split = pd.kb_split, p.n_ksplit = pd.n_ksplit, p.kc = pd.kc;
+  p.packed_tiles = d.D / 16, p.kb_total = d.F / 32, p.kb_split = pd.kb_split, p.n_ksplit = pd.n_ksplit, p.kc = pd.kc;
   p.n_stages = pd.n_stages, p.chunk_stride = pd.chunk_stride, p.frag_stride = pd.frag_stride, p.frag_cols = pd.frag_cols;
   p.out = pd.n_ksplit > 1 ? parts : d.y;
   // the weighted combine of the layer rides on the same launch when the caller asked for it

@@ -15,13 +15,14 @@
 //        [lane L][16 B] = quant bytes 4t..4t+3 of (slot g, blk 2p), (slot g+8, blk 2p),
 //                         (slot g, blk 2p+1), (slot g+8, blk 2p+1)                          (512 B)
 //        [g][4 x f16]   = scales in the same order                                          (64 B)
+//     and, when K / 32 is odd, the last block alone, 288 B: [lane L][8 B], [g][2 x f16]
 //   (g = lane / 4 and t = lane % 4 are the mma.sync m16n8k16 fragment coordinates.)
-//   Inside a record the 16-byte piece of lane L = (g, t) sits at position g*4 + ((t + g/2) % 4), not at L: the
+//   Inside a record the 16-byte (single block: 8-byte) piece of lane L = (g, t) sits at position g*4 + ((t + g/2) % 4), not at L: the
 //   streaming kernels read one piece per lane (any bijection is conflict-free for them), while the GEMM kernels'
 //   dequantisers read the four pieces of ONE row slot in four steps, all lanes at the same t; the rotation spreads the
 //   eight row slots of a step over all 32 banks of shared memory (without it: 8-way bank conflicts).
 //
-// Shapes whose rows are not multiples of 256 columns keep the reference's flat stream.
+// Shapes whose rows are not whole 32-value blocks keep the reference's flat stream.
 #pragma once
 
 #include <stdint.h>
@@ -56,6 +57,10 @@ __host__ __device__ inline PackedAddr packed_locate(uint32_t D, uint32_t F, int 
     const uint32_t bip = kb & 1u, jj = j & 15u, t = jj >> 2;
     a.quant = rec + (size_t)packed_piece(g, t) * 16 + bip * 8 + half * 4 + (jj & 3u);
     a.scale = rec + 512 + g * 8 + bip * 4 + half * 2;
+    if (kb == K / 32 - 1 && bip == 0) {  // odd K / 32: the last block has no partner
+      a.quant = rec + (size_t)packed_piece(g, t) * 8 + half * 4 + (jj & 3u);
+      a.scale = rec + 256 + g * 4 + half * 2;
+    }
   } else {
     const size_t rec = tile_base + (size_t)kb * 544;
     const uint32_t t = j >> 3;

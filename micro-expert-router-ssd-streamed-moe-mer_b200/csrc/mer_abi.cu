@@ -1975,10 +1975,10 @@ MER_EXPORT int mer_set_kernel_path(mer_backend *b, int path) {
   if (!b || path < 0 || path > 3) return MER_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(b->mu);
   if (path == 2 && !b->d_stream_scratch)
-    return fail(b, MER_ERR_INELIGIBLE, 0, MER_NONE, "streaming kernels need d_model and d_ff to be multiples of 256");
+    return fail(b, MER_ERR_INELIGIBLE, 0, MER_NONE, "streaming kernels need d_model and d_ff to be multiples of 32");
   if (path == 3 && !b->d_gemm_scratch)
     return fail(b, MER_ERR_INELIGIBLE, 0, MER_NONE,
-                "the GEMM kernels need d_model and d_ff to be multiples of 256 and a backend of at least %u tokens", 12u);
+                "the GEMM kernels need d_model and d_ff to be multiples of 128 and a backend of at least %u tokens", 12u);
   b->kernel_path = path;
   drop_graphs(b);
   return MER_OK;
