@@ -125,7 +125,8 @@ struct BlockBytes {
 };
 
 // --------------------------------------------------------------------------- main kernel
-template <int DT, int NT>
+// RAGGED: the last group of 16 tiles is not full, or K is no multiple of four blocks (the checks cost the even shapes 1 to 3 %).
+template <int DT, int NT, bool RAGGED>
 __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr uint32_t BB = BlockBytes<DT>::value;
@@ -199,7 +200,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       const uint8_t *src = base + (p.phase == 0 ? 0 : 2 * proj_bytes) + (size_t)(CONSUMER_WARPS * tile + my_tile) * tile_bytes;
       // tiles of this producer that exist (none: the stage's other half still completes the barrier's second arrival)
       const uint32_t first = CONSUMER_WARPS * tile + (warp - CONSUMER_WARPS) * TILES_PER_PRODUCER;
-      const uint32_t live = first >= p.packed_tiles ? 0u : min(TILES_PER_PRODUCER, p.packed_tiles - first);
+      const uint32_t live = !RAGGED ? TILES_PER_PRODUCER : first >= p.packed_tiles ? 0u : min(TILES_PER_PRODUCER, p.packed_tiles - first);
       for (uint32_t c0 = 0; c0 < kbn && ok; c0 += p.kc) {
         uint32_t nb = min(p.kc, kbn - c0);
         if (round > 0) ok = mbar_wait(&empty[stage], (round - 1) & 1);
@@ -307,8 +308,8 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         float *seed_dst = s_init + (size_t)my_tok * seed_stride;
         // float4 groups of this K split: 8 per block; a warp converts 4 blocks per step
 #pragma unroll 1
-        for (uint32_t q = my_sub * 32 + lane; q < ((kbn + 3) & ~3u) * 8; q += wpt * 32) {  // whole warps, the shuffles below need them
-          const bool inside = q < kbn * 8;
+        for (uint32_t q = my_sub * 32 + lane; q < (RAGGED ? (kbn + 3) & ~3u : kbn) * 8; q += wpt * 32) {  // whole warps, the shuffles below need them
+          const bool inside = !RAGGED || q < kbn * 8;
           float4 v = inside ? __ldg(reinterpret_cast<const float4 *>(row + (size_t)kb0 * 32) + q) : make_float4(0, 0, 0, 0);
           v.x *= sc, v.y *= sc, v.z *= sc, v.w *= sc;  // exact (power of two) unless it overflows
           const uint32_t kbl = q >> 3, j0 = (q & 7u) * 4;
@@ -343,7 +344,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       const uint32_t rows_here = (p.phase == 0 ? 8u : 16u) * CONSUMER_WARPS;
       for (uint32_t i = threadIdx.x; i < rows_here * pcount; i += CONSUMER_WARPS * 32) {
         const uint32_t pair = d.perm[pstart + i / rows_here], row = tile * rows_here + i % rows_here;
-        if (row >= p.packed_tiles * (p.phase == 0 ? 8u : 16u)) continue;
+        if (RAGGED && row >= p.packed_tiles * (p.phase == 0 ? 8u : 16u)) continue;
         if (split_gate_up) {
           float *gp = p.out + ((size_t)ks * n_pairs + pair) * 2 * d.F;
           gp[row] = 0.0f, gp[d.F + row] = 0.0f;
@@ -434,7 +435,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       }
     };
 
-    const bool my_tile_exists = CONSUMER_WARPS * tile + warp < p.packed_tiles;
+    const bool my_tile_exists = !RAGGED || CONSUMER_WARPS * tile + warp < p.packed_tiles;
     for (uint32_t c0 = 0; c0 < kbn; c0 += p.kc) {
       const uint32_t nb = min(p.kc, kbn - c0);
       if (!dead && !mbar_wait(&full[stage], round & 1)) dead = true;
@@ -450,7 +451,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
           do_pair(rec, kb);
           if (pr + 1 < np) do_pair(rec + PAIR_BYTES, kb + 2);
         }
-        if (nb & 1) do_last(stage0 + stage * stage_bytes + np * PAIR_BYTES, c0 + nb - 1);
+        if (RAGGED && (nb & 1)) do_last(stage0 + stage * stage_bytes + np * PAIR_BYTES, c0 + nb - 1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[stage]);
@@ -622,9 +623,9 @@ __device__ void ffn_stream_tail(const StreamParams &p) {
   }
 }
 
-template <int DT, int NT>
+template <int DT, int NT, bool RAGGED>
 __global__ void __launch_bounds__(THREADS, 1) k_ffn_stream(StreamParams p) {
-  ffn_stream_body<DT, NT>(p);
+  ffn_stream_body<DT, NT, RAGGED>(p);
   if (p.tail != TAIL_NONE) ffn_stream_tail(p);
 }
 
@@ -777,7 +778,9 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
 
 template <int DT>
 cudaError_t launch_phase(const StreamParams &p, uint32_t nt, size_t smem, int grid, cudaStream_t s) {
-  void (*kern)(StreamParams) = nt == 2 ? k_ffn_stream<DT, 2> : k_ffn_stream<DT, 1>;
+  const bool ragged = p.packed_tiles % CONSUMER_WARPS != 0 || p.kb_total % 4 != 0;
+  void (*kern)(StreamParams) = ragged ? (nt == 2 ? k_ffn_stream<DT, 2, true> : k_ffn_stream<DT, 1, true>)
+                                      : (nt == 2 ? k_ffn_stream<DT, 2, false> : k_ffn_stream<DT, 1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   if (p.tail != TAIL_NONE) {
