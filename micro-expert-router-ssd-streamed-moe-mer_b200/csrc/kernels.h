@@ -147,7 +147,23 @@ cudaError_t launch_dequant(int dtype, const uint8_t *src, float *dst, size_t n_w
 // Dequantises projection `matrix` (0 gate, 1 up, 2 down) of a packed expert into row-major f32.
 cudaError_t launch_dequant_packed(int dtype, const uint8_t *expert, int matrix, uint32_t D, uint32_t F, float *dst, cudaStream_t s);
 // Flat gate||up||down block stream -> tile-major fragment layout (same bytes, permuted).
-cudaError_t launch_repack(int dtype, const uint8_t *flat, uint8_t *packed, uint32_t D, uint32_t F, cudaStream_t s);
+// What an admission leaves beside the payload: the slot's header and the expert's table entry (slot null: only the entry).
+struct SlotHeader {  // at the start of every occupied slot
+  uint64_t epoch;
+  uint32_t expert_id;
+  uint32_t dtype;
+  uint64_t payload_bytes;
+};
+struct SlotWrite {
+  uint8_t *slot;
+  const uint8_t *payload;
+  const uint8_t **entry;
+  uint64_t epoch;
+  uint32_t expert_id, dtype;
+  uint64_t payload_bytes;
+};
+cudaError_t launch_repack(int dtype, const uint8_t *flat, uint8_t *packed, uint32_t D, uint32_t F, const SlotWrite &sw, cudaStream_t s);
+cudaError_t launch_slot_write(const SlotWrite &sw, cudaStream_t s);
 cudaError_t launch_raw_matvec(int dtype, const uint8_t *w, const float *x, float *y, size_t rows, size_t cols, cudaStream_t s);
 cudaError_t launch_f16_to_f32(const uint16_t *src, float *dst, size_t n, cudaStream_t s);
 cudaError_t launch_f32_to_f16(const float *src, uint16_t *dst, size_t n, cudaStream_t s);

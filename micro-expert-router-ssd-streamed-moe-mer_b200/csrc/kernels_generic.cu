@@ -1092,9 +1092,16 @@ __global__ void k_dequant_packed(const uint8_t *__restrict__ expert, int matrix,
   }
 }
 
+__device__ __forceinline__ void write_slot(const SlotWrite &sw) {
+  if (sw.slot) *reinterpret_cast<SlotHeader *>(sw.slot) = SlotHeader{sw.epoch, sw.expert_id, sw.dtype, sw.payload_bytes};
+  *sw.entry = sw.payload;
+}
+__global__ void k_slot_write(SlotWrite sw) { write_slot(sw); }
+
 // One thread per source block: copies its scale and its quant bytes to their packed places.
 template <int DT>
-__global__ void k_repack(const uint8_t *__restrict__ flat, uint8_t *__restrict__ packed, uint32_t D, uint32_t F) {
+__global__ void k_repack(const uint8_t *__restrict__ flat, uint8_t *__restrict__ packed, uint32_t D, uint32_t F, SlotWrite sw) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) write_slot(sw);  // readers wait for the event behind this kernel
   constexpr uint32_t BB = DT == MER_DTYPE_Q8_0 ? MER_Q8_BLOCK_BYTES : MER_Q4_BLOCK_BYTES;
   const size_t per_matrix = (size_t)D * F / 32;
   const size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -1273,11 +1280,15 @@ cudaError_t launch_dequant_packed(int dtype, const uint8_t *expert, int matrix, 
   return cudaGetLastError();
 }
 
-cudaError_t launch_repack(int dtype, const uint8_t *flat, uint8_t *packed, uint32_t D, uint32_t F, cudaStream_t s) {
+cudaError_t launch_repack(int dtype, const uint8_t *flat, uint8_t *packed, uint32_t D, uint32_t F, const SlotWrite &sw, cudaStream_t s) {
   if (dtype == MER_DTYPE_Q8_0)
-    k_repack<MER_DTYPE_Q8_0><<<148 * 8, 256, 0, s>>>(flat, packed, D, F);
+    k_repack<MER_DTYPE_Q8_0><<<148 * 8, 256, 0, s>>>(flat, packed, D, F, sw);
   else
-    k_repack<MER_DTYPE_Q4_0><<<148 * 8, 256, 0, s>>>(flat, packed, D, F);
+    k_repack<MER_DTYPE_Q4_0><<<148 * 8, 256, 0, s>>>(flat, packed, D, F, sw);
+  return cudaGetLastError();
+}
+cudaError_t launch_slot_write(const SlotWrite &sw, cudaStream_t s) {
+  k_slot_write<<<1, 1, 0, s>>>(sw);
   return cudaGetLastError();
 }
 

@@ -2,19 +2,23 @@
 // Host code only; kernels live in kernels_*.cu.  See include/mer_b200.h for the contract and
 // the reference interfaces each entry point replaces.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <thread>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <unordered_map>
 #include <vector>
 
 #include "../../include/mer_b200.h"
+#include "copy_pool.h"
 #include "kernels.h"
 
 #define MER_EXPORT extern "C" __attribute__((visibility("default")))
@@ -23,15 +27,9 @@ namespace {
 
 constexpr size_t SLOT_HEADER_BYTES = 256;  // {epoch, expert id, payload bytes}; payload stays 256-B aligned
 constexpr size_t SLOT_ALIGN = 4096;        // page-aligned slot stride (block_align of the reference's blobs)
-constexpr size_t STAGE_BYTES = 16u << 20;  // two pinned staging buffers for pageable host blobs
+constexpr size_t STAGE_BYTES = 32u << 20;  // pinned staging memory for pageable host blobs, used as STAGE_BUFS chunks
+constexpr size_t STAGE_BUFS = 8, STAGE_PIECE = 256u << 10;  // a piece is what one thread copies at a time
 constexpr uint32_t MAX_DIM = 1u << 20;
-
-struct SlotHeader {  // written at the start of every occupied slot
-  uint64_t epoch;
-  uint32_t expert_id;
-  uint32_t dtype;
-  uint64_t payload_bytes;
-};
 
 struct Slot {
   bool used = false, anchor = false;
@@ -58,7 +56,7 @@ struct mer_backend {
   int sm_count = 0;
   size_t expert_bytes = 0;
   cudaStream_t compute = nullptr, copy = nullptr;
-  cudaEvent_t ev_compute_done = nullptr, ev_copy_done = nullptr, ev_stage[2] = {nullptr, nullptr};
+  cudaEvent_t ev_compute_done = nullptr, ev_copy_done = nullptr, ev_stage[STAGE_BUFS] = {};
   bool copy_pending = false;
 
   // VRAM tier
@@ -67,9 +65,9 @@ struct mer_backend {
   std::vector<Slot> slots;
   std::unordered_map<uint32_t, size_t> id2slot;
   const uint8_t **d_expert_ptr = nullptr;  // device table: global id -> payload
-  const uint8_t **h_expert_ptr = nullptr;  // pinned mirror
-  uint8_t *h_stage[2] = {nullptr, nullptr};
-  SlotHeader *h_hdr = nullptr;  // pinned, one per slot
+  std::vector<const uint8_t *> h_expert_ptr;  // host mirror
+  uint8_t *h_stage = nullptr;                 // pinned, STAGE_BYTES
+  std::unique_ptr<CopyPool> copy_pool;
   uint64_t tick = 0;
 
   // workspace
@@ -382,7 +380,7 @@ void free_all(mer_backend *b) {
   F(b->arena), F(b->d_expert_ptr), F(b->d_x), F(b->d_out), F(b->d_h), F(b->d_y), F(b->d_pair_weight), F(b->d_logits);
   F(b->d_pair_expert), F(b->d_group_expert), F(b->d_offsets), F(b->d_perm), F(b->d_status), F(b->d_counters), F(b->d_group_count);
   F(b->d_f16), F(b->d_stream_scratch), F(b->d_gemm_scratch), F(b->d_dequant), F(b->d_raw_stage), F(b->d_xn), F(b->d_shared_scale);
-  H(b->h_expert_ptr), H(b->h_stage[0]), H(b->h_stage[1]), H(b->h_hdr), H(b->h_u32), H(b->h_f32);
+  H(b->h_stage), H(b->h_u32), H(b->h_f32);
   if (b->ev_compute_done) cudaEventDestroy(b->ev_compute_done);
   if (b->ev_copy_done) cudaEventDestroy(b->ev_copy_done);
   for (auto &e : b->ev_stage)
@@ -442,8 +440,7 @@ int acquire_slot(mer_backend *b, uint32_t id, uint64_t generation, uint32_t flag
     Slot &v = b->slots[victim];
     b->id2slot.erase(v.expert_id);
     b->h_expert_ptr[v.expert_id] = nullptr;
-    cudaMemcpyAsync((void *)(b->d_expert_ptr + v.expert_id), (void *)(b->h_expert_ptr + v.expert_id), sizeof(void *),
-                    cudaMemcpyHostToDevice, b->copy);
+    CU(MER_ERR_UPLOAD, "table kernel", launch_slot_write(SlotWrite{nullptr, nullptr, b->d_expert_ptr + v.expert_id, 0, v.expert_id, 0, 0}, b->copy));
     v.used = false;
     b->ctr.evictions++;
   }
@@ -454,6 +451,78 @@ int acquire_slot(mer_backend *b, uint32_t id, uint64_t generation, uint32_t flag
 
 // Fills `dst` with bytes [off, off + n) of the expert's gate||up||down stream; false = the source ran short.
 using ChunkReader = std::function<bool(size_t off, size_t n, uint8_t *dst)>;
+
+// Pageable bytes (or a reader's) -> pinned chunks -> `landing`, on the copy stream.  Several threads fill the chunks piece by
+// piece while the copy engine drains the finished ones; the calling thread enqueues chunks in order, hands freed buffers out
+// again, and copies pieces itself in between.  8-thread copies keep up with the link: 99 MB 8.4 ms -> 2.3 ms.
+int upload_staged(mer_backend *b, uint32_t id, uint8_t *landing, const uint8_t *src, const ChunkReader *reader) {
+  const uint32_t layer = 0, expert = id;
+  const size_t bytes = b->expert_bytes;
+  // about eight chunks per expert, so that the first one is on its way soon, of whole pieces
+  const size_t chunk = std::min(STAGE_BYTES / STAGE_BUFS, std::max((bytes / 8 + STAGE_PIECE - 1) / STAGE_PIECE, (size_t)1) * STAGE_PIECE);
+  const size_t n_chunks = (bytes + chunk - 1) / chunk, per_chunk = chunk / STAGE_PIECE, n_pieces = (bytes + STAGE_PIECE - 1) / STAGE_PIECE;
+  std::vector<std::atomic<uint32_t>> done(n_chunks);
+  for (auto &d : done) d.store(0, std::memory_order_relaxed);
+  std::atomic<size_t> next{0}, open{0};  // next piece to take; chunks whose buffer is free to be filled
+  std::atomic<bool> failed{false};
+  auto copy_piece = [&](size_t piece) {
+    const size_t off = piece * STAGE_PIECE, n = std::min(STAGE_PIECE, bytes - off), c = piece / per_chunk;
+    uint8_t *dst = b->h_stage + (c % STAGE_BUFS) * chunk + off % chunk;
+    if (!reader)
+      memcpy(dst, src + off, n);
+    else if (!(*reader)(off, n, dst))  // e.g. pread from an expert file, straight into the pinned staging memory
+      failed.store(true, std::memory_order_relaxed);
+    done[c].fetch_add(1, std::memory_order_release);
+  };
+  const std::function<void()> job = [&] {
+    for (;;) {
+      const size_t piece = next.fetch_add(1, std::memory_order_relaxed);
+      if (piece >= n_pieces) return;
+      while (open.load(std::memory_order_acquire) <= piece / per_chunk) {
+        if (failed.load(std::memory_order_relaxed)) return;
+        std::this_thread::yield();
+      }
+      copy_piece(piece);
+    }
+  };
+  const bool pool = n_pieces >= 4;
+  if (pool) {
+    if (!b->copy_pool) b->copy_pool.reset(new (std::nothrow) CopyPool());
+    if (b->copy_pool) b->copy_pool->start(&job);
+  }
+  cudaError_t e = cudaSuccess;
+  for (size_t c = 0; c < n_chunks && e == cudaSuccess && !failed.load(std::memory_order_relaxed);) {
+    const size_t ready = open.load(std::memory_order_relaxed);
+    if (ready < n_chunks && ready < c + STAGE_BUFS) {  // the buffer's previous chunk (of this or an earlier admission) has left it?
+      const cudaError_t q = cudaEventQuery(b->ev_stage[ready % STAGE_BUFS]);
+      if (q == cudaSuccess)
+        open.store(ready + 1, std::memory_order_release);
+      else if (q != cudaErrorNotReady)
+        e = q;
+    }
+    const uint32_t pieces = (uint32_t)std::min(per_chunk, n_pieces - c * per_chunk);
+    if (done[c].load(std::memory_order_acquire) == pieces) {
+      e = cudaMemcpyAsync(landing + c * chunk, b->h_stage + (c % STAGE_BUFS) * chunk, std::min(chunk, bytes - c * chunk), cudaMemcpyHostToDevice, b->copy);
+      if (e == cudaSuccess) e = cudaEventRecord(b->ev_stage[c % STAGE_BUFS], b->copy);
+      c++;
+      continue;
+    }
+    // a piece whose buffer is open, if one is left
+    size_t piece = next.load(std::memory_order_relaxed);
+    if (piece < n_pieces && piece / per_chunk < open.load(std::memory_order_relaxed)) {
+      if (next.compare_exchange_strong(piece, piece + 1, std::memory_order_relaxed)) copy_piece(piece);
+    }
+  }
+  const bool short_source = failed.load();
+  if (e != cudaSuccess) failed.store(true);
+  next.store(n_pieces);  // nothing more to take
+  open.store(n_chunks, std::memory_order_release);
+  if (pool && b->copy_pool) b->copy_pool->wait();
+  cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(b, MER_ERR_UPLOAD, layer, expert, "cudaMemcpyAsync(H2D staged)", e);
+  if (short_source || failed.load()) return fail(b, MER_ERR_UPLOAD, layer, expert, "the expert source ended before byte %zu", bytes);
+  return MER_OK;
+}
 
 int admit_impl(mer_backend *b, uint32_t id, uint64_t generation, const void *blob, size_t bytes, uint32_t flags,
                bool from_device, const ChunkReader *reader = nullptr) {
@@ -498,34 +567,19 @@ int admit_impl(mer_backend *b, uint32_t id, uint64_t generation, const void *blo
       CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(H2D pinned)",
          cudaMemcpyAsync(landing, src, b->expert_bytes, cudaMemcpyHostToDevice, b->copy));
     } else {
-      int which = 0;
-      for (size_t off = 0; off < b->expert_bytes; off += STAGE_BYTES, which ^= 1) {
-        size_t n = std::min(STAGE_BYTES, b->expert_bytes - off);
-        CU(MER_ERR_UPLOAD, "cudaEventSynchronize(stage)", cudaEventSynchronize(b->ev_stage[which]));
-        if (reader) {  // e.g. pread from an expert file, straight into the pinned staging buffer
-          if (!(*reader)(off, n, b->h_stage[which]))
-            return fail(b, MER_ERR_UPLOAD, layer, expert, "the expert source ended before byte %zu of %zu", off + n, b->expert_bytes);
-        } else {
-          memcpy(b->h_stage[which], src + off, n);
-        }
-        CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(H2D staged)",
-           cudaMemcpyAsync(landing + off, b->h_stage[which], n, cudaMemcpyHostToDevice, b->copy));
-        CU(MER_ERR_UPLOAD, "cudaEventRecord(stage)", cudaEventRecord(b->ev_stage[which], b->copy));
-      }
+      int rc = upload_staged(b, id, landing, src, reader);
+      if (rc) return rc;
     }
   }
+  // the slot header and the table entry are written by the kernel that fills the slot (a copy from a host mirror would read
+  // it whenever the copy stream gets there, by then perhaps changed by the next eviction)
+  const SlotWrite sw{slot_base, payload, b->d_expert_ptr + id, generation, id, (uint32_t)b->cfg.dtype, b->expert_bytes};
   if (b->packed)
     CU(MER_ERR_UPLOAD, "repack kernel",
-       launch_repack(b->cfg.dtype, landing, payload, (uint32_t)b->cfg.d_model, (uint32_t)b->cfg.d_ff, b->copy));
-  SlotHeader *hdr = b->h_hdr + si;
-  hdr->epoch = generation;
-  hdr->expert_id = id;
-  hdr->dtype = (uint32_t)b->cfg.dtype;
-  hdr->payload_bytes = b->expert_bytes;
-  CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(header)", cudaMemcpyAsync(slot_base, hdr, sizeof(SlotHeader), cudaMemcpyHostToDevice, b->copy));
+       launch_repack(b->cfg.dtype, landing, payload, (uint32_t)b->cfg.d_model, (uint32_t)b->cfg.d_ff, sw, b->copy));
+  else
+    CU(MER_ERR_UPLOAD, "table kernel", launch_slot_write(sw, b->copy));
   b->h_expert_ptr[id] = payload;
-  CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(table)",
-     cudaMemcpyAsync((void *)(b->d_expert_ptr + id), (void *)(b->h_expert_ptr + id), sizeof(void *), cudaMemcpyHostToDevice, b->copy));
   CU(MER_ERR_UPLOAD, "cudaEventRecord(copy)", cudaEventRecord(b->ev_copy_done, b->copy));
   b->copy_pending = true;
   s.used = true;
@@ -665,11 +719,8 @@ MER_EXPORT int mer_backend_create(const mer_backend_cfg *cfg, mer_backend **out)
   CB(cudaMalloc((void **)&b->arena, b->n_slots * b->slot_stride));
   CB(cudaMalloc((void **)&b->d_expert_ptr, sizeof(void *) * cfg->max_experts));
   CB(cudaMemset((void *)b->d_expert_ptr, 0, sizeof(void *) * cfg->max_experts));
-  CB(cudaHostAlloc((void **)&b->h_expert_ptr, sizeof(void *) * cfg->max_experts, cudaHostAllocDefault));
-  memset((void *)b->h_expert_ptr, 0, sizeof(void *) * cfg->max_experts);
-  CB(cudaHostAlloc((void **)&b->h_stage[0], STAGE_BYTES, cudaHostAllocDefault));
-  CB(cudaHostAlloc((void **)&b->h_stage[1], STAGE_BYTES, cudaHostAllocDefault));
-  CB(cudaHostAlloc((void **)&b->h_hdr, sizeof(SlotHeader) * b->n_slots, cudaHostAllocDefault));
+  b->h_expert_ptr.assign(cfg->max_experts, nullptr);
+  CB(cudaHostAlloc((void **)&b->h_stage, STAGE_BYTES, cudaHostAllocDefault));
   const size_t D = cfg->d_model, F = cfg->d_ff, T = cfg->max_tokens;
   b->max_pairs = cfg->max_tokens * cfg->max_top_k;
   const size_t P = b->max_pairs;
@@ -802,8 +853,9 @@ MER_EXPORT int mer_expert_admit_file(mer_backend *b, uint32_t expert_id, uint64_
   ChunkReader reader = [&](size_t off, size_t n, uint8_t *dst) -> bool {
     while (n) {  // canonical offset -> (projection, offset inside it) -> file offset
       const size_t pi = off / proj, in = off % proj, take = std::min<size_t>(n, proj - in);
-      if (pi >= 3 || fseeko(f, (off_t)(payload_off + range_off[pi] + in), SEEK_SET) != 0 || fread(dst, 1, take, f) != take) return false;
-      off += take, dst += take, n -= take;
+      const ssize_t got = pi < 3 ? pread(fileno(f), dst, take, (off_t)(payload_off + range_off[pi] + in)) : -1;  // several threads read
+      if (got <= 0) return false;
+      off += (size_t)got, dst += got, n -= (size_t)got;
     }
     return true;
   };
@@ -819,9 +871,7 @@ MER_EXPORT int mer_expert_retire(mer_backend *b, uint32_t expert_id, uint64_t ge
   CU(MER_ERR_UPLOAD, "cudaSetDevice", cudaSetDevice(b->cfg.device));
   CU(MER_ERR_UPLOAD, "order the copy stream after the readers", copy_waits_for_readers(b));
   b->h_expert_ptr[expert_id] = nullptr;
-  CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(table)",
-     cudaMemcpyAsync((void *)(b->d_expert_ptr + expert_id), (void *)(b->h_expert_ptr + expert_id), sizeof(void *),
-                     cudaMemcpyHostToDevice, b->copy));
+  CU(MER_ERR_UPLOAD, "table kernel", launch_slot_write(SlotWrite{nullptr, nullptr, b->d_expert_ptr + expert_id, 0, expert_id, 0, 0}, b->copy));
   CU(MER_ERR_UPLOAD, "cudaEventRecord(copy)", cudaEventRecord(b->ev_copy_done, b->copy));
   b->copy_pending = true;
   b->slots[it->second] = Slot{};
@@ -846,8 +896,7 @@ int retire_physical_locked(mer_backend *b, uint32_t id, uint32_t flags) {
   CU(MER_ERR_UPLOAD, "cudaSetDevice", cudaSetDevice(b->cfg.device));
   if (!(flags & MER_ADMIT_NO_READER_WAIT)) CU(MER_ERR_UPLOAD, "order the copy stream after the readers", copy_waits_for_readers(b));
   b->h_expert_ptr[id] = nullptr;
-  CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(table)",
-     cudaMemcpyAsync((void *)(b->d_expert_ptr + id), (void *)(b->h_expert_ptr + id), sizeof(void *), cudaMemcpyHostToDevice, b->copy));
+  CU(MER_ERR_UPLOAD, "table kernel", launch_slot_write(SlotWrite{nullptr, nullptr, b->d_expert_ptr + id, 0, id, 0, 0}, b->copy));
   CU(MER_ERR_UPLOAD, "cudaEventRecord(copy)", cudaEventRecord(b->ev_copy_done, b->copy));
   b->copy_pending = true;
   b->slots[it->second] = Slot{};
