@@ -1,21 +1,27 @@
-// Host threads that fill the pinned staging buffers of an admission: one thread copies pageable memory at about 11 GB/s, a fifth
+// Host threads that fill the pinned staging memory of an admission: one thread copies pageable memory at about 11 GB/s, a fifth
 // of what the PCIe link takes.  A pool belongs to one backend, is created on its first large pageable admission, holds at
-// most MAX_WORKERS threads that sleep between admissions, and ends with the backend.
+// most MAX_WORKERS threads, and ends with the backend.  Waking a sleeping thread costs 50 to 100 us in a virtual machine,
+// about what a 5 MB expert takes on the link: after a job the workers stay awake for SPIN_US, so that a run of admissions
+// finds them running, and nobody ever waits for a worker that woke too late to find work (jobs are shared, not borrowed).
 #pragma once
 
 #include <sched.h>
 
 #include <algorithm>
 #include <atomic>
+#include <chrono>
 #include <condition_variable>
 #include <functional>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <vector>
 
 class CopyPool {
  public:
-  static constexpr unsigned MAX_WORKERS = 8;
+  static constexpr unsigned MAX_WORKERS = 6;
+  static constexpr int SPIN_US = 500;
+  using Job = std::shared_ptr<const std::function<void()>>;  // owns everything it touches once its work is done
 
   CopyPool() {
     cpu_set_t set;
@@ -31,6 +37,7 @@ class CopyPool {
     {
       std::lock_guard<std::mutex> l(mu_);
       stop_ = true;
+      epoch_.fetch_add(1);
     }
     wake_.notify_all();
     for (auto &t : threads_) t.join();
@@ -38,39 +45,50 @@ class CopyPool {
   CopyPool(const CopyPool &) = delete;
   CopyPool &operator=(const CopyPool &) = delete;
 
-  // Every worker runs `job` once; wait() returns when all of them have left it.
-  void start(const std::function<void()> *job) {
-    std::lock_guard<std::mutex> l(mu_);
-    job_ = job, running_ = threads_.size(), epoch_++;
-    wake_.notify_all();
+  // Every worker that is awake, or wakes in time, runs `job` once.
+  void start(Job job) {
+    bool sleepers;
+    {
+      std::lock_guard<std::mutex> l(mu_);
+      job_ = std::move(job);
+      epoch_.fetch_add(1, std::memory_order_release);
+      sleepers = sleeping_ > 0;
+    }
+    if (sleepers) wake_.notify_all();
   }
-  void wait() {
-    std::unique_lock<std::mutex> l(mu_);
-    idle_.wait(l, [this] { return running_ == 0; });
-    job_ = nullptr;
+  // Lets go of the current job.
+  void finish() {
+    std::lock_guard<std::mutex> l(mu_);
+    job_.reset();
   }
 
  private:
   void loop() {
     uint64_t seen = 0;
-    std::unique_lock<std::mutex> l(mu_);
     for (;;) {
-      wake_.wait(l, [&] { return stop_ || epoch_ != seen; });
-      if (stop_) return;
-      seen = epoch_;
-      const std::function<void()> *job = job_;
-      l.unlock();
-      (*job)();
-      l.lock();
-      if (--running_ == 0) idle_.notify_all();
+      const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(SPIN_US);
+      while (epoch_.load(std::memory_order_acquire) == seen && std::chrono::steady_clock::now() < until) std::this_thread::yield();
+      Job job;
+      {
+        std::unique_lock<std::mutex> l(mu_);
+        if (epoch_.load() == seen) {
+          sleeping_++;
+          wake_.wait(l, [&] { return epoch_.load() != seen; });
+          sleeping_--;
+        }
+        if (stop_) return;
+        seen = epoch_.load();
+        job = job_;
+      }
+      if (job) (*job)();
     }
   }
 
   std::vector<std::thread> threads_;
   std::mutex mu_;
-  std::condition_variable wake_, idle_;
-  const std::function<void()> *job_ = nullptr;
-  size_t running_ = 0;
-  uint64_t epoch_ = 0;
+  std::condition_variable wake_;
+  Job job_;
+  std::atomic<uint64_t> epoch_{0};
+  unsigned sleeping_ = 0;
   bool stop_ = false;
 };

@@ -27,7 +27,7 @@ namespace {
 
 constexpr size_t SLOT_HEADER_BYTES = 256;  // {epoch, expert id, payload bytes}; payload stays 256-B aligned
 constexpr size_t SLOT_ALIGN = 4096;        // page-aligned slot stride (block_align of the reference's blobs)
-constexpr size_t STAGE_BYTES = 32u << 20;  // pinned staging memory for pageable host blobs, used as STAGE_BUFS chunks
+constexpr size_t STAGE_BYTES = 16u << 20;  // pinned staging memory for pageable host blobs, used as STAGE_BUFS chunks
 constexpr size_t STAGE_BUFS = 8, STAGE_PIECE = 256u << 10;  // a piece is what one thread copies at a time
 constexpr uint32_t MAX_DIM = 1u << 20;
 
@@ -454,73 +454,82 @@ using ChunkReader = std::function<bool(size_t off, size_t n, uint8_t *dst)>;
 
 // Pageable bytes (or a reader's) -> pinned chunks -> `landing`, on the copy stream.  Several threads fill the chunks piece by
 // piece while the copy engine drains the finished ones; the calling thread enqueues chunks in order, hands freed buffers out
-// again, and copies pieces itself in between.  8-thread copies keep up with the link: 99 MB 8.4 ms -> 2.3 ms.
+// again, and copies pieces itself in between.  Pageable 99 MB: 8.4 ms with one thread, 2.35 ms here, 1.95 ms from pinned memory; 5 MB: 0.36, 0.24, 0.12 ms.  (16 MB of chunks: with 8 MB the 99 MB took 3.1 ms, with 32 MB 2.85.)
 int upload_staged(mer_backend *b, uint32_t id, uint8_t *landing, const uint8_t *src, const ChunkReader *reader) {
   const uint32_t layer = 0, expert = id;
   const size_t bytes = b->expert_bytes;
   // about eight chunks per expert, so that the first one is on its way soon, of whole pieces
   const size_t chunk = std::min(STAGE_BYTES / STAGE_BUFS, std::max((bytes / 8 + STAGE_PIECE - 1) / STAGE_PIECE, (size_t)1) * STAGE_PIECE);
   const size_t n_chunks = (bytes + chunk - 1) / chunk, per_chunk = chunk / STAGE_PIECE, n_pieces = (bytes + STAGE_PIECE - 1) / STAGE_PIECE;
-  std::vector<std::atomic<uint32_t>> done(n_chunks);
-  for (auto &d : done) d.store(0, std::memory_order_relaxed);
-  std::atomic<size_t> next{0}, open{0};  // next piece to take; chunks whose buffer is free to be filled
-  std::atomic<bool> failed{false};
-  auto copy_piece = [&](size_t piece) {
+  struct State {  // shared with workers that may look at it after this call has returned (and find nothing left to do)
+    std::vector<std::atomic<uint32_t>> done;
+    std::atomic<size_t> next{0}, open{0};  // next piece to take; chunks whose buffer is free to be filled
+    std::atomic<bool> failed{false};
+    explicit State(size_t n) : done(n) {}
+  };
+  const auto st = std::make_shared<State>(n_chunks);
+  uint8_t *const stage = b->h_stage;
+  auto copy_piece = [st, stage, src, reader, bytes, chunk, per_chunk](size_t piece) {
     const size_t off = piece * STAGE_PIECE, n = std::min(STAGE_PIECE, bytes - off), c = piece / per_chunk;
-    uint8_t *dst = b->h_stage + (c % STAGE_BUFS) * chunk + off % chunk;
+    uint8_t *dst = stage + (c % STAGE_BUFS) * chunk + off % chunk;
     if (!reader)
       memcpy(dst, src + off, n);
     else if (!(*reader)(off, n, dst))  // e.g. pread from an expert file, straight into the pinned staging memory
-      failed.store(true, std::memory_order_relaxed);
-    done[c].fetch_add(1, std::memory_order_release);
+      st->failed.store(true, std::memory_order_relaxed);
+    st->done[c].fetch_add(1, std::memory_order_release);
   };
-  const std::function<void()> job = [&] {
-    for (;;) {
-      const size_t piece = next.fetch_add(1, std::memory_order_relaxed);
-      if (piece >= n_pieces) return;
-      while (open.load(std::memory_order_acquire) <= piece / per_chunk) {
-        if (failed.load(std::memory_order_relaxed)) return;
-        std::this_thread::yield();
-      }
-      copy_piece(piece);
-    }
+  // A worker takes a piece only when its buffer is open, so every piece that has been taken is being copied.
+  auto take = [st, n_pieces, per_chunk](size_t *piece) {
+    size_t p = st->next.load(std::memory_order_relaxed);
+    while (p < n_pieces && p / per_chunk < st->open.load(std::memory_order_acquire))
+      if (st->next.compare_exchange_weak(p, p + 1, std::memory_order_relaxed)) return *piece = p, true;
+    return false;
   };
   const bool pool = n_pieces >= 4;
   if (pool) {
     if (!b->copy_pool) b->copy_pool.reset(new (std::nothrow) CopyPool());
-    if (b->copy_pool) b->copy_pool->start(&job);
+    if (b->copy_pool)
+      b->copy_pool->start(std::make_shared<const std::function<void()>>([st, take, copy_piece, n_pieces] {
+        while (st->next.load(std::memory_order_relaxed) < n_pieces) {
+          size_t piece;
+          if (take(&piece))
+            copy_piece(piece);
+          else
+            std::this_thread::yield();
+        }
+      }));
   }
   cudaError_t e = cudaSuccess;
-  for (size_t c = 0; c < n_chunks && e == cudaSuccess && !failed.load(std::memory_order_relaxed);) {
-    const size_t ready = open.load(std::memory_order_relaxed);
-    if (ready < n_chunks && ready < c + STAGE_BUFS) {  // the buffer's previous chunk (of this or an earlier admission) has left it?
-      const cudaError_t q = cudaEventQuery(b->ev_stage[ready % STAGE_BUFS]);
-      if (q == cudaSuccess)
-        open.store(ready + 1, std::memory_order_release);
-      else if (q != cudaErrorNotReady)
-        e = q;
-    }
+  size_t c = 0;  // chunks enqueued
+  while (c < n_chunks && e == cudaSuccess && !st->failed.load(std::memory_order_relaxed)) {
     const uint32_t pieces = (uint32_t)std::min(per_chunk, n_pieces - c * per_chunk);
-    if (done[c].load(std::memory_order_acquire) == pieces) {
-      e = cudaMemcpyAsync(landing + c * chunk, b->h_stage + (c % STAGE_BUFS) * chunk, std::min(chunk, bytes - c * chunk), cudaMemcpyHostToDevice, b->copy);
+    if (st->done[c].load(std::memory_order_acquire) == pieces) {
+      e = cudaMemcpyAsync(landing + c * chunk, stage + (c % STAGE_BUFS) * chunk, std::min(chunk, bytes - c * chunk), cudaMemcpyHostToDevice, b->copy);
       if (e == cudaSuccess) e = cudaEventRecord(b->ev_stage[c % STAGE_BUFS], b->copy);
       c++;
       continue;
     }
-    // a piece whose buffer is open, if one is left
-    size_t piece = next.load(std::memory_order_relaxed);
-    if (piece < n_pieces && piece / per_chunk < open.load(std::memory_order_relaxed)) {
-      if (next.compare_exchange_strong(piece, piece + 1, std::memory_order_relaxed)) copy_piece(piece);
+    const size_t ready = st->open.load(std::memory_order_relaxed);
+    if (ready < n_chunks && ready < c + STAGE_BUFS) {  // has the buffer's previous chunk (of this or an earlier admission) left it?
+      const cudaError_t q = cudaEventQuery(b->ev_stage[ready % STAGE_BUFS]);
+      if (q == cudaSuccess)
+        st->open.store(ready + 1, std::memory_order_release);
+      else if (q != cudaErrorNotReady)
+        e = q;
+      if (q == cudaSuccess) continue;
     }
+    size_t piece;
+    if (take(&piece)) copy_piece(piece);
   }
-  const bool short_source = failed.load();
-  if (e != cudaSuccess) failed.store(true);
-  next.store(n_pieces);  // nothing more to take
-  open.store(n_chunks, std::memory_order_release);
-  if (pool && b->copy_pool) b->copy_pool->wait();
+  // on an early end: nothing more is taken, and what has been taken is copied to its end before the source may go away
+  for (size_t taken = st->next.exchange(n_pieces), k = 0; c < n_chunks && k < n_chunks; k++) {
+    const size_t first = k * per_chunk, last = std::min(std::min(first + per_chunk, n_pieces), taken);
+    while (first < last && st->done[k].load(std::memory_order_acquire) < last - first) std::this_thread::yield();
+  }
+  if (pool && b->copy_pool) b->copy_pool->finish();
   cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(b, MER_ERR_UPLOAD, layer, expert, "cudaMemcpyAsync(H2D staged)", e);
-  if (short_source || failed.load()) return fail(b, MER_ERR_UPLOAD, layer, expert, "the expert source ended before byte %zu", bytes);
+  if (st->failed.load()) return fail(b, MER_ERR_UPLOAD, layer, expert, "the expert source ended before byte %zu", bytes);
   return MER_OK;
 }
 
