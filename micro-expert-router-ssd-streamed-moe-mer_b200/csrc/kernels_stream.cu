@@ -33,6 +33,7 @@
 #include <type_traits>
 
 #include "../../include/mer_b200.h"
+#include "decode.cuh"
 #include "layout.cuh"
 #include "ptx.cuh"
 
@@ -42,7 +43,6 @@ constexpr int CONSUMER_WARPS = 16;
 constexpr int PRODUCER_WARPS = 2;  // each issues the bulk copies of half a stage's tiles: one warp alone was busy ~90 % of the time
 constexpr int THREADS = (CONSUMER_WARPS + PRODUCER_WARPS) * 32;
 constexpr uint32_t HEADER_BYTES = 1024;  // mbarriers and per-pass token tables at the start of shared memory
-constexpr float POW2_24 = 16777216.0f;
 
 constexpr int TAIL_NONE = 0, TAIL_FINALIZE = 1, TAIL_COMBINE = 2, TAIL_REDUCE = 3;
 
@@ -69,13 +69,6 @@ struct StreamParams {
   uint32_t *grid_counter;    // arrival counter of that barrier, zeroed by the grouping kernel
 };
 
-// D = A * B + C with separate C so that a seed / zero needs no register moves.
-__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                        uint32_t b1, float c0, float c1, float c2, float c3) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
-}
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMER_WARPS * 32) : "memory"); }
 
 
@@ -98,27 +91,7 @@ __device__ __forceinline__ void frag_slot(uint32_t j, uint32_t &pos, float &slot
   }
 }
 
-__device__ __forceinline__ float nan_max(float a, float b) { return (b > a || b != b) ? b : a; }  // NaN sticks
-
 // ------------------------------------------------------------------------ weight unpacking
-// Eight weights of one row slot of one block -> four f16x2 registers holding the integer fields as
-// subnormals: {MMA0.k(2t,2t+1), MMA0.k(2t+8,2t+9), MMA1.k(2t,2t+1), MMA1.k(2t+8,2t+9)}.
-__device__ __forceinline__ void unpack_q4(uint32_t v, uint32_t (&r)[4]) {
-  const uint32_t v8 = v >> 8;
-  r[0] = v & 0x000F000Fu;   // low nibbles of bytes 0, 2  -> elements 4t, 4t+2
-  r[1] = v8 & 0x000F000Fu;  // low nibbles of bytes 1, 3  -> elements 4t+1, 4t+3
-  r[2] = v & 0x00F000F0u;   // high nibbles -> elements 16 + ... (x16, undone on the activation side)
-  r[3] = v8 & 0x00F000F0u;
-}
-__device__ __forceinline__ void unpack_q8(uint32_t lo, uint32_t hi, uint32_t (&r)[4]) {
-  // int8 -> biased unsigned byte (q + 128) in the low mantissa bits
-  r[0] = (lo ^ 0x80808080u) & 0x00FF00FFu;
-  r[1] = ((lo >> 8) ^ 0x00808080u) & 0x00FF00FFu;
-  r[2] = (hi ^ 0x80808080u) & 0x00FF00FFu;
-  r[3] = ((hi >> 8) ^ 0x00808080u) & 0x00FF00FFu;
-}
-__device__ __forceinline__ float2 h2_to_f2(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2 *>(&v)); }
-
 template <int DT>
 struct BlockBytes {
   static constexpr uint32_t value = DT == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
@@ -501,12 +474,6 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     *(volatile uint32_t *)s_abort = 1;
     atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
   }
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
 }
 
 // Grid-wide barrier of a cooperative launch: every CTA arrives once; waits are bounded by wall-clock time.

@@ -34,6 +34,7 @@ constexpr size_t OFF_PERM = H_BYTES + 192;         // uint32 [MAX_TOKENS]
 constexpr size_t OFF_PAIR_EXPERT = H_BYTES + 320;  // uint32 [MAX_TOKENS]
 constexpr size_t OFF_PAIR_WEIGHT = H_BYTES + 448;  // float  [MAX_TOKENS]
 constexpr size_t OFF_STATUS = H_BYTES + 576;       // uint32 [1]
+constexpr size_t OFF_BAR = H_BYTES + 640;          // uint32 [2], zero between calls
 
 // Device code may name the array directly.  Everything a call depends on is rewritten here, because
 // the array still holds whatever the previous call left in it.
@@ -56,6 +57,7 @@ __global__ void k_noalloc_setup(const uint8_t *expert, uint32_t n_tokens) {
 constexpr int MAX_DEVICES = 64;
 std::mutex g_mu;
 unsigned char *g_scratch_ptr[MAX_DEVICES] = {};
+int g_sm_count[MAX_DEVICES] = {};
 
 void set_err(char *err, size_t err_len, const char *msg) {
   if (err && err_len) snprintf(err, err_len, "%s", msg);
@@ -90,6 +92,7 @@ MER_EXPORT int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint6
     return MER_ERR_DEVICE_LOST;
   }
   unsigned char *scratch;
+  int sm_count;
   {
     // First call on this device: resolve the device address of the static array (no allocation).
     std::lock_guard<std::mutex> lock(g_mu);
@@ -101,11 +104,20 @@ MER_EXPORT int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint6
         cudaGetLastError();
         return MER_ERR_RUNTIME_INVARIANT;
       }
+      if (cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sm_count[dev] = 0;
       g_scratch_ptr[dev] = p;
     }
     scratch = g_scratch_ptr[dev];
+    sm_count = g_sm_count[dev];
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (sm_count > 0 && flat_expert_supported(d_expert_blob, d_x, (uint32_t)d_model, (uint32_t)d_ff, (uint32_t)n_tokens)) {
+    cudaError_t e = launch_flat_expert(dtype, static_cast<const uint8_t *>(d_expert_blob), d_x, reinterpret_cast<float *>(scratch), d_out, (uint32_t)d_model,
+                                       (uint32_t)d_ff, (uint32_t)n_tokens, swiglu_limit, reinterpret_cast<uint32_t *>(scratch + OFF_BAR),
+                                       reinterpret_cast<uint32_t *>(scratch + OFF_STATUS), sm_count, s);
+    if (e == cudaSuccess) return MER_OK;
+    cudaGetLastError();  // no cooperative launch to be had: the kernels for any shape below
+  }
   MoeDispatch d{};
   d.expert_ptr = reinterpret_cast<const uint8_t *const *>(scratch + OFF_EXPERT_PTR);
   d.max_experts = 1;

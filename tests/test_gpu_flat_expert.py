@@ -1,0 +1,33 @@
+"""The one-launch kernel behind mer_expert_forward_noalloc, at the sizes where it can go wrong: rows that start off a 16-byte
+boundary, one block, several K ranges with a short last one, more and fewer tiles than CTAs, one to eight tokens."""
+import importlib
+
+import numpy as np
+import pytest
+
+import mer_b200
+import oracle
+
+pytestmark = pytest.mark.gpu
+synth = importlib.import_module("mer_b200.synth")
+
+
+@pytest.mark.parametrize("dtype,D,F,n", [
+    (mer_b200.DTYPE_Q4_0, 32, 32, 1), (mer_b200.DTYPE_Q4_0, 96, 160, 4), (mer_b200.DTYPE_Q4_0, 256, 512, 5),
+    (mer_b200.DTYPE_Q4_0, 4352, 288, 8), (mer_b200.DTYPE_Q4_0, 256, 4864, 3), (mer_b200.DTYPE_Q8_0, 64, 96, 8),
+    (mer_b200.DTYPE_Q8_0, 2304, 288, 2), (mer_b200.DTYPE_Q8_0, 512, 2336, 7), (mer_b200.DTYPE_Q8_0, 2048, 768, 4)])
+def test_flat_expert_matches_the_oracle(dtype, D, F, n):
+    import torch
+    blob = synth.make_expert_blob(dtype, D, F, 91, 0, 0)
+    x = synth.make_activations(n, D, 91)
+    x[0] *= 1e-3
+    d_blob, d_x = torch.from_numpy(blob).cuda(), torch.from_numpy(x).cuda()
+    d_out = torch.full((n, D), float("nan"), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for _ in range(2):
+        mer_b200.expert_forward_noalloc(dtype, D, F, d_blob.data_ptr(), d_x.data_ptr(), n, d_out.data_ptr(), 0.0, stream)
+    torch.cuda.synchronize()
+    got = d_out.cpu().numpy()
+    for t in range(n):
+        ref = oracle.expert_forward(dtype, blob, x[t], D, F)
+        assert np.abs(got[t] - ref).max() <= 1e-3 * np.sqrt(np.mean(ref.astype(np.float64) ** 2))
