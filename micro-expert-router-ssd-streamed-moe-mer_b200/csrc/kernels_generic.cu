@@ -7,12 +7,9 @@
 #include "kernels.h"
 
 #include <cuda_fp16.h>
-#include <math_constants.h>
-
-#include <climits>
-
 #include "../../include/mer_b200.h"
 #include "layout.cuh"
+#include "route.cuh"
 
 namespace {
 
@@ -64,15 +61,6 @@ __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + expf(-x));
 __device__ __forceinline__ float clamp_gate(float g, float limit) {
   if (limit > 0.0f && isfinite(limit) && g == g) g = fminf(fmaxf(g, -limit), limit);  // NaN stays NaN
   return g;
-}
-
-// Order of f32::total_cmp as a signed integer key (gating.rs:283-294 compares with total_cmp).
-__device__ __forceinline__ int total_key(float f) {
-  int b = __float_as_int(f);
-  return b ^ (int)(((unsigned)(b >> 31)) >> 1);
-}
-__device__ __forceinline__ bool better(int ka, uint32_t ia, int kb, uint32_t ib) {
-  return ka > kb || (ka == kb && ia < ib);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -406,210 +394,6 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
   if (d.pass_group) build_passes_block(d, s_off);
 }
 
-// Scoring, group filter, top-k and mixing weights of one token by one warp.
-// s_score / s_sel / s_ok are this warp's shared arrays of E entries; logits are already in s_score.
-__device__ void route_token(const RouterDev &r, const MoeDispatch &d, uint32_t token, float *s_score, float *s_sel,
-                            uint8_t *s_ok, uint32_t *s_groups, float *s_gscore, bool count_groups) {
-  const uint32_t E = r.num_experts, lane = threadIdx.x & 31;
-  constexpr int REG_E = 8;  // up to 32 * REG_E experts: selection keys live in registers
-  const bool small = E <= 32 * REG_E;
-  float cbias[REG_E];  // correction bias, fetched now so that its latency hides behind the scoring
-#pragma unroll
-  for (int j = 0; j < REG_E; j++) cbias[j] = (small && r.correction_bias && lane + 32 * j < E) ? __ldg(r.correction_bias + lane + 32 * j) : 0.0f;
-  if (r.logit_bias)
-#pragma unroll 1
-    for (uint32_t i = lane; i < E; i += 32) s_score[i] += __ldg(r.logit_bias + i);
-  __syncwarp();
-  if (r.scoring == MER_SCORE_SOFTMAX) {
-    // softmax_inplace (transformer.rs:2747-2819)
-    float mx = -CUDART_INF_F;
-    int nan = 0;
-#pragma unroll 1
-    for (uint32_t i = lane; i < E; i += 32) {
-      float v = s_score[i];
-      if (v != v)
-        nan = 1;
-      else if (v > mx)
-        mx = v;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      nan |= __shfl_xor_sync(0xffffffffu, nan, o);
-    }
-    if (nan || !isfinite(mx)) {
-#pragma unroll 1
-      for (uint32_t i = lane; i < E; i += 32) s_score[i] = 1.0f / (float)E;
-      if (lane == 0) atomicOr(d.status, MER_DEVSTAT_NONFINITE_ROUTER);
-    } else {
-#pragma unroll 1
-      for (uint32_t i = lane; i < E; i += 32) s_score[i] = expf(s_score[i] - mx);
-      __syncwarp();
-      float sum = 0.0f;
-      if (lane == 0) {  // the reference sums left to right; keep that order
-        if ((E & 3u) == 0) {
-          const float4 *s4 = reinterpret_cast<const float4 *>(s_score);  // E % 4 == 0 keeps every warp's array 16-byte aligned
-#pragma unroll 4
-          for (uint32_t i = 0; i < E / 4; i++) {
-            const float4 v = s4[i];
-            sum += v.x, sum += v.y, sum += v.z, sum += v.w;
-          }
-        } else {
-#pragma unroll 1
-          for (uint32_t i = 0; i < E; i++) sum += s_score[i];
-        }
-      }
-      sum = __shfl_sync(0xffffffffu, sum, 0);
-      if (sum > 0.0f)
-#pragma unroll 1
-        for (uint32_t i = lane; i < E; i += 32) s_score[i] = s_score[i] / sum;
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t i = lane; i < E; i += 32) s_score[i] = 1.0f / (1.0f + expf(-s_score[i]));
-  }
-  __syncwarp();
-  if (small) {
-#pragma unroll
-    for (int j = 0; j < REG_E; j++) {
-      const uint32_t i = lane + 32 * j;
-      if (i < E) s_sel[i] = r.correction_bias ? s_score[i] + cbias[j] : s_score[i], s_ok[i] = 1;
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t i = lane; i < E; i += 32) {
-      s_sel[i] = r.correction_bias ? s_score[i] + r.correction_bias[i] : s_score[i];
-      s_ok[i] = 1;
-    }
-  }
-  __syncwarp();
-  // group_filter_shape + select_top_groups (gating.rs:335-376)
-  const uint32_t ng = r.n_group < 1 ? 1 : r.n_group;
-  const bool grouped = ng > 1 && r.topk_group > 0 && r.topk_group < ng && (E % ng) == 0 && ng <= 64;
-  if (grouped) {
-    const uint32_t gs = E / ng;
-#pragma unroll 1
-    for (uint32_t gi = lane; gi < ng; gi += 32) {
-      float top1 = -CUDART_INF_F, top2 = -CUDART_INF_F;
-#pragma unroll 1
-      for (uint32_t i = 0; i < gs; i++) {
-        float s = s_sel[gi * gs + i];
-        if (s > top1) {
-          top2 = top1;
-          top1 = s;
-        } else if (s > top2) {
-          top2 = s;
-        }
-      }
-      s_gscore[gi] = top1 + (isfinite(top2) ? top2 : 0.0f);
-    }
-    __syncwarp();
-    if (lane == 0) {
-      uint64_t taken = 0;
-#pragma unroll 1
-      for (uint32_t n = 0; n < r.topk_group; n++) {
-        int bk = 0;
-        uint32_t bi = MER_NONE;
-#pragma unroll 1
-        for (uint32_t g = 0; g < ng; g++) {
-          if (taken >> g & 1) continue;
-          int k = total_key(s_gscore[g]);
-          if (bi == MER_NONE || better(k, g, bk, bi)) bk = k, bi = g;
-        }
-        taken |= 1ull << bi;
-        s_groups[n] = bi;
-      }
-    }
-    __syncwarp();
-#pragma unroll 1
-    for (uint32_t i = lane; i < E; i += 32) {
-      bool ok = false;
-#pragma unroll 1
-      for (uint32_t n = 0; n < r.topk_group; n++) ok |= (s_groups[n] == i / gs);
-      s_ok[i] = ok;
-    }
-    __syncwarp();
-  }
-  // top-k by (selection desc, id asc), non-finite skipped (gating.rs:315-333, 429-441)
-  const uint32_t S = d.slots, k = r.top_k;
-  uint32_t my_id = MER_NONE;  // lane i keeps the i-th pick
-  uint32_t n_sel = 0;
-  if (small) {
-    // keys in registers: lane l holds experts l, l + 32, ...; a taken or disallowed expert bids INT_MIN
-    int keys[REG_E];
-#pragma unroll
-    for (int j = 0; j < REG_E; j++) {
-      const uint32_t i = lane + 32 * j;
-      const float sv = i < E ? s_sel[i] : 0.0f;
-      keys[j] = (i < E && s_ok[i] && isfinite(sv)) ? total_key(sv) : INT_MIN;
-    }
-#pragma unroll 1
-    for (uint32_t n = 0; n < k; n++) {
-      int bk = INT_MIN;
-      uint32_t bj = 0;
-#pragma unroll
-      for (int j = 0; j < REG_E; j++)
-        if (keys[j] > bk) bk = keys[j], bj = j;  // ascending j keeps the lowest id on ties
-      const int top_key = __reduce_max_sync(0xffffffffu, bk);
-      if (top_key == INT_MIN) break;  // nothing left to pick
-      const uint32_t top_id = __reduce_min_sync(0xffffffffu, bk == top_key ? lane + 32 * bj : MER_NONE);
-      if (lane == (top_id & 31u)) {
-#pragma unroll
-        for (int j = 0; j < REG_E; j++)
-          if ((uint32_t)j == (top_id >> 5)) keys[j] = INT_MIN;
-      }
-      if (lane == (n & 31)) my_id = top_id;
-      n_sel++;
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t n = 0; n < k; n++) {
-      int bk = 0;
-      uint32_t bi = MER_NONE;
-#pragma unroll 1
-      for (uint32_t i = lane; i < E; i += 32) {
-        float s = s_sel[i];
-        if (!s_ok[i] || !isfinite(s)) continue;
-        int key = total_key(s);
-        if (bi == MER_NONE || key > bk) bk = key, bi = i;  // ascending scan keeps the lowest id on ties
-      }
-      // warp arg-max by (key desc, id asc): two warp reductions; lanes without a candidate bid the lowest key
-      const int my_key = bi == MER_NONE ? INT_MIN : bk;
-      const int top_key = __reduce_max_sync(0xffffffffu, my_key);
-      const uint32_t top_id = __reduce_min_sync(0xffffffffu, (bi != MER_NONE && my_key == top_key) ? bi : MER_NONE);
-      bk = top_key, bi = top_id;
-      if (bi == MER_NONE) break;
-      if (lane == 0) s_ok[bi] = 0;
-      if (lane == (n & 31)) my_id = bi;
-      n_sel++;
-      __syncwarp();
-    }
-  }
-  // mixing weights = unbiased scores; renormalise; scale (gating.rs:443-474)
-  float w = (lane < n_sel && my_id != MER_NONE) ? s_score[my_id] : 0.0f;
-  if (r.normalise) {
-    float sum = 0.0f;
-#pragma unroll 1
-    for (uint32_t i = 0; i < n_sel; i++) sum += __shfl_sync(0xffffffffu, w, i);  // slot order
-    if (isfinite(sum) && sum > 0.0f) w = w / sum;
-  }
-  if (r.scaling != 1.0f && isfinite(r.scaling)) w = w * r.scaling;
-  if (lane < k) {
-    bool have = lane < n_sel;
-    d.pair_expert[(size_t)token * S + lane] = have ? r.id_base + my_id : MER_NONE;
-    d.pair_weight[(size_t)token * S + lane] = have ? w : 0.0f;
-    if (count_groups && have) atomicAdd(d.group_count + my_id, 1u);  // the grid-wide grouping's count step, done here
-  }
-  if (lane == 0) {
-    if (n_sel < k) atomicOr(d.status, MER_DEVSTAT_SHORT_SELECTION);
-    if (S > k) {
-      if (count_groups) atomicAdd(d.group_count + E, 1u);
-      d.pair_expert[(size_t)token * S + k] = r.shared_expert_id;
-      d.pair_weight[(size_t)token * S + k] = r.shared_scale ? r.shared_scale[token] : 1.0f;
-    }
-  }
-}
-
 // Router logits of a large batch as a tiled fp32 GEMM: logits[t][e] = x[t] . w[e].  A CTA computes 32 tokens x 64
 // experts; K runs in chunks of 256 values that cp.async double-buffers in shared memory.  Eight warps split every
 // chunk (32 values of K each); a thread holds 8 tokens x 8 experts (rows ty + 4 i and tx + 8 j: neighbouring lanes read
@@ -816,7 +600,18 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
       for (uint32_t i = lane; i < E; i += 32) s_score[i] = single ? s_logit[warp][i] : __ldcg(d.logits + (size_t)token * E + i);
     }
     __syncwarp();
-    route_token(r, d, token, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], group_here == 2);
+    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], d.status);
+    const size_t p0 = (size_t)token * d.slots;
+    if (lane < r.top_k) {
+      d.pair_expert[p0 + lane] = pick.id == MER_NONE ? MER_NONE : r.id_base + pick.id;
+      d.pair_weight[p0 + lane] = pick.weight;
+      if (group_here == 2 && pick.id != MER_NONE) atomicAdd(d.group_count + pick.id, 1u);  // the grid-wide grouping's count step, done here
+    }
+    if (lane == 0 && d.slots > r.top_k) {
+      if (group_here == 2) atomicAdd(d.group_count + E, 1u);
+      d.pair_expert[p0 + r.top_k] = r.shared_expert_id;
+      d.pair_weight[p0 + r.top_k] = r.shared_scale ? r.shared_scale[token] : 1.0f;
+    }
   }
   if (group_here != 1) return;  // a large dispatch is grouped by the grid-wide kernels that follow (2: their count step is done above)
   __syncthreads();
