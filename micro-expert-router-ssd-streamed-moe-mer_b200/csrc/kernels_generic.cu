@@ -647,6 +647,7 @@ __global__ void k_groups_from_pairs(MoeDispatch d, int single_group) {
     }
   }
   if (threadIdx.x == 0) {
+    *d.status = 0;
     if (single_group) {
       d.group_expert[0] = d.pair_expert[0];
       d.offsets[0] = 0;

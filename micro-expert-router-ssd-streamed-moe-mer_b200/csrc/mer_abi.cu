@@ -83,6 +83,12 @@ struct mer_backend {
   uint32_t max_groups = 0, max_router_experts = 0;
   uint32_t *h_u32 = nullptr;  // pinned [max_pairs + 1]: ids up/down, status
   float *h_f32 = nullptr;     // pinned [max_pairs]
+  // host entry points: what goes up and what comes back lies together, so that each way is one copy of a captured sequence
+  float *d_step = nullptr, *h_step = nullptr;  // one token: [x D | ids | weights] (step_words floats), then [out D | status]
+  size_t step_words = 0;
+  float *h_rows = nullptr;     // pinned rows in, then rows out, rows_floats each (allocated on the first call that needs it)
+  size_t rows_floats = 0;
+  uint32_t *h_route = nullptr;  // pinned [3 x max_pairs]: routing, mixing weights, status
   float *d_dequant = nullptr;
   bool packed = false;          // slots hold the tile-major fragment layout (block-aligned shapes)
   uint8_t *d_raw_stage = nullptr;  // device copy of one flat blob, source of the repack at admission
@@ -115,8 +121,7 @@ struct mer_backend {
   struct GraphEntry {
     uint32_t layer;
     size_t n_tokens;
-    const void *x, *out, *ids, *w;
-    cudaStream_t stream;
+    const void *x, *out, *ids, *w;  // the buffers a caller passed, or a tag in `ids` for the other entry points
     cudaGraphExec_t exec;
     int launches;
   };
@@ -124,12 +129,15 @@ struct mer_backend {
   bool graphs_ok = true;
   // Streams other than `compute` that device entry points were last enqueued on, each with an event recorded after
   // the call: an admission or a retire makes the copy stream wait for all of them before it touches a slot.
+  // The legacy default stream is never destroyed: its event is recorded when an admission needs it, not on every call.
   struct UserStream {
     cudaStream_t stream;
     cudaEvent_t done;
     uint64_t last_use;
   };
   std::vector<UserStream> user_streams;
+  cudaEvent_t ev_legacy = nullptr;
+  bool legacy_used = false;
   // stage timing: sets of 5 events {start, after router, mid FFN, after FFN, after combine}
   bool timing_on = false;
   std::vector<cudaEvent_t> timing_events;
@@ -210,6 +218,10 @@ constexpr size_t MAX_USER_STREAMS = 8;
 // Records that work reading the slot arena was just enqueued on caller stream `s`.
 cudaError_t note_stream_use(mer_backend *b, cudaStream_t s) {
   if (s == b->compute) return cudaSuccess;  // ordered through ev_compute_done
+  if (s == nullptr || s == cudaStreamLegacy) {
+    b->legacy_used = true;
+    return cudaSuccess;
+  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -246,6 +258,12 @@ cudaError_t copy_waits_for_readers(mer_backend *b) {
   if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, b->ev_compute_done, 0);
   for (auto &u : b->user_streams)
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, u.done, 0);
+  if (e == cudaSuccess && b->legacy_used) {
+    if (!b->ev_legacy) e = cudaEventCreateWithFlags(&b->ev_legacy, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(b->ev_legacy, cudaStreamLegacy);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, b->ev_legacy, 0);
+    b->legacy_used = false;
+  }
   return e;
 }
 
@@ -329,6 +347,51 @@ void drop_graphs(mer_backend *b) {
   b->graphs.clear();
 }
 
+// Tags of captured sequences that are not mer_moe_layer_forward_device's.
+const void *graph_tag(uintptr_t n) { return reinterpret_cast<const void *>(n); }
+constexpr uintptr_t TAG_HOST_LAYER = 1, TAG_EP = 2, TAG_ROUTE = 3, TAG_STEP = 4, TAG_HOST_STAGED = 5;
+
+// The captured launch sequence of `key`, captured now on the backend's own stream if need be (`enqueue(&launches)` issues it
+// there); *out stays null where capture is not to be had.  A graph is launched into whatever stream the caller brings, the
+// legacy default stream included, which itself cannot be captured.
+template <typename Enqueue>
+int captured_graph(mer_backend *b, mer_backend::GraphEntry key, Enqueue enqueue, mer_backend::GraphEntry **out) {
+  *out = nullptr;
+  for (auto &g : b->graphs)
+    if (g.layer == key.layer && g.n_tokens == key.n_tokens && g.x == key.x && g.out == key.out && g.ids == key.ids && g.w == key.w) {
+      *out = &g;
+      return MER_OK;
+    }
+  if (b->graphs.size() >= 256) drop_graphs(b);
+  cudaGraph_t graph = nullptr;
+  int rc = MER_OK;
+  bool ok = cudaStreamBeginCapture(b->compute, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+  if (ok) {
+    rc = enqueue(&key.launches);
+    const cudaError_t ce = cudaStreamEndCapture(b->compute, &graph);
+    ok = ce == cudaSuccess && graph != nullptr;
+  }
+  if (rc == MER_OK && ok) ok = cudaGraphInstantiate(&key.exec, graph, 0) == cudaSuccess;
+  if (graph) cudaGraphDestroy(graph);
+  if (rc != MER_OK || !ok) cudaGetLastError();
+  if (rc != MER_OK) return rc;
+  if (!ok) {
+    b->graphs_ok = false;  // plain launches from now on
+    return MER_OK;
+  }
+  b->graphs.push_back(key);
+  *out = &b->graphs.back();
+  return MER_OK;
+}
+bool graphs_usable(const mer_backend *b) { return b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS); }
+// Whether the caller is capturing `s` into a graph of its own: then plain launches, which become part of it.
+bool caller_captures(cudaStream_t s) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) return false;
+  cudaGetLastError();
+  return true;
+}
+
 int check_device_status(mer_backend *b, uint32_t status, uint32_t layer, uint32_t expert) {
   b->err.device_status = status;
   if (status & MER_DEVSTAT_RESIDENCY_MISS)
@@ -377,10 +440,10 @@ void free_all(mer_backend *b) {
     F(kv.second.d_shared_gate);
   }
   b->routers.clear();
-  F(b->arena), F(b->d_expert_ptr), F(b->d_x), F(b->d_out), F(b->d_h), F(b->d_y), F(b->d_pair_weight), F(b->d_logits);
-  F(b->d_pair_expert), F(b->d_group_expert), F(b->d_offsets), F(b->d_perm), F(b->d_status), F(b->d_counters), F(b->d_group_count);
+  F(b->arena), F(b->d_expert_ptr), F(b->d_x), F(b->d_out), F(b->d_h), F(b->d_y), F(b->d_logits), F(b->d_step);
+  F(b->d_pair_expert), F(b->d_group_expert), F(b->d_offsets), F(b->d_perm), F(b->d_counters), F(b->d_group_count);
   F(b->d_f16), F(b->d_stream_scratch), F(b->d_gemm_scratch), F(b->d_dequant), F(b->d_raw_stage), F(b->d_xn), F(b->d_shared_scale);
-  H(b->h_stage), H(b->h_u32), H(b->h_f32);
+  H(b->h_stage), H(b->h_u32), H(b->h_f32), H(b->h_step), H(b->h_rows), H(b->h_route);
   if (b->ev_compute_done) cudaEventDestroy(b->ev_compute_done);
   if (b->ev_copy_done) cudaEventDestroy(b->ev_copy_done);
   for (auto &e : b->ev_stage)
@@ -391,6 +454,7 @@ void free_all(mer_backend *b) {
   b->timing_events.clear();
   for (auto &u : b->user_streams) cudaEventDestroy(u.done);
   b->user_streams.clear();
+  if (b->ev_legacy) cudaEventDestroy(b->ev_legacy);
   for (auto &a : b->aslots) {
     F(a.d_x), F(a.d_out), F(a.d_status), H(a.h_status);
     if (a.ev_in) cudaEventDestroy(a.ev_in);
@@ -603,6 +667,20 @@ int admit_impl(mer_backend *b, uint32_t id, uint64_t generation, const void *blo
   return MER_OK;
 }
 
+// Groups the pairs whose routing is in d.pair_expert / d.pair_weight and runs the FFN; clears the status word.
+int run_given_routing(mer_backend *b, uint32_t layer, uint32_t expert, MoeDispatch &d, size_t n_pairs, bool single_group, int *launches,
+                      bool combine_follows) {
+  d.n_groups = single_group ? 1u : (uint32_t)n_pairs;
+  d.max_group_tokens = single_group ? (uint32_t)n_pairs : 1u;
+  d.active_groups_hint = d.n_groups;
+  bind_ffn(b, d);
+  CU(MER_ERR_SUBMISSION, "group kernel", launch_groups_from_pairs(d, b->compute, launches));
+  d.fuse_combine = combine_follows ? 1 : 0;
+  CU(MER_ERR_SUBMISSION, "expert FFN kernels", run_ffn(b, d, b->compute, launches));
+  if (!combine_follows) CU(MER_ERR_SUBMISSION, "partial-sum kernel", launch_reduce_parts(d, b->compute, launches));
+  return MER_OK;
+}
+
 // Shared tail of the host entry points whose routing comes from the caller: upload ids and
 // weights, group, run the FFN.  `single_group` = all pairs run the same expert.
 int dispatch_given_routing(mer_backend *b, uint32_t layer, MoeDispatch &d, const uint32_t *ids, const float *weights,
@@ -614,26 +692,78 @@ int dispatch_given_routing(mer_backend *b, uint32_t layer, MoeDispatch &d, const
      cudaMemcpyAsync(b->d_pair_expert, b->h_u32, n_pairs * 4, cudaMemcpyHostToDevice, b->compute));
   CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(weights)",
      cudaMemcpyAsync(b->d_pair_weight, b->h_f32, n_pairs * 4, cudaMemcpyHostToDevice, b->compute));
-  CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, b->compute));
-  d.n_groups = single_group ? 1u : (uint32_t)n_pairs;
-  d.max_group_tokens = single_group ? (uint32_t)n_pairs : 1u;
-  d.active_groups_hint = d.n_groups;
-  bind_ffn(b, d);
   CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
-  CU(MER_ERR_SUBMISSION, "group kernel", launch_groups_from_pairs(d, b->compute, launches));
-  d.fuse_combine = combine_follows ? 1 : 0;
-  CU(MER_ERR_SUBMISSION, "expert FFN kernels", run_ffn(b, d, b->compute, launches));
-  if (!combine_follows) CU(MER_ERR_SUBMISSION, "partial-sum kernel", launch_reduce_parts(d, b->compute, launches));
-  return MER_OK;
+  return run_given_routing(b, layer, expert, d, n_pairs, single_group, launches, combine_follows);
 }
 
-int finish_host_call(mer_backend *b, uint32_t layer, uint32_t expert, int launches, size_t n_experts_run) {
-  CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)",
-     cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, b->compute));
+// Routing, mixing weights and status word of `pairs` pairs into h_route, [3][pairs], in one copy.
+int enqueue_routing_readback(mer_backend *b, uint32_t layer, size_t pairs) {
+  const uint32_t expert = MER_NONE;
+  CU(MER_ERR_READBACK_MAP, "cudaMemcpy2DAsync(routing)",
+     cudaMemcpy2DAsync(b->h_route, pairs * 4, b->d_pair_expert, (size_t)b->max_pairs * 4, pairs * 4, 3, cudaMemcpyDeviceToHost, b->compute));
+  return MER_OK;
+}
+// h_route -> the caller's [n_tokens x top_k] arrays (either may be null): routed columns, local ids.
+void unpack_routing(const mer_backend *b, const RouterDev &r, uint32_t slots, size_t n_tokens, uint32_t *ids, float *weights) {
+  const uint32_t *h_ids = b->h_route;
+  const float *h_w = reinterpret_cast<const float *>(b->h_route + n_tokens * slots);
+  for (size_t t = 0; t < n_tokens; t++)
+    for (uint32_t s = 0; s < r.top_k; s++) {
+      if (ids) {
+        const uint32_t g = h_ids[t * slots + s];
+        ids[t * r.top_k + s] = g == MER_NONE ? MER_NONE : g - r.id_base;
+      }
+      if (weights) weights[t * r.top_k + s] = h_w[t * slots + s];
+    }
+}
+
+constexpr size_t ROWS_MAX_BYTES = 32u << 20;  // host rows go through pinned memory of at most this size each way
+// Whether `bytes` of host rows can be staged (each way); allocates the pinned rows on the first such call.
+bool stage_rows(mer_backend *b, size_t bytes) {
+  if (!b->h_rows) {
+    const size_t want = std::min(ROWS_MAX_BYTES, (size_t)b->cfg.max_tokens * b->cfg.d_model * 4);
+    if (cudaHostAlloc((void **)&b->h_rows, 2 * want, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      b->h_rows = nullptr;
+      return false;
+    }
+    b->rows_floats = want / 4;
+  }
+  return bytes <= b->rows_floats * 4;
+}
+
+// Host copy, by several threads from 2 MB on.
+void copy_host(mer_backend *b, void *dst, const void *src, size_t n) {
+  static constexpr size_t PIECE = 256u << 10;
+  if (n < (2u << 20)) {
+    memcpy(dst, src, n);
+    return;
+  }
+  struct State {
+    std::atomic<size_t> next{0}, done{0};
+  };
+  const auto st = std::make_shared<State>();
+  const size_t n_pieces = (n + PIECE - 1) / PIECE;
+  auto work = [st, dst, src, n, n_pieces] {
+    for (size_t i; (i = st->next.fetch_add(1)) < n_pieces; st->done.fetch_add(1, std::memory_order_release))
+      memcpy(static_cast<char *>(dst) + i * PIECE, static_cast<const char *>(src) + i * PIECE, std::min(PIECE, n - i * PIECE));
+  };
+  if (!b->copy_pool) b->copy_pool.reset(new (std::nothrow) CopyPool());
+  if (b->copy_pool) b->copy_pool->start(std::make_shared<const std::function<void()>>(work));
+  work();
+  while (st->done.load(std::memory_order_acquire) < n_pieces) std::this_thread::yield();
+  if (b->copy_pool) b->copy_pool->finish();
+}
+
+// `status`: where a copy that is already enqueued leaves the status word (null: read it back here).
+int finish_host_call(mer_backend *b, uint32_t layer, uint32_t expert, int launches, size_t n_experts_run, const uint32_t *status = nullptr) {
+  if (!status)
+    CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)",
+       cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, b->compute));
   CU(MER_ERR_READBACK_MAP, "cudaStreamSynchronize", cudaStreamSynchronize(b->compute));
   b->ctr.kernel_launches += (uint64_t)launches;
   b->ctr.gpu_dispatch_attempts += n_experts_run;
-  int rc = check_device_status(b, b->h_u32[b->max_pairs], layer, expert);
+  int rc = check_device_status(b, status ? *status : b->h_u32[b->max_pairs], layer, expert);
   if (rc && rc != MER_ERR_NUMERICAL) {
     b->ctr.gpu_dispatch_failures += n_experts_run;  // counted once, never replayed (engine.rs:6624-6642)
     return rc;
@@ -739,21 +869,25 @@ MER_EXPORT int mer_backend_create(const mer_backend_cfg *cfg, mer_backend **out)
   CB(cudaMalloc((void **)&b->d_out, T * D * 4));
   CB(cudaMalloc((void **)&b->d_h, P * F * 4));
   CB(cudaMalloc((void **)&b->d_y, P * D * 4));
-  CB(cudaMalloc((void **)&b->d_pair_weight, P * 4));
-  CB(cudaMalloc((void **)&b->d_pair_expert, P * 4));
+  CB(cudaMalloc((void **)&b->d_pair_expert, 3 * P * 4));  // routing [P], mixing weights [P], status word: one strided copy reads all three
+  b->d_pair_weight = reinterpret_cast<float *>(b->d_pair_expert + P);
+  b->d_status = b->d_pair_expert + 2 * P;
   CB(cudaMalloc((void **)&b->d_group_expert, (size_t)b->max_groups * 4));
   CB(cudaMalloc((void **)&b->d_offsets, ((size_t)b->max_groups + 1) * 4));
   CB(cudaMalloc((void **)&b->d_group_count, (size_t)b->max_groups * 2 * 4));
   CB(cudaMemset(b->d_group_count, 0, (size_t)b->max_groups * 2 * 4));
   CB(cudaMalloc((void **)&b->d_perm, P * 4));
   CB(cudaMalloc((void **)&b->d_logits, T * b->max_router_experts * 4));
-  CB(cudaMalloc((void **)&b->d_status, 4));
   CB(cudaMalloc((void **)&b->d_counters, (T + 1) * 4));
   CB(cudaMemset(b->d_status, 0, 4));
   CB(cudaMemset(b->d_counters, 0, (T + 1) * 4));
   CB(cudaMalloc((void **)&b->d_f16, std::max(P, T) * D * 2));
   CB(cudaHostAlloc((void **)&b->h_u32, (P + 1) * 4, cudaHostAllocDefault));
   CB(cudaHostAlloc((void **)&b->h_f32, P * 4, cudaHostAllocDefault));
+  CB(cudaHostAlloc((void **)&b->h_route, 3 * P * 4, cudaHostAllocDefault));
+  b->step_words = (D + 2 * cfg->max_top_k + 1 + 63) / 64 * 64;
+  CB(cudaMalloc((void **)&b->d_step, 2 * b->step_words * 4));
+  CB(cudaHostAlloc((void **)&b->h_step, 2 * b->step_words * 4, cudaHostAllocDefault));
   if (stream_ffn_supported(cfg->dtype, (uint32_t)D, (uint32_t)F)) {
     b->packed = true;
     CB(cudaMalloc((void **)&b->d_raw_stage, b->expert_bytes));
@@ -1144,7 +1278,7 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   }
   if (re.layer_flags & MER_LAYER_RESIDUAL) d.residual = d_x, d.routed_slots = r.top_k;
   const RouterDev &r2 = rl;
-  CU(MER_ERR_SUBMISSION, "router kernel", launch_router(r2, d, b->cfg.max_tokens, s, launches));
+  CU(MER_ERR_SUBMISSION, "router kernel", launch_router(r2, d, b->cfg.max_tokens, s, launches, run_ffn_too));
   if (run_ffn_too) {
     if (ev) cudaEventRecord(ev[1], s);
     d.fuse_combine = 1;
@@ -1166,24 +1300,40 @@ MER_EXPORT int mer_router_route(mer_backend *b, uint32_t layer, const float *x, 
   CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
   if (n_tokens == 0 || n_tokens > b->cfg.max_tokens)
     return fail(b, MER_ERR_VALIDATION_DISPATCH, layer, expert, "n_tokens %zu outside 1..=%u", n_tokens, b->cfg.max_tokens);
-  CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)",
-     cudaMemcpyAsync(b->d_x, x, n_tokens * b->cfg.d_model * 4, cudaMemcpyHostToDevice, b->compute));
-  int launches = 0;
-  MoeDispatch d;
-  int rc = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, &launches, &d);
-  if (rc) return rc;
-  const RouterDev &r = b->routers[layer].dev;
-  // ids/weights on the device are [n_tokens x slots]; the caller gets the top_k routed columns with local ids
-  size_t P = n_tokens * d.slots;
-  CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(ids)", cudaMemcpyAsync(b->h_u32, b->d_pair_expert, P * 4, cudaMemcpyDeviceToHost, b->compute));
-  CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(w)", cudaMemcpyAsync(b->h_f32, b->d_pair_weight, P * 4, cudaMemcpyDeviceToHost, b->compute));
-  rc = finish_host_call(b, layer, expert, launches, 0);
-  for (size_t t = 0; t < n_tokens; t++)
-    for (uint32_t s = 0; s < r.top_k; s++) {
-      uint32_t g = b->h_u32[t * d.slots + s];
-      ids[t * r.top_k + s] = g == MER_NONE ? MER_NONE : g - r.id_base;
-      weights[t * r.top_k + s] = b->h_f32[t * d.slots + s];
-    }
+  auto it = b->routers.find(layer);
+  if (it == b->routers.end()) return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "no router installed for layer %u", layer);
+  const RouterDev &r = it->second.dev;
+  const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
+  const size_t P = n_tokens * slots, bytes = n_tokens * b->cfg.d_model * 4;
+  int rc, launches = 0;
+  mer_backend::GraphEntry *hit = nullptr;
+  if (graphs_usable(b) && stage_rows(b, bytes)) {
+    CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
+    rc = captured_graph(
+        b, {layer, n_tokens, nullptr, nullptr, graph_tag(TAG_ROUTE), nullptr, nullptr, 0},
+        [&](int *n) -> int {
+          MoeDispatch d;
+          CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
+          const int e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, n, &d, true);
+          return e ? e : enqueue_routing_readback(b, layer, P);
+        },
+        &hit);
+    if (rc) return rc;
+  }
+  if (hit) {
+    copy_host(b, b->h_rows, x, bytes);
+    CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
+    launches = hit->launches;
+  } else {
+    CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, bytes, cudaMemcpyHostToDevice, b->compute));
+    MoeDispatch d;
+    rc = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, &launches, &d);
+    if (rc == MER_OK) rc = enqueue_routing_readback(b, layer, P);
+    if (rc) return rc;
+  }
+  rc = finish_host_call(b, layer, expert, launches, 0, b->h_route + 2 * P);
+  // ids / weights on the device are [n_tokens x slots]; the caller gets the top_k routed columns with local ids
+  unpack_routing(b, r, slots, n_tokens, ids, weights);
   b->ctr.hidden_upload_bytes += n_tokens * b->cfg.d_model * 4;
   b->ctr.readback_bytes += P * 8;
   return rc;
@@ -1281,21 +1431,44 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
       return rc;
     }
   const size_t D = b->cfg.d_model;
-  CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, D * 4, cudaMemcpyHostToDevice, b->compute));
-  MoeDispatch d = base_dispatch(b);
-  d.n_tokens = 1;
-  d.slots = (uint32_t)n_slots;
-  d.x = b->d_x;
-  d.out = b->d_out;
+  // [x | ids | weights] up in one copy, [out | status] back in one; the sequence depends on the number of slots only
+  uint32_t *h_status = reinterpret_cast<uint32_t *>(b->h_step + b->step_words + D);
+  memcpy(b->h_step, x, D * 4);
+  memcpy(b->h_step + D, expert_ids, n_slots * 4);
+  memcpy(b->h_step + D + n_slots, weights, n_slots * 4);
+  auto enqueue = [&](int *n) -> int {
+    CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_step, b->h_step, (D + 2 * n_slots) * 4, cudaMemcpyHostToDevice, b->compute));
+    MoeDispatch d = base_dispatch(b);
+    d.n_tokens = 1;
+    d.slots = (uint32_t)n_slots;
+    d.x = b->d_step;
+    d.pair_expert = reinterpret_cast<uint32_t *>(b->d_step + D);
+    d.pair_weight = b->d_step + D + n_slots;
+    d.out = b->d_step + b->step_words;
+    d.status = reinterpret_cast<uint32_t *>(b->d_step + b->step_words + D);
+    const int e = run_given_routing(b, layer, expert, d, n_slots, false, n, true);
+    if (e) return e;
+    CU(MER_ERR_SUBMISSION, "combine kernel", launch_combine(d, b->compute, n));
+    CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)",
+       cudaMemcpyAsync(b->h_step + b->step_words, b->d_step + b->step_words, (D + 1) * 4, cudaMemcpyDeviceToHost, b->compute));
+    return MER_OK;
+  };
+  CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
   int launches = 0;
-  rc = dispatch_given_routing(b, layer, d, expert_ids, weights, n_slots, false, &launches, true);
-  if (rc) return rc;
-  CU(MER_ERR_SUBMISSION, "combine kernel", launch_combine(d, b->compute, &launches));
-  CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(out, b->d_out, D * 4, cudaMemcpyDeviceToHost, b->compute));
+  mer_backend::GraphEntry *hit = nullptr;
+  if (graphs_usable(b) && (rc = captured_graph(b, {0, n_slots, nullptr, nullptr, graph_tag(TAG_STEP), nullptr, nullptr, 0}, enqueue, &hit)) != MER_OK) return rc;
+  if (hit) {
+    CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
+    launches = hit->launches;
+  } else if ((rc = enqueue(&launches)) != MER_OK) {
+    return rc;
+  }
   b->ctr.batch_calls += 1;
   b->ctr.hidden_upload_bytes += D * 4;
   b->ctr.readback_bytes += D * 4;
-  return finish_host_call(b, layer, expert, launches, n_slots);
+  rc = finish_host_call(b, layer, expert, launches, n_slots, h_status);
+  memcpy(out, b->h_step + b->step_words, D * 4);
+  return rc;
 }
 
 MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float *x, size_t n_tokens, float *out, uint32_t *ids,
@@ -1310,49 +1483,28 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
   const size_t D = b->cfg.d_model;
   // Pinned host buffers and no routing wanted back: upload, layer, read-back and the status word are captured once
   // per (layer, n_tokens, x, out) and replayed as one graph launch (the call stays synchronous).
-  if (!ids && !weights && b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS) && b->routers.count(layer)) {
+  if (!ids && !weights && graphs_usable(b) && b->routers.count(layer)) {
     cudaPointerAttributes ax{}, ao{};
     const bool pinned = cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost &&
                         cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost;
     cudaGetLastError();
     if (pinned) {
       cudaStream_t s = b->compute;
-      const void *host_tag = reinterpret_cast<const void *>(uintptr_t(1));  // marks host-entry graphs in the cache
       CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
       mer_backend::GraphEntry *hit = nullptr;
-      for (auto &g : b->graphs)
-        if (g.layer == layer && g.n_tokens == n_tokens && g.x == x && g.out == out && g.ids == host_tag && g.stream == s) hit = &g;
-      if (!hit) {
-        if (b->graphs.size() >= 256) drop_graphs(b);
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        int launches = 0, rc = MER_OK;
-        bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-        if (ok) {
-          ok = cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, s) == cudaSuccess;
-          MoeDispatch d;
-          if (ok) rc = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, s, &launches, &d, true);
-          if (ok && rc == MER_OK) ok = cudaMemcpyAsync(out, b->d_out, n_tokens * D * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
-          if (ok && rc == MER_OK)
-            ok = cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
-          cudaError_t ce = cudaStreamEndCapture(s, &graph);
-          ok = ok && ce == cudaSuccess && graph != nullptr;
-        }
-        if (rc != MER_OK) {
-          if (graph) cudaGraphDestroy(graph);
-          cudaGetLastError();
-          return rc;
-        }
-        if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-        if (graph) cudaGraphDestroy(graph);
-        if (ok) {
-          b->graphs.push_back({layer, n_tokens, x, out, host_tag, nullptr, s, exec, launches});
-          hit = &b->graphs.back();
-        } else {
-          cudaGetLastError();
-          b->graphs_ok = false;  // capture is not available here: plain launches from now on
-        }
-      }
+      const int rc = captured_graph(
+          b, {layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr, nullptr, 0},
+          [&](int *n) -> int {
+            MoeDispatch d;
+            CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, s));
+            const int r = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, s, n, &d, true);
+            if (r) return r;
+            CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(out, b->d_out, n_tokens * D * 4, cudaMemcpyDeviceToHost, s));
+            CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)", cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, s));
+            return MER_OK;
+          },
+          &hit);
+      if (rc != MER_OK) return rc;
       if (hit) {
         const RouterDev &r = b->routers[layer].dev;
         const size_t P = n_tokens * (r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u));
@@ -1371,6 +1523,38 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
         b->ctr.gpu_dispatch_successes += P;
         return rc;
       }
+    }
+  }
+  if (graphs_usable(b) && b->routers.count(layer) && stage_rows(b, n_tokens * D * 4)) {
+    // ordinary host memory: rows through pinned memory, the sequence (routing included) captured per (layer, n_tokens)
+    const RouterDev &r = b->routers[layer].dev;
+    const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
+    const size_t P = n_tokens * slots, bytes = n_tokens * D * 4;
+    float *h_out = b->h_rows + b->rows_floats;
+    CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
+    mer_backend::GraphEntry *hit = nullptr;
+    int rc = captured_graph(
+        b, {layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr, nullptr, 0},
+        [&](int *n) -> int {
+          MoeDispatch d;
+          CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
+          const int e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, b->compute, n, &d, true);
+          if (e) return e;
+          CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(h_out, b->d_out, bytes, cudaMemcpyDeviceToHost, b->compute));
+          return enqueue_routing_readback(b, layer, P);
+        },
+        &hit);
+    if (rc) return rc;
+    if (hit) {
+      copy_host(b, b->h_rows, x, bytes);
+      CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
+      b->ctr.selected_routed_experts += P;
+      rc = finish_host_call(b, layer, expert, hit->launches, P, b->h_route + 2 * P);
+      copy_host(b, out, h_out, bytes);
+      unpack_routing(b, r, slots, n_tokens, ids, weights);
+      b->ctr.hidden_upload_bytes += bytes;
+      b->ctr.readback_bytes += bytes + (ids ? P * 4 : 0) + (weights ? P * 4 : 0);
+      return rc;
     }
   }
   CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, b->compute));
@@ -1419,49 +1603,26 @@ int layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *d_x
   const uint32_t expert = MER_NONE;
   int launches = 0;
   size_t P = 0;
-  const bool use_graph = b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS);
   bool replayed = false;
-  if (use_graph) {
+  if (graphs_usable(b) && !caller_captures(s)) {
     auto it = b->routers.find(layer);
     if (it == b->routers.end()) return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "no router installed for layer %u", layer);
     P = n_tokens * (it->second.dev.top_k + (it->second.dev.shared_expert_id != MER_NONE ? 1u : 0u));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
     mer_backend::GraphEntry *hit = nullptr;
-    for (auto &g : b->graphs)
-      if (g.layer == layer && g.n_tokens == n_tokens && g.x == d_x && g.out == d_out && g.ids == d_ids && g.w == d_weights &&
-          g.stream == s)
-        hit = &g;
-    if (!hit) {
-      // first call with these arguments: capture the launch sequence once
-      if (b->graphs.size() >= 256) drop_graphs(b);
-      cudaGraph_t graph = nullptr;
-      cudaGraphExec_t exec = nullptr;
-      bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-      int rc = MER_OK;
-      if (ok) {
-        MoeDispatch d;
-        rc = enqueue_layer(b, layer, d_x, n_tokens, d_out, true, s, &launches, &d, true);
-        if (rc == MER_OK && d_ids) ok = cudaMemcpyAsync(d_ids, b->d_pair_expert, P * 4, cudaMemcpyDeviceToDevice, s) == cudaSuccess;
-        if (rc == MER_OK && ok && d_weights)
-          ok = cudaMemcpyAsync(d_weights, b->d_pair_weight, P * 4, cudaMemcpyDeviceToDevice, s) == cudaSuccess;
-        cudaError_t ce = cudaStreamEndCapture(s, &graph);
-        ok = ok && ce == cudaSuccess && graph != nullptr;
-      }
-      if (rc != MER_OK) {
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        return rc;
-      }
-      if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-      if (graph) cudaGraphDestroy(graph);
-      if (ok) {
-        b->graphs.push_back({layer, n_tokens, d_x, d_out, d_ids, d_weights, s, exec, launches});
-        hit = &b->graphs.back();
-      } else {
-        cudaGetLastError();
-        b->graphs_ok = false;  // capture is not available here: plain launches from now on
-      }
-    }
+    const int rc = captured_graph(
+        b, {layer, n_tokens, d_x, d_out, d_ids, d_weights, nullptr, 0},
+        [&](int *n) -> int {
+          MoeDispatch d;
+          int r = enqueue_layer(b, layer, d_x, n_tokens, d_out, true, b->compute, n, &d, true);
+          if (r == MER_OK && d_ids && cudaMemcpyAsync(d_ids, b->d_pair_expert, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
+            r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the expert ids");
+          if (r == MER_OK && d_weights && cudaMemcpyAsync(d_weights, b->d_pair_weight, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
+            r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the mixing weights");
+          return r;
+        },
+        &hit);
+    if (rc != MER_OK) return rc;
     if (hit) {
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, s));
       launches = hit->launches;
@@ -1873,40 +2034,15 @@ int ep_enqueue(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens
 int ep_layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens, float *d_out, cudaStream_t s) {
   const uint32_t expert = MER_NONE;
   int launches = 0;
-  const void *ep_tag = reinterpret_cast<const void *>(uintptr_t(2));  // marks expert-parallel graphs in the cache
   bool replayed = false;
-  if (b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS) && b->ep_on && b->ep_attached) {
+  if (graphs_usable(b) && b->ep_on && b->ep_attached && !caller_captures(s)) {
     CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
     mer_backend::GraphEntry *hit = nullptr;
-    for (auto &g : b->graphs)
-      if (g.layer == layer && g.n_tokens == n_tokens && g.x == d_x && g.out == d_out && g.ids == ep_tag && g.stream == s) hit = &g;
-    if (!hit) {
-      if (b->graphs.size() >= 256) drop_graphs(b);
-      cudaGraph_t graph = nullptr;
-      cudaGraphExec_t exec = nullptr;
-      int rc = MER_OK;
-      bool ok = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-      if (ok) {
-        rc = ep_enqueue(b, layer, d_x, n_tokens, d_out, s, &launches, true);
-        cudaError_t ce = cudaStreamEndCapture(s, &graph);
-        ok = ce == cudaSuccess && graph != nullptr;
-      }
-      if (rc != MER_OK) {
-        if (graph) cudaGraphDestroy(graph);
-        cudaGetLastError();
-        return rc;
-      }
-      if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
-      if (graph) cudaGraphDestroy(graph);
-      if (ok) {
-        b->graphs.push_back({layer, n_tokens, d_x, d_out, ep_tag, nullptr, s, exec, launches});
-        hit = &b->graphs.back();
-      } else {
-        cudaGetLastError();
-        b->graphs_ok = false;  // capture is not available here: plain launches from now on
-      }
-    }
+    const int rc = captured_graph(
+        b, {layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr, nullptr, 0},
+        [&](int *n) -> int { return ep_enqueue(b, layer, d_x, n_tokens, d_out, b->compute, n, true); }, &hit);
+    if (rc != MER_OK) return rc;
     if (hit) {
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, s));
       launches = hit->launches;
