@@ -124,8 +124,12 @@ struct mer_backend {
     const void *x, *out, *ids, *w;  // the buffers a caller passed, or a tag in `ids` for the other entry points
     cudaGraphExec_t exec;
     int launches;
+    bool same_call(const GraphEntry &o) const {
+      return layer == o.layer && n_tokens == o.n_tokens && x == o.x && out == o.out && ids == o.ids && w == o.w;
+    }
   };
   std::vector<GraphEntry> graphs;
+  std::vector<GraphEntry> graph_calls;  // calls seen lately and not captured yet, by hash; `launches` counts them
   bool graphs_ok = true;
   // Streams other than `compute` that device entry points were last enqueued on, each with an event recorded after
   // the call: an admission or a retire makes the copy stream wait for all of them before it touches a slot.
@@ -351,14 +355,32 @@ void drop_graphs(mer_backend *b) {
 const void *graph_tag(uintptr_t n) { return reinterpret_cast<const void *>(n); }
 constexpr uintptr_t TAG_HOST_LAYER = 1, TAG_EP = 2, TAG_ROUTE = 3, TAG_STEP = 4, TAG_HOST_STAGED = 5;
 
-// The captured launch sequence of `key`, captured now on the backend's own stream if need be (`enqueue(&launches)` issues it
-// there); *out stays null where capture is not to be had.  A graph is launched into whatever stream the caller brings, the
-// legacy default stream included, which itself cannot be captured.
+bool graphs_usable(const mer_backend *b) { return b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS); }
+
+// Whether the call `key` is to be replayed from a graph.  Capturing costs 0.1 to 0.3 ms and a replay saves 10 to 30 us, so a
+// call is captured at its third occurrence; rows of ever new addresses or lengths never are.
+bool replays(mer_backend *b, const mer_backend::GraphEntry &key) {
+  constexpr size_t CALLS = 1024;
+  if (!graphs_usable(b)) return false;
+  for (auto &g : b->graphs)
+    if (g.same_call(key)) return true;
+  if (b->graph_calls.empty()) b->graph_calls.resize(CALLS, {MER_NONE, 0, nullptr, nullptr, nullptr, nullptr, nullptr, 0});
+  uint64_t h = key.layer;
+  for (const uint64_t v : {(uint64_t)key.n_tokens, (uint64_t)key.x, (uint64_t)key.out, (uint64_t)key.ids, (uint64_t)key.w})
+    h = (h ^ v) * 0x9e3779b97f4a7c15ull, h ^= h >> 29;
+  auto &seen = b->graph_calls[h % CALLS];
+  if (!seen.same_call(key)) seen = key;
+  return ++seen.launches >= 3;
+}
+
+// The captured launch sequence of `key` (which replays()), captured now on the backend's own stream if need be
+// (`enqueue(&launches)` issues it there); *out stays null where capture is not to be had.  A graph is launched into whatever
+// stream the caller brings, the legacy default stream included, which itself cannot be captured.
 template <typename Enqueue>
 int captured_graph(mer_backend *b, mer_backend::GraphEntry key, Enqueue enqueue, mer_backend::GraphEntry **out) {
   *out = nullptr;
   for (auto &g : b->graphs)
-    if (g.layer == key.layer && g.n_tokens == key.n_tokens && g.x == key.x && g.out == key.out && g.ids == key.ids && g.w == key.w) {
+    if (g.same_call(key)) {
       *out = &g;
       return MER_OK;
     }
@@ -383,7 +405,6 @@ int captured_graph(mer_backend *b, mer_backend::GraphEntry key, Enqueue enqueue,
   *out = &b->graphs.back();
   return MER_OK;
 }
-bool graphs_usable(const mer_backend *b) { return b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS); }
 // Whether the caller is capturing `s` into a graph of its own: then plain launches, which become part of it.
 bool caller_captures(cudaStream_t s) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1307,10 +1328,11 @@ MER_EXPORT int mer_router_route(mer_backend *b, uint32_t layer, const float *x, 
   const size_t P = n_tokens * slots, bytes = n_tokens * b->cfg.d_model * 4;
   int rc, launches = 0;
   mer_backend::GraphEntry *hit = nullptr;
-  if (graphs_usable(b) && stage_rows(b, bytes)) {
+  const mer_backend::GraphEntry key{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_ROUTE), nullptr, nullptr, 0};
+  if (replays(b, key) && stage_rows(b, bytes)) {
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
     rc = captured_graph(
-        b, {layer, n_tokens, nullptr, nullptr, graph_tag(TAG_ROUTE), nullptr, nullptr, 0},
+        b, key,
         [&](int *n) -> int {
           MoeDispatch d;
           CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
@@ -1456,7 +1478,8 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
   CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
   int launches = 0;
   mer_backend::GraphEntry *hit = nullptr;
-  if (graphs_usable(b) && (rc = captured_graph(b, {0, n_slots, nullptr, nullptr, graph_tag(TAG_STEP), nullptr, nullptr, 0}, enqueue, &hit)) != MER_OK) return rc;
+  const mer_backend::GraphEntry key{0, n_slots, nullptr, nullptr, graph_tag(TAG_STEP), nullptr, nullptr, 0};
+  if (replays(b, key) && (rc = captured_graph(b, key, enqueue, &hit)) != MER_OK) return rc;
   if (hit) {
     CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
     launches = hit->launches;
@@ -1488,12 +1511,13 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
     const bool pinned = cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost &&
                         cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost;
     cudaGetLastError();
-    if (pinned) {
+    const mer_backend::GraphEntry key{layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr, nullptr, 0};
+    if (pinned && replays(b, key)) {
       cudaStream_t s = b->compute;
       CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
       mer_backend::GraphEntry *hit = nullptr;
       const int rc = captured_graph(
-          b, {layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr, nullptr, 0},
+          b, key,
           [&](int *n) -> int {
             MoeDispatch d;
             CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, s));
@@ -1525,7 +1549,8 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
       }
     }
   }
-  if (graphs_usable(b) && b->routers.count(layer) && stage_rows(b, n_tokens * D * 4)) {
+  const mer_backend::GraphEntry key{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr, nullptr, 0};
+  if (b->routers.count(layer) && replays(b, key) && stage_rows(b, n_tokens * D * 4)) {
     // ordinary host memory: rows through pinned memory, the sequence (routing included) captured per (layer, n_tokens)
     const RouterDev &r = b->routers[layer].dev;
     const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
@@ -1534,7 +1559,7 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
     mer_backend::GraphEntry *hit = nullptr;
     int rc = captured_graph(
-        b, {layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr, nullptr, 0},
+        b, key,
         [&](int *n) -> int {
           MoeDispatch d;
           CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
@@ -1604,14 +1629,15 @@ int layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *d_x
   int launches = 0;
   size_t P = 0;
   bool replayed = false;
-  if (graphs_usable(b) && !caller_captures(s)) {
+  const mer_backend::GraphEntry key{layer, n_tokens, d_x, d_out, d_ids, d_weights, nullptr, 0};
+  if (!caller_captures(s) && replays(b, key)) {
     auto it = b->routers.find(layer);
     if (it == b->routers.end()) return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "no router installed for layer %u", layer);
     P = n_tokens * (it->second.dev.top_k + (it->second.dev.shared_expert_id != MER_NONE ? 1u : 0u));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
     mer_backend::GraphEntry *hit = nullptr;
     const int rc = captured_graph(
-        b, {layer, n_tokens, d_x, d_out, d_ids, d_weights, nullptr, 0},
+        b, key,
         [&](int *n) -> int {
           MoeDispatch d;
           int r = enqueue_layer(b, layer, d_x, n_tokens, d_out, true, b->compute, n, &d, true);
@@ -2035,12 +2061,13 @@ int ep_layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *
   const uint32_t expert = MER_NONE;
   int launches = 0;
   bool replayed = false;
-  if (graphs_usable(b) && b->ep_on && b->ep_attached && !caller_captures(s)) {
+  const mer_backend::GraphEntry key{layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr, nullptr, 0};
+  if (b->ep_on && b->ep_attached && !caller_captures(s) && replays(b, key)) {
     CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
     mer_backend::GraphEntry *hit = nullptr;
     const int rc = captured_graph(
-        b, {layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr, nullptr, 0},
+        b, key,
         [&](int *n) -> int { return ep_enqueue(b, layer, d_x, n_tokens, d_out, b->compute, n, true); }, &hit);
     if (rc != MER_OK) return rc;
     if (hit) {
