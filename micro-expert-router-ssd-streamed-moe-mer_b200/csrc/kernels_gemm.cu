@@ -25,6 +25,7 @@
 //     take alternate blocks), 18 = producer of the weight stages (lanes 0..7 copy one packed tile each).
 // Every wait is bounded; on expiry the CTA latches MER_DEVSTAT_TIMEOUT, stops issuing work, waits
 // (bounded) for its copies and MMAs in flight, frees its TMEM and returns.
+#include <cuda.h>
 #include <cuda_fp16.h>
 
 #include <type_traits>
@@ -36,33 +37,38 @@
 
 namespace {
 
-constexpr int G_WARPS = 19, G_THREADS = G_WARPS * 32;
-constexpr int W_PRODUCER = 0, W_MMA = 1, W_EPI0 = 2, W_DQ0 = 10, W_WEIGHTS = 18;
-constexpr int EPI_WARPS = 4, DQ_WARPS = 8;  // EPI_WARPS per accumulator
+constexpr int G_WARPS = 27, G_THREADS = G_WARPS * 32;
+constexpr int W_PRODUCER = 0, W_MMA = 1, W_EPI0 = 2, W_DQ0 = 10, W_WEIGHTS = 26;
+constexpr int EPI_WARPS = 4, DQ_WARPS = 16;  // EPI_WARPS per accumulator
+constexpr uint32_t PAIR = 2;             // CTAs of a cluster: they share the B operand, each holding half of its rows
 constexpr uint32_t RAW_BLOCKS = 4;       // blocks of K per weight stage (per packed tile: one bulk copy)
 constexpr uint32_t G_HEADER = 5120;      // mbarriers, TMEM base, and from byte 1024 the epilogue groups' per-pass tables (2 KB each)
 constexpr uint32_t TMEM_COLS = 512;      // [0, 256): two accumulator buffers of up to 128 columns; [256, 512): A stages
 constexpr uint32_t TMEM_A0 = 256, A_STAGES = 8, A_STAGE_COLS = 32;  // a stage = one block: 16 columns hi + 16 columns lo
 constexpr uint32_t MAX_RING = 8;
-// The MMA issuer synchronises with its producers once per GROUP blocks of K: it waits for a whole group of A stages
-// and for the group's activation stage (both complete the same barrier, a_full: eight dequantiser arrivals, the
-// producer's expect-tx arrival and the bytes of its two copies), issues the group's MMAs and commits done[], which releases
-// both.  A waiter is never two phases behind a done[] barrier: the issuer leads its producers by at most two groups.
-constexpr uint32_t GROUP = 4, DONE_RING = 8;
-static_assert(GROUP == RAW_BLOCKS, "a weight stage holds exactly one group of blocks");
+// The MMA issuer synchronises with its producers once per GROUP blocks of K: it waits for the group's A stages of both
+// CTAs (a_full: every dequantiser warp of the pair) and for its activation stage (b_full: the bytes of both CTAs'
+// copies), issues the group's MMAs and commits done[] in both CTAs, which releases all of it.
+constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16;
+constexpr uint32_t CHUNK_K = 64, CHUNKS = GROUP * 32 / CHUNK_K;  // a row's piece of a chunk is 128 bytes, the swizzle span
+constexpr uint32_t PASS_TOKENS = 128;    // tokens of a pass at most: N of one MMA, and the columns of an accumulator buffer
+constexpr uint32_t PART_BYTES = PASS_TOKENS / PAIR * 128, CHUNK_BYTES = 2 * PART_BYTES, B_STAGE = CHUNKS * CHUNK_BYTES;  // hi rows, then lo rows
+static_assert(RAW_BLOCKS % GROUP == 0 && A_STAGES % GROUP == 0 && GROUP * 32 % CHUNK_K == 0, "whole groups per stage");
 constexpr float POW2_SCALE_TARGET = 9;   // activations are scaled so that the row maximum lies in [256, 512)
 
 struct GemmParams {
   MoeDispatch d;
   int phase;               // 0 = gate/up (+SiLU*mul), 1 = down
-  const uint8_t *act_img;  // [pass][K / 64] images of {hi, lo} activation tiles
-  const float *unscale;    // [pass][bn] 1 / scale of each token row
+  const float *unscale;    // 1 / scale of each activation row
   uint32_t rows;           // F (gate/up) or D (down)
   uint32_t kb_total;       // 32-value blocks per weight row
-  uint32_t bn;             // token columns per pass (16, 32, 64 or 128)
-  uint32_t b_lbo;          // bn * 16 + 32: a chunk slot of the activation ring and of the image array holds 16 of these
   uint32_t n_raw, n_b;     // ring depths (weights, activations)
   float *out;              // phase 0: h [P x F]; phase 1: y [P x D]
+};
+
+// The activation matrix in boxes of 8, 16 .. 64 rows (half a pass's width) x 64 values.
+struct ActMaps {
+  CUtensorMap m[PASS_TOKENS / 16];
 };
 
 // ------------------------------------------------------------------------------ tcgen05 PTX
@@ -81,23 +87,43 @@ __device__ __forceinline__ uint32_t elect_one() {
 __device__ __forceinline__ void tc_commit(uint32_t leader, uint64_t *bar) {
   asm volatile(
       "{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
-      " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(smem_u32(bar)),
-      "r"(leader)
+      " @q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n}\n" ::"r"(smem_u32(bar)),
+      "r"(leader), "h"((uint16_t)3)
       : "memory");
 }
-// K-major, no swizzle: 8-row x 16-byte core matrices; LBO = step between core matrices along K,
-// SBO = step between 8-row groups.  Bits: start >> 4 [0,14), LBO >> 4 [16,30), SBO >> 4 [32,46), version 1 [46,48).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
+// K-major rows of 128 bytes, swizzled in atoms of 8 rows (1024 bytes).  Bits: start >> 4 [0,14), LBO (not used) [16,30),
+// SBO = 1024 >> 4 between atoms [32,46), version 1 [46,48), 128-byte swizzle = 2 [61,64).
+__device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
+  return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// f16 x f16 -> f32, both operands K-major, M = 128, N = n.
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24); }
+// f16 x f16 -> f32, both operands K-major, M = 256 (128 rows in each CTA of the pair), N = n.
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t n) { return (1u << 4) | ((n >> 3) << 17) | ((256u >> 4) << 24); }
+// The same shared-memory address in the pair's first CTA, which issues the MMAs and holds the barriers it waits on.
+__device__ __forceinline__ uint32_t leader_addr(const void *p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// The box of `map` at (column x, row r) of the activation matrix into this CTA's shared memory (128-byte rows, swizzled);
+// the bytes are counted on a barrier of the pair's first CTA.
+__device__ __forceinline__ void tile_g2s(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t r, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+      "l"(map), "r"(x), "r"(r), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 // A operand read from tensor memory (lane = row, a 32-bit column = two consecutive values of K), B through a descriptor.
 // Called by the whole (converged) warp; only the lane with leader != 0 issues.
 __device__ __forceinline__ void tc_mma_ts(uint32_t leader, uint32_t d_tmem, uint32_t a_tmem, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p, q;\n setp.ne.b32 q, %5, 0;\n setp.ne.b32 p, %4, 0;\n"
-      " @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
+      " @q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
       "r"(a_tmem), "l"(b), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
@@ -116,16 +142,13 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&v)[32])
       : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// 32 columns of this thread's TMEM lane (lane = 32 * (warp % 4) + lane id).
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+// 16 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
       "tcgen05.wait::ld.sync.aligned;\n"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-        "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-        "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(taddr)
       : "memory");
 }
@@ -141,19 +164,8 @@ __device__ __forceinline__ void dq2(uint32_t biased, __half2 zp1024, __half2 d2,
   lo = h2_bits(__hfma2(d2, q, __hneg2(h)));
 }
 
-// Token columns a pass occupies in its activation image and in the accumulator: its count rounded up to 16, at most bn.
-__host__ __device__ constexpr uint32_t pass_width(uint32_t bn, uint32_t count) {
-  const uint32_t w = (count + 15u) & ~15u;
-  return w < bn ? w : bn;
-}
-// Bytes between two K core-matrix columns of a pass's image: the hi rows, then the lo rows, then a 32-byte skew.
-__host__ __device__ constexpr uint32_t pass_lbo(uint32_t width) { return 2u * width * 16u + 32u; }
-// The passes of a group of at most MERGE_TOKENS tokens (always a single pass) multiply W_hi by [x_hi | x_lo] in one
-// instruction of twice the pass's width (two column sets of one accumulator buffer, added in the epilogue): two
-// instructions per 16 values of K instead of three.  The rule looks at the group, not at the pass, so that the order
-// of a token's additions depends only on how many tokens its expert received, never on which pass it landed in:
-// results stay bit-identical from run to run although large dispatches are grouped with atomics.
-constexpr uint32_t MERGE_TOKENS = 64;
+// Token columns of a pass: its count rounded up to 16.
+__host__ __device__ constexpr uint32_t pass_width(uint32_t count) { return (count + 15u) & ~15u; }
 
 struct Ring {
   uint32_t stage = 0, round = 0, n;
@@ -164,48 +176,50 @@ struct Ring {
 };
 
 template <int DT>
-__global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
-  extern __shared__ __align__(128) uint8_t smem[];
+__global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_ffn_gemm(const GemmParams p, const __grid_constant__ ActMaps maps) {
+  extern __shared__ __align__(1024) uint8_t smem[];
   constexpr uint32_t BB = DT == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
   constexpr uint32_t TILE_RAW = RAW_BLOCKS * 16 * BB;  // bytes of RAW_BLOCKS blocks of one packed tile (2304 / 4352)
   constexpr uint32_t RAW_BYTES = 8 * TILE_RAW;
   const MoeDispatch &d = p.d;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  const uint32_t rank = blockIdx.x & 1;
   const uint32_t m_tiles = p.rows / (p.phase == 0 ? 64u : 128u);  // 128-row MMA tiles (8 packed tiles each)
-  const uint32_t n_chunks = p.kb_total / 2, n_groups = p.kb_total / GROUP;
+  const uint32_t m_pairs = (m_tiles + 1) / 2;                     // the second CTA of an odd last pair repeats the last tile, unwritten
+  const uint32_t n_groups = p.kb_total / GROUP;
   const uint32_t n_passes = *d.n_passes;
-  // Items (pass, 128-row tile) are dealt round-robin: the CTAs running at any moment work on a dozen
-  // neighbouring passes, so the activation images they all re-read stay in L2.
-  const uint32_t n_items = n_passes * m_tiles;
-  const uint32_t item_beg = blockIdx.x, item_step = gridDim.x;
+  // Items (pass, 256 rows) are dealt round-robin: the pairs running at any moment work on a dozen
+  // neighbouring passes, so the activation rows they all re-read stay in L2.
+  const uint32_t n_items = n_passes * m_pairs;
+  const uint32_t item_beg = blockIdx.x / PAIR, item_step = gridDim.x / PAIR;
   if (item_beg >= n_items) return;
 
   uint64_t *bars = reinterpret_cast<uint64_t *>(smem);
-  uint64_t *raw_full = bars, *raw_empty = bars + 8, *a_full = bars + 16, *done = bars + 24,
+  uint64_t *raw_full = bars, *raw_empty = bars + 8, *a_full = bars + 16, *b_full = bars + 24, *done = bars + 32,
            *acc_full = bars + 48, *acc_empty = bars + 50, *drain = bars + 52;
   uint32_t *s_tmem = reinterpret_cast<uint32_t *>(smem + 512);
   volatile uint32_t *s_abort = reinterpret_cast<volatile uint32_t *>(smem + 516);
-  uint8_t *s_raw = smem + G_HEADER;
-  uint8_t *s_b = s_raw + p.n_raw * RAW_BYTES;
-  const uint32_t b_stage = 16 * p.b_lbo;  // ring slot and image slot of one 64-value chunk of K: what the widest pass needs
+  uint8_t *s_b = smem + G_HEADER;
+  uint8_t *s_raw = s_b + p.n_b * B_STAGE;
 
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < MAX_RING; s++) {
       mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], DQ_WARPS);  // filled by the weight producer, left by every dequantiser warp
-      mbar_init(&a_full[s], DQ_WARPS + 1), mbar_init(&done[s], 1);  // per group: every dequantiser warp + the activation producer
+      mbar_init(&a_full[s], PAIR * DQ_WARPS), mbar_init(&b_full[s], 1);
     }
-    for (uint32_t s = 0; s < 2; s++) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], EPI_WARPS);
+    for (uint32_t s = 0; s < DONE_RING; s++) mbar_init(&done[s], 1);
+    for (uint32_t s = 0; s < 2; s++) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], PAIR * EPI_WARPS);
     mbar_init(drain, 1);
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == W_MMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(s_tmem)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();
   tc_fence_after();
   // The CTA owns all 512 columns of its SM's tensor memory, so the allocation starts at lane 0, column 0.  Using the
   // constant instead of the value read back lets every TMEM address below be computed in uniform registers: with the
@@ -213,7 +227,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
   // the kernel gives the columns back, latches the error status and leaves.
   constexpr uint32_t tmem_base = 0;
   if (*s_tmem != tmem_base) {
-    if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*s_tmem), "r"(TMEM_COLS) : "memory");
+    if (warp == W_MMA) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(*s_tmem), "r"(TMEM_COLS) : "memory");
     if (threadIdx.x == 0) atomicOr(p.d.status, MER_DEVSTAT_TIMEOUT);
     return;
   }
@@ -229,15 +243,18 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
 
   if (warp == W_PRODUCER) {
     // ------------------------------------------------------------------------ producer of the activation stages
-    // one stage = one group of blocks of K of the pass's activation image: two chunks of 64 values, one bulk copy each.
-    // A stage is free again when the MMAs of the group that used it have run: the issuer's done[] commit says so.
+    // one stage = one group of blocks of K of this CTA's half of the pass's rows; lane l copies chunk l / 2, the hi parts
+    // (even l) or the lo parts.  A stage is free again when the MMAs of the group that used it have run: the
+    // issuer's done[] commit says so.
     Ring rb(p.n_b);
     uint32_t pg = 0;  // groups issued so far, over all items (the issuer counts the same way)
+    const uint32_t chunk = lane >> 1, part = lane & 1, K = p.kb_total * 32;
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_tiles;
+      const uint32_t pass = item / m_pairs;
       if (!expert_base(pass)) continue;
-      const uint8_t *bsrc = p.act_img + (size_t)pass * n_chunks * b_stage;
-      const uint32_t bytes = 8 * pass_lbo(pass_width(p.bn, __ldg(d.pass_count + pass)));  // a narrow pass has a small image
+      const uint32_t width = pass_width(__ldg(d.pass_count + pass));
+      const uint32_t row = __ldg(d.pass_start + pass) + rank * (width / PAIR);
+      const CUtensorMap *map = &maps.m[width / 16 - 1];
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, pg++) {
         if (pg >= p.n_b) {
           const uint32_t sp = pg - p.n_b;
@@ -246,20 +263,23 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(&a_full[rb.stage], 2 * bytes);  // stage = group parity: the barrier the group's A stages complete too
+        if (rank == 0 && lane == 0) mbar_expect_tx(&b_full[rb.stage], CHUNKS * width * 2 * 128);  // both CTAs' bytes
         __syncwarp();
-        if (lane < 2)
-          bulk_g2s(s_b + ((size_t)rb.stage * 2 + lane) * b_stage, bsrc + ((size_t)gi * 2 + lane) * b_stage, bytes, &a_full[rb.stage]);
+        if (lane < 2 * CHUNKS)
+          tile_g2s(smem_u32(s_b) + rb.stage * B_STAGE + chunk * CHUNK_BYTES + part * PART_BYTES, map,
+                   part * K + (gi * CHUNKS + chunk) * CHUNK_K, row, leader_addr(&b_full[rb.stage]));
         rb.advance();
       }
     }
     if (!ok) {
       if (lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
-      // copies already in flight get a bounded chance to land before the CTA's shared memory is released
-      for (uint32_t s = 0; s < p.n_b; s++) (void)mbar_wait(&a_full[s], 0), (void)mbar_wait(&a_full[s], 1);
+      // copies already in flight get a bounded chance to land before the pair's shared memory is released
+      if (rank == 0)
+        for (uint32_t s = 0; s < p.n_b; s++) (void)mbar_wait(&b_full[s], 0), (void)mbar_wait(&b_full[s], 1);
     }
   } else if (warp == W_MMA) {
-    // -------------------------------------------------------------------------- MMA issuer
+    // -------------------------------------------------------------------------- MMA issuer (of the pair: its first CTA)
+    if (rank == 0) {
     // The whole warp walks the loops and waits (every value it computes is warp-uniform); the elected lane issues.
     // one step = one 32-value block of K: two instructions of 16 values for each of the three operand pairings
     Ring rb(p.n_b);
@@ -268,23 +288,20 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
     uint32_t grp = 0;     // groups of GROUP blocks issued so far, over all items; A-stage half = grp & 1
     // B descriptors differ only in their start-address field: one base, then 64-bit adds of (byte offset >> 4).
     // (The ring lies well inside the 256 KB the 14-bit field spans, so the adds never carry out of it.)
-    const uint32_t stage16 = b_stage >> 4;
+    const uint64_t b_desc0 = smem_desc(smem_u32(s_b));
     // One item's K loop for a pass of WIDTH columns.  WIDTH is a template argument because everything the MMA instruction
     // takes (descriptors, TMEM addresses) must sit in uniform registers: values derived from kernel parameters and
     // constants are computed there directly, values derived from a loaded pass count had to be moved over per
     // instruction (measured: +25 % issue time).
-    auto run_item = [&](auto width_tag, auto merged_tag) {
-      constexpr uint32_t width = decltype(width_tag)::value, lbo = pass_lbo(width);
-      constexpr bool merged = decltype(merged_tag)::value;
-      constexpr uint32_t idesc = instr_desc(width), idesc2 = instr_desc(2 * width);
-      constexpr uint32_t half16 = (4 * lbo) >> 4, j16 = (2 * lbo) >> 4, lo16 = width;  // the lo rows follow the hi rows: width * 16 bytes
-      const uint64_t b_desc0 = smem_desc(smem_u32(s_b), lbo, 128);
+    auto run_item = [&](auto width_tag) {
+      constexpr uint32_t idesc = instr_desc(decltype(width_tag)::value);
       const uint32_t buf = n_done & 1, use = n_done >> 1;
       const uint32_t d_tmem = tmem_base + buf * 128;
       for (uint32_t st = 0; st < p.kb_total && ok; st += GROUP, grp++) {
-        const uint32_t ag = grp & 1;
-        if (st == 0 && use > 0) ok = mbar_wait(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
-        if (ok) ok = mbar_wait(&a_full[ag], (grp >> 1) & 1);
+        const uint32_t ag = grp % A_RING;
+        if (st == 0 && use > 0) ok = mbar_wait_cluster(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
+        if (ok) ok = mbar_wait_cluster(&b_full[rb.stage], rb.round & 1);
+        if (ok) ok = mbar_wait_cluster(&a_full[ag], (grp / A_RING) & 1);
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the vote also tells the compiler so
         if (!ok) break;
@@ -292,54 +309,35 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
 #pragma unroll
         for (uint32_t b4 = 0; b4 < GROUP; b4++) {
           const uint32_t a_hi = tmem_base + TMEM_A0 + (ag * GROUP + b4) * A_STAGE_COLS, a_lo = a_hi + 16;
-          const uint64_t b_blk = b_desc0 + (uint64_t)((rb.stage * 2 + (b4 >> 1)) * stage16 + (b4 & 1) * half16);
+          const uint64_t b_blk = b_desc0 + (uint64_t)((rb.stage * B_STAGE + (b4 >> 1) * CHUNK_BYTES + (b4 & 1) * 64) >> 4);
 #pragma unroll
-          for (uint32_t j = 0; j < 2; j++) {  // 16 values of K per instruction: 8 TMEM columns of A, two core-matrix columns of B
-            const uint64_t dbh = b_blk + (uint64_t)(j * j16), dbl = dbh + lo16;
+          for (uint32_t j = 0; j < 2; j++) {  // 16 values of K per instruction: 8 TMEM columns of A, 32 bytes of a row of B
+            const uint64_t dbh = b_blk + (uint64_t)(j * 2), dbl = dbh + (PART_BYTES >> 4);
             const uint32_t acc = (b4 == 0 && j == 0) ? (st != 0) : 1u;  // the item's first MMA overwrites the accumulator
-            if (merged) {
-              tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc2, acc);  // columns [0, width): W_hi x_hi; [width, 2 width): W_hi x_lo
-            } else {
-              tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc, acc);
-              tc_mma_ts_acc(leader, d_tmem, a_hi + j * 8, dbl, idesc);
-            }
+            tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc, acc);
+            tc_mma_ts_acc(leader, d_tmem, a_hi + j * 8, dbl, idesc);
             tc_mma_ts_acc(leader, d_tmem, a_lo + j * 8, dbh, idesc);
           }
         }
         rb.advance();
-        tc_commit(leader, &done[grp % DONE_RING]);  // frees the group's A stages and its activation stage
+        tc_commit(leader, &done[grp % DONE_RING]);  // frees the group's A stages and its activation stage, in both CTAs
         if (st + GROUP >= p.kb_total) tc_commit(leader, &acc_full[buf]);
       }
       n_done++;
     };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_tiles;
+      const uint32_t pass = item / m_pairs;
       if (!expert_base(pass)) continue;
-      // the MMA is as wide as the pass has tokens (rounded up to 16 columns): a ragged last pass of a group costs
-      // its share, not a full tile
-      const uint32_t grp_id = __ldg(d.pass_group + pass);
-      const bool merged = __ldg(d.offsets + grp_id + 1) - __ldg(d.offsets + grp_id) <= MERGE_TOKENS;
-      const uint32_t w16 = pass_width(p.bn, __ldg(d.pass_count + pass)) >> 4;
-      using T = std::true_type;
-      using F = std::false_type;
-      if (merged) {
-        switch (w16) {
-          case 1: run_item(std::integral_constant<uint32_t, 16>{}, T{}); break;
-          case 2: run_item(std::integral_constant<uint32_t, 32>{}, T{}); break;
-          case 3: run_item(std::integral_constant<uint32_t, 48>{}, T{}); break;
-          default: run_item(std::integral_constant<uint32_t, 64>{}, T{}); break;
-        }
-      } else {
-        switch (w16) {
-          case 1: run_item(std::integral_constant<uint32_t, 16>{}, F{}); break;
-          case 2: run_item(std::integral_constant<uint32_t, 32>{}, F{}); break;
-          case 3: run_item(std::integral_constant<uint32_t, 48>{}, F{}); break;
-          case 4: run_item(std::integral_constant<uint32_t, 64>{}, F{}); break;
-          case 5: run_item(std::integral_constant<uint32_t, 80>{}, F{}); break;
-          case 6: run_item(std::integral_constant<uint32_t, 96>{}, F{}); break;
-          case 7: run_item(std::integral_constant<uint32_t, 112>{}, F{}); break;
-          default: run_item(std::integral_constant<uint32_t, 128>{}, F{}); break;
-        }
+      // the MMA is as wide as the pass has tokens (rounded up to 16 columns)
+      switch (pass_width(__ldg(d.pass_count + pass)) >> 4) {
+        case 1: run_item(std::integral_constant<uint32_t, 16>{}); break;
+        case 2: run_item(std::integral_constant<uint32_t, 32>{}); break;
+        case 3: run_item(std::integral_constant<uint32_t, 48>{}); break;
+        case 4: run_item(std::integral_constant<uint32_t, 64>{}); break;
+        case 5: run_item(std::integral_constant<uint32_t, 80>{}); break;
+        case 6: run_item(std::integral_constant<uint32_t, 96>{}); break;
+        case 7: run_item(std::integral_constant<uint32_t, 112>{}); break;
+        default: run_item(std::integral_constant<uint32_t, 128>{}); break;
       }
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
@@ -348,15 +346,17 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
     tc_commit(leader, drain);
     (void)mbar_wait(drain, 0);
     __syncwarp();
+    }
   } else if (warp == W_WEIGHTS) {
     // ------------------------------------------------------------------------ producer of the weight stages
-    // one stage = one group of RAW_BLOCKS blocks of the item's eight packed tiles; lane m < 8 copies tile m's chunk
+    // one stage = RAW_BLOCKS blocks of K of the item's eight packed tiles; lane m < 8 copies tile m's chunk
     Ring raw(p.n_raw);
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint8_t *base = expert_base(item / m_tiles);
+      const uint8_t *base = expert_base(item / m_pairs);
       if (!base) continue;
-      const uint8_t *src = base + region + (size_t)((item % m_tiles) * 8 + (lane & 7)) * tile_bytes;
-      for (uint32_t gi = 0; gi < n_groups && ok; gi++) {
+      const uint32_t mt = min((item % m_pairs) * PAIR + rank, m_tiles - 1);
+      const uint8_t *src = base + region + (size_t)(mt * 8 + (lane & 7)) * tile_bytes;
+      for (uint32_t gi = 0; gi < p.kb_total / RAW_BLOCKS && ok; gi++) {
         if (raw.round > 0) ok = mbar_wait(&raw_empty[raw.stage], (raw.round - 1) & 1);  // every dequantiser warp has left the stage
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
@@ -379,18 +379,20 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
     // 16 columns of hi and 16 of lo.  The two warps of a quarter take alternate blocks.
     Ring raw(p.n_raw);
     uint32_t gblk = 0;  // blocks of K seen so far, over all items (A stage = gblk % A_STAGES)
-    const uint32_t q = warp & 3, mine = (warp - W_DQ0) >> 2;
+    const uint32_t q = warp & 3, mine = (warp - W_DQ0) >> 2;  // lanes of TMEM; block of every DQ_WARPS / 4
     const uint32_t T = 2 * q + (lane >> 4), g = lane & 7, half = (lane >> 3) & 1;
     const __half2 zp = DT == MER_DTYPE_Q4_0 ? __floats2half2_rn(1032.0f, 1032.0f) : __floats2half2_rn(1152.0f, 1152.0f);
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_tiles;
+      const uint32_t pass = item / m_pairs;
       if (!expert_base(pass)) continue;
-      // one group (= one weight stage) at a time: this warp's two blocks of it, one wait on each side
+      // a group of blocks at a time, RAW_BLOCKS / GROUP of them per weight stage; this warp takes every other block
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, gblk += GROUP) {
-        ok = mbar_wait(&raw_full[raw.stage], raw.round & 1);
+        constexpr uint32_t PER = RAW_BLOCKS / GROUP;
+        const uint32_t in_stage = gi % PER;
+        if (in_stage == 0) ok = mbar_wait(&raw_full[raw.stage], raw.round & 1);
         if (ok && gblk >= A_STAGES) {
-          // the group's A stages were last read by the MMAs of group gblk / GROUP - 2
-          const uint32_t sp = gblk / GROUP - A_STAGES / GROUP;
+          // the group's A stages were last read by the MMAs of the group A_RING before it
+          const uint32_t sp = gblk / GROUP - A_RING;
           ok = mbar_wait(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
         }
         if (*s_abort) ok = false;
@@ -399,8 +401,8 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
         tc_fence_after();
         const uint32_t tile_src = smem_u32(s_raw) + raw.stage * RAW_BYTES + T * TILE_RAW;
 #pragma unroll
-        for (uint32_t hb = 0; hb < GROUP / 2; hb++) {
-          const uint32_t sub = mine + 2 * hb;  // block of the group handled here
+        for (uint32_t hb = 0; hb < GROUP * 4 / DQ_WARPS; hb++) {
+          const uint32_t in_group = mine + DQ_WARPS / 4 * hb, sub = in_stage * GROUP + in_group;  // block of the group and of the weight stage
           uint32_t v[32];  // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
           if (DT == MER_DTYPE_Q8_0) {
             const uint32_t src = tile_src + sub * 544;
@@ -431,16 +433,16 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
               dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
             }
           }
-          tc_st32(tmem_base + ((q * 32u) << 16) + TMEM_A0 + ((gblk + sub) % A_STAGES) * A_STAGE_COLS, v);
+          tc_st32(tmem_base + ((q * 32u) << 16) + TMEM_A0 + ((gblk + in_group) % A_STAGES) * A_STAGE_COLS, v);
         }
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          mbar_arrive(&a_full[(gblk / GROUP) & 1]);
-          mbar_arrive(&raw_empty[raw.stage]);
+          arrive_cluster(leader_addr(&a_full[(gblk / GROUP) % A_RING]));
+          if (in_stage == PER - 1) mbar_arrive(&raw_empty[raw.stage]);
         }
-        raw.advance();
+        if (in_stage == PER - 1) raw.advance();
       }
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
@@ -451,7 +453,6 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
     const uint32_t q = warp & 3;         // a warp reads the TMEM lanes 32 * (warp % 4) ..
     const uint32_t row = q * 32 + lane;  // row of the item's 128-row tile
     const uint32_t buf = (warp - W_EPI0) >> 2, gw = (warp - W_EPI0) & 3;  // group, warp within the group
-    uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 1024 + buf * 2048);
     float *s_un = reinterpret_cast<float *>(smem + 1024 + buf * 2048 + 512);
     float **s_row = reinterpret_cast<float **>(smem + 1024 + buf * 2048 + 1024);  // down phase: each token's output row
     uint32_t n_item = 0, used = 0;  // resident items seen by the CTA; uses of this group's buffer
@@ -459,7 +460,7 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
     // that the group's named barriers always see all four warps.
     bool dead = false;
     for (uint32_t item = item_beg; item < n_items; item += item_step) {
-      const uint32_t pass = item / m_tiles, mt = item % m_tiles;
+      const uint32_t pass = item / m_pairs, mt = (item % m_pairs) * PAIR + rank;
       const bool resident = expert_base(pass) != nullptr;
       if (resident) {
         if ((n_item++ & 1) != buf) continue;  // the other group's item
@@ -473,11 +474,10 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
       {
         const uint32_t c = gw * 32 + lane;
         const bool have = c < pcount;
-        const uint32_t pr = have ? __ldg(d.perm + pstart + c) : 0u;
-        const float un = have ? __ldg(p.unscale + (size_t)pass * p.bn + c) : 0.0f;
+        const float un = have ? __ldg(p.unscale + pstart + c) : 0.0f;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + buf) : "memory");  // the group has finished reading the previous item's tables
-        s_pair[c] = pr, s_un[c] = un;
-        if (p.phase == 1) s_row[c] = have ? pair_output_row(d, p.out, pr) : nullptr;
+        s_un[c] = un;
+        if (p.phase == 1) s_row[c] = have ? pair_output_row(d, p.out, __ldg(d.perm + pstart + c)) : nullptr;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + buf) : "memory");
       }
       if (resident && !dead) {
@@ -490,267 +490,219 @@ __global__ void __launch_bounds__(G_THREADS, 1) k_ffn_gemm(GemmParams p) {
         atomicOr(d.status, MER_DEVSTAT_RESIDENCY_MISS);  // fail closed: zeros below
       }
       const uint32_t acc_addr = tmem_base + ((q * 32u) << 16) + buf * 128;
-      const uint32_t width = pass_width(p.bn, pcount);
-      const uint32_t grp_id = d.pass_group[pass];
-      const bool merged = d.offsets[grp_id + 1] - d.offsets[grp_id] <= MERGE_TOKENS;
       const bool is_gate = (lane & 8) == 0;
       const bool clamp = d.swiglu_limit > 0.0f && isfinite(d.swiglu_limit);
-      for (uint32_t cbase = 0; cbase < pcount; cbase += 32) {  // 32 columns (tokens) at a time
-        uint32_t v[32];
-        float val[32];
+      constexpr int EC = 16;  // columns (tokens) at a time
+      for (uint32_t cbase = 0; cbase < pcount && mt < m_tiles; cbase += EC) {
+        float val[EC];
         if (resident && !dead) {
-          tc_ld32(acc_addr + cbase, v);
+          uint32_t v[EC];
+          tc_ld16(acc_addr + cbase, v);
 #pragma unroll
-          for (int i = 0; i < 32; i++) val[i] = __uint_as_float(v[i]);
-          if (merged) {  // the W_hi x_lo column set of the same tokens
-            tc_ld32(acc_addr + width + cbase, v);
-#pragma unroll
-            for (int i = 0; i < 32; i++) val[i] += __uint_as_float(v[i]);
-          }
+          for (int i = 0; i < EC; i++) val[i] = __uint_as_float(v[i]);
         } else {
 #pragma unroll
-          for (int i = 0; i < 32; i++) val[i] = 0.0f;
+          for (int i = 0; i < EC; i++) val[i] = 0.0f;
         }
         // the steps run column-batched (all multiplies, then all shuffles, ...): warp-synchronous operations are kept in
         // program order, so a column-by-column loop would serialise on the latency of every single one
 #pragma unroll
-        for (int i = 0; i < 32; i++) val[i] *= s_un[cbase + i];
+        for (int i = 0; i < EC; i++) val[i] *= s_un[cbase + i];
         if (p.phase == 0) {
           // rows come in packed tiles of 16: slots 0..7 gate rows, 8..15 the matching up rows
-          float up[32];
+          float up[EC];
 #pragma unroll
-          for (int i = 0; i < 32; i++) up[i] = __shfl_down_sync(0xffffffffu, val[i], 8);
+          for (int i = 0; i < EC; i++) up[i] = __shfl_down_sync(0xffffffffu, val[i], 8);
 #pragma unroll
-          for (int i = 0; i < 32; i++) {
+          for (int i = 0; i < EC; i++) {
             float gate = val[i];
             if (clamp && gate == gate) gate = fminf(fmaxf(gate, -d.swiglu_limit), d.swiglu_limit);
             val[i] = __fdividef(gate, 1.0f + __expf(-gate)) * up[i];
           }
-          float *dst = p.out + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
+          // h in the order of the groups: its rows are then the rows of the down phase's passes
+          float *dst = p.out + (size_t)(pstart + cbase) * d.F + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
 #pragma unroll
-          for (int i = 0; i < 32; i++)
-            if (is_gate && cbase + i < pcount) dst[(size_t)s_pair[cbase + i] * d.F] = val[i];
+          for (int i = 0; i < EC; i++)
+            if (is_gate && cbase + i < pcount) dst[(size_t)i * d.F] = val[i];
         } else {
           const uint32_t off = mt * 128 + row;
 #pragma unroll
-          for (int i = 0; i < 32; i++)
+          for (int i = 0; i < EC; i++)
             if (cbase + i < pcount) s_row[cbase + i][off] = val[i];
         }
       }
       if (resident && !dead) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        if (lane == 0) arrive_cluster(leader_addr(&acc_empty[buf]));
       }
     }
     if (dead && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
   }
 
+  // neither CTA may leave while the other's MMAs read its memory or its warps signal barriers here
   tc_fence_before();
-  __syncthreads();
+  cluster_sync();
   if (warp == W_MMA) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
 }
 
-// Per-token row maximum of |x| (the gate/up activations' scale source).  One warp per token.
-__global__ void __launch_bounds__(256) k_row_amax(const float *__restrict__ x, uint32_t n_tokens, uint32_t K, uint32_t *__restrict__ amax) {
-  const uint32_t tok = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (tok >= n_tokens) return;
-  const float4 *r4 = reinterpret_cast<const float4 *>(x + (size_t)tok * K);
+// Rows of activations -> rows of their f16 hi parts and lo parts, [hi K | lo K], after an exact power-of-two scaling of the
+// row, and its inverse.  Row i of the output belongs to the i-th pair in group order, so that a pass is a run of rows and
+// one copy fetches a chunk of all of them; its source is row i of h, or with `perm` row perm[i] / slots of the tokens
+// (a token that eight experts share is converted eight times; rows picked by the GEMM's own copies instead,
+// four per gather, took 80 cycles per four rows and doubled the GEMM's time).  TPR threads per row.
+template <int TPR>
+__global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ act, uint32_t K, const uint32_t *__restrict__ perm,
+                                                    uint32_t slots, const uint32_t *__restrict__ n_grouped, uint16_t *__restrict__ out,
+                                                    float *__restrict__ unscale) {
+  const uint32_t i = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, t = threadIdx.x % TPR;
+  const bool have = i < *n_grouped;  // fewer than the pairs of the dispatch under expert parallelism
+  if (TPR <= 32 && !have) return;
+  const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)(have && perm ? perm[i] / slots : i) * K);
   float mx = 0.0f;
   bool nan = false;
-  for (uint32_t i = lane; i < K / 4; i += 32) {
-    const float4 v = __ldg(r4 + i);
-    nan |= (v.x != v.x) | (v.y != v.y) | (v.z != v.z) | (v.w != v.w);
-    mx = fmaxf(fmaxf(fmaxf(fmaxf(mx, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
+  if (have) {
+#pragma unroll 4
+    for (uint32_t k = t; k < K / 4; k += TPR) {
+      const float4 v = __ldg(src + k);
+      nan |= (v.x != v.x) | (v.y != v.y) | (v.z != v.z) | (v.w != v.w);
+      mx = fmaxf(fmaxf(fmaxf(fmaxf(mx, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  nan = __any_sync(0xffffffffu, nan);
-  if (lane == 0) amax[tok] = nan ? 0x7fc00000u : __float_as_uint(mx);
+  if (__any_sync(0xffffffffu, nan)) mx = __uint_as_float(0x7fc00000u);
+  if (TPR > 32) {
+    __shared__ float s_mx[8];
+    if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    mx = s_mx[0];
+    for (int w = 1; w < 8; w++) mx = s_mx[w] != s_mx[w] || mx != mx ? __uint_as_float(0x7fc00000u) : fmaxf(mx, s_mx[w]);
+    if (!have) return;
+  }
+  float sc = 1.0f;
+  if (mx > 0.0f && isfinite(mx)) {
+    int e;
+    frexpf(mx, &e);
+    sc = ldexpf(1.0f, (int)POW2_SCALE_TARGET - e);  // mx * sc in [256, 512)
+  } else if (mx != mx || isinf(mx)) {
+    sc = mx;  // non-finite activations poison the row, as they would in fp32
+  }
+  if (t == 0) unscale[i] = 1.0f / sc;
+  uint2 *hi = reinterpret_cast<uint2 *>(out + (size_t)i * 2 * K), *lo = hi + K / 4;
+#pragma unroll 4
+  for (uint32_t k = t; k < K / 4; k += TPR) {
+    const float4 v = __ldg(src + k);
+    const float a = v.x * sc, b = v.y * sc, c = v.z * sc, e = v.w * sc;
+    const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, e);
+    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+    hi[k] = make_uint2(h2_bits(h0), h2_bits(h1));
+    lo[k] = make_uint2(h2_bits(__floats2half2_rn(a - f0.x, b - f0.y)), h2_bits(__floats2half2_rn(c - f1.x, e - f1.y)));
+  }
 }
 
-// Row maxima of the grouped rows of h only (perm lists them): in an expert-parallel dispatch most pairs belong to other
-// ranks and their rows of h are never written or read.
-__global__ void __launch_bounds__(256) k_row_amax_grouped(MoeDispatch d, const float *__restrict__ h, uint32_t K, uint32_t *__restrict__ amax) {
-  const uint32_t i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (i >= d.offsets[d.n_groups]) return;
-  const uint32_t pair = d.perm[i];
-  const float4 *r4 = reinterpret_cast<const float4 *>(h + (size_t)pair * K);
-  float mx = 0.0f;
-  bool nan = false;
-  for (uint32_t k = lane; k < K / 4; k += 32) {
-    const float4 v = __ldg(r4 + k);
-    nan |= (v.x != v.x) | (v.y != v.y) | (v.z != v.z) | (v.w != v.w);
-    mx = fmaxf(fmaxf(fmaxf(fmaxf(mx, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  nan = __any_sync(0xffffffffu, nan);
-  if (lane == 0) amax[pair] = nan ? 0x7fc00000u : __float_as_uint(mx);
+void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *perm, uint32_t slots, const uint32_t *n_grouped,
+                       uint16_t *out, float *unscale, cudaStream_t s) {
+  // a warp per row keeps short rows of large batches cheap; long rows, and few of them, want more loads in flight
+  if (K <= 2048 && n_rows >= 2048)
+    k_split_rows<32><<<(n_rows + 7) / 8, 256, 0, s>>>(act, K, perm, slots, n_grouped, out, unscale);
+  else
+    k_split_rows<256><<<n_rows, 256, 0, s>>>(act, K, perm, slots, n_grouped, out, unscale);
 }
 
-// Builds, for every token pass, the activation operand images the GEMM kernel copies chunk by chunk.  A chunk is 64
-// values of K = 8 core-matrix columns; a column holds the pass's rows as 16-byte pieces, the f16 hi parts of all rows
-// first, then the lo parts (+32 B skew): [hi row 0 .. hi row w-1 | lo row 0 .. lo row w-1], w = the pass's width
-// (its token count rounded up to 16), so one descriptor of 2w rows covers [x_hi | x_lo] and a narrow pass is a small
-// image.  grid = (pass capacity, K / 64).
-__global__ void __launch_bounds__(256) k_gemm_act_image(MoeDispatch d, int phase, const float *__restrict__ act, uint32_t K, uint32_t bn,
-                                                        uint32_t b_lbo, const uint32_t *__restrict__ amax_tok, uint8_t *__restrict__ img,
-                                                        float *__restrict__ unscale) {
-  const uint32_t pass = blockIdx.x, chunk = blockIdx.y;
-  if (pass >= *d.n_passes) return;
-  const uint32_t pstart = d.pass_start[pass], pcount = d.pass_count[pass];
-  const uint32_t n_chunks = K / 64;
-  uint8_t *dst0 = img + ((size_t)pass * n_chunks + chunk) * 16 * b_lbo;  // slots are as large as the widest pass needs
-  const uint32_t width = pass_width(bn, pcount), lbo = pass_lbo(width);
-  // per row of the pass, once: where it comes from and its scale
-  __shared__ float s_scale[128];
-  __shared__ uint32_t s_src[128];
-  for (uint32_t j = threadIdx.x; j < width; j += blockDim.x) {
-    float sc = 0.0f;  // rows beyond the pass's count are zero rows
-    uint32_t rowi = 0;
-    if (j < pcount) {
-      const uint32_t pair = d.perm[pstart + j];
-      rowi = phase == 0 ? pair / d.slots : pair;
-      const float mx = __uint_as_float(phase == 0 ? amax_tok[rowi] : d.amax[pair]);
-      sc = 1.0f;
-      if (mx > 0.0f && isfinite(mx)) {
-        int e;
-        frexpf(mx, &e);
-        sc = ldexpf(1.0f, (int)POW2_SCALE_TARGET - e);  // mx * sc in [256, 512)
-      } else if (mx != mx || isinf(mx)) {
-        sc = mx;  // non-finite activations poison the row, as they would in fp32
-      }
-    }
-    s_scale[j] = sc, s_src[j] = rowi;
-    if (chunk == 0) unscale[(size_t)pass * bn + j] = j < pcount ? 1.0f / sc : 0.0f;
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                 const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// The driver's encoder, looked up once; null when the driver has none.
+EncodeTiled encode_tiled() {
+  static const EncodeTiled fn = [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<EncodeTiled>(p) : nullptr;
+  }();
+  return fn;
+}
+// Rows of [hi K | lo K] f16.  Rows past the end read as zeros.
+bool activation_maps(ActMaps *maps, void *base, uint32_t rows, uint32_t K) {
+  const EncodeTiled fn = encode_tiled();
+  bool ok = fn != nullptr;
+  for (uint32_t i = 0; i < PASS_TOKENS / 16 && ok; i++) {
+    const cuuint64_t dims[2] = {2ull * K, rows}, strides[1] = {4ull * K};
+    const cuuint32_t box[2] = {CHUNK_K, 8 * (i + 1)}, step[2] = {1, 1};
+    ok = fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
-  __syncthreads();
-  for (uint32_t idx = threadIdx.x; idx < width * 8; idx += blockDim.x) {
-    const uint32_t k8 = idx / width, j = idx - k8 * width;
-    uint4 hi = make_uint4(0, 0, 0, 0), lo = make_uint4(0, 0, 0, 0);
-    if (j < pcount) {
-      const float sc = s_scale[j];
-      const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)s_src[j] * K + chunk * 64 + k8 * 8);
-      const float4 a = __ldg(src), b = __ldg(src + 1);
-      const float vs[8] = {a.x * sc, a.y * sc, a.z * sc, a.w * sc, b.x * sc, b.y * sc, b.z * sc, b.w * sc};
-      uint32_t h[4], l[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const __half2 hh = __floats2half2_rn(vs[2 * i], vs[2 * i + 1]);
-        const float2 back = __half22float2(hh);
-        h[i] = h2_bits(hh);
-        l[i] = h2_bits(__floats2half2_rn(vs[2 * i] - back.x, vs[2 * i + 1] - back.y));
-      }
-      hi = make_uint4(h[0], h[1], h[2], h[3]), lo = make_uint4(l[0], l[1], l[2], l[3]);
-    }
-    uint8_t *dst = dst0 + (size_t)k8 * lbo + j * 16;
-    *reinterpret_cast<uint4 *>(dst) = hi;
-    *reinterpret_cast<uint4 *>(dst + width * 16) = lo;
-  }
+  return ok;
 }
 
 struct GemmPlan {
-  uint32_t n_raw, n_b, b_lbo;
+  uint32_t n_raw, n_b;
   size_t smem;
 };
 
-GemmPlan gemm_plan(int dtype, uint32_t bn) {
+GemmPlan gemm_plan(int dtype) {
   const uint32_t tile_raw = RAW_BLOCKS * 16 * (dtype == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES);
   GemmPlan pl{};
-  pl.b_lbo = bn * 16 + 32;
-  pl.n_raw = 4, pl.n_b = 2;  // weight stages (one group each); activation stages (one group = two chunk slots each)
-  pl.smem = G_HEADER + (size_t)pl.n_raw * 8 * tile_raw + (size_t)pl.n_b * 2 * 16 * pl.b_lbo;
+  pl.n_raw = 4, pl.n_b = 4;  // weight stages of four blocks; activation stages of one group
+  pl.smem = G_HEADER + (size_t)pl.n_raw * 8 * tile_raw + (size_t)pl.n_b * B_STAGE;
   return pl;
 }
 
-struct GemmScratch {
-  uint32_t *amax_tok;
-  float *unscale;
-  uint8_t *img;
-  size_t img_bytes;
-};
-
-GemmScratch gemm_scratch(void *scratch, size_t scratch_bytes, uint32_t max_tokens, uint32_t max_pairs) {
-  GemmScratch g{};
-  uint8_t *p = reinterpret_cast<uint8_t *>(scratch);
-  g.amax_tok = reinterpret_cast<uint32_t *>(p);
-  size_t off = ((size_t)max_tokens * 4 + 255) & ~(size_t)255;
-  g.unscale = reinterpret_cast<float *>(p + off);
-  off += ((size_t)3 * max_pairs * 4 + 128 * 4 + 255) & ~(size_t)255;
-  g.img = p + off;
-  g.img_bytes = scratch_bytes > off ? scratch_bytes - off : 0;
-  return g;
-}
+size_t unscale_bytes(uint32_t max_pairs) { return ((size_t)max_pairs * 4 + 255) & ~(size_t)255; }
 
 }  // namespace
 
 bool gemm_ffn_supported(int dtype, uint32_t D, uint32_t F) {
-  return (dtype == MER_DTYPE_Q4_0 || dtype == MER_DTYPE_Q8_0) && D % 128 == 0 && F % 128 == 0;  // whole 128-row tiles, whole groups of four blocks
+  return (dtype == MER_DTYPE_Q4_0 || dtype == MER_DTYPE_Q8_0) && D % 128 == 0 && F % 128 == 0;  // whole 128-row tiles, whole weight stages
 }
 
-// Activation images: rows padded to whole passes (at most 3 x max_pairs rows), 4 bytes per value plus the skew.
-size_t gemm_ffn_scratch_bytes(uint32_t max_tokens, uint32_t max_pairs, uint32_t D, uint32_t F) {
-  const size_t kmax = D > F ? D : F;
-  const size_t rows = (size_t)3 * max_pairs + 128;
-  return (((size_t)max_tokens * 4 + 255) & ~(size_t)255) + ((rows * 4 + 255) & ~(size_t)255) + rows * kmax * 4 + (rows / 16 + 1) * (kmax / 64) * 512 +
-         4096;
+// Scales and split rows of the pairs, for gate/up and then for down.
+size_t gemm_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F) {
+  return unscale_bytes(max_pairs) + (size_t)max_pairs * (D > F ? D : F) * 4;
 }
 
-// Tokens per pass for a dispatch: about 1.5 x the mean group size, within what the image scratch holds.
-// Returns 0 when the dispatch is better served by the streaming kernels.
+// Tokens per pass at most, or 0 when the dispatch is better served by the streaming kernels.
 uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
   const uint64_t P = (uint64_t)d.n_tokens * d.slots;
   const uint32_t groups = d.active_groups_hint ? d.active_groups_hint : 1;
   const uint64_t mean = (d.expected_pairs ? d.expected_pairs : P) / groups;
-  if (mean < min_mean_tokens) return 0;
-  uint32_t bn = mean <= 12 ? 16 : mean <= 24 ? 32 : mean <= 56 ? 64 : 128;
-  const uint64_t gmax = d.n_groups < P ? d.n_groups : P;
-  while (bn > 16 && P + gmax * (bn - 1) > (uint64_t)3 * d.scratch_pairs) bn >>= 1;
-  if (P + gmax * (bn - 1) > (uint64_t)3 * d.scratch_pairs + 128) return 0;
-  return bn;
+  return mean < min_mean_tokens ? 0 : PASS_TOKENS;
 }
 
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) {
-  stream_bind(d, stream_scratch, sm_count);  // pass tables and the per-pair max cells live in the streaming scratch
+  stream_bind(d, stream_scratch, sm_count);  // pass tables live in the streaming scratch
   d.tokens_per_pass = bn;
 }
 
-cudaError_t launch_ffn_gemm(MoeDispatch &d, void *gemm_scratch_ptr, size_t gemm_scratch_bytes, uint32_t max_tokens, int sm_count,
-                            cudaStream_t s, int *launches, cudaEvent_t ev_mid) {
-  const uint32_t bn = d.tokens_per_pass;
-  const GemmPlan pl = gemm_plan(d.dtype, bn);
-  const GemmScratch gs = gemm_scratch(gemm_scratch_ptr, gemm_scratch_bytes, max_tokens, d.scratch_pairs);
+cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid) {
+  const GemmPlan pl = gemm_plan(d.dtype);
   const uint32_t P = d.n_tokens * d.slots;
-  const uint32_t gmax = d.n_groups < P ? d.n_groups : P;
-  const uint32_t pass_cap = P / bn + gmax;  // upper bound on the number of passes
+  float *unscale = reinterpret_cast<float *>(scratch);
+  const size_t off = unscale_bytes(d.scratch_pairs);
+  uint16_t *rows = reinterpret_cast<uint16_t *>(static_cast<uint8_t *>(scratch) + off);
+  if (P > d.scratch_pairs || off + (size_t)P * (d.D > d.F ? d.D : d.F) * 4 > scratch_bytes) return cudaErrorInvalidConfiguration;
   auto kern = d.dtype == MER_DTYPE_Q4_0 ? k_ffn_gemm<MER_DTYPE_Q4_0> : k_ffn_gemm<MER_DTYPE_Q8_0>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
   if (e != cudaSuccess) return e;
 
-  k_row_amax<<<(d.n_tokens + 7) / 8, 256, 0, s>>>(d.x, d.n_tokens, d.D, gs.amax_tok);
   for (int phase = 0; phase < 2; phase++) {
     const uint32_t K = phase == 0 ? d.D : d.F;
-    const float *act = phase == 0 ? d.x : d.h;
-    k_gemm_act_image<<<dim3(pass_cap, K / 64), 256, 0, s>>>(d, phase, act, K, bn, pl.b_lbo, gs.amax_tok, gs.img, gs.unscale);
+    launch_split_rows(phase == 0 ? d.x : d.h, P, K, phase == 0 ? d.perm : nullptr, d.slots, d.offsets + d.n_groups, rows, unscale, s);
+    ActMaps maps;
+    if (!activation_maps(&maps, rows, P, K)) return cudaErrorNotSupported;
     GemmParams p{};
-    p.d = d, p.phase = phase, p.act_img = gs.img, p.unscale = gs.unscale;
+    p.d = d, p.phase = phase, p.unscale = unscale;
     p.rows = phase == 0 ? d.F : d.D;
     p.kb_total = K / 32;
-    p.bn = bn, p.b_lbo = pl.b_lbo, p.n_raw = pl.n_raw, p.n_b = pl.n_b;
+    p.n_raw = pl.n_raw, p.n_b = pl.n_b;
     p.out = phase == 0 ? d.h : d.y;
-    kern<<<sm_count, G_THREADS, pl.smem, s>>>(p);
-    if (phase == 0) {
-      // row maxima of h = SiLU(gate) * up, the scale source of the down phase's operand image (the GEMM epilogue does
-      // not collect them: a warp reduction per column sat on its critical path)
-      k_row_amax_grouped<<<(P + 7) / 8, 256, 0, s>>>(d, d.h, d.F, d.amax);
-      if (ev_mid) cudaEventRecord(ev_mid, s);
-    }
+    kern<<<sm_count / PAIR * PAIR, G_THREADS, pl.smem, s>>>(p, maps);
+    if (phase == 0 && ev_mid) cudaEventRecord(ev_mid, s);
   }
   d.y_parts = nullptr, d.y_nparts = 1;
-  if (launches) (*launches) += 6;
+  if (launches) (*launches) += 4;
   return cudaGetLastError();
 }

@@ -113,9 +113,13 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
 #pragma unroll 1
   for (uint32_t g = g0; g < g1; g++) {
     const uint32_t beg = off[g], end = off[g + 1];
+    // the GEMM kernels work at a width of the pass's tokens, 16 at a time: several passes of a group share its tokens
+    // evenly, as a narrow last pass would still have all the weights to dequantise
+    const uint32_t n = (end - beg + tpp - 1) >> tpp_shift;
+    const uint32_t step = tpp >= 16 && n > 1 ? ((end - beg + n - 1) / n + 15) & ~15u : tpp;
 #pragma unroll 1
-    for (uint32_t st = beg; st < end; st += tpp) {
-      const uint32_t cnt = min(tpp, end - st);
+    for (uint32_t st = beg; st < end; st += step) {
+      const uint32_t cnt = min(step, end - st);
       d.pass_group[np] = g;
       d.pass_start[np] = st;
       d.pass_count[np] = cnt;

@@ -300,7 +300,7 @@ cudaError_t run_ffn(mer_backend *b, MoeDispatch &d, cudaStream_t s, int *launche
   d.y_parts = nullptr, d.y_nparts = 1;
   d.combined = 0;
   if (d.gemm_bn)
-    return launch_ffn_gemm(d, b->d_gemm_scratch, b->gemm_scratch_bytes, std::max(b->cfg.max_tokens, b->max_pairs), b->sm_count, s, launches,
+    return launch_ffn_gemm(d, b->d_gemm_scratch, b->gemm_scratch_bytes, b->sm_count, s, launches,
                            ev_mid);
   if (use_stream_path(b, d)) return launch_ffn_stream(d, b->d_stream_scratch, b->sm_count, s, launches, ev_mid);
   return launch_ffn_generic(d, s, launches, ev_mid);
@@ -918,8 +918,7 @@ MER_EXPORT int mer_backend_create(const mer_backend_cfg *cfg, mer_backend **out)
       CB(cudaMemset(b->d_stream_scratch, 0, sb));
     }
     if (sb && T >= 12 && gemm_ffn_supported(cfg->dtype, (uint32_t)D, (uint32_t)F)) {
-      // token rows of a dispatch may be (token, slot) pairs of other ranks (NCCL all-to-all mode): size per-row scratch by pairs
-      b->gemm_scratch_bytes = gemm_ffn_scratch_bytes((uint32_t)std::max(T, P), (uint32_t)P, (uint32_t)D, (uint32_t)F);
+      b->gemm_scratch_bytes = gemm_ffn_scratch_bytes((uint32_t)P, (uint32_t)D, (uint32_t)F);
       CB(cudaMalloc(&b->d_gemm_scratch, b->gemm_scratch_bytes));
     }
   }
