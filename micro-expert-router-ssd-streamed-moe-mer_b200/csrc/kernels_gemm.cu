@@ -53,7 +53,7 @@ constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16;
 constexpr uint32_t CHUNK_K = 64, CHUNKS = GROUP * 32 / CHUNK_K;  // a row's piece of a chunk is 128 bytes, the swizzle span
 constexpr uint32_t PASS_TOKENS = 128;    // tokens of a pass at most: N of one MMA, and the columns of an accumulator buffer
 constexpr uint32_t PART_BYTES = PASS_TOKENS / PAIR * 128, CHUNK_BYTES = 2 * PART_BYTES, B_STAGE = CHUNKS * CHUNK_BYTES;  // hi rows, then lo rows
-static_assert(RAW_BLOCKS % GROUP == 0 && A_STAGES % GROUP == 0 && GROUP * 32 % CHUNK_K == 0, "whole groups per stage");
+static_assert(RAW_BLOCKS % GROUP == 0 && DQ_WARPS == 4 * RAW_BLOCKS && A_STAGES % RAW_BLOCKS == 0, "a block of a weight stage for each of a quarter's warps");
 constexpr float POW2_SCALE_TARGET = 9;   // activations are scaled so that the row maximum lies in [256, 512)
 
 struct GemmParams {
@@ -206,7 +206,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < MAX_RING; s++) {
       mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], DQ_WARPS);  // filled by the weight producer, left by every dequantiser warp
-      mbar_init(&a_full[s], PAIR * DQ_WARPS), mbar_init(&b_full[s], 1);
+      mbar_init(&a_full[s], PAIR * 4 * GROUP), mbar_init(&b_full[s], 1);
     }
     for (uint32_t s = 0; s < DONE_RING; s++) mbar_init(&done[s], 1);
     for (uint32_t s = 0; s < 2; s++) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], PAIR * EPI_WARPS);
@@ -235,10 +235,26 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
   const size_t proj_bytes = (size_t)d.D * d.F / 32 * BB;
   const size_t tile_bytes = (size_t)p.kb_total * 16 * BB;
   const size_t region = p.phase == 0 ? 0 : 2 * proj_bytes;
-  auto expert_base = [&](uint32_t pass) -> const uint8_t * {
-    const uint32_t eid = d.group_expert[d.pass_group[pass]];
-    return eid < d.max_experts ? d.expert_ptr[eid] : nullptr;
+  // What a role needs to know of its items, fetched for 32 of them at a time, one per lane: the three dependent loads
+  // behind an expert's address would otherwise stall every role at the start of every item.
+  struct Items {
+    uint64_t base = 0;
+    uint32_t start = 0, count = 0;
+    __device__ void fetch(const MoeDispatch &d, uint32_t item, uint32_t n_items, uint32_t m_pairs) {
+      if (item >= n_items) return;
+      const uint32_t pass = item / m_pairs, eid = d.group_expert[__ldg(d.pass_group + pass)];
+      start = __ldg(d.pass_start + pass), count = __ldg(d.pass_count + pass);
+      base = eid < d.max_experts ? reinterpret_cast<uint64_t>(d.expert_ptr[eid]) : 0;
+    }
+  } items;
+  uint32_t item_no = 0;  // running number of the role's item
+  auto next_item = [&](uint32_t item, uint32_t &start, uint32_t &count) -> const uint8_t * {
+    const uint32_t k = item_no++ & 31;
+    if (k == 0) items.fetch(d, item + lane * item_step, n_items, m_pairs);
+    start = __shfl_sync(0xffffffffu, items.start, k), count = __shfl_sync(0xffffffffu, items.count, k);
+    return reinterpret_cast<const uint8_t *>(__shfl_sync(0xffffffffu, items.base, k));
   };
+  uint32_t pstart, pcount;
   bool ok = true;
 
   if (warp == W_PRODUCER) {
@@ -250,10 +266,8 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     uint32_t pg = 0;  // groups issued so far, over all items (the issuer counts the same way)
     const uint32_t chunk = lane >> 1, part = lane & 1, K = p.kb_total * 32;
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_pairs;
-      if (!expert_base(pass)) continue;
-      const uint32_t width = pass_width(__ldg(d.pass_count + pass));
-      const uint32_t row = __ldg(d.pass_start + pass) + rank * (width / PAIR);
+      if (!next_item(item, pstart, pcount)) continue;
+      const uint32_t width = pass_width(pcount), row = pstart + rank * (width / PAIR);
       const CUtensorMap *map = &maps.m[width / 16 - 1];
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, pg++) {
         if (pg >= p.n_b) {
@@ -302,7 +316,6 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         if (st == 0 && use > 0) ok = mbar_wait_cluster(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
         if (ok) ok = mbar_wait_cluster(&b_full[rb.stage], rb.round & 1);
         if (ok) ok = mbar_wait_cluster(&a_full[ag], (grp / A_RING) & 1);
-        if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the vote also tells the compiler so
         if (!ok) break;
         tc_fence_after();
@@ -326,10 +339,9 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       n_done++;
     };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_pairs;
-      if (!expert_base(pass)) continue;
+      if (!next_item(item, pstart, pcount)) continue;
       // the MMA is as wide as the pass has tokens (rounded up to 16 columns)
-      switch (pass_width(__ldg(d.pass_count + pass)) >> 4) {
+      switch (pass_width(pcount) >> 4) {
         case 1: run_item(std::integral_constant<uint32_t, 16>{}); break;
         case 2: run_item(std::integral_constant<uint32_t, 32>{}); break;
         case 3: run_item(std::integral_constant<uint32_t, 48>{}); break;
@@ -352,7 +364,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // one stage = RAW_BLOCKS blocks of K of the item's eight packed tiles; lane m < 8 copies tile m's chunk
     Ring raw(p.n_raw);
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint8_t *base = expert_base(item / m_pairs);
+      const uint8_t *base = next_item(item, pstart, pcount);
       if (!base) continue;
       const uint32_t mt = min((item % m_pairs) * PAIR + rank, m_tiles - 1);
       const uint8_t *src = base + region + (size_t)(mt * 8 + (lane & 7)) * tile_bytes;
@@ -376,73 +388,68 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // ------------------------------------------------------------------------ dequantisers
     // A thread owns one weight row of the item: TMEM lane 32 * (warp % 4) + lane, i.e. packed tile 2q + lane / 16,
     // row slot lane % 16.  Per block it reads the row's 32 quants from the tile chunk in shared memory and stores
-    // 16 columns of hi and 16 of lo.  The two warps of a quarter take alternate blocks.
+    // 16 columns of hi and 16 of lo.  The four warps of a quarter take one block of a weight stage each.
     Ring raw(p.n_raw);
     uint32_t gblk = 0;  // blocks of K seen so far, over all items (A stage = gblk % A_STAGES)
-    const uint32_t q = warp & 3, mine = (warp - W_DQ0) >> 2;  // lanes of TMEM; block of every DQ_WARPS / 4
+    const uint32_t q = warp & 3, mine = (warp - W_DQ0) >> 2;  // quarter of the rows; block of every weight stage
     const uint32_t T = 2 * q + (lane >> 4), g = lane & 7, half = (lane >> 3) & 1;
     const __half2 zp = DT == MER_DTYPE_Q4_0 ? __floats2half2_rn(1032.0f, 1032.0f) : __floats2half2_rn(1152.0f, 1152.0f);
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      const uint32_t pass = item / m_pairs;
-      if (!expert_base(pass)) continue;
-      // a group of blocks at a time, RAW_BLOCKS / GROUP of them per weight stage; this warp takes every other block
-      for (uint32_t gi = 0; gi < n_groups && ok; gi++, gblk += GROUP) {
-        constexpr uint32_t PER = RAW_BLOCKS / GROUP;
-        const uint32_t in_stage = gi % PER;
-        if (in_stage == 0) ok = mbar_wait(&raw_full[raw.stage], raw.round & 1);
-        if (ok && gblk >= A_STAGES) {
+      if (!next_item(item, pstart, pcount)) continue;
+      // One weight stage at a time, of which this warp converts one block.  It waits for the A stage only when the
+      // block is ready in registers: the conversion of the next blocks is then off the cycle of MMAs -> done -> store -> MMAs.
+      for (uint32_t gi = 0; gi < p.kb_total / RAW_BLOCKS && ok; gi++, gblk += RAW_BLOCKS) {
+        ok = mbar_wait(&raw_full[raw.stage], raw.round & 1);
+        const uint32_t tile_src = smem_u32(s_raw) + raw.stage * RAW_BYTES + T * TILE_RAW;
+        uint32_t v[32];  // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
+        if (DT == MER_DTYPE_Q8_0) {
+          const uint32_t src = tile_src + mine * 544;
+          const uint32_t sc2 = lds32(src + 512 + g * 4);
+          const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
+#pragma unroll
+          for (int t = 0; t < 4; t++) {  // values 8t .. 8t+7
+            const uint2 w = lds64(src + packed_piece(g, t) * 16 + half * 8);
+            const uint32_t w0 = w.x ^ 0x80808080u, w1 = w.y ^ 0x80808080u;
+            dq2(__byte_perm(w0, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
+            dq2(__byte_perm(w0, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
+            dq2(__byte_perm(w1, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
+            dq2(__byte_perm(w1, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
+          }
+        } else {
+          // block-pair record: 16 bytes per (g, t) = words (slot g, blk 0), (slot g+8, blk 0), (slot g, blk 1), (slot g+8, blk 1);
+          // byte i of a word holds values 4t+i (low nibble) and 16+4t+i (high nibble) of its block
+          const uint32_t src = tile_src + (mine >> 1) * 576, blk = mine & 1;
+          const uint32_t sc2 = lds32(src + 512 + g * 8 + blk * 4);
+          const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
+#pragma unroll
+          for (int t = 0; t < 4; t++) {
+            const uint32_t w = lds32(src + packed_piece(g, t) * 16 + (blk * 2 + half) * 4);
+            const uint32_t lows = w & 0x0F0F0F0Fu, highs = (w >> 4) & 0x0F0F0F0Fu;
+            dq2(__byte_perm(lows, 0x64646464u, 0x4140), zp, dd, v[2 * t + 0], v[16 + 2 * t + 0]);
+            dq2(__byte_perm(lows, 0x64646464u, 0x4342), zp, dd, v[2 * t + 1], v[16 + 2 * t + 1]);
+            dq2(__byte_perm(highs, 0x64646464u, 0x4140), zp, dd, v[8 + 2 * t + 0], v[24 + 2 * t + 0]);
+            dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 32; i++) asm volatile("" : "+r"(v[i]));  // the conversion stays ahead of the wait below
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
+        raw.advance();
+        const uint32_t grp = (gblk + mine) / GROUP;
+        if (grp >= A_RING && ok) {
           // the group's A stages were last read by the MMAs of the group A_RING before it
-          const uint32_t sp = gblk / GROUP - A_RING;
+          const uint32_t sp = grp - A_RING;
           ok = mbar_wait(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
         }
-        if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t tile_src = smem_u32(s_raw) + raw.stage * RAW_BYTES + T * TILE_RAW;
-#pragma unroll
-        for (uint32_t hb = 0; hb < GROUP * 4 / DQ_WARPS; hb++) {
-          const uint32_t in_group = mine + DQ_WARPS / 4 * hb, sub = in_stage * GROUP + in_group;  // block of the group and of the weight stage
-          uint32_t v[32];  // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
-          if (DT == MER_DTYPE_Q8_0) {
-            const uint32_t src = tile_src + sub * 544;
-            const uint32_t sc2 = lds32(src + 512 + g * 4);
-            const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
-#pragma unroll
-            for (int t = 0; t < 4; t++) {  // values 8t .. 8t+7
-              const uint2 w = lds64(src + packed_piece(g, t) * 16 + half * 8);
-              const uint32_t w0 = w.x ^ 0x80808080u, w1 = w.y ^ 0x80808080u;
-              dq2(__byte_perm(w0, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
-              dq2(__byte_perm(w0, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
-              dq2(__byte_perm(w1, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
-              dq2(__byte_perm(w1, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
-            }
-          } else {
-            // block-pair record: 16 bytes per (g, t) = words (slot g, blk 0), (slot g+8, blk 0), (slot g, blk 1), (slot g+8, blk 1);
-            // byte i of a word holds values 4t+i (low nibble) and 16+4t+i (high nibble) of its block
-            const uint32_t src = tile_src + (sub >> 1) * 576, blk = sub & 1;
-            const uint32_t sc2 = lds32(src + 512 + g * 8 + blk * 4);
-            const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-              const uint32_t w = lds32(src + packed_piece(g, t) * 16 + (blk * 2 + half) * 4);
-              const uint32_t lows = w & 0x0F0F0F0Fu, highs = (w >> 4) & 0x0F0F0F0Fu;
-              dq2(__byte_perm(lows, 0x64646464u, 0x4140), zp, dd, v[2 * t + 0], v[16 + 2 * t + 0]);
-              dq2(__byte_perm(lows, 0x64646464u, 0x4342), zp, dd, v[2 * t + 1], v[16 + 2 * t + 1]);
-              dq2(__byte_perm(highs, 0x64646464u, 0x4140), zp, dd, v[8 + 2 * t + 0], v[24 + 2 * t + 0]);
-              dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
-            }
-          }
-          tc_st32(tmem_base + ((q * 32u) << 16) + TMEM_A0 + ((gblk + in_group) % A_STAGES) * A_STAGE_COLS, v);
-        }
+        tc_st32(tmem_base + ((q * 32u) << 16) + TMEM_A0 + ((gblk + mine) % A_STAGES) * A_STAGE_COLS, v);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          arrive_cluster(leader_addr(&a_full[(gblk / GROUP) % A_RING]));
-          if (in_stage == PER - 1) mbar_arrive(&raw_empty[raw.stage]);
-        }
-        if (in_stage == PER - 1) raw.advance();
+        if (lane == 0) arrive_cluster(leader_addr(&a_full[grp % A_RING]));
       }
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
@@ -460,14 +467,13 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // that the group's named barriers always see all four warps.
     bool dead = false;
     for (uint32_t item = item_beg; item < n_items; item += item_step) {
-      const uint32_t pass = item / m_pairs, mt = (item % m_pairs) * PAIR + rank;
-      const bool resident = expert_base(pass) != nullptr;
+      const uint32_t mt = (item % m_pairs) * PAIR + rank;
+      const bool resident = next_item(item, pstart, pcount) != nullptr;
       if (resident) {
         if ((n_item++ & 1) != buf) continue;  // the other group's item
       } else if (buf != 0) {
         continue;  // items of missing experts are zero-filled by group 0
       }
-      const uint32_t pstart = d.pass_start[pass], pcount = d.pass_count[pass];
       // The pass's pair indices and un-scale factors go to shared memory (one column per thread of the group), fetched
       // before the accumulator is waited for so that their latency hides behind the item's MMAs; the column loop then
       // reads them as broadcasts.
@@ -507,23 +513,29 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         // the steps run column-batched (all multiplies, then all shuffles, ...): warp-synchronous operations are kept in
         // program order, so a column-by-column loop would serialise on the latency of every single one
 #pragma unroll
-        for (int i = 0; i < EC; i++) val[i] *= s_un[cbase + i];
+        for (int i = 0; i < EC; i += 4) {
+          const float4 un = *reinterpret_cast<const float4 *>(s_un + cbase + i);
+          val[i] *= un.x, val[i + 1] *= un.y, val[i + 2] *= un.z, val[i + 3] *= un.w;
+        }
         if (p.phase == 0) {
-          // rows come in packed tiles of 16: slots 0..7 gate rows, 8..15 the matching up rows
-          float up[EC];
+          // rows come in packed tiles of 16: slots 0..7 gate rows, 8..15 the matching up rows.  The two lanes of a
+          // gate/up pair exchange halves: the gate lane finishes the first eight columns, the up lane the others.
+          float h[EC / 2];
 #pragma unroll
-          for (int i = 0; i < EC; i++) up[i] = __shfl_down_sync(0xffffffffu, val[i], 8);
+          for (int i = 0; i < EC / 2; i++) h[i] = __shfl_xor_sync(0xffffffffu, is_gate ? val[EC / 2 + i] : val[i], 8);
 #pragma unroll
-          for (int i = 0; i < EC; i++) {
-            float gate = val[i];
+          for (int i = 0; i < EC / 2; i++) {
+            float gate = is_gate ? val[i] : h[i];
+            const float up = is_gate ? h[i] : val[EC / 2 + i];
             if (clamp && gate == gate) gate = fminf(fmaxf(gate, -d.swiglu_limit), d.swiglu_limit);
-            val[i] = __fdividef(gate, 1.0f + __expf(-gate)) * up[i];
+            h[i] = __fdividef(gate, 1.0f + __expf(-gate)) * up;
           }
           // h in the order of the groups: its rows are then the rows of the down phase's passes
-          float *dst = p.out + (size_t)(pstart + cbase) * d.F + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
+          const uint32_t col = cbase + (is_gate ? 0 : EC / 2);
+          float *dst = p.out + (size_t)(pstart + col) * d.F + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
 #pragma unroll
-          for (int i = 0; i < EC; i++)
-            if (is_gate && cbase + i < pcount) dst[(size_t)i * d.F] = val[i];
+          for (int i = 0; i < EC / 2; i++)
+            if (col + i < pcount) dst[(size_t)i * d.F] = h[i];
         } else {
           const uint32_t off = mt * 128 + row;
 #pragma unroll
