@@ -166,6 +166,12 @@ __device__ __forceinline__ void dq2(uint32_t biased, __half2 zp1024, __half2 d2,
 
 // Token columns of a pass: its count rounded up to 16.
 __host__ __device__ constexpr uint32_t pass_width(uint32_t count) { return (count + 15u) & ~15u; }
+// A group of at most SPLIT_TOKENS tokens (always a single pass) leaves half of its accumulator buffer free: the two small
+// products go there and are added at the end, so that the large one is rounded by its own additions only.  The
+// rule looks at the group, not at the pass, so that the order of a token's additions depends only on how many tokens its
+// expert received, never on which pass it landed in: results stay bit-identical from run to run although large
+// dispatches are grouped with atomics.
+constexpr uint32_t SPLIT_TOKENS = PASS_TOKENS / 2;
 
 struct Ring {
   uint32_t stage = 0, round = 0, n;
@@ -239,22 +245,25 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
   // behind an expert's address would otherwise stall every role at the start of every item.
   struct Items {
     uint64_t base = 0;
-    uint32_t start = 0, count = 0;
+    uint32_t start = 0, count = 0, split = 0;
     __device__ void fetch(const MoeDispatch &d, uint32_t item, uint32_t n_items, uint32_t m_pairs) {
       if (item >= n_items) return;
-      const uint32_t pass = item / m_pairs, eid = d.group_expert[__ldg(d.pass_group + pass)];
+      const uint32_t pass = item / m_pairs, g = __ldg(d.pass_group + pass), eid = d.group_expert[g];
+      split = __ldg(d.offsets + g + 1) - __ldg(d.offsets + g) <= SPLIT_TOKENS;
       start = __ldg(d.pass_start + pass), count = __ldg(d.pass_count + pass);
       base = eid < d.max_experts ? reinterpret_cast<uint64_t>(d.expert_ptr[eid]) : 0;
     }
   } items;
   uint32_t item_no = 0;  // running number of the role's item
-  auto next_item = [&](uint32_t item, uint32_t &start, uint32_t &count) -> const uint8_t * {
+  auto next_item = [&](uint32_t item, uint32_t &start, uint32_t &count, bool *split = nullptr) -> const uint8_t * {
     const uint32_t k = item_no++ & 31;
     if (k == 0) items.fetch(d, item + lane * item_step, n_items, m_pairs);
     start = __shfl_sync(0xffffffffu, items.start, k), count = __shfl_sync(0xffffffffu, items.count, k);
+    if (split) *split = __shfl_sync(0xffffffffu, items.split, k) != 0;
     return reinterpret_cast<const uint8_t *>(__shfl_sync(0xffffffffu, items.base, k));
   };
   uint32_t pstart, pcount;
+  bool split;
   bool ok = true;
 
   if (warp == W_PRODUCER) {
@@ -307,7 +316,8 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // takes (descriptors, TMEM addresses) must sit in uniform registers: values derived from kernel parameters and
     // constants are computed there directly, values derived from a loaded pass count had to be moved over per
     // instruction (measured: +25 % issue time).
-    auto run_item = [&](auto width_tag) {
+    auto run_item = [&](auto width_tag, auto split_tag) {
+      constexpr uint32_t LO = decltype(split_tag)::value ? SPLIT_TOKENS : 0;  // columns of the small products
       constexpr uint32_t idesc = instr_desc(decltype(width_tag)::value);
       const uint32_t buf = n_done & 1, use = n_done >> 1;
       const uint32_t d_tmem = tmem_base + buf * 128;
@@ -328,8 +338,8 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
             const uint64_t dbh = b_blk + (uint64_t)(j * 2), dbl = dbh + (PART_BYTES >> 4);
             const uint32_t acc = (b4 == 0 && j == 0) ? (st != 0) : 1u;  // the item's first MMA overwrites the accumulator
             tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc, acc);
-            tc_mma_ts_acc(leader, d_tmem, a_hi + j * 8, dbl, idesc);
-            tc_mma_ts_acc(leader, d_tmem, a_lo + j * 8, dbh, idesc);
+            tc_mma_ts(leader, d_tmem + LO, a_hi + j * 8, dbl, idesc, LO ? acc : 1u);
+            tc_mma_ts_acc(leader, d_tmem + LO, a_lo + j * 8, dbh, idesc);
           }
         }
         rb.advance();
@@ -339,17 +349,29 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       n_done++;
     };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
-      if (!next_item(item, pstart, pcount)) continue;
+      if (!next_item(item, pstart, pcount, &split)) continue;
       // the MMA is as wide as the pass has tokens (rounded up to 16 columns)
-      switch (pass_width(pcount) >> 4) {
-        case 1: run_item(std::integral_constant<uint32_t, 16>{}); break;
-        case 2: run_item(std::integral_constant<uint32_t, 32>{}); break;
-        case 3: run_item(std::integral_constant<uint32_t, 48>{}); break;
-        case 4: run_item(std::integral_constant<uint32_t, 64>{}); break;
-        case 5: run_item(std::integral_constant<uint32_t, 80>{}); break;
-        case 6: run_item(std::integral_constant<uint32_t, 96>{}); break;
-        case 7: run_item(std::integral_constant<uint32_t, 112>{}); break;
-        default: run_item(std::integral_constant<uint32_t, 128>{}); break;
+      using T = std::true_type;
+      using F = std::false_type;
+      const uint32_t w16 = pass_width(pcount) >> 4;
+      if (split) {
+        switch (w16) {
+          case 1: run_item(std::integral_constant<uint32_t, 16>{}, T{}); break;
+          case 2: run_item(std::integral_constant<uint32_t, 32>{}, T{}); break;
+          case 3: run_item(std::integral_constant<uint32_t, 48>{}, T{}); break;
+          default: run_item(std::integral_constant<uint32_t, 64>{}, T{}); break;
+        }
+      } else {
+        switch (w16) {
+          case 1: run_item(std::integral_constant<uint32_t, 16>{}, F{}); break;
+          case 2: run_item(std::integral_constant<uint32_t, 32>{}, F{}); break;
+          case 3: run_item(std::integral_constant<uint32_t, 48>{}, F{}); break;
+          case 4: run_item(std::integral_constant<uint32_t, 64>{}, F{}); break;
+          case 5: run_item(std::integral_constant<uint32_t, 80>{}, F{}); break;
+          case 6: run_item(std::integral_constant<uint32_t, 96>{}, F{}); break;
+          case 7: run_item(std::integral_constant<uint32_t, 112>{}, F{}); break;
+          default: run_item(std::integral_constant<uint32_t, 128>{}, F{}); break;
+        }
       }
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
@@ -468,7 +490,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     bool dead = false;
     for (uint32_t item = item_beg; item < n_items; item += item_step) {
       const uint32_t mt = (item % m_pairs) * PAIR + rank;
-      const bool resident = next_item(item, pstart, pcount) != nullptr;
+      const bool resident = next_item(item, pstart, pcount, &split) != nullptr;
       if (resident) {
         if ((n_item++ & 1) != buf) continue;  // the other group's item
       } else if (buf != 0) {
@@ -506,6 +528,11 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
           tc_ld16(acc_addr + cbase, v);
 #pragma unroll
           for (int i = 0; i < EC; i++) val[i] = __uint_as_float(v[i]);
+          if (split) {
+            tc_ld16(acc_addr + SPLIT_TOKENS + cbase, v);
+#pragma unroll
+            for (int i = 0; i < EC; i++) val[i] += __uint_as_float(v[i]);
+          }
         } else {
 #pragma unroll
           for (int i = 0; i < EC; i++) val[i] = 0.0f;
