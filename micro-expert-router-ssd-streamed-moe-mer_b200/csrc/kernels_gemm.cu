@@ -714,6 +714,7 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) {
   stream_bind(d, stream_scratch, sm_count);  // pass tables live in the streaming scratch
   d.tokens_per_pass = bn;
+  d.item_bounds = nullptr;  // items are dealt round-robin
 }
 
 cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid) {

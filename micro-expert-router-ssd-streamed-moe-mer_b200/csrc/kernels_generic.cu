@@ -64,18 +64,68 @@ __device__ __forceinline__ float clamp_gate(float g, float limit) {
 }
 
 // ---------------------------------------------------------------------------------------
-// Router.  One CTA computes the logits of 8 experts for a tile of 4 tokens (every warp takes an
-// eighth of the columns of all 8 rows, so W is read once per token tile and each lane has many
+// Router.  One CTA computes the logits of 1 to 8 experts for a tile of 4 tokens (every warp takes an
+// eighth of the columns of all its rows, so W is read once per token tile and each lane has many
 // independent loads in flight).  The last CTA to finish a token tile scores, filters and picks
 // top-k for its tokens, one warp per token (LinearGate::route_with_scratch, gating.rs:395-476);
 // the last tile overall groups the (token, slot) pairs by expert.
 // ---------------------------------------------------------------------------------------
 constexpr int ROUTER_THREADS = 256;
-constexpr int ROUTER_ROWS = ROUTER_THREADS / 32;  // expert rows per CTA
+constexpr int ROUTER_WARPS = ROUTER_THREADS / 32;
 constexpr int ROUTER_TT = 4;                      // tokens per CTA
 constexpr uint32_t SMALL_P = 4096;                // pair keys staged in shared memory below this many pairs
 constexpr uint32_t STABLE_G = 512;
 constexpr uint32_t GRID_GROUPING_PAIRS = 8192;    // from this many pairs the grouping runs grid-wide (count / scan / scatter)                // stable (token, slot)-ordered grouping up to this many groups
+
+// ---- work split of the streaming kernels: one contiguous item range per CTA and phase.  An item of a pass with
+// more than four tokens multiplies two token tiles instead of one, which measures as ~1.3x the time: cost 13 vs 10.
+// `s_cum`: running cost before each pass and after the last, or null: all passes cost the same.  One CTA of 256 threads.
+__device__ void build_item_bounds(const MoeDispatch &d, uint32_t n_passes, const uint32_t *s_cum) {
+  const uint32_t G = d.n_ctas;
+#pragma unroll 1
+  for (uint32_t i = threadIdx.x; i < 2 * (G + 1); i += 256) {
+    const uint32_t phase = i / (G + 1), b = i % (G + 1);
+    const uint32_t ipp = d.items_per_pass[phase];
+    const uint64_t n_items = (uint64_t)n_passes * ipp;
+    uint32_t bound;
+    if (!s_cum) {
+      bound = n_items * G <= 0xFFFFFFFFull ? (uint32_t)n_items * b / G : (uint32_t)(n_items * b / G);
+    } else if ((uint64_t)s_cum[n_passes] * ipp * G <= 0xFFFFFFFFull) {
+      // the usual case: everything fits 32 bits (64-bit divisions cost a few hundred cycles each, and this loop sits
+      // on the critical path of every decode layer)
+      const uint32_t total = s_cum[n_passes] * ipp, target = total * b / G;
+      uint32_t lo = 0, hi = n_passes;  // largest pass index with cum[pass] * ipp <= target
+#pragma unroll 1
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
+      }
+      if (lo >= n_passes) {
+        bound = (uint32_t)n_items;
+      } else {
+        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
+        const uint32_t rem = target - s_cum[lo] * ipp;
+        bound = lo * ipp + min(ipp, (rem + w - 1) / w);
+      }
+    } else {
+      const uint64_t total = (uint64_t)s_cum[n_passes] * ipp, target = total * b / G;
+      uint32_t lo = 0, hi = n_passes;
+#pragma unroll 1
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if ((uint64_t)s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
+      }
+      if (lo >= n_passes) {
+        bound = (uint32_t)n_items;
+      } else {
+        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
+        const uint64_t rem = target - (uint64_t)s_cum[lo] * ipp;
+        bound = lo * ipp + (uint32_t)min((uint64_t)ipp, (rem + w - 1) / w);
+      }
+    }
+    d.item_bounds[phase * MER_MAX_CTAS1 + b] = bound;
+  }
+}
 
 // Cuts every group into passes of at most d.tokens_per_pass pairs (the unit the streaming FFN works
 // on) and clears the per-pair max cells.  One CTA of 256 threads; `off` = the group offsets.
@@ -132,10 +182,8 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
     d.n_passes[1] = d.n_passes[2] = 0;  // arrival counters of the streaming kernels' grid-wide barriers
   }
   if (!d.item_bounds) return;
-  // ---- work split of the streaming kernels: one contiguous item range per CTA and phase.  An item of a pass with
-  // more than four tokens multiplies two token tiles instead of one, which measures as ~1.3x the time: cost 13 vs 10.
   __shared__ uint32_t s_cum[1025];
-  const uint32_t n_passes = s_pcnt[256], G = d.n_ctas;
+  const uint32_t n_passes = s_pcnt[256];
   __syncthreads();  // s_cost[] written above is read back below
   const bool weighted = n_passes <= 1024 && tpp == 8;
   if (weighted) {
@@ -174,49 +222,7 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
     if (threadIdx.x == 255) s_cum[1024] = acc;
     __syncthreads();
   }
-#pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < 2 * (G + 1); i += 256) {
-    const uint32_t phase = i / (G + 1), b = i % (G + 1);
-    const uint32_t ipp = d.items_per_pass[phase];
-    const uint64_t n_items = (uint64_t)n_passes * ipp;
-    uint32_t bound;
-    if (!weighted) {
-      bound = (uint32_t)(n_items * b / G);
-    } else if ((uint64_t)s_cum[n_passes] * ipp * G <= 0xFFFFFFFFull) {
-      // the usual case: everything fits 32 bits (64-bit divisions cost a few hundred cycles each, and this loop sits
-      // on the critical path of every decode layer)
-      const uint32_t total = s_cum[n_passes] * ipp, target = total * b / G;
-      uint32_t lo = 0, hi = n_passes;  // largest pass index with cum[pass] * ipp <= target
-#pragma unroll 1
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
-      }
-      if (lo >= n_passes) {
-        bound = (uint32_t)n_items;
-      } else {
-        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
-        const uint32_t rem = target - s_cum[lo] * ipp;
-        bound = lo * ipp + min(ipp, (rem + w - 1) / w);
-      }
-    } else {
-      const uint64_t total = (uint64_t)s_cum[n_passes] * ipp, target = total * b / G;
-      uint32_t lo = 0, hi = n_passes;
-#pragma unroll 1
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if ((uint64_t)s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
-      }
-      if (lo >= n_passes) {
-        bound = (uint32_t)n_items;
-      } else {
-        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
-        const uint64_t rem = target - (uint64_t)s_cum[lo] * ipp;
-        bound = lo * ipp + (uint32_t)min((uint64_t)ipp, (rem + w - 1) / w);
-      }
-    }
-    d.item_bounds[phase * MER_MAX_CTAS1 + b] = bound;
-  }
+  build_item_bounds(d, n_passes, weighted ? s_cum : nullptr);
 }
 
 // Group of pair p: local expert index, the shared-expert group, or MER_NONE for an unfilled / foreign slot.
@@ -281,15 +287,64 @@ __global__ void k_group_clear(MoeDispatch d) {
   for (uint32_t g = threadIdx.x; g < d.n_groups; g += blockDim.x) d.group_cursor[g] = 0;
 }
 
+// The same for at most 32 pairs of the streaming kernels, in registers of one warp: sorted position of every pair, the pairs
+// that start a pass, their order.  The general form's dozen block-wide steps took 4 us on B200 for one token's eight pairs, as long
+// as the kernels that follow need for the weights of half of them.
+__device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
+  __shared__ uint32_t s_np, s_cum[33];
+  const uint32_t P = d.n_tokens * d.slots, tpp = d.tokens_per_pass;
+  const bool weighted = tpp == 8;
+  if (threadIdx.x < 32) {
+    const uint32_t p = threadIdx.x, before = (1u << p) - 1;
+    const uint32_t eid = p < P ? __ldcg(d.pair_expert + p) : MER_NONE;
+    uint32_t key = eid;  // group index; unfilled slots sort last
+    if (eid != MER_NONE) key = p % d.slots >= r.top_k || eid == r.shared_expert_id ? r.num_experts : eid - r.id_base;
+    const uint32_t same = __match_any_sync(0xffffffffu, key), rank = __popc(same & before);
+    uint32_t pos = rank;
+#pragma unroll 4
+    for (uint32_t j = 0; j < P; j++) pos += __shfl_sync(0xffffffffu, key, j) < key;
+    const bool valid = key != MER_NONE, starts = valid && rank % tpp == 0;
+    const uint32_t starters = __reduce_or_sync(0xffffffffu, starts ? 1u << pos : 0u);
+    const uint32_t np = __popc(starters), n_valid = __popc(__ballot_sync(0xffffffffu, valid));
+    if (valid) {
+      d.perm[pos] = p;
+      if (rank == 0) d.group_expert[key] = eid;
+    }
+    const uint32_t count = min(tpp, __popc(same) - rank), pass = __popc(starters & ((1u << pos) - 1));
+    if (starts) d.pass_group[pass] = key, d.pass_start[pass] = pos, d.pass_count[pass] = count;
+    if (p < P) d.amax[p] = 0;
+    if (p == 0) {
+      d.offsets[d.n_groups] = n_valid;  // all of the offsets that anyone reads after the streaming kernels
+      d.n_passes[0] = s_np = np;
+      d.n_passes[1] = d.n_passes[2] = 0;
+    }
+    if (weighted) {
+      if (starts) s_cum[pass + 1] = count > 4 ? 13 : 10;
+      __syncwarp();
+      uint32_t incl = p < np ? s_cum[p + 1] : 0;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (p >= (uint32_t)o) incl += up;
+      }
+      s_cum[p + 1] = incl;
+      if (p == 0) s_cum[0] = 0;
+    }
+  }
+  __syncthreads();
+  build_item_bounds(d, s_np, weighted ? s_cum : nullptr);
+}
+
 // Runs in one CTA after every token has been routed: groups pairs by expert.
 __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uint32_t *s_u32) {
   const uint32_t P = d.n_tokens * d.slots;
+  if (P <= 32 && d.item_bounds) return build_groups_small(r, d);
   const uint32_t G = d.n_groups;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *s_off = s_u32;                    // [G + 1]
   uint32_t *s_cnt = s_u32 + G + 1;            // [8 warps][G] (stable path) or [G]
   const bool stable = G <= STABLE_G;
-  uint32_t *s_key = s_cnt + (stable ? ROUTER_ROWS * G : G);  // [min(P, SMALL_P)]
+  uint32_t *s_key = s_cnt + (stable ? ROUTER_WARPS * G : G);  // [min(P, SMALL_P)]
   const bool staged = P <= SMALL_P;
   auto key_global = [&](uint32_t p) -> uint32_t {
     uint32_t e = __ldcg(d.pair_expert + p);
@@ -301,14 +356,14 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
 #pragma unroll 1
   for (uint32_t g = tid; g < G; g += nt) d.group_expert[g] = (g < r.num_experts) ? r.id_base + g : r.shared_expert_id;
 #pragma unroll 1
-  for (uint32_t i = tid; i < (stable ? ROUTER_ROWS * G : G); i += nt) s_cnt[i] = 0;
+  for (uint32_t i = tid; i < (stable ? ROUTER_WARPS * G : G); i += nt) s_cnt[i] = 0;
   if (staged)
 #pragma unroll 1
     for (uint32_t p = tid; p < P; p += nt) s_key[p] = key_global(p);
   __syncthreads();
   if (stable) {
     // every warp owns a contiguous run of pairs, so (warp, position in run) order = (token, slot) order
-    const uint32_t chunk = ((P + ROUTER_ROWS - 1) / ROUTER_ROWS + 31) / 32 * 32;
+    const uint32_t chunk = ((P + ROUTER_WARPS - 1) / ROUTER_WARPS + 31) / 32 * 32;
     const uint32_t p0 = warp * chunk, p1 = min(P, p0 + chunk);
 #pragma unroll 1
     for (uint32_t p = p0 + lane; p < p1; p += 32) {
@@ -320,7 +375,7 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
     for (uint32_t g = tid; g < G; g += nt) {  // per group: exclusive scan over the warps, total into s_off
       uint32_t run = 0;
 #pragma unroll 1
-      for (uint32_t w = 0; w < ROUTER_ROWS; w++) {
+      for (uint32_t w = 0; w < ROUTER_WARPS; w++) {
         uint32_t c = s_cnt[w * G + g];
         s_cnt[w * G + g] = run;
         run += c;
@@ -493,41 +548,42 @@ __global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r,
   }
 }
 
+template <int ROWS>
 __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int pre, int group_here) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t E = r.num_experts, D = d.D;
   const uint32_t tile = blockIdx.y, t0 = tile * ROUTER_TT;
   const uint32_t n_here = min((uint32_t)ROUTER_TT, d.n_tokens - t0);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t e0 = blockIdx.x * ROUTER_ROWS;
-  __shared__ float s_part[ROUTER_ROWS][ROUTER_TT][ROUTER_ROWS + 1];  // [row][token][warp]
-  __shared__ float s_logit[ROUTER_TT][ROUTER_ROWS];                  // used when one CTA covers all experts
+  const uint32_t e0 = blockIdx.x * ROWS;
+  __shared__ float s_part[ROWS][ROUTER_TT][ROUTER_WARPS + 1];  // [row][token][warp]
+  __shared__ float s_logit[ROUTER_TT][ROWS];                  // used when one CTA covers all experts
   const bool single = gridDim.x == 1 && !pre;
 
   if (pre) {
     // logits are already in d.logits (k_router_logits_tiled)
   } else if ((D & 1023u) == 0) {
-    const uint32_t slice4 = D / 4 / ROUTER_ROWS;  // float4 per warp slice
-    float acc[ROUTER_ROWS][ROUTER_TT];
+    const uint32_t slice4 = D / 4 / ROUTER_WARPS;  // float4 per warp slice
+    float acc[ROWS][ROUTER_TT];
 #pragma unroll
-    for (int rr = 0; rr < ROUTER_ROWS; rr++)
+    for (int rr = 0; rr < ROWS; rr++)
 #pragma unroll
       for (int tt = 0; tt < ROUTER_TT; tt++) acc[rr][tt] = 0.0f;
-#pragma unroll 2
+#pragma unroll (ROWS >= 8 ? 2 : 4)
     for (uint32_t i = lane; i < slice4; i += 32) {
-      float4 b[ROUTER_TT], a[ROUTER_ROWS];
+      float4 b[ROUTER_TT], a[ROWS];
 #pragma unroll
       for (int tt = 0; tt < ROUTER_TT; tt++) {
         b[tt] = make_float4(0, 0, 0, 0);
         if ((uint32_t)tt < n_here) b[tt] = __ldg(reinterpret_cast<const float4 *>(d.x + (size_t)(t0 + tt) * D) + warp * slice4 + i);
       }
 #pragma unroll
-      for (int rr = 0; rr < ROUTER_ROWS; rr++) {
+      for (int rr = 0; rr < ROWS; rr++) {
         const uint32_t row = min(e0 + rr, E - 1);
         a[rr] = __ldg(reinterpret_cast<const float4 *>(r.w + (size_t)row * D) + warp * slice4 + i);
       }
 #pragma unroll
-      for (int rr = 0; rr < ROUTER_ROWS; rr++)
+      for (int rr = 0; rr < ROWS; rr++)
 #pragma unroll
         for (int tt = 0; tt < ROUTER_TT; tt++) {
           acc[rr][tt] = fmaf(a[rr].x, b[tt].x, acc[rr][tt]);
@@ -537,18 +593,19 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
         }
     }
 #pragma unroll
-    for (int rr = 0; rr < ROUTER_ROWS; rr++)
+    for (int rr = 0; rr < ROWS; rr++)
 #pragma unroll
       for (int tt = 0; tt < ROUTER_TT; tt++) {
+        if ((uint32_t)tt >= n_here) continue;
         float v = warp_sum(acc[rr][tt]);
         if (lane == 0) s_part[rr][tt][warp] = v;
       }
     __syncthreads();
-    if (threadIdx.x < ROUTER_ROWS * ROUTER_TT) {
+    if (threadIdx.x < ROWS * ROUTER_TT) {
       const uint32_t rr = threadIdx.x / ROUTER_TT, tt = threadIdx.x % ROUTER_TT;
       float v = 0.0f;
 #pragma unroll
-      for (int w = 0; w < ROUTER_ROWS; w++) v += s_part[rr][tt][w];
+      for (int w = 0; w < ROUTER_WARPS; w++) v += s_part[rr][tt][w];
       if (single)
         s_logit[tt][rr] = v;
       else if (e0 + rr < E && tt < n_here)
@@ -556,7 +613,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     }
   } else {
     // any d_model: warp = expert row, tokens one after the other
-    const uint32_t e = e0 + warp;
+    const uint32_t e = warp < ROWS ? e0 + warp : E;
     for (uint32_t tt = 0; tt < n_here; tt++) {
       float acc = 0.0f;
       if (e < E) {
@@ -961,13 +1018,9 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   const uint32_t E = r.num_experts, G = d.n_groups;
   const uint32_t P = d.n_tokens * d.slots;
   size_t smem_topk = (size_t)ROUTER_TT * E * 9;
-  size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_ROWS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
+  size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   size_t smem = smem_topk > smem_grp ? smem_topk : smem_grp;
   smem = (smem + 15) & ~(size_t)15;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_router, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
   const bool tiled = d.n_tokens >= 256 && (d.D % RL_KC) == 0;  // from a few hundred tokens: logits as a tiled GEMM first
   uint32_t ksplit = 1;
   if (tiled) {
@@ -983,9 +1036,19 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     k_router_logits_tiled<<<lgrid, RL_THREADS, RL_SMEM, s>>>(r, d, ksplit);
     if (launches) (*launches)++;
   }
-  dim3 grid(tiled ? 1 : (E + ROUTER_ROWS - 1) / ROUTER_ROWS, (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT);
+  // Expert rows per CTA: eight share the loads of x best, but a small call wants its few rows on as many SMs as there are
+  // (one token, 128 experts of 2048: 13.4 us with a row per CTA, 16.6 us with eight).
+  const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
+  uint32_t rows = 8;
+  while (!tiled && rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < 120) rows >>= 1;
+  const dim3 grid(tiled ? 1 : (E + rows - 1) / rows, tiles);
   const bool grid_grouping = group && P >= GRID_GROUPING_PAIRS && d.group_count != nullptr;
-  k_router<<<grid, ROUTER_THREADS, smem, s>>>(r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0);
+  auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  kern<<<grid, ROUTER_THREADS, smem, s>>>(r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0);
   if (launches) (*launches)++;
   if (grid_grouping) {  // the router has counted the pairs per group
     const unsigned blocks = (P + 1023) / 1024;
@@ -1010,7 +1073,7 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
     if (launches) (*launches) += counted ? 3 : 4;
     return cudaGetLastError();
   }
-  size_t smem = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_ROWS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
+  size_t smem = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   smem = (smem + 15) & ~(size_t)15;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(k_groups_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -46,8 +46,9 @@ __device__ Pick route_token_reg(const RouterDev &r, float *s_score, float *s_sel
 #pragma unroll
     for (int j = 0; j < EJ; j++)
       if (lane + 32 * j < E) mx = fmaxf(mx, sc[j]), nan |= sc[j] != sc[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    // the maximum of the total-order keys is the maximum of the values (-0 sorts below 0 and exponentiates alike)
+    const int mk = __reduce_max_sync(0xffffffffu, total_key(mx));
+    mx = __int_as_float(mk ^ (int)(((unsigned)(mk >> 31)) >> 1));
     nan = __any_sync(0xffffffffu, nan);
     if (nan || !isfinite(mx)) {
 #pragma unroll
@@ -141,21 +142,31 @@ __device__ Pick route_token_reg(const RouterDev &r, float *s_score, float *s_sel
       if (keys[j] > bk) bk = keys[j], bj = j;  // ascending j keeps the lowest id on ties
     const int top_key = __reduce_max_sync(0xffffffffu, bk);
     if (top_key == INT_MIN) break;  // nothing left to pick
-    const uint32_t top_id = __reduce_min_sync(0xffffffffu, bk == top_key ? lane + 32 * bj : MER_NONE);
-    if (lane == (top_id & 31u)) {
+    const uint32_t tied = __ballot_sync(0xffffffffu, bk == top_key);
+    uint32_t top_lane = __ffs(tied) - 1;
+    if (tied & (tied - 1))  // equal keys in several lanes: the lowest id wins
+      top_lane = __reduce_min_sync(0xffffffffu, bk == top_key ? lane + 32 * bj : MER_NONE) & 31u;
+    const uint32_t top_j = __shfl_sync(0xffffffffu, bj, top_lane);
+    if (lane == top_lane) {
 #pragma unroll
       for (int j = 0; j < EJ; j++)
-        if ((uint32_t)j == (top_id >> 5)) keys[j] = INT_MIN;
+        if ((uint32_t)j == bj) keys[j] = INT_MIN;
     }
-    if (lane == (n & 31)) my_id = top_id;
+    if (lane == (n & 31)) my_id = top_lane + 32 * top_j;
     n_sel++;
   }
   // mixing weights = unbiased scores; renormalise; scale (gating.rs:443-474)
   float w = (lane < n_sel && my_id != MER_NONE) ? s_score[my_id] : 0.0f;
   if (r.normalise) {
     float sum = 0.0f;
-#pragma unroll 1
-    for (uint32_t i = 0; i < n_sel; i++) sum += __shfl_sync(0xffffffffu, w, i);  // slot order
+    for (uint32_t i0 = 0; i0 < n_sel; i0 += 8) {  // slot order; the shuffles of eight slots are in flight together
+      float v[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) v[i] = __shfl_sync(0xffffffffu, w, (i0 + i) & 31);
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+        if (i0 + i < n_sel) sum += v[i];
+    }
     if (isfinite(sum) && sum > 0.0f) w = w / sum;
   }
   if (r.scaling != 1.0f && isfinite(r.scaling)) w = w * r.scaling;
