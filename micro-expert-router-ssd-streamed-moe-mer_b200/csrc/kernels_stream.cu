@@ -9,7 +9,7 @@
 //     4-bit or 8-bit field masked into the low mantissa bits of an f16 IS the subnormal value
 //     q * 2^-24 (q * 2^-20 for a field at bits 4..7), so unpacking is one LOP3 per two weights and
 //     the integers are exact.  The zero point (8 for Q4_0, 128 for the sign-flipped Q8_0 byte) is
-//     folded in as the accumulator's initial value -zp * sum(x_block).
+//     added four blocks at a time as the product of the blocks' scales and -zp * sum(x_block).
 //   * Activations are pre-split into f16 hi + lo parts (22+ significant bits) after an exact
 //     power-of-two per-token scaling; hi and lo are two columns of the n=8 MMA tile, so one tile
 //     carries 4 tokens.  Products are exact, accumulation is fp32 in the tensor core.
@@ -42,6 +42,7 @@ namespace {
 constexpr int CONSUMER_WARPS = 16;
 constexpr int PRODUCER_WARPS = 2;  // each issues the bulk copies of half a stage's tiles: one warp alone was busy ~90 % of the time
 constexpr int THREADS = (CONSUMER_WARPS + PRODUCER_WARPS) * 32;
+constexpr int BATCH = 4;  // activation loads a lane has in flight while fragments are built
 constexpr uint32_t HEADER_BYTES = 1024;  // mbarriers and per-pass token tables at the start of shared memory
 
 constexpr int TAIL_NONE = 0, TAIL_FINALIZE = 1, TAIL_COMBINE = 2, TAIL_REDUCE = 3;
@@ -68,6 +69,10 @@ struct StreamParams {
                              // TAIL_REDUCE (phase 1, K split): y[pair] = sum of its partials, grouped pairs only
   uint32_t *grid_counter;    // arrival counter of that barrier, zeroed by the grouping kernel
 };
+
+// Words between two columns of zero-point terms: 4 mod 8, so that the eight columns and four blocks a warp reads together lie in
+// different banks.
+__host__ __device__ constexpr uint32_t seed_words(uint32_t kb_split) { return ((kb_split + 7) & ~7u) + 4; }
 
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(CONSUMER_WARPS * 32) : "memory"); }
 
@@ -98,7 +103,7 @@ struct BlockBytes {
 };
 
 // --------------------------------------------------------------------------- main kernel
-// RAGGED: the last group of 16 tiles is not full, or K is no multiple of four blocks (the checks cost the even shapes 1 to 3 %).
+// RAGGED: the last group of 16 tiles is not full, or K or a stage is no multiple of four blocks (the checks cost the even shapes 1 to 3 %).
 template <int DT, int NT, bool RAGGED>
 __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   extern __shared__ __align__(128) uint8_t smem[];
@@ -114,12 +119,10 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 160);  // [TP] pair index of each token of the current pass
   float *s_un = reinterpret_cast<float *>(smem + 192);          // [TP] its 2^24 / scale
   uint32_t *s_amax = reinterpret_cast<uint32_t *>(smem + 224);  // [TP] max |activation| of its row, as float bits
-  // per-block accumulator seeds, [TP][about kb_split + 2]: the four token rows a warp reads together (one per t) must not start
-  // in the same bank (a stride of 32 blocks put every 64-bit read four-deep on one bank pair: 25 % more shared-memory
-  // wavefronts in the whole gate/up phase)
-  const uint32_t seed_stride = (p.kb_split + 3) & ~1u;  // even: seeds are read two at a time
+  // the zero point's share of every block, [2 TP columns: token, hi / lo][seed_stride]
+  const uint32_t seed_stride = seed_words(p.kb_split);
   float *s_init = reinterpret_cast<float *>(smem + HEADER_BYTES);
-  uint8_t *s_frag = reinterpret_cast<uint8_t *>(s_init + seed_stride * TP);  // [TP*2][frag_stride]
+  uint8_t *s_frag = reinterpret_cast<uint8_t *>(s_init + seed_stride * 2 * TP);  // [TP*2][frag_stride]
   s_frag = reinterpret_cast<uint8_t *>(((size_t)s_frag + 127) & ~(size_t)127);
   uint8_t *s_stage = s_frag + (size_t)p.frag_cols * p.frag_stride;          // [n_stages][16 tiles][chunk_stride]
   const uint32_t stage_bytes = CONSUMER_WARPS * p.chunk_stride;
@@ -203,7 +206,9 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   const uint32_t g = lane >> 2, t = lane & 3;
   const uint32_t piece16 = packed_piece(g, t) * 16;  // byte offset of this lane's 16-byte piece inside a block record
   const uint32_t stage0 = smem_u32(s_stage) + warp * p.chunk_stride;  // this warp's tile chunk in stage 0
-  const uint32_t frag0 = smem_u32(s_frag) + t * 16, init0 = smem_u32(s_init);
+  const uint32_t frag0 = smem_u32(s_frag) + t * 16, init0 = smem_u32(s_init) + t * 4;
+  // scales {row slot g, slot g+8} of block t of four, from the record of the first
+  const uint32_t scale4 = DT == MER_DTYPE_Q4_0 ? (t >> 1) * 576 + 512 + g * 8 + (t & 1) * 4 : t * 544 + 512 + g * 4;
   uint32_t stage = 0, round = 0;
   uint32_t cur_pp = MER_NONE, cur_ks = MER_NONE;
   // A warp whose bounded wait expired goes "dead": it stops computing and waiting but still walks
@@ -232,7 +237,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       cur_pp = pp, cur_ks = ks;
       // The pass's activation rows become MMA B fragments here, in shared memory: an exact power-of-two
       // scaling that puts max |a| of the row in [256, 512), an f16 hi/lo split in fragment order, and the
-      // per-block accumulator seed -zp * 2^-24 * sum(block).  Warps share the rows: 16 / pcount per row; every
+      // per-block zero-point term -zp * 2^-24 * sum(block).  Warps share the rows: 16 / pcount per row; every
       // warp looks up its own row, so the only barriers are the one above, one for the row maxima (gate/up
       // phase) and the final one.
       const uint32_t K = p.kb_total * 32;
@@ -251,10 +256,16 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         float mx = 0.0f;
         if (has_row) {
           const float4 *r4 = reinterpret_cast<const float4 *>(row);
+          const uint32_t step = wpt * 32;
 #pragma unroll 1
-          for (uint32_t i = my_sub * 32 + lane; i < K / 4; i += wpt * 32) {
-            const float4 v = __ldg(r4 + i);
-            mx = nan_max(nan_max(nan_max(nan_max(mx, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
+          for (uint32_t i0 = my_sub * 32 + lane; i0 < K / 4; i0 += BATCH * step) {
+            float4 v[BATCH];
+#pragma unroll
+            for (int u = 0; u < BATCH; u++)
+              v[u] = i0 + u * step < K / 4 ? __ldg(r4 + i0 + u * step) : make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (int u = 0; u < BATCH; u++)
+              mx = nan_max(nan_max(nan_max(nan_max(mx, fabsf(v[u].x)), fabsf(v[u].y)), fabsf(v[u].z)), fabsf(v[u].w));
           }
         }
 #pragma unroll
@@ -278,33 +289,41 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         const float sc = row_scale;
         const float zp = DT == MER_DTYPE_Q4_0 ? 8.0f : 128.0f;
         uint8_t *hi_dst = s_frag + (size_t)(2 * my_tok) * p.frag_stride, *lo_dst = hi_dst + p.frag_stride;
-        float *seed_dst = s_init + (size_t)my_tok * seed_stride;
-        // float4 groups of this K split: 8 per block; a warp converts 4 blocks per step
+        float *seed_dst = s_init + (size_t)(2 * my_tok) * seed_stride;
+        const uint32_t n4 = kbn * 8, limit = RAGGED ? (kbn + 3) / 4 * 32 : n4, step = wpt * 32;  // whole warps, the shuffles below need them
+        const float4 *src = reinterpret_cast<const float4 *>(row + (size_t)kb0 * 32);
+        // a warp's loads of BATCH steps are in flight together (one at a time, eight rows of 3584 values took 19 us)
 #pragma unroll 1
-        for (uint32_t q = my_sub * 32 + lane; q < (RAGGED ? (kbn + 3) & ~3u : kbn) * 8; q += wpt * 32) {  // whole warps, the shuffles below need them
-          const bool inside = !RAGGED || q < kbn * 8;
-          float4 v = inside ? __ldg(reinterpret_cast<const float4 *>(row + (size_t)kb0 * 32) + q) : make_float4(0, 0, 0, 0);
-          v.x *= sc, v.y *= sc, v.z *= sc, v.w *= sc;  // exact (power of two) unless it overflows
-          const uint32_t kbl = q >> 3, j0 = (q & 7u) * 4;
-          uint32_t pos;
-          float ss;
-          frag_slot<DT>(j0, pos, ss);  // the four elements land at pos + {0, 2, 1, 3}
-          const float vs[4] = {v.x * ss, v.z * ss, v.y * ss, v.w * ss};
-          uint32_t hi[4], lo[4];
+        for (uint32_t q0 = my_sub * 32 + lane; q0 < limit; q0 += BATCH * step) {
+          float4 in[BATCH];
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const __half h = __float2half_rn(vs[i]);
-            hi[i] = __half_as_ushort(h);
-            lo[i] = __half_as_ushort(__float2half_rn(vs[i] - __half2float(h)));
-          }
-          if (inside) {
-            *reinterpret_cast<uint2 *>(hi_dst + kbl * 64 + pos * 2) = make_uint2(hi[0] | hi[1] << 16, hi[2] | hi[3] << 16);
-            *reinterpret_cast<uint2 *>(lo_dst + kbl * 64 + pos * 2) = make_uint2(lo[0] | lo[1] << 16, lo[2] | lo[3] << 16);
-          }
-          float sum = (v.x + v.y) + (v.z + v.w);  // eight consecutive lanes hold one block
+          for (int u = 0; u < BATCH; u++) in[u] = q0 + u * step < n4 ? __ldg(src + q0 + u * step) : make_float4(0, 0, 0, 0);
 #pragma unroll
-          for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-          if (inside && (lane & 7) == 0) seed_dst[kbl] = -zp * sum * (1.0f / POW2_24);
+          for (int u = 0; u < BATCH; u++) {
+            const uint32_t q = q0 + u * step;
+            if (q >= limit) break;  // uniform
+            const bool inside = !RAGGED || q < n4;
+            float4 v = in[u];
+            v.x *= sc, v.y *= sc, v.z *= sc, v.w *= sc;  // exact (power of two) unless it overflows
+            const uint32_t kbl = q >> 3, j0 = (q & 7u) * 4;
+            uint32_t pos;
+            float ss;
+            frag_slot<DT>(j0, pos, ss);  // the four elements land at pos + {0, 2, 1, 3}
+            const __half2 h0 = __floats2half2_rn(v.x * ss, v.z * ss), h1 = __floats2half2_rn(v.y * ss, v.w * ss);
+            const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+            const __half2 l0 = __floats2half2_rn(v.x * ss - f0.x, v.z * ss - f0.y), l1 = __floats2half2_rn(v.y * ss - f1.x, v.w * ss - f1.y);
+            if (inside) {
+              *reinterpret_cast<uint2 *>(hi_dst + kbl * 64 + pos * 2) = make_uint2(h2_bits(h0), h2_bits(h1));
+              *reinterpret_cast<uint2 *>(lo_dst + kbl * 64 + pos * 2) = make_uint2(h2_bits(l0), h2_bits(l1));
+            }
+            float sum = (v.x + v.y) + (v.z + v.w);  // eight consecutive lanes hold one block
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+            if (inside && (lane & 7) == 0) {
+              const float seed = -zp * sum * (1.0f / POW2_24), hi = tf32_round(seed);
+              seed_dst[kbl] = hi, seed_dst[seed_stride + kbl] = tf32_round(seed - hi);
+            }
+          }
         }
       }
       consumer_sync();  // fragments, seeds, s_pair, s_un visible to every warp
@@ -335,12 +354,27 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
 #pragma unroll
     for (int n = 0; n < NT; n++) {
       fa[n] = frag0 + (n * 8 + g) * p.frag_stride;  // column g of N-tile n = (token n*4 + g/2, part g&1)
-      ia[n] = init0 + (n * 4 + t) * seed_stride * 4;
+      ia[n] = init0 + (n * 8 + g) * seed_stride * 4;
     }
     float acc[NT][4];
 #pragma unroll
     for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
     const uint32_t n_live = (pcount + 3) >> 2;  // N-tiles that hold tokens
+
+    // The zero point's share of `left` (at most 4) blocks: acc += scales[16 rows x 4 blocks] * terms[4 blocks x 8 columns] in
+    // one MMA (a scale's 11 bits are exact in tf32, a term is two columns, hi and lo).  As the initial value of every
+    // block's own MMA it cost four register moves a block, a sixth of the loop's instructions.
+    auto do_zero = [&](uint32_t rec, uint32_t kb, uint32_t left, bool single_last) {
+      uint32_t sa = rec + scale4;
+      if (RAGGED && DT == MER_DTYPE_Q4_0 && single_last && t + 1 == left) sa = rec + (t >> 1) * 576 + 256 + g * 4;  // odd K: half a pair record
+      const bool in = !RAGGED || t < left;
+      const float2 sc = h2_to_f2(in ? lds32(sa) : 0u);
+#pragma unroll
+      for (int n = 0; n < NT; n++) {
+        if (n > 0 && (uint32_t)n >= n_live) break;  // uniform
+        mma_tf32(acc[n], __float_as_uint(sc.x), __float_as_uint(sc.y), in ? lds32(ia[n] + kb * 4) : 0u);
+      }
+    };
 
     // two adjacent blocks (kb, kb + 1; kb even) of both row slots against every live N-tile.
     // rec = shared address of the pair's first record in this warp's tile chunk.
@@ -362,11 +396,9 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       for (int n = 0; n < NT; n++) {
         if (n > 0 && (uint32_t)n >= n_live) break;  // uniform
         const uint4 bf0 = lds128(fa[n] + kb * 64), bf1 = lds128(fa[n] + kb * 64 + 64);
-        const uint2 sd = lds64(ia[n] + kb * 4);
-        const float seed0 = __uint_as_float(sd.x), seed1 = __uint_as_float(sd.y);
         float c1[4], c2[4], e1[4], e2[4];
-        mma_f16(c1, a0[0], a0h[0], a0[1], a0h[1], bf0.x, bf0.y, seed0, 0.0f, seed0, 0.0f);
-        mma_f16(e1, a1[0], a1h[0], a1[1], a1h[1], bf1.x, bf1.y, seed1, 0.0f, seed1, 0.0f);
+        mma_f16(c1, a0[0], a0h[0], a0[1], a0h[1], bf0.x, bf0.y, 0.0f, 0.0f, 0.0f, 0.0f);
+        mma_f16(e1, a1[0], a1h[0], a1[1], a1h[1], bf1.x, bf1.y, 0.0f, 0.0f, 0.0f, 0.0f);
         mma_f16(c2, a0[2], a0h[2], a0[3], a0h[3], bf0.z, bf0.w, c1[0], c1[1], c1[2], c1[3]);
         mma_f16(e2, a1[2], a1h[2], a1[3], a1h[3], bf1.z, bf1.w, e1[0], e1[1], e1[2], e1[3]);
         acc[n][0] = fmaf(d0.x, c2[0], acc[n][0]);
@@ -397,9 +429,8 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       for (int n = 0; n < NT; n++) {
         if (n > 0 && (uint32_t)n >= n_live) break;  // uniform
         const uint4 bf = lds128(fa[n] + kb * 64);
-        const float seed = __uint_as_float(lds32(ia[n] + kb * 4));
         float c1[4], c2[4];
-        mma_f16(c1, a[0], ah[0], a[1], ah[1], bf.x, bf.y, seed, 0.0f, seed, 0.0f);
+        mma_f16(c1, a[0], ah[0], a[1], ah[1], bf.x, bf.y, 0.0f, 0.0f, 0.0f, 0.0f);
         mma_f16(c2, a[2], ah[2], a[3], ah[3], bf.z, bf.w, c1[0], c1[1], c1[2], c1[3]);
         acc[n][0] = fmaf(ds.x, c2[0], acc[n][0]);
         acc[n][1] = fmaf(ds.x, c2[1], acc[n][1]);
@@ -415,16 +446,23 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       dead = __any_sync(0xffffffffu, dead);
       if (!dead && my_tile_exists) {
         constexpr uint32_t PAIR_BYTES = 2 * 16 * BB;  // 576 (Q4_0) / 1088 (Q8_0)
-        const uint32_t np = nb >> 1;                  // block pairs in this chunk
         uint32_t rec = stage0 + stage * stage_bytes;
-        uint32_t kb = c0;
-        // two pairs per iteration keep independent MMA chains in flight
+        // four blocks per iteration keep independent MMA chains in flight
 #pragma unroll 1
-        for (uint32_t pr = 0; pr < np; pr += 2, rec += 2 * PAIR_BYTES, kb += 4) {
-          do_pair(rec, kb);
-          if (pr + 1 < np) do_pair(rec + PAIR_BYTES, kb + 2);
+        for (uint32_t b = 0; b < nb; b += 4, rec += 2 * PAIR_BYTES) {
+          const uint32_t left = nb - b;
+          do_zero(rec, c0 + b, left < 4 ? left : 4, left < 4 && (left & 1));
+          if (RAGGED && left == 1) {
+            do_last(rec, c0 + b);
+            continue;
+          }
+          do_pair(rec, c0 + b);
+          if (RAGGED && left < 4) {
+            if (left == 3) do_last(rec + PAIR_BYTES, c0 + b + 2);
+            continue;
+          }
+          do_pair(rec + PAIR_BYTES, c0 + b + 2);
         }
-        if (RAGGED && (nb & 1)) do_last(stage0 + stage * stage_bytes + np * PAIR_BYTES, c0 + nb - 1);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[stage]);
@@ -685,7 +723,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   for (;;) {
     const uint32_t frag_cols = 2 * (max_group_tokens < tp ? max_group_tokens : tp);
     const uint32_t frag_stride = kb_split * 64 + 64;
-    const size_t fixed = HEADER_BYTES + (size_t)(kb_split + 3) * tp * 4 + 128 + (size_t)frag_cols * frag_stride;
+    const size_t fixed = HEADER_BYTES + (size_t)seed_words(kb_split) * 2 * tp * 4 + 128 + (size_t)frag_cols * frag_stride;
     if (fixed < SMEM_LIMIT) {
       const size_t avail = SMEM_LIMIT - fixed;
       for (uint32_t ppw = 4; ppw >= 1; ppw >>= 1) {
@@ -745,7 +783,7 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
 
 template <int DT>
 cudaError_t launch_phase(const StreamParams &p, uint32_t nt, size_t smem, int grid, cudaStream_t s) {
-  const bool ragged = p.packed_tiles % CONSUMER_WARPS != 0 || p.kb_total % 4 != 0;
+  const bool ragged = p.packed_tiles % CONSUMER_WARPS != 0 || p.kb_total % 4 != 0 || p.kc % 4 != 0;
   void (*kern)(StreamParams) = ragged ? (nt == 2 ? k_ffn_stream<DT, 2, true> : k_ffn_stream<DT, 1, true>)
                                       : (nt == 2 ? k_ffn_stream<DT, 2, false> : k_ffn_stream<DT, 1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
