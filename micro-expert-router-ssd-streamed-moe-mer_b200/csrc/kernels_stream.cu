@@ -687,6 +687,12 @@ constexpr uint32_t MAX_KSPLIT = 64;
 //    `max_ksplit` (what the partial-sum scratch can hold);
 //  * a stage holds 4 block pairs per warp if at least three stages then fit, else 2, else 1;
 //  * fragment arrays are sized by the most tokens any group can hold in this dispatch.
+// Shared memory of a plan without its ring.
+size_t fixed_smem(uint32_t kb_split, uint32_t nt, uint32_t max_group_tokens) {
+  const uint32_t tp = 4 * nt, frag_cols = 2 * (max_group_tokens < tp ? max_group_tokens : tp);
+  return HEADER_BYTES + (size_t)seed_words(kb_split) * 2 * tp * 4 + 128 + (size_t)frag_cols * (kb_split * 64 + 64);
+}
+
 Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt, uint32_t max_group_tokens,
                uint32_t active_groups, int n_ctas, uint32_t max_ksplit) {
   const uint32_t bb = dtype == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
@@ -712,6 +718,9 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
       seen_split = split;
       const uint32_t nn = (kb_total + split - 1) / split;
       if (nn > max_ksplit) continue;
+      // a ring of less than three stages of eight blocks loses more than a smaller split
+      const uint32_t stage_blocks = split < 8 ? split : 8;
+      if (fixed_smem(split, nt, max_group_tokens) + (size_t)3 * CONSUMER_WARPS * stage_blocks * 16 * bb > SMEM_LIMIT && split > 16 && n < max_ksplit) continue;
       const uint64_t items = items_per_split * nn;
       const double per_cta = (double)((items + n_ctas - 1) / n_ctas);
       const double units = (per_cta - 1.0) / tile_groups + 1.0;
@@ -723,7 +732,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   for (;;) {
     const uint32_t frag_cols = 2 * (max_group_tokens < tp ? max_group_tokens : tp);
     const uint32_t frag_stride = kb_split * 64 + 64;
-    const size_t fixed = HEADER_BYTES + (size_t)seed_words(kb_split) * 2 * tp * 4 + 128 + (size_t)frag_cols * frag_stride;
+    const size_t fixed = fixed_smem(kb_split, nt, max_group_tokens);
     if (fixed < SMEM_LIMIT) {
       const size_t avail = SMEM_LIMIT - fixed;
       for (uint32_t ppw = 4; ppw >= 1; ppw >>= 1) {
