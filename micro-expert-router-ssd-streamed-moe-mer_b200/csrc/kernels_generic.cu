@@ -885,44 +885,69 @@ __global__ void __launch_bounds__(256) k_combine_rows4(MoeDispatch d) {
 // RMSNorm of every token row and / or the shared expert's gate scalar (RmsNorm::forward_inplace, transformer.rs:62-74;
 // SharedExpert::forward, transformer.rs:2224-2231).  One CTA per token; sums are block tree reductions (the
 // reference adds left to right: rounding differs in the last bits only).
-__global__ void __launch_bounds__(256) k_pre_moe(const float *__restrict__ x, uint32_t D, const float *__restrict__ rms_weight, float eps,
-                                                 const float *__restrict__ shared_gate, float *__restrict__ xn,
-                                                 float *__restrict__ shared_scale) {
-  __shared__ float s_red[8];
-  __shared__ float s_bcast;
-  const uint32_t token = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+constexpr int PRE_THREADS = 512;
+// VEC: D is a multiple of four and the rows are read and written four values at a time (16 tokens of 7168: 5 us, 18 us one by one).
+template <bool VEC>
+__global__ void __launch_bounds__(PRE_THREADS) k_pre_moe(const float *__restrict__ x, uint32_t D, const float *__restrict__ rms_weight, float eps,
+                                                         const float *__restrict__ shared_gate, float *__restrict__ xn,
+                                                         float *__restrict__ shared_scale) {
+  constexpr int W = VEC ? 4 : 1;
+  __shared__ float s_red[2][PRE_THREADS / 32];
+  const uint32_t token = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = D / W;
   const float *row = x + (size_t)token * D;
-  auto block_sum = [&](float v) -> float {
-    v = warp_sum(v);
-    __syncthreads();  // s_red / s_bcast of a previous reduction have been read
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      float t = 0.0f;
-      for (int w = 0; w < 8; w++) t += s_red[w];
-      s_bcast = t;
+  auto load = [](const float *p, uint32_t i, float (&v)[W]) {
+    if (VEC) {
+      const float4 q = __ldg(reinterpret_cast<const float4 *>(p) + i);
+      v[0] = q.x, v[1 % W] = q.y, v[2 % W] = q.z, v[3 % W] = q.w;
+    } else {
+      v[0] = __ldg(p + i);
     }
+  };
+  auto block_sum = [&](float v, int k) -> float {
+    v = warp_sum(v);
+    if (lane == 0) s_red[k][warp] = v;
     __syncthreads();
-    return s_bcast;
+    float t = 0.0f;
+#pragma unroll
+    for (int w = 0; w < PRE_THREADS / 32; w++) t += s_red[k][w];
+    return t;
   };
   float scale = 1.0f;
   if (rms_weight) {
     float sq = 0.0f;
-    for (uint32_t i = threadIdx.x; i < D; i += blockDim.x) sq = fmaf(row[i], row[i], sq);
-    sq = block_sum(sq);
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < n; i += PRE_THREADS) {
+      float v[W];
+      load(row, i, v);
+#pragma unroll
+      for (int j = 0; j < W; j++) sq = fmaf(v[j], v[j], sq);
+    }
+    sq = block_sum(sq, 0);
     scale = 1.0f / sqrtf(sq / (float)D + eps);
   }
   float dot = 0.0f;
-  for (uint32_t i = threadIdx.x; i < D; i += blockDim.x) {
-    float v = row[i];
+#pragma unroll 4
+  for (uint32_t i = threadIdx.x; i < n; i += PRE_THREADS) {
+    float v[W], g[W];
+    load(row, i, v);
     if (rms_weight) {
-      v = __fmul_rn(__fmul_rn(v, scale), rms_weight[i]);  // x * scale * weight, rounded after each product
-      xn[(size_t)token * D + i] = v;
+      load(rms_weight, i, g);
+#pragma unroll
+      for (int j = 0; j < W; j++) v[j] = __fmul_rn(__fmul_rn(v[j], scale), g[j]);  // x * scale * weight, rounded after each product
+      float *dst = xn + (size_t)token * D + (size_t)i * W;
+      if (VEC)
+        *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1 % W], v[2 % W], v[3 % W]);
+      else
+        *dst = v[0];
     }
-    if (shared_gate) dot = fmaf(shared_gate[i], v, dot);
+    if (shared_gate) {
+      load(shared_gate, i, g);
+#pragma unroll
+      for (int j = 0; j < W; j++) dot = fmaf(g[j], v[j], dot);
+    }
   }
   if (shared_gate) {
-    dot = block_sum(dot);
+    dot = block_sum(dot, 1);
     if (threadIdx.x == 0) shared_scale[token] = 1.0f / (1.0f + expf(-dot));
   }
 }
@@ -1120,7 +1145,8 @@ cudaError_t launch_combine(const MoeDispatch &d, cudaStream_t s, int *launches) 
 cudaError_t launch_pre_moe(const float *x, uint32_t n_tokens, uint32_t D, const float *rms_weight, float eps, const float *shared_gate,
                            float *xn, float *shared_scale, cudaStream_t s, int *launches) {
   if (!rms_weight && !shared_gate) return cudaSuccess;
-  k_pre_moe<<<n_tokens, 256, 0, s>>>(x, D, rms_weight, eps, shared_gate, xn, shared_scale);
+  const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(rms_weight) | reinterpret_cast<uintptr_t>(shared_gate) | reinterpret_cast<uintptr_t>(xn);
+  (D % 4 == 0 && at % 16 == 0 ? k_pre_moe<true> : k_pre_moe<false>)<<<n_tokens, PRE_THREADS, 0, s>>>(x, D, rms_weight, eps, shared_gate, xn, shared_scale);
   if (launches) (*launches)++;
   return cudaGetLastError();
 }
