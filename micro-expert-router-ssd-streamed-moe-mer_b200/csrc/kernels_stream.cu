@@ -379,7 +379,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     // two adjacent blocks (kb, kb + 1; kb even) of both row slots against every live N-tile.
     // rec = shared address of the pair's first record in this warp's tile chunk.
     auto do_pair = [&](uint32_t rec, uint32_t kb, auto nl) {
-      constexpr int NL = decltype(nl)::value;  // N-tiles at most
+      constexpr int NL = decltype(nl)::value;  // N-tiles that hold tokens, 0: n_live
       uint32_t a0[4], a0h[4], a1[4], a1h[4];  // block kb: slots g / g+8; block kb+1: slots g / g+8
       float2 d0, d1;                          // {scale slot g, scale slot g+8} of each block
       if (DT == MER_DTYPE_Q4_0) {
@@ -395,7 +395,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       }
 #pragma unroll
       for (int n = 0; n < NT; n++) {
-        if (n >= NL || (n > 0 && (uint32_t)n >= n_live)) break;  // uniform
+        if (NL ? n >= NL : (n > 0 && (uint32_t)n >= n_live)) break;  // uniform
         const uint4 bf0 = lds128(fa[n] + kb * 64), bf1 = lds128(fa[n] + kb * 64 + 64);
         float c1[4], c2[4], e1[4], e2[4];
         mma_f16(c1, a0[0], a0h[0], a0[1], a0h[1], bf0.x, bf0.y, 0.0f, 0.0f, 0.0f, 0.0f);
@@ -448,16 +448,24 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       if (!dead && my_tile_exists) {
         constexpr uint32_t PAIR_BYTES = 2 * 16 * BB;  // 576 (Q4_0) / 1088 (Q8_0)
         uint32_t rec = stage0 + stage * stage_bytes;
-        using All = std::integral_constant<int, NT>;
+        using Live = std::integral_constant<int, 0>;
         using One = std::integral_constant<int, 1>;
-        // Four blocks per iteration keep independent MMA chains in flight.  A single N-tile of Q4_0 takes eight (2 % on 16
-        // tokens of 8 x 14336 x 4096; with two N-tiles, or Q8_0, the longer loop costs as much).
+        using All = std::integral_constant<int, NT>;
+        // Four blocks per iteration keep independent MMA chains in flight.  Q4_0 has loops of its own for one N-tile, eight
+        // blocks long, and for two (2 to 3 % on 16 tokens of 8 x 14336 x 4096); Q8_0 loses 2 % with them.
         if (!RAGGED && DT == MER_DTYPE_Q4_0 && (NT == 1 || n_live == 1)) {
 #pragma unroll 2
           for (uint32_t b = 0; b < nb; b += 4, rec += 2 * PAIR_BYTES) {
             do_zero(rec, c0 + b, 4, false);
             do_pair(rec, c0 + b, One{});
             do_pair(rec + PAIR_BYTES, c0 + b + 2, One{});
+          }
+        } else if (!RAGGED && DT == MER_DTYPE_Q4_0) {
+#pragma unroll 1
+          for (uint32_t b = 0; b < nb; b += 4, rec += 2 * PAIR_BYTES) {
+            do_zero(rec, c0 + b, 4, false);
+            do_pair(rec, c0 + b, All{});
+            do_pair(rec + PAIR_BYTES, c0 + b + 2, All{});
           }
         } else
 #pragma unroll 1
@@ -468,12 +476,12 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
             do_last(rec, c0 + b);
             continue;
           }
-          do_pair(rec, c0 + b, All{});
+          do_pair(rec, c0 + b, Live{});
           if (RAGGED && left < 4) {
             if (left == 3) do_last(rec + PAIR_BYTES, c0 + b + 2);
             continue;
           }
-          do_pair(rec + PAIR_BYTES, c0 + b + 2, All{});
+          do_pair(rec + PAIR_BYTES, c0 + b + 2, Live{});
         }
       }
       __syncwarp();
