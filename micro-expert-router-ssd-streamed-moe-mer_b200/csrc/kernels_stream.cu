@@ -574,8 +574,8 @@ __device__ void ffn_stream_tail(const StreamParams &p) {
       float mx = 0.0f;
       if (f0 < F) {
         float4 g = make_float4(0, 0, 0, 0), up = make_float4(0, 0, 0, 0);
-#pragma unroll 1
-        for (uint32_t k = 0; k < p.n_ksplit; k++) {
+#pragma unroll 4
+        for (uint32_t k = 0; k < p.n_ksplit; k++) {  // loads of several splits in flight, added in order
           const float *base = parts + ((size_t)k * P + pair) * 2 * F;
           const float4 a = __ldcg(reinterpret_cast<const float4 *>(base + f0)), b = __ldcg(reinterpret_cast<const float4 *>(base + F + f0));
           g.x += a.x, g.y += a.y, g.z += a.z, g.w += a.w;
@@ -608,22 +608,38 @@ __device__ void ffn_stream_tail(const StreamParams &p) {
         const float4 r = __ldg(reinterpret_cast<const float4 *>(d.residual) + (size_t)token * D4 + i4);
         acc.x = __fadd_rn(r.x, acc.x), acc.y = __fadd_rn(r.y, acc.y), acc.z = __fadd_rn(r.z, acc.z), acc.w = __fadd_rn(r.w, acc.w);
       };
+      // four slots at a time: their loads are in flight together (one by one, the eight partial sums of two slots took 3 us)
+      constexpr uint32_t S = 4;
 #pragma unroll 1
-      for (uint32_t sl = 0; sl < d.slots; sl++) {
-        if (d.residual && sl == d.routed_slots) add_residual();
-        const size_t pr = (size_t)token * d.slots + sl;
-        const float w = d.pair_weight[pr];
-        if (d.pair_expert[pr] == MER_NONE || w == 0.0f) continue;
-        float4 yv = __ldcg(yp + pr * D4 + i4);
-#pragma unroll 1
-        for (uint32_t k = 1; k < p.n_ksplit; k++) {
-          const float4 t = __ldcg(yp + (size_t)k * part4 + pr * D4 + i4);
-          yv.x += t.x, yv.y += t.y, yv.z += t.z, yv.w += t.w;
+      for (uint32_t s0 = 0; s0 < d.slots; s0 += S) {
+        float w[S];
+        float4 yv[S];
+#pragma unroll
+        for (uint32_t j = 0; j < S; j++) {
+          const size_t pr = (size_t)token * d.slots + s0 + j;
+          w[j] = s0 + j < d.slots && d.pair_expert[pr] != MER_NONE ? d.pair_weight[pr] : 0.0f;
         }
-        acc.x = __fadd_rn(acc.x, __fmul_rn(w, yv.x));
-        acc.y = __fadd_rn(acc.y, __fmul_rn(w, yv.y));
-        acc.z = __fadd_rn(acc.z, __fmul_rn(w, yv.z));
-        acc.w = __fadd_rn(acc.w, __fmul_rn(w, yv.w));
+#pragma unroll
+        for (uint32_t j = 0; j < S; j++)
+          yv[j] = w[j] != 0.0f ? __ldcg(yp + ((size_t)token * d.slots + s0 + j) * D4 + i4) : make_float4(0, 0, 0, 0);
+#pragma unroll 2
+        for (uint32_t k = 1; k < p.n_ksplit; k++) {
+#pragma unroll
+          for (uint32_t j = 0; j < S; j++) {
+            if (w[j] == 0.0f) continue;
+            const float4 t = __ldcg(yp + (size_t)k * part4 + ((size_t)token * d.slots + s0 + j) * D4 + i4);
+            yv[j].x += t.x, yv[j].y += t.y, yv[j].z += t.z, yv[j].w += t.w;
+          }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < S; j++) {
+          if (d.residual && s0 + j == d.routed_slots && s0 + j < d.slots) add_residual();
+          if (w[j] == 0.0f) continue;
+          acc.x = __fadd_rn(acc.x, __fmul_rn(w[j], yv[j].x));
+          acc.y = __fadd_rn(acc.y, __fmul_rn(w[j], yv[j].y));
+          acc.z = __fadd_rn(acc.z, __fmul_rn(w[j], yv[j].z));
+          acc.w = __fadd_rn(acc.w, __fmul_rn(w[j], yv[j].w));
+        }
       }
       if (d.residual && d.routed_slots >= d.slots) add_residual();
       reinterpret_cast<float4 *>(d.out)[(size_t)token * D4 + i4] = acc;
