@@ -134,6 +134,22 @@ cudaError_t launch_a2a_combine(uint32_t n_tokens, uint32_t D, uint32_t slots, ui
 bool groups_layer_on_grid(const MoeDispatch &d);
 cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaStream_t s, int *launches, bool counted = false);
 // group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
+// Launches `kern` so that it may start while its predecessor in the stream still runs (the kernel waits for it itself).  Between the
+// three or four short kernels of a decode layer this hides launch and set-up, 1 to 2 us each.
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t s, bool cooperative, A... args) {
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeCooperative;
+  at[1].val.cooperative = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(block), cfg.dynamicSmemBytes = smem, cfg.stream = s;
+  cfg.attrs = at, cfg.numAttrs = cooperative ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+bool router_sets_status(const MoeDispatch &d);
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s, int *launches,
                           bool group = true);
 cudaError_t launch_groups_from_pairs(const MoeDispatch &d, cudaStream_t s, int *launches);

@@ -5,6 +5,7 @@
 // d_ff not a multiple of 32, e.g. the reference's 37x45 test shape) and are the on-device
 // cross-check for the streaming kernels.
 #include "kernels.h"
+#include "ptx.cuh"
 
 #include <cuda_fp16.h>
 #include "../../include/mer_b200.h"
@@ -646,6 +647,10 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   __shared__ float s_part[ROWS][ROUTER_TT][ROUTER_WARPS + 1];  // [row][token][warp]
   __shared__ float s_logit[ROUTER_TT][ROWS];                  // used when one CTA covers all experts
   const bool single = gridDim.x == 1 && !pre;
+  // With the grouping done here, status bits gather in a scratch word, which the last CTA publishes: no launch clears them.
+  uint32_t *const status = group_here == 1 ? d.counters + max_tokens + 1 : d.status;
+  grid_dep_wait();
+  grid_dep_launch();
 
   if (pre) {
     // logits are already in d.logits (k_router_logits_tiled)
@@ -748,7 +753,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
       for (uint32_t i = lane; i < E; i += 32) s_score[i] = single ? s_logit[warp][i] : __ldcg(d.logits + (size_t)token * E + i);
     }
     __syncwarp();
-    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], d.status);
+    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], status);
     const size_t p0 = (size_t)token * d.slots;
     if (lane < r.top_k) {
       d.pair_expert[p0 + lane] = pick.id == MER_NONE ? MER_NONE : r.id_base + pick.id;
@@ -775,6 +780,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     if (!s_flag) return;
     __threadfence();
   }
+  if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
   build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
 }
 
@@ -1000,6 +1006,8 @@ __global__ void __launch_bounds__(PRE_THREADS) k_pre_moe(const float *__restrict
     return t;
   };
   float scale = 1.0f;
+  grid_dep_wait();
+  grid_dep_launch();
   if (rms_weight) {
     float sq = 0.0f;
 #pragma unroll 4
@@ -1125,6 +1133,9 @@ __global__ void k_f32_to_f16(const float *__restrict__ src, uint16_t *__restrict
 
 }  // namespace
 
+// Whether launch_router leaves d.status written by itself (it groups in its last CTA): no need to clear it first.
+bool router_sets_status(const MoeDispatch &d) { return d.n_tokens * d.slots < GRID_GROUPING_PAIRS || d.group_count == nullptr; }
+
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s,
                           int *launches, bool group) {
   const uint32_t E = r.num_experts, G = d.n_groups;
@@ -1160,7 +1171,8 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  kern<<<grid, ROUTER_THREADS, smem, s>>>(r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0);
+  cudaError_t e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0);
+  if (e != cudaSuccess) return e;
   if (launches) (*launches)++;
   if (grid_grouping) {  // the router has counted the pairs per group
     const unsigned blocks = (P + 1023) / 1024;
@@ -1233,7 +1245,9 @@ cudaError_t launch_pre_moe(const float *x, uint32_t n_tokens, uint32_t D, const 
                            float *xn, float *shared_scale, cudaStream_t s, int *launches) {
   if (!rms_weight && !shared_gate) return cudaSuccess;
   const uintptr_t at = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(rms_weight) | reinterpret_cast<uintptr_t>(shared_gate) | reinterpret_cast<uintptr_t>(xn);
-  (D % 4 == 0 && at % 16 == 0 ? k_pre_moe<true> : k_pre_moe<false>)<<<n_tokens, PRE_THREADS, 0, s>>>(x, D, rms_weight, eps, shared_gate, xn, shared_scale);
+  const cudaError_t e = launch_overlapped(D % 4 == 0 && at % 16 == 0 ? k_pre_moe<true> : k_pre_moe<false>, dim3(n_tokens), PRE_THREADS, 0, s, false, x, D,
+                                          rms_weight, eps, shared_gate, xn, shared_scale);
+  if (e != cudaSuccess) return e;
   if (launches) (*launches)++;
   return cudaGetLastError();
 }

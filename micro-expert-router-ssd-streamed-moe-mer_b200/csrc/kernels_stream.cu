@@ -135,6 +135,8 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  grid_dep_wait();
+  grid_dep_launch();
   __syncthreads();
 
   const uint32_t n_tiles = (p.packed_tiles + CONSUMER_WARPS - 1) / CONSUMER_WARPS;  // items per (pass, K split); the last one may hold fewer tiles
@@ -833,14 +835,8 @@ cudaError_t launch_phase(const StreamParams &p, uint32_t nt, size_t smem, int gr
                                       : (nt == 2 ? k_ffn_stream<DT, 2, false> : k_ffn_stream<DT, 1, false>);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  if (p.tail != TAIL_NONE) {
-    // the tail waits for every CTA of the grid: a cooperative launch guarantees that they are all resident
-    StreamParams q = p;
-    void *args[] = {&q};
-    return cudaLaunchCooperativeKernel((const void *)kern, dim3(grid), dim3(THREADS), args, smem, s);
-  }
-  kern<<<grid, THREADS, smem, s>>>(p);
-  return cudaGetLastError();
+  // the tail waits for every CTA of the grid: a cooperative launch guarantees that they are all resident
+  return launch_overlapped(kern, dim3(grid), THREADS, smem, s, p.tail != TAIL_NONE, p);
 }
 
 }  // namespace

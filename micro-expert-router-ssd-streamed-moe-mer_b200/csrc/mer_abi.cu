@@ -899,9 +899,9 @@ MER_EXPORT int mer_backend_create(const mer_backend_cfg *cfg, mer_backend **out)
   CB(cudaMemset(b->d_group_count, 0, (size_t)b->max_groups * 2 * 4));
   CB(cudaMalloc((void **)&b->d_perm, P * 4));
   CB(cudaMalloc((void **)&b->d_logits, T * b->max_router_experts * 4));
-  CB(cudaMalloc((void **)&b->d_counters, (T + 1) * 4));
+  CB(cudaMalloc((void **)&b->d_counters, (T + 2) * 4));
   CB(cudaMemset(b->d_status, 0, 4));
-  CB(cudaMemset(b->d_counters, 0, (T + 1) * 4));
+  CB(cudaMemset(b->d_counters, 0, (T + 2) * 4));
   CB(cudaMalloc((void **)&b->d_f16, std::max(P, T) * D * 2));
   CB(cudaHostAlloc((void **)&b->h_u32, (P + 1) * 4, cudaHostAllocDefault));
   CB(cudaHostAlloc((void **)&b->h_f32, P * 4, cudaHostAllocDefault));
@@ -1281,7 +1281,7 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   if (run_ffn_too) bind_ffn(b, d);
   d.x = d_x;
   d.out = d_out;
-  CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
+  if (!run_ffn_too || !router_sets_status(d)) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
   if (!capturing) CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
   cudaEvent_t *ev = (run_ffn_too && !capturing) ? next_timing_set(b) : nullptr;
   if (ev) cudaEventRecord(ev[0], s);

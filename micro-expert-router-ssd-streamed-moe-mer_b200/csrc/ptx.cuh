@@ -8,6 +8,11 @@ namespace {
 
 constexpr uint32_t SPIN_LIMIT = 1u << 16;  // polls per bounded wait; a poll suspends for tens of microseconds
 
+// Programmatic dependent launch: a kernel launched with the attribute starts while its predecessor runs and waits here, before
+// it touches anything the predecessor reads or writes; without the attribute both are no-ops.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
