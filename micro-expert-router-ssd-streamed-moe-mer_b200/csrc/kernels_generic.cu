@@ -725,14 +725,12 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   __syncthreads();
   if (!single && !pre) {
     if (threadIdx.x == 0) {
-      __threadfence();
-      uint32_t prev = atomicAdd(&d.counters[tile], 1u);
+      const uint32_t prev = arrive_acq_rel(&d.counters[tile]);
       s_flag = (prev == gridDim.x - 1);
       if (s_flag) d.counters[tile] = 0;  // re-arm for the next launch
     }
     __syncthreads();
     if (!s_flag) return;
-    __threadfence();
   }
 
   // ---- this CTA holds the last logits of the token tile: one warp routes one token ----
@@ -771,14 +769,12 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   const uint32_t n_tiles = gridDim.y;
   if (n_tiles > 1) {
     if (threadIdx.x == 0) {
-      __threadfence();
-      uint32_t prev = atomicAdd(&d.counters[max_tokens], 1u);
+      const uint32_t prev = arrive_acq_rel(&d.counters[max_tokens]);
       s_flag = (prev == n_tiles - 1);
       if (s_flag) d.counters[max_tokens] = 0;
     }
     __syncthreads();
     if (!s_flag) return;
-    __threadfence();
   }
   if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
   build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));

@@ -541,18 +541,12 @@ __device__ bool grid_barrier(uint32_t *counter, uint32_t *status) {
   __shared__ int s_ok;
   __syncthreads();  // this CTA's stores are issued
   if (threadIdx.x == 0) {
-    __threadfence();
-    atomicAdd(counter, 1u);
+    bool ok = arrive_acq_rel(counter) + 1 >= gridDim.x;
     const uint64_t t0 = global_ns();
-    bool ok = true;
-    while (*(volatile uint32_t *)counter < gridDim.x) {
-      __nanosleep(64);
-      if (global_ns() - t0 > 2000000000ull) {
-        ok = false;
-        break;
-      }
+    for (uint32_t polls = 0; !ok; polls++) {
+      ok = load_acquire(counter) >= gridDim.x;
+      if (!ok && (polls & 31) == 31 && global_ns() - t0 > 2000000000ull) break;
     }
-    __threadfence();
     if (!ok) atomicOr(status, MER_DEVSTAT_TIMEOUT);
     s_ok = ok;
   }

@@ -8,6 +8,18 @@ namespace {
 
 constexpr uint32_t SPIN_LIMIT = 1u << 16;  // polls per bounded wait; a poll suspends for tens of microseconds
 
+// Arrival counters between CTAs: what the CTA wrote before (a __syncthreads() in front) is visible to whoever acquires the count.
+__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t *counter) {
+  uint32_t v;
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(counter) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t load_acquire(const uint32_t *p) {
+  uint32_t v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Programmatic dependent launch: a kernel launched with the attribute starts while its predecessor runs and waits here, before
 // it touches anything the predecessor reads or writes; without the attribute both are no-ops.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
