@@ -717,7 +717,7 @@ constexpr uint32_t MAX_KSPLIT = 64;
 //  * K split: the largest split (whole K, K/2, K/4, ... in multiples of 8 blocks, at least 16 blocks)
 //    that still leaves about eight items per CTA for the expected number of active experts, within
 //    `max_ksplit` (what the partial-sum scratch can hold);
-//  * a stage holds 4 block pairs per warp if at least three stages then fit, else 2, else 1;
+//  * a stage holds 8 (Q4_0) or 4 block pairs per warp if at least three stages then fit, else half of that, and so on (8: 2 % on one token);
 //  * fragment arrays are sized by the most tokens any group can hold in this dispatch.
 // Shared memory of a plan without its ring.
 size_t fixed_smem(uint32_t kb_split, uint32_t nt, uint32_t max_group_tokens) {
@@ -739,7 +739,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   // (epilogue) and one activation-fragment rebuild per (pass, K split) unit its contiguous range touches; a rebuild
   // measures about 4 us, i.e. ~10 block steps of Q8_0 or ~20 of Q4_0 at the rate one SM streams.
   {
-    const double rebuild = dtype == MER_DTYPE_Q4_0 ? 20.0 : 10.0, per_item = 2.0;
+    const double rebuild = dtype == MER_DTYPE_Q4_0 ? 20.0 : 10.0, per_item = 6.0;
     double best = 1e30;
     uint32_t seen_split = 0;
     for (uint32_t n = 1; n <= max_ksplit; n++) {
@@ -767,7 +767,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
     const size_t fixed = fixed_smem(kb_split, nt, max_group_tokens);
     if (fixed < SMEM_LIMIT) {
       const size_t avail = SMEM_LIMIT - fixed;
-      for (uint32_t ppw = 4; ppw >= 1; ppw >>= 1) {
+      for (uint32_t ppw = dtype == MER_DTYPE_Q4_0 ? 8 : 4; ppw >= 1; ppw >>= 1) {
         uint32_t kc = 2 * ppw;
         if (kc > kb_split) kc = kb_split;
         const uint32_t chunk = kc * 16 * bb;
