@@ -249,9 +249,12 @@ __global__ void __launch_bounds__(256) k_group_count(RouterDev r, MoeDispatch d)
 }
 __global__ void __launch_bounds__(256) k_group_scan(RouterDev r, MoeDispatch d) {
   const uint32_t G = d.n_groups;
-  for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) d.group_expert[g] = (g < r.num_experts) ? r.id_base + g : r.shared_expert_id;
-  // the counts go through shared memory in slabs: one thread adds them up, everybody loads and stores
-  __shared__ uint32_t s_cnt[1024];
+  for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) {
+    d.group_expert[g] = (g < r.num_experts) ? r.id_base + g : r.shared_expert_id;
+    d.group_cursor[g] = 0;  // of the scatter that follows
+  }
+  // the counts go through shared memory in slabs
+  __shared__ uint32_t s_cnt[1024], s_warp[8];
   __shared__ uint32_t s_run;
   if (threadIdx.x == 0) s_run = 0;
   for (uint32_t g0 = 0; g0 < G; g0 += 1024) {
@@ -262,14 +265,31 @@ __global__ void __launch_bounds__(256) k_group_scan(RouterDev r, MoeDispatch d) 
       d.group_count[g0 + i] = 0;  // zero again for the next dispatch's count
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t acc = s_run;
-      for (uint32_t i = 0; i < n; i++) {
-        const uint32_t c = s_cnt[i];
-        s_cnt[i] = acc;
-        acc += c;
+    {  // exclusive scan, four counts per thread
+      uint32_t c[4], run = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) c[i] = threadIdx.x * 4 + i < n ? s_cnt[threadIdx.x * 4 + i] : 0, run += c[i];
+      uint32_t incl = run;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((threadIdx.x & 31) >= (uint32_t)o) incl += up;
       }
-      s_run = acc;
+      if ((threadIdx.x & 31) == 31) s_warp[threadIdx.x >> 5] = incl;
+      __syncthreads();
+      uint32_t acc = s_run + incl - run, total = s_run;
+#pragma unroll
+      for (uint32_t w = 0; w < 8; w++) {
+        if (w < threadIdx.x >> 5) acc += s_warp[w];
+        total += s_warp[w];
+      }
+#pragma unroll
+      for (uint32_t i = 0; i < 4; i++) {
+        if (threadIdx.x * 4 + i < n) s_cnt[threadIdx.x * 4 + i] = acc;
+        acc += c[i];
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) s_run = total;
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) d.offsets[g0 + i] = s_cnt[i];
@@ -287,11 +307,6 @@ __global__ void __launch_bounds__(256) k_group_scatter(RouterDev r, MoeDispatch 
     if (k != MER_NONE) d.perm[d.offsets[k] + atomicAdd(d.group_cursor + k, 1u)] = p;
   }
 }
-// Clears the scatter cursors after use, so that group_count / group_cursor are zero between dispatches.
-__global__ void k_group_clear(MoeDispatch d) {
-  for (uint32_t g = threadIdx.x; g < d.n_groups; g += blockDim.x) d.group_cursor[g] = 0;
-}
-
 // The same for at most 32 pairs of the streaming kernels, in registers of one warp: sorted position of every pair, the pairs
 // that start a pass, their order.  The general form's dozen block-wide steps took 4 us on B200 for one token's eight pairs, as long
 // as the kernels that follow need for the weights of half of them.
@@ -541,39 +556,48 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
   if (d.pass_group) build_passes_block(d, s_off);
 }
 
-// Router logits of a large batch as a tiled fp32 GEMM: logits[t][e] = x[t] . w[e].  A CTA computes 32 tokens x 64
-// experts; K runs in chunks of 256 values that cp.async double-buffers in shared memory.  Eight warps split every
-// chunk (32 values of K each); a thread holds 8 tokens x 8 experts (rows ty + 4 i and tx + 8 j: neighbouring lanes read
-// neighbouring rows, whose stride of 260 floats keeps every 128-bit load conflict-free), i.e. 16 shared 128-bit loads per 256 FMAs (the
-// 4 x 4 form before it, 8 loads per 64 FMAs, was bound by shared-memory bandwidth: 45 us for 1 GFLOP).  The eight
-// partial sums are added at the end in warp order.  k_router then runs with `pre` set and only scores / selects.
+// Router logits of a large batch as a tiled fp32 GEMM: logits[t][e] = x[t] . w[e].  A CTA computes TT tokens x TE experts; K
+// runs in chunks of KC values that cp.async double-buffers in shared memory.  A warp owns 32 tokens x 64 experts over a
+// slice of every chunk; a thread holds 8 tokens x 8 experts (rows ty + 4 i and tx + 8 j: neighbouring lanes read neighbouring
+// rows, whose stride of 4 mod 32 floats keeps every 128-bit load conflict-free), i.e. 16 shared 128-bit loads per 256 FMAs.
+// The slices' partial sums are added at the end in warp order.  k_router then runs with `pre` set and only scores / selects.
+// What bounds it is reading operand rows from L2: the 64 x 128 tile reads half as much per FMA as 32 x 64
+// (4096 x 256 x 7168 with selection and grouping: 710 us before, 614 now).
 constexpr int RL_WARPS = 8, RL_THREADS = 32 * RL_WARPS;
-constexpr int RL_TT = 32, RL_TE = 64, RL_KC = 32 * RL_WARPS, RL_LD = RL_KC + 4;  // row stride = 4 mod 32 floats: conflict-free 128-bit loads
-constexpr size_t RL_BUF = (size_t)(RL_TT + RL_TE) * RL_LD;                       // floats per buffer
-constexpr size_t RL_SMEM = 2 * RL_BUF * 4;
+template <int TT, int TE, int KC>
+struct LogitsTile {
+  static constexpr int SPATIAL = TT / 32 * (TE / 64), SLICES = RL_WARPS / SPATIAL, SLICE_K = KC / SLICES, LD = KC + 4;
+  static constexpr size_t BUF = (size_t)(TT + TE) * LD, SMEM = 2 * BUF * 4;  // floats per buffer; bytes
+};
+template <int TT, int TE, int KC>
 __global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r, MoeDispatch d, uint32_t ksplit) {
+  using S = LogitsTile<TT, TE, KC>;
+  constexpr int RL_TT = TT, RL_TE = TE, RL_KC = KC, RL_LD = S::LD, PIECES = KC / 4, STEP = RL_THREADS / PIECES;
+  constexpr size_t RL_BUF = S::BUF;
   extern __shared__ __align__(16) float sm[];
   const uint32_t E = r.num_experts, D = d.D, T = d.n_tokens;
   const uint32_t t0 = blockIdx.y * RL_TT, e0 = blockIdx.x * RL_TE;
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, ty = lane >> 3, tx = lane & 7;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t where = warp % S::SPATIAL, slice = warp / S::SPATIAL;
+  const uint32_t ty = where % (TT / 32) * 32 + (lane >> 3), tx = where / (TT / 32) * 64 + (lane & 7);
   float acc[8][8];
 #pragma unroll
   for (int i = 0; i < 8; i++)
 #pragma unroll
     for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
-  // global -> shared: a thread copies one 16-byte piece of every fourth row (64 pieces per 256-value row)
-  const uint32_t lr = tid >> 6, lc = (tid & 63) * 4;
+  // global -> shared: a thread copies one 16-byte piece of every STEP-th row
+  const uint32_t lr = tid / PIECES, lc = tid % PIECES * 4;
   auto issue_chunk = [&](uint32_t k0, uint32_t buf) {
     float *xs = sm + buf * RL_BUF, *ws = xs + RL_TT * RL_LD;
 #pragma unroll
-    for (int i = 0; i < RL_TT / 4; i++) {
-      const uint32_t row = 4 * i + lr;
+    for (int i = 0; i < RL_TT / STEP; i++) {
+      const uint32_t row = STEP * i + lr;
       const float *src = d.x + (size_t)min(t0 + row, T - 1) * D + k0 + lc;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + row * RL_LD + lc)), "l"(src) : "memory");
     }
 #pragma unroll
-    for (int j = 0; j < RL_TE / 4; j++) {
-      const uint32_t row = 4 * j + lr;
+    for (int j = 0; j < RL_TE / STEP; j++) {
+      const uint32_t row = STEP * j + lr;
       const float *src = r.w + (size_t)min(e0 + row, E - 1) * D + k0 + lc;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(ws + row * RL_LD + lc)), "l"(src) : "memory");
     }
@@ -593,8 +617,8 @@ __global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r,
     __syncthreads();  // ... and everybody else's
     const float *xs = sm + (c & 1) * RL_BUF, *ws = xs + RL_TT * RL_LD;
 #pragma unroll 2
-    for (int kk = 0; kk < RL_KC / RL_WARPS; kk += 4) {
-      const int k = warp * (RL_KC / RL_WARPS) + kk;
+    for (int kk = 0; kk < S::SLICE_K; kk += 4) {
+      const int k = slice * S::SLICE_K + kk;
       float4 a[8], b[8];
 #pragma unroll
       for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(xs + (ty + 4 * i) * RL_LD + k);
@@ -612,24 +636,24 @@ __global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r,
     }
     __syncthreads();  // the buffer may be refilled two iterations from now
   }
-  // partial sums of warps 1..7 through shared memory (the operand buffers are done with), added to warp 0's in warp order
-  float *red = sm;  // [RL_WARPS - 1][RL_TT * RL_TE]
-  static_assert((RL_WARPS - 1) * RL_TT * RL_TE <= 2 * RL_BUF, "the partial sums fit the operand buffers");
-  if (warp > 0) {
+  // partial sums of slices 1.. through shared memory (the operand buffers are done with), added to slice 0's in order
+  float *red = sm;  // [SLICES - 1][RL_TT * RL_TE]
+  static_assert((S::SLICES - 1) * RL_TT * RL_TE <= 2 * RL_BUF, "the partial sums fit the operand buffers");
+  if (slice > 0) {
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
-      for (int j = 0; j < 8; j++) red[(warp - 1) * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j] = acc[i][j];
+      for (int j = 0; j < 8; j++) red[(slice - 1) * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j] = acc[i][j];
   }
   __syncthreads();
-  if (warp == 0) {
+  if (slice == 0) {
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         float v = acc[i][j];
 #pragma unroll
-        for (int g = 0; g < RL_WARPS - 1; g++) v += red[g * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j];
+        for (int g = 0; g < S::SLICES - 1; g++) v += red[g * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j];
         const uint32_t t = t0 + ty + 4 * i, e = e0 + tx + 8 * j;
         if (t < T && e < E) d.logits[((size_t)blockIdx.z * T + t) * E + e] = v;
       }
@@ -1140,19 +1164,32 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   size_t smem = smem_topk > smem_grp ? smem_topk : smem_grp;
   smem = (smem + 15) & ~(size_t)15;
-  const bool tiled = d.n_tokens >= 256 && (d.D % RL_KC) == 0;  // from a few hundred tokens: logits as a tiled GEMM first
+  // From a few hundred tokens the logits are a tiled GEMM of their own, unless the experts are so few that most of a tile would be
+  // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel).
+  const bool tiled = d.n_tokens >= 256 && d.D % 256 == 0 && (E > 16 || d.D % 1024 != 0);
   uint32_t ksplit = 1;
   if (tiled) {
-    dim3 lgrid((E + RL_TE - 1) / RL_TE, (d.n_tokens + RL_TT - 1) / RL_TT);
     // split K over blockIdx.z while the tiles alone leave SMs idle (the partial sets must fit the logits scratch,
     // which holds max_tokens x 4096 floats, and a slice is a whole number of chunks)
-    const uint32_t n_chunks = d.D / RL_KC, tiles = lgrid.x * lgrid.y;
-    for (uint32_t ks = 2; ks <= 8 && ks <= n_chunks; ks++)
-      if (n_chunks % ks == 0 && tiles * ks <= 160 && (size_t)ks * E <= 4096) ksplit = ks;
-    lgrid.z = ksplit;
-    cudaError_t e = cudaFuncSetAttribute(k_router_logits_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RL_SMEM);
+    auto plan = [&](uint32_t tt, uint32_t te, uint32_t kc, dim3 &grid) {
+      grid = dim3((E + te - 1) / te, (d.n_tokens + tt - 1) / tt);
+      const uint32_t n_chunks = d.D / kc, tiles = grid.x * grid.y;
+      for (uint32_t ks = 2; ks <= 8 && ks <= n_chunks; ks++)
+        if (n_chunks % ks == 0 && tiles * ks <= 160 && (size_t)ks * E <= 4096) grid.z = ks;
+    };
+    auto run = [&](auto kern, size_t bytes, dim3 grid) {
+      ksplit = grid.z;
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+      if (e == cudaSuccess) kern<<<grid, RL_THREADS, bytes, s>>>(r, d, ksplit);
+      return e;
+    };
+    // the large tile where it fills the chip and the experts fill it
+    dim3 big, small;
+    plan(64, 128, 128, big), plan(32, 64, 256, small);
+    const bool use_big = E > 64 && (E % 128 == 0 || E > 512) && big.x * big.y * big.z >= 120;
+    const cudaError_t e = use_big ? run(k_router_logits_tiled<64, 128, 128>, LogitsTile<64, 128, 128>::SMEM, big)
+                                  : run(k_router_logits_tiled<32, 64, 256>, LogitsTile<32, 64, 256>::SMEM, small);
     if (e != cudaSuccess) return e;
-    k_router_logits_tiled<<<lgrid, RL_THREADS, RL_SMEM, s>>>(r, d, ksplit);
     if (launches) (*launches)++;
   }
   // Expert rows per CTA: eight share the loads of x best, but a small call wants its few rows on as many SMs as there are
@@ -1174,8 +1211,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     const unsigned blocks = (P + 1023) / 1024;
     k_group_scan<<<1, 256, 0, s>>>(r, d);
     k_group_scatter<<<blocks, 256, 0, s>>>(r, d);
-    k_group_clear<<<1, 256, 0, s>>>(d);
-    if (launches) (*launches) += 3;
+    if (launches) (*launches) += 2;
   }
   return cudaGetLastError();
 }
@@ -1189,8 +1225,7 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
     if (!counted) k_group_count<<<blocks, 256, 0, s>>>(r, d);
     k_group_scan<<<1, 256, 0, s>>>(r, d);
     k_group_scatter<<<blocks, 256, 0, s>>>(r, d);
-    k_group_clear<<<1, 256, 0, s>>>(d);
-    if (launches) (*launches) += counted ? 3 : 4;
+    if (launches) (*launches) += counted ? 2 : 3;
     return cudaGetLastError();
   }
   size_t smem = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
