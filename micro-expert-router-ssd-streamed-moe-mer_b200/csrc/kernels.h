@@ -149,6 +149,8 @@ inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, unsigned blo
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+cudaError_t launch_host_in(const void *src, void *dst, size_t words, uint32_t *status, cudaStream_t s, int *launches);
+cudaError_t launch_host_out(const void *src, size_t stride, size_t rows, size_t words, void *dst, uint32_t *count, uint32_t *done, cudaStream_t s, int *launches);
 bool router_sets_status(const MoeDispatch &d);
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s, int *launches,
                           bool group = true);

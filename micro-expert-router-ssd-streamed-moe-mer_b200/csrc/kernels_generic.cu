@@ -998,6 +998,28 @@ __global__ void __launch_bounds__(256) k_combine_rows4(MoeDispatch d) {
 // RMSNorm of every token row and / or the shared expert's gate scalar (RmsNorm::forward_inplace, transformer.rs:62-74;
 // SharedExpert::forward, transformer.rs:2224-2231).  One CTA per token; sums are block tree reductions (the
 // reference adds left to right: rounding differs in the last bits only).
+// A few KB between pinned host memory and the device, as kernels of the call's own sequence: a copy node waits 3 to 4 us for the copy
+// engine on either side.  `status` (may be null) is cleared on the way in; on the way out `done` is written last, for a host
+// that polls it.
+constexpr int HOST_COPY_THREADS = 1024;
+__global__ void __launch_bounds__(HOST_COPY_THREADS) k_host_in(const uint32_t *__restrict__ src, uint32_t *__restrict__ dst, uint32_t n, uint32_t *status) {
+  grid_dep_launch();
+  if (blockIdx.x == 0 && threadIdx.x == 0 && status) *status = 0;
+  const uint32_t n4 = n / 4, i = blockIdx.x * HOST_COPY_THREADS + threadIdx.x;
+  if (i < n4) reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
+  if (i < n % 4) dst[n4 * 4 + i] = src[n4 * 4 + i];
+}
+__global__ void __launch_bounds__(HOST_COPY_THREADS) k_host_out(const uint32_t *src, uint32_t stride, uint32_t rows, uint32_t n, uint32_t *dst, uint32_t *count,
+                                                                uint32_t *done) {
+  grid_dep_wait();
+  for (uint32_t r = 0; r < rows; r++)
+    for (uint32_t i = threadIdx.x; i < n; i += HOST_COPY_THREADS) dst[r * n + i] = __ldcg(src + (size_t)r * stride + i);
+  if (!done) return;
+  __threadfence_system();
+  __syncthreads();
+  if (threadIdx.x == 0) *(volatile uint32_t *)done = ++*count;
+}
+
 constexpr int PRE_THREADS = 512;
 // VEC: D is a multiple of four and the rows are read and written four values at a time (16 tokens of 7168: 5 us, 18 us one by one).
 template <bool VEC>
@@ -1322,6 +1344,17 @@ cudaError_t launch_raw_matvec(int dtype, const uint8_t *w, const float *x, float
   return cudaGetLastError();
 }
 
+cudaError_t launch_host_in(const void *src, void *dst, size_t words, uint32_t *status, cudaStream_t s, int *launches) {
+  const unsigned blocks = (unsigned)((words + 4 * HOST_COPY_THREADS - 1) / (4 * HOST_COPY_THREADS));
+  k_host_in<<<blocks ? blocks : 1, HOST_COPY_THREADS, 0, s>>>(static_cast<const uint32_t *>(src), static_cast<uint32_t *>(dst), (uint32_t)words, status);
+  if (launches) (*launches)++;
+  return cudaGetLastError();
+}
+cudaError_t launch_host_out(const void *src, size_t stride, size_t rows, size_t words, void *dst, uint32_t *count, uint32_t *done, cudaStream_t s, int *launches) {
+  if (launches) (*launches)++;
+  return launch_overlapped(k_host_out, dim3(1), HOST_COPY_THREADS, 0, s, false, static_cast<const uint32_t *>(src), (uint32_t)stride, (uint32_t)rows,
+                           (uint32_t)words, static_cast<uint32_t *>(dst), count, done);
+}
 cudaError_t launch_f16_to_f32(const uint16_t *src, float *dst, size_t n, cudaStream_t s) {
   k_f16_to_f32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(src, dst, n);
   return cudaGetLastError();

@@ -89,6 +89,7 @@ struct mer_backend {
   float *h_rows = nullptr;     // pinned rows in, then rows out, rows_floats each (allocated on the first call that needs it)
   size_t rows_floats = 0;
   uint32_t *h_route = nullptr;  // pinned [3 x max_pairs]: routing, mixing weights, status
+  uint32_t *h_done = nullptr, *d_done_count = nullptr;  // pinned word that the last kernel of a small host call changes; its source
   float *d_dequant = nullptr;
   bool packed = false;          // slots hold the tile-major fragment layout (block-aligned shapes)
   uint8_t *d_raw_stage = nullptr;  // device copy of one flat blob, source of the repack at admission
@@ -464,7 +465,7 @@ void free_all(mer_backend *b) {
   F(b->arena), F(b->d_expert_ptr), F(b->d_x), F(b->d_out), F(b->d_h), F(b->d_y), F(b->d_logits), F(b->d_step);
   F(b->d_pair_expert), F(b->d_group_expert), F(b->d_offsets), F(b->d_perm), F(b->d_counters), F(b->d_group_count);
   F(b->d_f16), F(b->d_stream_scratch), F(b->d_gemm_scratch), F(b->d_dequant), F(b->d_raw_stage), F(b->d_xn), F(b->d_shared_scale);
-  H(b->h_stage), H(b->h_u32), H(b->h_f32), H(b->h_step), H(b->h_rows), H(b->h_route);
+  H(b->h_stage), H(b->h_u32), H(b->h_f32), H(b->h_step), H(b->h_rows), H(b->h_route), H(b->h_done), F(b->d_done_count);
   if (b->ev_compute_done) cudaEventDestroy(b->ev_compute_done);
   if (b->ev_copy_done) cudaEventDestroy(b->ev_copy_done);
   for (auto &e : b->ev_stage)
@@ -717,12 +718,44 @@ int dispatch_given_routing(mer_backend *b, uint32_t layer, MoeDispatch &d, const
   return run_given_routing(b, layer, expert, d, n_pairs, single_group, launches, combine_follows);
 }
 
-// Routing, mixing weights and status word of `pairs` pairs into h_route, [3][pairs], in one copy.
-int enqueue_routing_readback(mer_backend *b, uint32_t layer, size_t pairs) {
+constexpr size_t SMALL_COPY = 64u << 10;  // bytes up to which kernels move a host call's data (16 KB: 2 us, a copy node 5)
+
+// Pinned bytes (whole words) to the device; clears the status word if `clear_status`.
+int enqueue_upload(mer_backend *b, uint32_t layer, void *dst, const void *pinned, size_t bytes, bool clear_status, int *launches) {
   const uint32_t expert = MER_NONE;
-  CU(MER_ERR_READBACK_MAP, "cudaMemcpy2DAsync(routing)",
-     cudaMemcpy2DAsync(b->h_route, pairs * 4, b->d_pair_expert, (size_t)b->max_pairs * 4, pairs * 4, 3, cudaMemcpyDeviceToHost, b->compute));
+  if (bytes <= SMALL_COPY) {
+    CU(MER_ERR_SUBMISSION, "upload kernel", launch_host_in(pinned, dst, bytes / 4, clear_status ? b->d_status : nullptr, b->compute, launches));
+    return MER_OK;
+  }
+  CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(dst, pinned, bytes, cudaMemcpyHostToDevice, b->compute));
+  if (clear_status) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, b->compute));
   return MER_OK;
+}
+// Rows of `words` words to pinned memory, packed.  The `last` step of a call, if small, changes h_done when all is there.
+int enqueue_download(mer_backend *b, uint32_t layer, void *pinned, const void *src, size_t stride, size_t rows, size_t words, bool last, int *launches) {
+  const uint32_t expert = MER_NONE;
+  if (rows * words * 4 <= SMALL_COPY)
+    CU(MER_ERR_READBACK_MAP, "read-back kernel",
+       launch_host_out(src, stride, rows, words, pinned, b->d_done_count, last ? b->h_done : nullptr, b->compute, launches));
+  else
+    CU(MER_ERR_READBACK_MAP, "cudaMemcpy2DAsync(read-back)",
+       cudaMemcpy2DAsync(pinned, words * 4, src, stride * 4, words * 4, rows, cudaMemcpyDeviceToHost, b->compute));
+  return MER_OK;
+}
+// Routing, mixing weights and status word of `pairs` pairs into h_route, [3][pairs].
+int enqueue_routing_readback(mer_backend *b, uint32_t layer, size_t pairs, int *launches) {
+  return enqueue_download(b, layer, b->h_route, b->d_pair_expert, b->max_pairs, 3, pairs, true, launches);
+}
+// Waits for a call whose last step is enqueue_download(last): for h_done to leave `before`, polling while that is
+// shorter than a synchronisation's own 5 to 10 us of wake-up, else (large data, a long call, an error) for the stream.
+cudaError_t wait_for_download(mer_backend *b, uint32_t before) {
+  for (int i = 0; i < 200000; i++) {  // a few milliseconds
+    if (__atomic_load_n(b->h_done, __ATOMIC_ACQUIRE) != before) return cudaSuccess;
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+  }
+  return cudaStreamSynchronize(b->compute);
 }
 // h_route -> the caller's [n_tokens x top_k] arrays (either may be null): routed columns, local ids.
 void unpack_routing(const mer_backend *b, const RouterDev &r, uint32_t slots, size_t n_tokens, uint32_t *ids, float *weights) {
@@ -776,12 +809,13 @@ void copy_host(mer_backend *b, void *dst, const void *src, size_t n) {
   if (b->copy_pool) b->copy_pool->finish();
 }
 
-// `status`: where a copy that is already enqueued leaves the status word (null: read it back here).
-int finish_host_call(mer_backend *b, uint32_t layer, uint32_t expert, int launches, size_t n_experts_run, const uint32_t *status = nullptr) {
+// `polled`: the call ends in a small read-back, h_done was `done_before` in front of it.  `status`: where a copy that is already enqueued leaves the status word (null: read it back here).
+int finish_host_call(mer_backend *b, uint32_t layer, uint32_t expert, int launches, size_t n_experts_run, const uint32_t *status = nullptr,
+                     bool polled = false, uint32_t done_before = 0) {
   if (!status)
     CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)",
        cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, b->compute));
-  CU(MER_ERR_READBACK_MAP, "cudaStreamSynchronize", cudaStreamSynchronize(b->compute));
+  CU(MER_ERR_READBACK_MAP, "cudaStreamSynchronize", polled ? wait_for_download(b, done_before) : cudaStreamSynchronize(b->compute));
   b->ctr.kernel_launches += (uint64_t)launches;
   b->ctr.gpu_dispatch_attempts += n_experts_run;
   int rc = check_device_status(b, status ? *status : b->h_u32[b->max_pairs], layer, expert);
@@ -906,6 +940,10 @@ MER_EXPORT int mer_backend_create(const mer_backend_cfg *cfg, mer_backend **out)
   CB(cudaHostAlloc((void **)&b->h_u32, (P + 1) * 4, cudaHostAllocDefault));
   CB(cudaHostAlloc((void **)&b->h_f32, P * 4, cudaHostAllocDefault));
   CB(cudaHostAlloc((void **)&b->h_route, 3 * P * 4, cudaHostAllocDefault));
+  CB(cudaHostAlloc((void **)&b->h_done, 64, cudaHostAllocDefault));
+  *b->h_done = 0;
+  CB(cudaMalloc((void **)&b->d_done_count, 4));
+  CB(cudaMemset(b->d_done_count, 0, 4));
   b->step_words = (D + 2 * cfg->max_top_k + 1 + 63) / 64 * 64;
   CB(cudaMalloc((void **)&b->d_step, 2 * b->step_words * 4));
   CB(cudaHostAlloc((void **)&b->h_step, 2 * b->step_words * 4, cudaHostAllocDefault));
@@ -1265,7 +1303,7 @@ MER_EXPORT int mer_layer_install(mer_backend *b, uint32_t layer, const mer_layer
 namespace {
 // Enqueues router (+ optional FFN + combine) for device-resident x on stream s.
 int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens, float *d_out, bool run_ffn_too,
-                  cudaStream_t s, int *launches, MoeDispatch *out_d, bool capturing = false) {
+                  cudaStream_t s, int *launches, MoeDispatch *out_d, bool capturing = false, bool status_cleared = false) {
   const uint32_t expert = MER_NONE;
   auto it = b->routers.find(layer);
   if (it == b->routers.end()) return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "no router installed for layer %u", layer);
@@ -1281,7 +1319,7 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   if (run_ffn_too) bind_ffn(b, d);
   d.x = d_x;
   d.out = d_out;
-  if (!run_ffn_too || !router_sets_status(d)) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
+  if (!status_cleared && (!run_ffn_too || !router_sets_status(d))) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
   if (!capturing) CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
   cudaEvent_t *ev = (run_ffn_too && !capturing) ? next_timing_set(b) : nullptr;
   if (ev) cudaEventRecord(ev[0], s);
@@ -1334,13 +1372,15 @@ MER_EXPORT int mer_router_route(mer_backend *b, uint32_t layer, const float *x, 
         b, key,
         [&](int *n) -> int {
           MoeDispatch d;
-          CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
-          const int e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, n, &d, true);
-          return e ? e : enqueue_routing_readback(b, layer, P);
+          int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, true, n);
+          if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, n, &d, true, true);
+          return e ? e : enqueue_routing_readback(b, layer, P, n);
         },
         &hit);
     if (rc) return rc;
   }
+  const uint32_t done_before = *b->h_done;
+  const bool polled = 3 * P * 4 <= SMALL_COPY;
   if (hit) {
     copy_host(b, b->h_rows, x, bytes);
     CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
@@ -1349,10 +1389,10 @@ MER_EXPORT int mer_router_route(mer_backend *b, uint32_t layer, const float *x, 
     CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, bytes, cudaMemcpyHostToDevice, b->compute));
     MoeDispatch d;
     rc = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, &launches, &d);
-    if (rc == MER_OK) rc = enqueue_routing_readback(b, layer, P);
+    if (rc == MER_OK) rc = enqueue_routing_readback(b, layer, P, &launches);
     if (rc) return rc;
   }
-  rc = finish_host_call(b, layer, expert, launches, 0, b->h_route + 2 * P);
+  rc = finish_host_call(b, layer, expert, launches, 0, b->h_route + 2 * P, polled, done_before);
   // ids / weights on the device are [n_tokens x slots]; the caller gets the top_k routed columns with local ids
   unpack_routing(b, r, slots, n_tokens, ids, weights);
   b->ctr.hidden_upload_bytes += n_tokens * b->cfg.d_model * 4;
@@ -1458,7 +1498,8 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
   memcpy(b->h_step + D, expert_ids, n_slots * 4);
   memcpy(b->h_step + D + n_slots, weights, n_slots * 4);
   auto enqueue = [&](int *n) -> int {
-    CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_step, b->h_step, (D + 2 * n_slots) * 4, cudaMemcpyHostToDevice, b->compute));
+    int e = enqueue_upload(b, layer, b->d_step, b->h_step, (D + 2 * n_slots) * 4, false, n);
+    if (e) return e;
     MoeDispatch d = base_dispatch(b);
     d.n_tokens = 1;
     d.slots = (uint32_t)n_slots;
@@ -1467,13 +1508,11 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
     d.pair_weight = b->d_step + D + n_slots;
     d.out = b->d_step + b->step_words;
     d.status = reinterpret_cast<uint32_t *>(b->d_step + b->step_words + D);
-    const int e = run_given_routing(b, layer, expert, d, n_slots, false, n, true);
-    if (e) return e;
+    if ((e = run_given_routing(b, layer, expert, d, n_slots, false, n, true)) != MER_OK) return e;
     CU(MER_ERR_SUBMISSION, "combine kernel", launch_combine(d, b->compute, n));
-    CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)",
-       cudaMemcpyAsync(b->h_step + b->step_words, b->d_step + b->step_words, (D + 1) * 4, cudaMemcpyDeviceToHost, b->compute));
-    return MER_OK;
+    return enqueue_download(b, layer, b->h_step + b->step_words, b->d_step + b->step_words, D + 1, 1, D + 1, true, n);
   };
+  const uint32_t done_before = *b->h_done;
   CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
   int launches = 0;
   mer_backend::GraphEntry *hit = nullptr;
@@ -1488,7 +1527,7 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
   b->ctr.batch_calls += 1;
   b->ctr.hidden_upload_bytes += D * 4;
   b->ctr.readback_bytes += D * 4;
-  rc = finish_host_call(b, layer, expert, launches, n_slots, h_status);
+  rc = finish_host_call(b, layer, expert, launches, n_slots, h_status, (D + 1) * 4 <= SMALL_COPY, done_before);
   memcpy(out, b->h_step + b->step_words, D * 4);
   return rc;
 }
@@ -1561,19 +1600,19 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
         b, key,
         [&](int *n) -> int {
           MoeDispatch d;
-          CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, b->h_rows, bytes, cudaMemcpyHostToDevice, b->compute));
-          const int e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, b->compute, n, &d, true);
-          if (e) return e;
-          CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(h_out, b->d_out, bytes, cudaMemcpyDeviceToHost, b->compute));
-          return enqueue_routing_readback(b, layer, P);
+          int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, false, n);
+          if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, b->compute, n, &d, true);
+          if (!e) e = enqueue_download(b, layer, h_out, b->d_out, bytes / 4, 1, bytes / 4, false, n);
+          return e ? e : enqueue_routing_readback(b, layer, P, n);
         },
         &hit);
     if (rc) return rc;
     if (hit) {
+      const uint32_t done_before = *b->h_done;
       copy_host(b, b->h_rows, x, bytes);
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
       b->ctr.selected_routed_experts += P;
-      rc = finish_host_call(b, layer, expert, hit->launches, P, b->h_route + 2 * P);
+      rc = finish_host_call(b, layer, expert, hit->launches, P, b->h_route + 2 * P, 3 * P * 4 <= SMALL_COPY, done_before);
       copy_host(b, out, h_out, bytes);
       unpack_routing(b, r, slots, n_tokens, ids, weights);
       b->ctr.hidden_upload_bytes += bytes;
