@@ -1,0 +1,92 @@
+"""Sizes at which the dispatch changes its way of routing, grouping, multiplying or moving host data, against the CPU oracle."""
+import numpy as np
+import pytest
+
+import mer_b200
+import oracle
+
+pytestmark = pytest.mark.gpu
+synth = __import__("importlib").import_module("mer_b200.synth")
+
+FFN_TOL = 1e-3  # max-abs error relative to the RMS of the reference output
+
+
+def rel_rms_err(got, ref):
+    ref = np.asarray(ref, np.float64)
+    return float(np.max(np.abs(np.asarray(got, np.float64) - ref)) / (np.sqrt(np.mean(ref ** 2)) + 1e-30))
+
+
+def backend(dtype, D, F, n_experts, **kw):
+    stride = (256 + mer_b200.expert_bytes(dtype, D, F) + 4095) // 4096 * 4096
+    return mer_b200.Backend(dtype, D, F, stride * n_experts, n_experts, **kw)
+
+
+@pytest.mark.parametrize("E,k,B,D,F", [
+    (8, 2, 16, 64, 32), (8, 2, 17, 64, 32),        # 32 pairs are grouped in one warp, more in a block
+    (4, 1, 2048, 64, 32), (4, 1, 2049, 64, 32),    # the block's largest number of pairs
+    (512, 1, 40, 64, 32), (513, 1, 40, 64, 32),    # and of groups
+    (3, 1, 1, 1024, 32), (100, 2, 5, 1024, 32),    # one and two expert rows per router CTA
+    (16, 1, 300, 1024, 32), (17, 1, 300, 1024, 32),  # logits of a large batch: direct, in small tiles,
+    (128, 1, 1921, 512, 32),                       # in large ones
+    (2, 1, 4100, 128, 128), (130, 2, 4100, 64, 32),  # and grouped over the grid
+])
+def test_routing_and_grouping_edges(E, k, B, D, F):
+    dtype = oracle.Q8_0 if B % 2 else oracle.Q4_0
+    blobs = [synth.make_expert_blob(dtype, D, F, 91, 0, e) for e in range(E)]
+    W = synth.make_router(E, D, 91)
+    x = synth.make_activations(B, D, 91)
+    with backend(dtype, D, F, E, max_tokens=B, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, blobs[e])
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        out, ids, _ = b.moe_layer_forward(0, x)
+    ref, rids, _, _ = oracle.moe_layer_forward(dtype, oracle.LinearGate(W, E, D, k), blobs, x, F, n_threads=8)
+    same = (ids == rids).all(axis=1)  # scores within rounding of each other may swap
+    assert np.count_nonzero(~same) <= B // 1000
+    assert rel_rms_err(out[same], ref[same]) <= FFN_TOL
+
+
+@pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
+@pytest.mark.parametrize("D,F,n_tokens", [(128, 128, 1), (384, 128, 65), (128, 128, 128), (384, 256, 129), (128, 384, 257)])
+def test_gemm_pass_widths_and_odd_tile_counts(dtype, D, F, n_tokens):
+    blob = synth.make_expert_blob(dtype, D, F, 92, 0, 0)
+    x = synth.make_activations(n_tokens, D, 92)
+    with backend(dtype, D, F, 2, max_tokens=max(n_tokens, 16)) as b:
+        b.admit(1, 1, blob)
+        b.set_kernel_path(3)
+        got = b.expert_forward_f32(0, 1, x)
+    ref = np.stack([oracle.expert_forward(dtype, blob, x[t], D, F, oracle.FWD_AUTHORITATIVE) for t in range(n_tokens)])
+    assert rel_rms_err(got, ref) <= FFN_TOL
+
+
+@pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
+@pytest.mark.parametrize("D,F,n_tokens", [(32, 96, 3), (96, 544, 9), (160, 32, 8), (4128, 288, 5), (7168, 256, 12)])
+def test_streaming_remainders_of_four_blocks_and_of_sixteen_tiles(dtype, D, F, n_tokens):
+    blob = synth.make_expert_blob(dtype, D, F, 93, 0, 0)
+    x = synth.make_activations(n_tokens, D, 93) + 0.5  # block sums far from zero: the zero point's share matters
+    with backend(dtype, D, F, 2, max_tokens=n_tokens) as b:
+        b.admit(1, 1, blob)
+        b.set_kernel_path(2)
+        got = b.expert_forward_f32(0, 1, x)
+    ref = np.stack([oracle.expert_forward(dtype, blob, x[t], D, F, oracle.FWD_AUTHORITATIVE) for t in range(n_tokens)])
+    assert rel_rms_err(got, ref) <= FFN_TOL
+
+
+@pytest.mark.parametrize("B", [1, 64, 65])  # 64 rows of 256 values are moved by kernels, 65 by copies
+def test_repeated_host_calls_read_new_rows(B):
+    dtype, E, D, F, k = oracle.Q8_0, 16, 256, 64, 4
+    blobs = [synth.make_expert_blob(dtype, D, F, 94, 0, e) for e in range(E)]
+    W = synth.make_router(E, D, 94)
+    gate = oracle.LinearGate(W, E, D, k)
+    with backend(dtype, D, F, E, max_tokens=B, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, blobs[e])
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        for rep in range(5):  # plain launches, then the capture, then replays
+            x = synth.make_activations(B, D, 95 + rep)
+            ref, rids, rw, _ = oracle.moe_layer_forward(dtype, gate, blobs, x, F, n_threads=8)
+            ids, w = b.route(0, x)
+            assert (ids == rids).all() and np.allclose(w, rw, rtol=1e-5, atol=1e-7)
+            out, ids, _ = b.moe_layer_forward(0, x)
+            assert (ids == rids).all() and rel_rms_err(out, ref) <= FFN_TOL
+            assert rel_rms_err(b.moe_step_weighted_into(0, x[0], rids[0], rw[0]), ref[0]) <= FFN_TOL
