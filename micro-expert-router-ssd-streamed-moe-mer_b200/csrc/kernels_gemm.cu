@@ -1,28 +1,29 @@
 // Grouped expert FFN for token groups of a dozen tokens and more (prefill, expert-parallel decode):
-// tcgen05 tensor-core GEMM per (expert, 128 weight rows, up to 128 tokens) with TMEM accumulators.
+// tcgen05 tensor-core GEMM per (expert, 256 weight rows, up to 128 tokens) on pairs of CTAs, accumulators in TMEM.
 //
-//   D[128 weight rows x N tokens] += A[128 x 32] * B[N x 32]^T      per 32-value block of K
+//   D[256 weight rows x N tokens] += A[256 x 32] * B[N x 32]^T      per 32-value block of K
 //
+//   * Two CTAs (a cluster, cta_group::2) multiply 128 weight rows each against one B operand of which each holds half of the
+//     token rows: half the activation traffic and half the MMA instructions per weight row of single CTAs.
 //   * A never touches shared memory as an operand: the packed Q4_0 / Q8_0 tile chunks of layout.cuh
-//     are streamed global -> shared by bulk async copies, eight warps dequantise them block by block into
+//     are streamed global -> shared by bulk async copies, sixteen warps dequantise them block by block into
 //     two f16 operands, hi = f16(d*q) and lo = d*q - hi (exact: an 11-bit scale times an 8-bit integer
 //     has at most 19 significant bits), and store them straight into TENSOR MEMORY (tcgen05.st; a thread
 //     owns one weight row), from where the MMA reads its A operand.  Eight A stages live in TMEM beside
-//     the two accumulators.
-//   * B is the activation tile as f16 hi + lo parts (22 significant bits after an exact power-of-two
-//     per-row scaling), laid out in the K-major no-swizzle core-matrix order by k_gemm_act_image (per core-matrix
-//     column of K the hi pieces of the pass's rows, then the lo pieces; as wide as the pass, not as the widest one)
-//     and fetched with one bulk copy per 64 values of K, two per stage, into a two-stage shared-memory ring.
+//     the two accumulators; a block is converted before its stage is waited for.
+//   * B is the activation rows as f16 hi + lo parts (22 significant bits after an exact power-of-two
+//     per-row scaling), written once in group order by k_split_rows, so that a pass is a run of rows and one tiled copy
+//     fetches 64 values of all of them (128-byte swizzle; a tensor map per pass width).
 //   * Three products per 16 values of K (hi*hi, hi*lo, lo*hi; lo*lo is below fp32 resolution) accumulate
 //     in fp32 in TMEM, so the result matches the fp32 reference to ~1e-4 of the output RMS instead of f16's 2e-3.
-//     A group of at most 64 tokens issues them as two instructions: W_hi * [x_hi | x_lo] with twice the width
-//     (two column sets of the accumulator, added in the epilogue) and W_lo * x_hi.
-//   * Warp roles: 0 = producer of the activation stages, 1 = MMA issuer (one elected lane issues predicated
-//     instructions; every operand is computed in uniform registers) and TMEM owner,
-//     2..9 = epilogue (four warps per accumulator buffer: tcgen05.ld, un-scaling, SiLU(gate)*up or plain store; two
-//     buffers let the epilogue of one item overlap the MMAs of the next two),
-//     10..17 = dequantisers (a warp reaches the 32 TMEM lanes of its quarter; the two warps of a quarter
-//     take alternate blocks), 18 = producer of the weight stages (lanes 0..7 copy one packed tile each).
+//   * Warp roles: 0 = producer of the activation stages, 1 = MMA issuer (of the pair's first CTA; one elected lane issues
+//     predicated instructions; every operand is computed in uniform registers) and TMEM owner, 2..9 = epilogue (two groups
+//     of four, one per accumulator buffer), 10..25 = dequantisers (four per quarter of the rows, a block of every weight
+//     stage each), 26 = producer of the weight stages (lanes 0..7 copy one packed tile each).
+// What bounds it: full-width passes run the tensor pipe with the chip at its power limit (2048 tokens on 128 experts of
+// 2048 x 768: 990 W at 1.64 GHz, tensor pipe 63 % active, 345 us for gate/up against 416 us with single CTAs, two 66 KB activation stages
+// and eight dequantiser warps; 4096 tokens on 256 experts of 7168 x 2048: 5.7 ms, 6.6 ms before); passes of a few tokens are bound
+// by reading the weights and by their instructions.  Sorting the passes by width, widest first, changed neither.
 // Every wait is bounded; on expiry the CTA latches MER_DEVSTAT_TIMEOUT, stops issuing work, waits
 // (bounded) for its copies and MMAs in flight, frees its TMEM and returns.
 #include <cuda.h>
