@@ -74,57 +74,49 @@ __device__ __forceinline__ float clamp_gate(float g, float limit) {
 constexpr int ROUTER_THREADS = 256;
 constexpr int ROUTER_WARPS = ROUTER_THREADS / 32;
 constexpr int ROUTER_TT = 4;                      // tokens per CTA
+constexpr uint32_t ROUTER_CTAS = 240;             // rows per CTA are halved while there are fewer CTAs than this
 constexpr uint32_t SMALL_P = 4096;                // pair keys staged in shared memory below this many pairs
 constexpr uint32_t STABLE_G = 512;
 constexpr uint32_t GRID_GROUPING_PAIRS = 8192;    // from this many pairs the grouping runs grid-wide (count / scan / scatter)                // stable (token, slot)-ordered grouping up to this many groups
 
+// 64-bit divisions cost a few hundred cycles and much code, and this sits on the critical path of every decode layer: they are
+// kept out of line, for sizes that need them.
+__device__ __noinline__ uint32_t div64(uint64_t a, uint32_t b) { return (uint32_t)(a / b); }
+// ceil(a * b / c)
+__device__ __forceinline__ uint32_t scaled_ceil(uint32_t a, uint32_t b, uint32_t c) {
+  const uint64_t v = (uint64_t)a * b + c - 1;
+  return v <= 0xFFFFFFFFull ? (uint32_t)v / c : div64(v, c);
+}
 // ---- work split of the streaming kernels: one contiguous item range per CTA and phase.  An item of a pass with
 // more than four tokens multiplies two token tiles instead of one, which measures as ~1.3x the time: cost 13 vs 10.
 // `s_cum`: running cost before each pass and after the last, or null: all passes cost the same.  One CTA of 256 threads.
 __device__ void build_item_bounds(const MoeDispatch &d, uint32_t n_passes, const uint32_t *s_cum) {
-  const uint32_t G = d.n_ctas;
+  const uint32_t G = d.n_ctas, i0 = d.items_per_pass[0], i1 = d.items_per_pass[1];
+  const uint32_t total = s_cum ? s_cum[n_passes] : n_passes;  // at most 13 x 1024 weighted: products with G fit 32 bits
 #pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < 2 * (G + 1); i += 256) {
-    const uint32_t phase = i / (G + 1), b = i % (G + 1);
-    const uint32_t ipp = d.items_per_pass[phase];
-    const uint64_t n_items = (uint64_t)n_passes * ipp;
-    uint32_t bound;
-    if (!s_cum) {
-      bound = n_items * G <= 0xFFFFFFFFull ? (uint32_t)n_items * b / G : (uint32_t)(n_items * b / G);
-    } else if ((uint64_t)s_cum[n_passes] * ipp * G <= 0xFFFFFFFFull) {
-      // the usual case: everything fits 32 bits (64-bit divisions cost a few hundred cycles each, and this loop sits
-      // on the critical path of every decode layer)
-      const uint32_t total = s_cum[n_passes] * ipp, target = total * b / G;
-      uint32_t lo = 0, hi = n_passes;  // largest pass index with cum[pass] * ipp <= target
+  for (uint32_t b = threadIdx.x; b <= G; b += 256) {
+    uint32_t pass, b0, b1;  // first pass that is not wholly in front of the bound; items of it that are, in either phase
+    if (s_cum) {
+      const uint32_t target = total * b;
+      uint32_t lo = 0, hi = n_passes;  // largest pass index with cum[pass] * G <= target
 #pragma unroll 1
       while (lo < hi) {
         const uint32_t mid = (lo + hi + 1) >> 1;
-        if (s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
+        if (s_cum[mid] * G <= target) lo = mid; else hi = mid - 1;
       }
-      if (lo >= n_passes) {
-        bound = (uint32_t)n_items;
-      } else {
-        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
-        const uint32_t rem = target - s_cum[lo] * ipp;
-        bound = lo * ipp + min(ipp, (rem + w - 1) / w);
+      pass = lo, b0 = b1 = 0;
+      if (lo < n_passes) {
+        const uint32_t w = s_cum[lo + 1] - s_cum[lo], wg = w * G, rem = target - s_cum[lo] * G;  // rem < wg
+        b0 = scaled_ceil(rem, i0, wg), b1 = scaled_ceil(rem, i1, wg);
       }
     } else {
-      const uint64_t total = (uint64_t)s_cum[n_passes] * ipp, target = total * b / G;
-      uint32_t lo = 0, hi = n_passes;
-#pragma unroll 1
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if ((uint64_t)s_cum[mid] * ipp <= target) lo = mid; else hi = mid - 1;
-      }
-      if (lo >= n_passes) {
-        bound = (uint32_t)n_items;
-      } else {
-        const uint32_t w = s_cum[lo + 1] - s_cum[lo];
-        const uint64_t rem = target - (uint64_t)s_cum[lo] * ipp;
-        bound = lo * ipp + (uint32_t)min((uint64_t)ipp, (rem + w - 1) / w);
-      }
+      const uint64_t target = (uint64_t)total * b;
+      pass = target <= 0xFFFFFFFFull ? (uint32_t)target / G : div64(target, G);
+      const uint32_t rem = (uint32_t)(target - (uint64_t)pass * G);
+      b0 = scaled_ceil(rem, i0, G), b1 = scaled_ceil(rem, i1, G);
     }
-    d.item_bounds[phase * MER_MAX_CTAS1 + b] = bound;
+    d.item_bounds[b] = pass * i0 + b0;
+    d.item_bounds[MER_MAX_CTAS1 + b] = pass * i1 + b1;
   }
 }
 
@@ -352,7 +344,15 @@ __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
     }
   }
   __syncthreads();
-  build_item_bounds(d, s_np, weighted ? s_cum : nullptr);
+  if (weighted) return build_item_bounds(d, s_np, s_cum);
+  const uint32_t G = d.n_ctas;  // passes of equal cost
+  const uint32_t n0 = s_np * d.items_per_pass[0], n1 = s_np * d.items_per_pass[1];
+  if (threadIdx.x <= G && (uint64_t)max(n0, n1) * G <= 0xFFFFFFFFull && G < 256) {
+    d.item_bounds[threadIdx.x] = n0 * threadIdx.x / G;
+    d.item_bounds[MER_MAX_CTAS1 + threadIdx.x] = n1 * threadIdx.x / G;
+  } else if ((uint64_t)max(n0, n1) * G > 0xFFFFFFFFull || G >= 256) {
+    build_item_bounds(d, s_np, nullptr);
+  }
 }
 
 // The same for a batch of decode size (at most 2048 pairs, 512 groups): the counting atomics hand out the pairs' ranks, and
@@ -360,26 +360,26 @@ __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
 // the pairs inside a group is whatever the atomics give; every pair's result is independent of its position.  (The
 // general form: a dozen more block-wide steps, 7 us for 512 pairs of 128 groups.)
 constexpr uint32_t MID_PAIRS = 2048, MID_GROUPS = 512;
-__device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d) {
-  constexpr uint32_t PER_P = MID_PAIRS / 256, PER_G = MID_GROUPS / 256;
+// `s_pair` [P]: group (16 bits) and rank of every pair.  Loops stay rolled: the code runs once, cold.
+__device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint32_t *s_pair) {
+  constexpr uint32_t PER_G = MID_GROUPS / 256;
   __shared__ uint32_t s_cnt[MID_GROUPS], s_cum[MID_PAIRS / 8 + MID_GROUPS + 1];
   __shared__ uint64_t s_part[8];
   const uint32_t P = d.n_tokens * d.slots, G = d.n_groups, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t tpp = d.tokens_per_pass, shift = 31 - __clz(tpp);
   const bool bounds = d.item_bounds != nullptr;
-  uint32_t key[PER_P], rank[PER_P];
-#pragma unroll
-  for (uint32_t i = 0; i < PER_P; i++) key[i] = tid + i * 256 < P ? __ldcg(d.pair_expert + tid + i * 256) : MER_NONE;
-#pragma unroll
-  for (uint32_t i = 0; i < PER_G; i++) s_cnt[tid + i * 256] = 0;
+  for (uint32_t i = tid; i < MID_GROUPS; i += 256) s_cnt[i] = 0;
   __syncthreads();
-#pragma unroll
-  for (uint32_t i = 0; i < PER_P; i++) {
-    const uint32_t p = tid + i * 256;
-    if (p < P) d.amax[p] = 0;
-    if (key[i] == MER_NONE) continue;
-    key[i] = p % d.slots >= r.top_k || key[i] == r.shared_expert_id ? r.num_experts : key[i] - r.id_base;
-    rank[i] = atomicAdd(&s_cnt[key[i]], 1u);
+#pragma unroll 1
+  for (uint32_t p = tid; p < P; p += 256) {
+    d.amax[p] = 0;
+    const uint32_t eid = __ldcg(d.pair_expert + p);
+    uint32_t v = MER_NONE;
+    if (eid != MER_NONE) {
+      const uint32_t key = eid == r.shared_expert_id || p % d.slots >= r.top_k ? r.num_experts : eid - r.id_base;
+      v = key << 16 | atomicAdd(&s_cnt[key], 1u);
+    }
+    s_pair[p] = v;
   }
   __syncthreads();
   // packed: pairs (20 bits), passes (20 bits), cost; thread t owns groups t * PER_G ..
@@ -431,9 +431,11 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d) {
     if (bounds) s_cum[n_passes] = (uint32_t)(total >> 40);
   }
   __syncthreads();
-#pragma unroll
-  for (uint32_t i = 0; i < PER_P; i++)
-    if (key[i] != MER_NONE) d.perm[s_cnt[key[i]] + rank[i]] = tid + i * 256;
+#pragma unroll 1
+  for (uint32_t p = tid; p < P; p += 256) {
+    const uint32_t v = s_pair[p];
+    if (v != MER_NONE) d.perm[s_cnt[v >> 16] + (v & 0xFFFF)] = p;
+  }
   if (bounds) build_item_bounds(d, n_passes, tpp == 8 ? s_cum : nullptr);
 }
 
@@ -441,7 +443,7 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d) {
 __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uint32_t *s_u32) {
   const uint32_t P = d.n_tokens * d.slots;
   if (P <= 32 && d.item_bounds) return build_groups_small(r, d);
-  if (P <= MID_PAIRS && d.n_groups <= MID_GROUPS && d.pass_group) return build_groups_mid(r, d);
+  if (P <= MID_PAIRS && d.n_groups <= MID_GROUPS && d.pass_group) return build_groups_mid(r, d, s_u32);
   const uint32_t G = d.n_groups;
   const uint32_t tid = threadIdx.x, nt = blockDim.x, warp = tid >> 5, lane = tid & 31;
   uint32_t *s_off = s_u32;                    // [G + 1]
@@ -1218,7 +1220,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   // (one token, 128 experts of 2048: 13.4 us with a row per CTA, 16.6 us with eight).
   const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
   uint32_t rows = 8;
-  while (!tiled && rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < 120) rows >>= 1;
+  while (!tiled && rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
   const dim3 grid(tiled ? 1 : (E + rows - 1) / rows, tiles);
   const bool grid_grouping = group && P >= GRID_GROUPING_PAIRS && d.group_count != nullptr;
   auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
