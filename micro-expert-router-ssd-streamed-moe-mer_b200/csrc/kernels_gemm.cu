@@ -709,7 +709,7 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
   const uint64_t P = (uint64_t)d.n_tokens * d.slots;
   const uint32_t groups = d.active_groups_hint ? d.active_groups_hint : 1;
   const uint64_t mean = (d.expected_pairs ? d.expected_pairs : P) / groups;
-  return mean < min_mean_tokens ? 0 : PASS_TOKENS;
+  return mean < min_mean_tokens || P > d.scratch_pairs ? 0 : PASS_TOKENS;
 }
 
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) {
