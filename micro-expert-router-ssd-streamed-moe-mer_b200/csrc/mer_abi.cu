@@ -359,8 +359,9 @@ constexpr uintptr_t TAG_HOST_LAYER = 1, TAG_EP = 2, TAG_ROUTE = 3, TAG_STEP = 4,
 bool graphs_usable(const mer_backend *b) { return b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS); }
 
 // Whether the call `key` is to be replayed from a graph.  Capturing costs 0.1 to 0.3 ms and a replay saves 10 to 30 us, so a
-// call is captured at its third occurrence; rows of ever new addresses or lengths never are.
-bool replays(mer_backend *b, const mer_backend::GraphEntry &key) {
+// call is captured at its third occurrence; rows of ever new addresses or lengths never are.  (`from` = 1: pinned and
+// exchange buffers, which programs keep, at the first.)
+bool replays(mer_backend *b, const mer_backend::GraphEntry &key, int from = 3) {
   constexpr size_t CALLS = 1024;
   if (!graphs_usable(b)) return false;
   for (auto &g : b->graphs)
@@ -371,7 +372,7 @@ bool replays(mer_backend *b, const mer_backend::GraphEntry &key) {
     h = (h ^ v) * 0x9e3779b97f4a7c15ull, h ^= h >> 29;
   auto &seen = b->graph_calls[h % CALLS];
   if (!seen.same_call(key)) seen = key;
-  return ++seen.launches >= 3;
+  return ++seen.launches >= from;
 }
 
 // The captured launch sequence of `key` (which replays()), captured now on the backend's own stream if need be
@@ -1544,13 +1545,16 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
   const size_t D = b->cfg.d_model;
   // Pinned host buffers and no routing wanted back: upload, layer, read-back and the status word are captured once
   // per (layer, n_tokens, x, out) and replayed as one graph launch (the call stays synchronous).
-  if (!ids && !weights && graphs_usable(b) && b->routers.count(layer)) {
+  bool pinned = false;
+  if (((!ids && !weights) || n_tokens * D * 4 > SMALL_COPY) && graphs_usable(b) && b->routers.count(layer)) {
     cudaPointerAttributes ax{}, ao{};
-    const bool pinned = cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost &&
-                        cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost;
+    pinned = cudaPointerGetAttributes(&ax, x) == cudaSuccess && ax.type == cudaMemoryTypeHost &&
+             cudaPointerGetAttributes(&ao, out) == cudaSuccess && ao.type == cudaMemoryTypeHost;
     cudaGetLastError();
+  }
+  if (pinned && !ids && !weights) {
     const mer_backend::GraphEntry key{layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr, nullptr, 0};
-    if (pinned && replays(b, key)) {
+    if (replays(b, key, 1)) {
       cudaStream_t s = b->compute;
       CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
       mer_backend::GraphEntry *hit = nullptr;
@@ -1588,7 +1592,8 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
     }
   }
   const mer_backend::GraphEntry key{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr, nullptr, 0};
-  if (b->routers.count(layer) && replays(b, key) && stage_rows(b, n_tokens * D * 4)) {
+  // (pinned rows of some size go up and down directly: staging them would only add a copy)
+  if (b->routers.count(layer) && !(pinned && n_tokens * D * 4 > SMALL_COPY) && replays(b, key) && stage_rows(b, n_tokens * D * 4)) {
     // ordinary host memory: rows through pinned memory, the sequence (routing included) captured per (layer, n_tokens)
     const RouterDev &r = b->routers[layer].dev;
     const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
@@ -2100,7 +2105,7 @@ int ep_layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *
   int launches = 0;
   bool replayed = false;
   const mer_backend::GraphEntry key{layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr, nullptr, 0};
-  if (b->ep_on && b->ep_attached && !caller_captures(s) && replays(b, key)) {
+  if (b->ep_on && b->ep_attached && !caller_captures(s) && replays(b, key, 1)) {
     CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
     mer_backend::GraphEntry *hit = nullptr;
