@@ -25,6 +25,12 @@
 // takes a contiguous item range and rebuilds activation fragments only when its (pass, K split)
 // changes; no atomics on data, no inter-CTA waits.  Every mbarrier wait is bounded: on expiry the
 // warp stops computing, the CTA latches MER_DEVSTAT_TIMEOUT, drains its copies in flight and returns.
+//
+// What bounds it: the consumers' instructions.  Weights are waited for a tenth of the time; a block of 16 rows takes a warp about
+// 30 instructions (40 with the zero point as every block's accumulator start) at one issue in two cycles of a scheduler's four
+// warps, 38 GB/s per SM of the 44 that HBM gives.  Around the multiplication: first fragments 3 to 5 us, a rebuild 3, the grid
+// barrier 1.5 and its tail 0.5 to 4.  Measured, gate/up and down together: 64 tokens on 128 experts of 2048 x 768 (Q8_0) 172 -> 154 us;
+// 16 tokens on 8 of 4096 x 14336 (Q4_0) 285 -> 229; 16 on 256 of 7168 x 2048 589 -> 490; 1 on 8 of 4096 x 14336 76 -> 69.
 #include "kernels.h"
 
 #include <cuda_fp16.h>
