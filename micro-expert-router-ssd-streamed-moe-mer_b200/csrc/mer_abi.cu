@@ -134,15 +134,12 @@ struct mer_backend {
   bool graphs_ok = true;
   // Streams other than `compute` that device entry points were last enqueued on, each with an event recorded after
   // the call: an admission or a retire makes the copy stream wait for all of them before it touches a slot.
-  // The legacy default stream is never destroyed: its event is recorded when an admission needs it, not on every call.
   struct UserStream {
     cudaStream_t stream;
     cudaEvent_t done;
     uint64_t last_use;
   };
   std::vector<UserStream> user_streams;
-  cudaEvent_t ev_legacy = nullptr;
-  bool legacy_used = false;
   // stage timing: sets of 5 events {start, after router, mid FFN, after FFN, after combine}
   bool timing_on = false;
   std::vector<cudaEvent_t> timing_events;
@@ -220,13 +217,10 @@ cudaError_t order_after_copies(mer_backend *b, cudaStream_t s) {
 
 constexpr size_t MAX_USER_STREAMS = 8;
 
-// Records that work reading the slot arena was just enqueued on caller stream `s`.
+// Records that work reading the slot arena was just enqueued on caller stream `s`: behind the call itself, so that an admission
+// waits for the layer and not for whatever else the caller has put on the stream since.
 cudaError_t note_stream_use(mer_backend *b, cudaStream_t s) {
   if (s == b->compute) return cudaSuccess;  // ordered through ev_compute_done
-  if (s == nullptr || s == cudaStreamLegacy) {
-    b->legacy_used = true;
-    return cudaSuccess;
-  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -263,12 +257,6 @@ cudaError_t copy_waits_for_readers(mer_backend *b) {
   if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, b->ev_compute_done, 0);
   for (auto &u : b->user_streams)
     if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, u.done, 0);
-  if (e == cudaSuccess && b->legacy_used) {
-    if (!b->ev_legacy) e = cudaEventCreateWithFlags(&b->ev_legacy, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventRecord(b->ev_legacy, cudaStreamLegacy);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(b->copy, b->ev_legacy, 0);
-    b->legacy_used = false;
-  }
   return e;
 }
 
@@ -477,7 +465,6 @@ void free_all(mer_backend *b) {
   b->timing_events.clear();
   for (auto &u : b->user_streams) cudaEventDestroy(u.done);
   b->user_streams.clear();
-  if (b->ev_legacy) cudaEventDestroy(b->ev_legacy);
   for (auto &a : b->aslots) {
     F(a.d_x), F(a.d_out), F(a.d_status), H(a.h_status);
     if (a.ev_in) cudaEventDestroy(a.ev_in);

@@ -144,3 +144,35 @@ def test_admission_waits_for_a_layer_on_a_caller_stream():
         b.synchronize()
         for o in outs:
             assert rel_rms_err(o.cpu().numpy(), ref) <= 1e-3
+
+
+def test_admission_does_not_wait_for_work_enqueued_on_the_default_stream_behind_the_layer():
+    # a layer on the legacy default stream, then something long on it that reads no slot (a model's next layers): the
+    # upload is ordered after the layer alone
+    torch = pytest.importorskip("torch")
+    dtype, E, D, F, k, B = oracle.Q8_0, 4, 512, 512, 2, 8
+    blobs = [synth.make_expert_blob(dtype, D, F, 65, 0, e) for e in range(E)]
+    other = synth.make_expert_blob(dtype, D, F, 65, 1, 0)
+    W = synth.make_router(E, D, 65)
+    x = synth.make_activations(B, D, 65)
+    ref = oracle.moe_layer_forward(dtype, oracle.LinearGate(W, E, D, k), blobs, x, F)[0]
+    with make_backend(dtype, D, F, slots=E, max_tokens=B, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, blobs[e])
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        xd = torch.from_numpy(x).cuda()
+        out = torch.empty(B, D, device="cuda")
+        behind = torch.cuda.Event()
+        torch.cuda._sleep(1000)  # loads its kernel
+        for _ in range(4):  # plain launches, the capture, a replay
+            b.moe_layer_forward_device(0, xd.data_ptr(), B, out.data_ptr(), 0)
+        torch.cuda.synchronize()
+        b.moe_layer_forward_device(0, xd.data_ptr(), B, out.data_ptr(), 0)
+        torch.cuda._sleep(1_000_000_000)  # half a second
+        behind.record()
+        for e in range(E):
+            b.admit(e, 2, other)  # returns when the payload is in its slot
+        overlapped = not behind.query()
+        torch.cuda.synchronize()
+        assert overlapped, "the uploads waited for work behind the layer"
+        assert rel_rms_err(out.cpu().numpy(), ref) <= 1e-3
