@@ -20,6 +20,7 @@
 #include "../../include/mer_b200.h"
 #include "copy_pool.h"
 #include "kernels.h"
+#include "replay_table.h"
 
 #define MER_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -118,19 +119,7 @@ struct mer_backend {
   uint16_t *d_ep_owner = nullptr;       // placement table [max_experts] (mer_ep_set_placement), device copy
   std::vector<uint16_t> ep_owner_host;  // and host copy; empty = the contiguous rule
   void *ep_opened[MER_EP_MAX_WORLD] = {};  // mappings opened from IPC handles (closed at destroy)
-  // captured launch sequences of mer_moe_layer_forward_device, replayed with one cudaGraphLaunch
-  struct GraphEntry {
-    uint32_t layer;
-    size_t n_tokens;
-    const void *x, *out, *ids, *w;  // the buffers a caller passed, or a tag in `ids` for the other entry points
-    cudaGraphExec_t exec;
-    int launches;
-    bool same_call(const GraphEntry &o) const {
-      return layer == o.layer && n_tokens == o.n_tokens && x == o.x && out == o.out && ids == o.ids && w == o.w;
-    }
-  };
-  std::vector<GraphEntry> graphs;
-  std::vector<GraphEntry> graph_calls;  // calls seen lately and not captured yet, by hash; `launches` counts them
+  ReplayTable<cudaGraphExec_t> graphs;  // captured launch sequences, replayed with one cudaGraphLaunch
   bool graphs_ok = true;
   // Streams other than `compute` that device entry points were last enqueued on, each with an event recorded after
   // the call: an admission or a retire makes the copy stream wait for all of them before it touches a slot.
@@ -333,11 +322,13 @@ void drain_timing(mer_backend *b) {
   b->timing_used = 0;
 }
 
+using GraphCall = ReplayTable<cudaGraphExec_t>::Call;
+void destroy_graph(cudaGraphExec_t g) { cudaGraphExecDestroy(g); }  // one in flight is freed when it has run
+
 void drop_graphs(mer_backend *b) {
-  if (b->graphs.empty()) return;
+  if (b->graphs.graphs() == 0) return;
   cudaDeviceSynchronize();
-  for (auto &g : b->graphs) cudaGraphExecDestroy(g.exec);
-  b->graphs.clear();
+  b->graphs.drop(destroy_graph);
 }
 
 // Tags of captured sequences that are not mer_moe_layer_forward_device's.
@@ -346,53 +337,35 @@ constexpr uintptr_t TAG_HOST_LAYER = 1, TAG_EP = 2, TAG_ROUTE = 3, TAG_STEP = 4,
 
 bool graphs_usable(const mer_backend *b) { return b->graphs_ok && !b->timing_on && !(b->cfg.flags & MER_FLAG_NO_GRAPHS); }
 
-// Whether the call `key` is to be replayed from a graph.  Capturing costs 0.1 to 0.3 ms and a replay saves 10 to 30 us, so a
-// call is captured at its third occurrence; rows of ever new addresses or lengths never are.  (`from` = 1: pinned and
-// exchange buffers, which programs keep, at the first.)
-bool replays(mer_backend *b, const mer_backend::GraphEntry &key, int from = 3) {
-  constexpr size_t CALLS = 1024;
-  if (!graphs_usable(b)) return false;
-  for (auto &g : b->graphs)
-    if (g.same_call(key)) return true;
-  if (b->graph_calls.empty()) b->graph_calls.resize(CALLS, {MER_NONE, 0, nullptr, nullptr, nullptr, nullptr, nullptr, 0});
-  uint64_t h = key.layer;
-  for (const uint64_t v : {(uint64_t)key.n_tokens, (uint64_t)key.x, (uint64_t)key.out, (uint64_t)key.ids, (uint64_t)key.w})
-    h = (h ^ v) * 0x9e3779b97f4a7c15ull, h ^= h >> 29;
-  auto &seen = b->graph_calls[h % CALLS];
-  if (!seen.same_call(key)) seen = key;
-  return ++seen.launches >= from;
+// The call `key`, if it is to be replayed from a graph.  (`from` = 1: pinned and exchange buffers, which programs keep, at the
+// first occurrence.)
+GraphCall *replays(mer_backend *b, const CallKey &key, uint32_t from = 3) {
+  return graphs_usable(b) ? b->graphs.occurrence(key, from) : nullptr;
 }
 
-// The captured launch sequence of `key` (which replays()), captured now on the backend's own stream if need be
-// (`enqueue(&launches)` issues it there); *out stays null where capture is not to be had.  A graph is launched into whatever
+// Captures the launch sequence of a call that replays(), if that has not happened yet, on the backend's own stream
+// (`enqueue(&launches)` issues it there); call->exec stays null where capture is not to be had.  A graph is launched into whatever
 // stream the caller brings, the legacy default stream included, which itself cannot be captured.
 template <typename Enqueue>
-int captured_graph(mer_backend *b, mer_backend::GraphEntry key, Enqueue enqueue, mer_backend::GraphEntry **out) {
-  *out = nullptr;
-  for (auto &g : b->graphs)
-    if (g.same_call(key)) {
-      *out = &g;
-      return MER_OK;
-    }
-  if (b->graphs.size() >= 256) drop_graphs(b);
+int capture_once(mer_backend *b, GraphCall *call, Enqueue enqueue) {
+  if (call->exec) return MER_OK;
   cudaGraph_t graph = nullptr;
-  int rc = MER_OK;
+  cudaGraphExec_t exec = nullptr;
+  int rc = MER_OK, launches = 0;
   bool ok = cudaStreamBeginCapture(b->compute, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
   if (ok) {
-    rc = enqueue(&key.launches);
+    rc = enqueue(&launches);
     const cudaError_t ce = cudaStreamEndCapture(b->compute, &graph);
     ok = ce == cudaSuccess && graph != nullptr;
   }
-  if (rc == MER_OK && ok) ok = cudaGraphInstantiate(&key.exec, graph, 0) == cudaSuccess;
+  if (rc == MER_OK && ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
   if (graph) cudaGraphDestroy(graph);
   if (rc != MER_OK || !ok) cudaGetLastError();
   if (rc != MER_OK) return rc;
-  if (!ok) {
+  if (ok)
+    b->graphs.captured(call, exec, launches, destroy_graph);
+  else
     b->graphs_ok = false;  // plain launches from now on
-    return MER_OK;
-  }
-  b->graphs.push_back(key);
-  *out = &b->graphs.back();
   return MER_OK;
 }
 // Whether the caller is capturing `s` into a graph of its own: then plain launches, which become part of it.
@@ -459,8 +432,7 @@ void free_all(mer_backend *b) {
   if (b->ev_copy_done) cudaEventDestroy(b->ev_copy_done);
   for (auto &e : b->ev_stage)
     if (e) cudaEventDestroy(e);
-  for (auto &g : b->graphs) cudaGraphExecDestroy(g.exec);
-  b->graphs.clear();
+  b->graphs.drop(destroy_graph);
   for (auto &e : b->timing_events) cudaEventDestroy(e);
   b->timing_events.clear();
   for (auto &u : b->user_streams) cudaEventDestroy(u.done);
@@ -1352,24 +1324,20 @@ MER_EXPORT int mer_router_route(mer_backend *b, uint32_t layer, const float *x, 
   const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
   const size_t P = n_tokens * slots, bytes = n_tokens * b->cfg.d_model * 4;
   int rc, launches = 0;
-  mer_backend::GraphEntry *hit = nullptr;
-  const mer_backend::GraphEntry key{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_ROUTE), nullptr, nullptr, 0};
-  if (replays(b, key) && stage_rows(b, bytes)) {
+  GraphCall *hit = replays(b, CallKey{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_ROUTE), nullptr});
+  if (hit && stage_rows(b, bytes)) {
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
-    rc = captured_graph(
-        b, key,
-        [&](int *n) -> int {
-          MoeDispatch d;
-          int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, true, n);
-          if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, n, &d, true, true);
-          return e ? e : enqueue_routing_readback(b, layer, P, n);
-        },
-        &hit);
+    rc = capture_once(b, hit, [&](int *n) -> int {
+      MoeDispatch d;
+      int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, true, n);
+      if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, false, b->compute, n, &d, true, true);
+      return e ? e : enqueue_routing_readback(b, layer, P, n);
+    });
     if (rc) return rc;
   }
   const uint32_t done_before = *b->h_done;
   const bool polled = 3 * P * 4 <= SMALL_COPY;
-  if (hit) {
+  if (hit && hit->exec) {
     copy_host(b, b->h_rows, x, bytes);
     CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
     launches = hit->launches;
@@ -1503,10 +1471,9 @@ MER_EXPORT int mer_moe_step_weighted_into(mer_backend *b, uint32_t layer, const 
   const uint32_t done_before = *b->h_done;
   CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
   int launches = 0;
-  mer_backend::GraphEntry *hit = nullptr;
-  const mer_backend::GraphEntry key{0, n_slots, nullptr, nullptr, graph_tag(TAG_STEP), nullptr, nullptr, 0};
-  if (replays(b, key) && (rc = captured_graph(b, key, enqueue, &hit)) != MER_OK) return rc;
-  if (hit) {
+  GraphCall *hit = replays(b, CallKey{0, n_slots, nullptr, nullptr, graph_tag(TAG_STEP), nullptr});
+  if (hit && (rc = capture_once(b, hit, enqueue)) != MER_OK) return rc;
+  if (hit && hit->exec) {
     CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
     launches = hit->launches;
   } else if ((rc = enqueue(&launches)) != MER_OK) {
@@ -1540,25 +1507,20 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
     cudaGetLastError();
   }
   if (pinned && !ids && !weights) {
-    const mer_backend::GraphEntry key{layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr, nullptr, 0};
-    if (replays(b, key, 1)) {
+    if (GraphCall *hit = replays(b, CallKey{layer, n_tokens, x, out, graph_tag(TAG_HOST_LAYER), nullptr}, 1)) {
       cudaStream_t s = b->compute;
       CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
-      mer_backend::GraphEntry *hit = nullptr;
-      const int rc = captured_graph(
-          b, key,
-          [&](int *n) -> int {
-            MoeDispatch d;
-            CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, s));
-            const int r = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, s, n, &d, true);
-            if (r) return r;
-            CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(out, b->d_out, n_tokens * D * 4, cudaMemcpyDeviceToHost, s));
-            CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)", cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, s));
-            return MER_OK;
-          },
-          &hit);
+      const int rc = capture_once(b, hit, [&](int *n) -> int {
+        MoeDispatch d;
+        CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(x)", cudaMemcpyAsync(b->d_x, x, n_tokens * D * 4, cudaMemcpyHostToDevice, s));
+        const int r = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, s, n, &d, true);
+        if (r) return r;
+        CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(out)", cudaMemcpyAsync(out, b->d_out, n_tokens * D * 4, cudaMemcpyDeviceToHost, s));
+        CU(MER_ERR_READBACK_MAP, "cudaMemcpyAsync(status)", cudaMemcpyAsync(b->h_u32 + b->max_pairs, b->d_status, 4, cudaMemcpyDeviceToHost, s));
+        return MER_OK;
+      });
       if (rc != MER_OK) return rc;
-      if (hit) {
+      if (hit->exec) {
         const RouterDev &r = b->routers[layer].dev;
         const size_t P = n_tokens * (r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u));
         CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, s));
@@ -1578,28 +1540,26 @@ MER_EXPORT int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float
       }
     }
   }
-  const mer_backend::GraphEntry key{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr, nullptr, 0};
   // (pinned rows of some size go up and down directly: staging them would only add a copy)
-  if (b->routers.count(layer) && !(pinned && n_tokens * D * 4 > SMALL_COPY) && replays(b, key) && stage_rows(b, n_tokens * D * 4)) {
+  GraphCall *hit = nullptr;
+  if (b->routers.count(layer) && !(pinned && n_tokens * D * 4 > SMALL_COPY))
+    hit = replays(b, CallKey{layer, n_tokens, nullptr, nullptr, graph_tag(TAG_HOST_STAGED), nullptr});
+  if (hit && stage_rows(b, n_tokens * D * 4)) {
     // ordinary host memory: rows through pinned memory, the sequence (routing included) captured per (layer, n_tokens)
     const RouterDev &r = b->routers[layer].dev;
     const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
     const size_t P = n_tokens * slots, bytes = n_tokens * D * 4;
     float *h_out = b->h_rows + b->rows_floats;
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, b->compute));
-    mer_backend::GraphEntry *hit = nullptr;
-    int rc = captured_graph(
-        b, key,
-        [&](int *n) -> int {
-          MoeDispatch d;
-          int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, false, n);
-          if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, b->compute, n, &d, true);
-          if (!e) e = enqueue_download(b, layer, h_out, b->d_out, bytes / 4, 1, bytes / 4, false, n);
-          return e ? e : enqueue_routing_readback(b, layer, P, n);
-        },
-        &hit);
+    int rc = capture_once(b, hit, [&](int *n) -> int {
+      MoeDispatch d;
+      int e = enqueue_upload(b, layer, b->d_x, b->h_rows, bytes, false, n);
+      if (!e) e = enqueue_layer(b, layer, b->d_x, n_tokens, b->d_out, true, b->compute, n, &d, true);
+      if (!e) e = enqueue_download(b, layer, h_out, b->d_out, bytes / 4, 1, bytes / 4, false, n);
+      return e ? e : enqueue_routing_readback(b, layer, P, n);
+    });
     if (rc) return rc;
-    if (hit) {
+    if (hit->exec) {
       const uint32_t done_before = *b->h_done;
       copy_host(b, b->h_rows, x, bytes);
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, b->compute));
@@ -1659,27 +1619,23 @@ int layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *d_x
   int launches = 0;
   size_t P = 0;
   bool replayed = false;
-  const mer_backend::GraphEntry key{layer, n_tokens, d_x, d_out, d_ids, d_weights, nullptr, 0};
-  if (!caller_captures(s) && replays(b, key)) {
+  GraphCall *hit = caller_captures(s) ? nullptr : replays(b, CallKey{layer, n_tokens, d_x, d_out, d_ids, d_weights});
+  if (hit) {
     auto it = b->routers.find(layer);
     if (it == b->routers.end()) return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "no router installed for layer %u", layer);
     P = n_tokens * (it->second.dev.top_k + (it->second.dev.shared_expert_id != MER_NONE ? 1u : 0u));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
-    mer_backend::GraphEntry *hit = nullptr;
-    const int rc = captured_graph(
-        b, key,
-        [&](int *n) -> int {
-          MoeDispatch d;
-          int r = enqueue_layer(b, layer, d_x, n_tokens, d_out, true, b->compute, n, &d, true);
-          if (r == MER_OK && d_ids && cudaMemcpyAsync(d_ids, b->d_pair_expert, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
-            r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the expert ids");
-          if (r == MER_OK && d_weights && cudaMemcpyAsync(d_weights, b->d_pair_weight, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
-            r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the mixing weights");
-          return r;
-        },
-        &hit);
+    const int rc = capture_once(b, hit, [&](int *n) -> int {
+      MoeDispatch d;
+      int r = enqueue_layer(b, layer, d_x, n_tokens, d_out, true, b->compute, n, &d, true);
+      if (r == MER_OK && d_ids && cudaMemcpyAsync(d_ids, b->d_pair_expert, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
+        r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the expert ids");
+      if (r == MER_OK && d_weights && cudaMemcpyAsync(d_weights, b->d_pair_weight, P * 4, cudaMemcpyDeviceToDevice, b->compute) != cudaSuccess)
+        r = fail(b, MER_ERR_SUBMISSION, layer, expert, "copy of the mixing weights");
+      return r;
+    });
     if (rc != MER_OK) return rc;
-    if (hit) {
+    if (hit->exec) {
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, s));
       launches = hit->launches;
       replayed = true;
@@ -2091,16 +2047,14 @@ int ep_layer_forward_device_locked(mer_backend *b, uint32_t layer, const float *
   const uint32_t expert = MER_NONE;
   int launches = 0;
   bool replayed = false;
-  const mer_backend::GraphEntry key{layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr, nullptr, 0};
-  if (b->ep_on && b->ep_attached && !caller_captures(s) && replays(b, key, 1)) {
+  GraphCall *hit = nullptr;
+  if (b->ep_on && b->ep_attached && !caller_captures(s)) hit = replays(b, CallKey{layer, n_tokens, d_x, d_out, graph_tag(TAG_EP), nullptr}, 1);
+  if (hit) {
     CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
     CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));  // outside any capture
-    mer_backend::GraphEntry *hit = nullptr;
-    const int rc = captured_graph(
-        b, key,
-        [&](int *n) -> int { return ep_enqueue(b, layer, d_x, n_tokens, d_out, b->compute, n, true); }, &hit);
+    const int rc = capture_once(b, hit, [&](int *n) -> int { return ep_enqueue(b, layer, d_x, n_tokens, d_out, b->compute, n, true); });
     if (rc != MER_OK) return rc;
-    if (hit) {
+    if (hit->exec) {
       CU(MER_ERR_SUBMISSION, "cudaGraphLaunch", cudaGraphLaunch(hit->exec, s));
       launches = hit->launches;
       replayed = true;

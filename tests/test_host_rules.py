@@ -1,0 +1,98 @@
+"""Rules of the host layer and of the kernels' work split that need no GPU: the headers that hold them are compiled with the host
+compiler into a small library and called here."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "micro-expert-router-ssd-streamed-moe-mer_b200", "csrc")
+
+SOURCE = r"""
+#include "replay_table.h"
+using Table = ReplayTable<const char *>;
+static int g_destroyed;
+static const char *const GRAPH = "graph";
+extern "C" {
+void *table_new() { return new Table(); }
+void table_delete(void *t) { delete static_cast<Table *>(t); }
+// One call: 0 plain launches, 1 captured now, 2 replayed.
+int table_call(void *t, uint32_t layer, size_t n_tokens, size_t x, size_t out, size_t tag, uint32_t from) {
+  Table &tab = *static_cast<Table *>(t);
+  auto *c = tab.occurrence(CallKey{layer, n_tokens, (const void *)x, (const void *)out, (const void *)tag, nullptr}, from);
+  if (!c) return 0;
+  if (c->exec) return 2;
+  tab.captured(c, GRAPH, 3, [](const char *) { g_destroyed++; });
+  return 1;
+}
+int table_drop(void *t) {
+  g_destroyed = 0;
+  static_cast<Table *>(t)->drop([](const char *) { g_destroyed++; });
+  return g_destroyed;
+}
+size_t table_graphs(void *t) { return static_cast<Table *>(t)->graphs(); }
+size_t table_size(void *t) { return static_cast<Table *>(t)->size(); }
+size_t max_graphs() { return Table::MAX_GRAPHS; }
+size_t max_calls() { return Table::MAX_CALLS; }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    d = tmp_path_factory.mktemp("rules")
+    src, lib = d / "rules.cpp", d / "librules.so"
+    src.write_text(SOURCE)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)])
+    r = C.CDLL(str(lib))
+    r.table_new.restype = C.c_void_p
+    for name in ("table_graphs", "table_size", "max_graphs", "max_calls"):
+        getattr(r, name).restype = C.c_size_t
+    for name in ("table_delete", "table_drop", "table_graphs", "table_size"):
+        getattr(r, name).argtypes = [C.c_void_p]
+    r.table_call.argtypes = [C.c_void_p, C.c_uint32] + [C.c_size_t] * 4 + [C.c_uint32]
+    return r
+
+
+@pytest.fixture
+def table(rules):
+    t = rules.table_new()
+    yield t
+    rules.table_delete(t)
+
+
+@pytest.mark.parametrize("layers", [48, 61, 94])
+@pytest.mark.parametrize("batches", [1, 5])
+@pytest.mark.parametrize("device", [False, True])
+def test_every_layer_of_a_stack_is_replayed_from_its_fourth_pass_on(rules, table, layers, batches, device):
+    # the calls of a model alternate: none may push another one out of the table.  Device calls carry their buffers' addresses.
+    calls = [(l, n, *((0x7f0000000000 + (l * 5 + n) * 8192, 0x7f1000000000 + l * 65536, 0) if device else (0, 0, 5)))
+             for l in range(layers) for n in (1, 4, 16, 64, 256)[:batches]]
+    passes = [[rules.table_call(table, *c, 3) for c in calls] for _ in range(5)]
+    assert passes[0] == passes[1] == [0] * len(calls)
+    assert passes[2] == [1] * len(calls)
+    assert passes[3] == passes[4] == [2] * len(calls)
+    assert rules.table_drop(table) == len(calls) and rules.table_graphs(table) == 0
+    assert [rules.table_call(table, *c, 3) for c in calls] == [1] * len(calls)  # known calls are captured again at once
+
+
+def test_calls_with_ever_new_buffers_are_never_captured_and_do_not_grow_the_table(rules, table):
+    for i in range(3 * rules.max_calls()):
+        assert rules.table_call(table, 0, 1, 4096 * (i + 1), 0, 0, 3) == 0
+        assert rules.table_call(table, 7, 1, 1, 0, 0, 3) == min(i // 2, 1) + (i > 2)  # one among them that comes again
+        assert rules.table_size(table) <= rules.max_calls()
+    assert rules.table_graphs(table) == 1
+
+
+def test_a_full_table_keeps_what_it_has_until_that_is_idle(rules, table):
+    n, more = rules.max_graphs(), rules.max_graphs() + 200
+    for _ in range(3):
+        for l in range(more):
+            rules.table_call(table, l, 1, 0, 0, 1, 3)
+    assert rules.table_graphs(table) == n
+    for _ in range(3):  # a working set that does not fit: the same calls are replayed, nothing is captured
+        assert [rules.table_call(table, l, 1, 0, 0, 1, 3) for l in range(more)] == [2] * n + [0] * (more - n)
+    seen = [[rules.table_call(table, 10000 + l, 1, 0, 0, 1, 1) for l in range(100)] for _ in range(60)]  # another model
+    assert seen[0] == [0] * 100 and seen[-1] == [2] * 100 and sum(map(sum, ([v == 1 for v in s] for s in seen))) == 100
+    assert rules.table_graphs(table) == n
