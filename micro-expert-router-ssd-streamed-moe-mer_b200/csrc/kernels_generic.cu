@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 #include "../../include/mer_b200.h"
 #include "layout.cuh"
+#include "passes.cuh"
 #include "route.cuh"
 
 namespace {
@@ -120,13 +121,6 @@ __device__ void build_item_bounds(const MoeDispatch &d, uint32_t n_passes, const
   }
 }
 
-// Pairs per pass of a group of n pairs.  The GEMM kernels work at a width of the pass's tokens, 16 at a time: several passes of
-// a group share its tokens evenly, as a narrow last pass would still have all the weights to dequantise.
-__device__ __forceinline__ uint32_t pass_step(uint32_t n, uint32_t tpp, uint32_t tpp_shift) {
-  const uint32_t passes = (n + tpp - 1) >> tpp_shift;
-  return tpp >= 16 && passes > 1 ? ((n + passes - 1) / passes + 15) & ~15u : tpp;
-}
-
 // Cuts every group into passes of at most d.tokens_per_pass pairs (the unit the streaming FFN works
 // on) and clears the per-pair max cells.  One CTA of 256 threads; `off` = the group offsets.
 __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
@@ -163,15 +157,16 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
 #pragma unroll 1
   for (uint32_t g = g0; g < g1; g++) {
     const uint32_t beg = off[g], end = off[g + 1];
-    const uint32_t step = pass_step(end - beg, tpp, tpp_shift);
+    const PassCut cut(end - beg, tpp, tpp_shift);
+    uint32_t st = beg;
 #pragma unroll 1
-    for (uint32_t st = beg; st < end; st += step) {
-      const uint32_t cnt = min(step, end - st);
+    for (uint32_t i = 0; i < cut.passes; i++) {
+      const uint32_t cnt = cut.count(i, end - st);
       d.pass_group[np] = g;
       d.pass_start[np] = st;
       d.pass_count[np] = cnt;
       if (np < 1024) s_cost[np] = cnt > 4 ? 13 : 10;
-      np++;
+      np++, st += cnt;
     }
   }
   if (threadIdx.x == 0) {
@@ -414,11 +409,13 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
     if (g < G) {
       d.group_expert[g] = g < r.num_experts ? r.id_base + g : r.shared_expert_id;
       d.offsets[g] = beg;
-      const uint32_t step = pass_step(n, tpp, shift);
+      const PassCut cut(n, tpp, shift);
+      uint32_t st = 0;
 #pragma unroll 1
-      for (uint32_t st = 0; st < n; st += step, pass++) {
-        const uint32_t cnt = min(step, n - st);
+      for (uint32_t j = 0; j < cut.passes; j++, pass++) {
+        const uint32_t cnt = cut.count(j, n - st);
         d.pass_group[pass] = g, d.pass_start[pass] = beg + st, d.pass_count[pass] = cnt;
+        st += cnt;
         if (bounds) s_cum[pass] = cum, cum += cnt > 4 ? 13 : 10;
       }
     }

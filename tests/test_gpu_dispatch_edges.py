@@ -59,6 +59,21 @@ def test_gemm_pass_widths_and_odd_tile_counts(dtype, D, F, n_tokens):
     assert rel_rms_err(got, ref) <= FFN_TOL
 
 
+@pytest.mark.parametrize("n_tokens", [897, 1025])  # passes of unequal width
+def test_a_row_gives_the_same_bits_in_every_pass_of_a_large_group(n_tokens):
+    dtype, D, F = oracle.Q8_0, 256, 128
+    blob = synth.make_expert_blob(dtype, D, F, 96, 0, 0)
+    rows = synth.make_activations(7, D, 96)
+    which = np.arange(n_tokens) % 7
+    with backend(dtype, D, F, 1, max_tokens=n_tokens) as b:
+        b.admit(0, 1, blob)
+        b.set_kernel_path(3)
+        got = b.expert_forward_f32(0, 0, rows[which])
+    ref = np.stack([oracle.expert_forward(dtype, blob, r, D, F, oracle.FWD_AUTHORITATIVE) for r in rows])
+    assert rel_rms_err(got[:7], ref) <= FFN_TOL
+    assert np.array_equal(got, got[:7][which])
+
+
 @pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
 @pytest.mark.parametrize("D,F,n_tokens", [(32, 96, 3), (96, 544, 9), (160, 32, 8), (4128, 288, 5), (7168, 256, 12)])
 def test_streaming_remainders_of_four_blocks_and_of_sixteen_tiles(dtype, D, F, n_tokens):

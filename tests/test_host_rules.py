@@ -10,6 +10,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "micro-expert-router-ssd-streamed-moe-mer_b200", "csrc")
 
 SOURCE = r"""
+#include <cuda_runtime.h>
+#include "passes.cuh"
 #include "replay_table.h"
 using Table = ReplayTable<const char *>;
 static int g_destroyed;
@@ -33,6 +35,13 @@ int table_drop(void *t) {
 }
 size_t table_graphs(void *t) { return static_cast<Table *>(t)->graphs(); }
 size_t table_size(void *t) { return static_cast<Table *>(t)->size(); }
+// The passes of a group of n pairs, as the grouping kernels write them; returns their number.
+uint32_t cut(uint32_t n, uint32_t tpp, uint32_t *counts) {
+  const PassCut c(n, tpp, 31 - __builtin_clz(tpp));
+  uint32_t st = 0;
+  for (uint32_t i = 0; i < c.passes; i++) st += counts[i] = c.count(i, n - st);
+  return c.passes;
+}
 size_t max_graphs() { return Table::MAX_GRAPHS; }
 size_t max_calls() { return Table::MAX_CALLS; }
 }
@@ -44,7 +53,8 @@ def rules(tmp_path_factory):
     d = tmp_path_factory.mktemp("rules")
     src, lib = d / "rules.cpp", d / "librules.so"
     src.write_text(SOURCE)
-    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC, str(src), "-o", str(lib)])
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC,
+                           "-I", "/usr/local/cuda/include", str(src), "-o", str(lib)])
     r = C.CDLL(str(lib))
     r.table_new.restype = C.c_void_p
     for name in ("table_graphs", "table_size", "max_graphs", "max_calls"):
@@ -96,3 +106,17 @@ def test_a_full_table_keeps_what_it_has_until_that_is_idle(rules, table):
     seen = [[rules.table_call(table, 10000 + l, 1, 0, 0, 1, 1) for l in range(100)] for _ in range(60)]  # another model
     assert seen[0] == [0] * 100 and seen[-1] == [2] * 100 and sum(map(sum, ([v == 1 for v in s] for s in seen))) == 100
     assert rules.table_graphs(table) == n
+
+
+@pytest.mark.parametrize("tpp", [4, 8, 16, 32, 64, 128])
+def test_the_passes_of_a_group_share_its_pairs_evenly(rules, tpp):
+    counts = (C.c_uint32 * 4096)()
+    for n in list(range(0, 2600)) + [4095, 4096, 4097, 10000]:
+        k = rules.cut(n, tpp, counts)
+        got = counts[:k]
+        assert k == -(-n // tpp) and sum(got) == n and all(0 < c <= tpp for c in got), (n, got)
+        if tpp < 16:
+            assert got[:-1] == [tpp] * (k - 1)
+        elif k:
+            widths = [(c + 15) // 16 for c in got]  # of an MMA, in units of 16 columns
+            assert max(widths) - min(widths) <= 1 and sum(widths) == -(-n // 16), (n, got)
