@@ -74,6 +74,26 @@ def test_a_row_gives_the_same_bits_in_every_pass_of_a_large_group(n_tokens):
     assert np.array_equal(got, got[:7][which])
 
 
+# pairs grouped in one block by atomics (streaming and GEMM kernels), and over the grid
+@pytest.mark.parametrize("E,k,B,path", [(16, 4, 40, 2), (16, 4, 200, 3), (4, 2, 4100, 2), (4, 2, 4100, 3)])
+def test_a_grouping_whose_order_the_atomics_decide_gives_the_same_bits_every_time(E, k, B, path):
+    dtype, D, F = oracle.Q4_0, 256, 128
+    W = synth.make_router(E, D, 97)
+    x = synth.make_activations(B, D, 97)
+    x[1::2] = x[0:-1:2][:x[1::2].shape[0]]  # pairs of equal rows lie side by side
+    with backend(dtype, D, F, E, max_tokens=B, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, synth.make_expert_blob(dtype, D, F, 97, 0, e))
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        b.set_kernel_path(path)
+        first, ids, w = b.moe_layer_forward(0, x)
+        for _ in range(5):
+            again, ids2, w2 = b.moe_layer_forward(0, x)
+            assert np.array_equal(first, again) and np.array_equal(ids, ids2) and np.array_equal(w, w2)
+    n = B // 2 * 2
+    assert np.array_equal(first[0:n:2], first[1:n:2])
+
+
 @pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
 @pytest.mark.parametrize("D,F,n_tokens", [(32, 96, 3), (96, 544, 9), (160, 32, 8), (4128, 288, 5), (7168, 256, 12)])
 def test_streaming_remainders_of_four_blocks_and_of_sixteen_tiles(dtype, D, F, n_tokens):
