@@ -5,8 +5,10 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
+#include <condition_variable>
 #include <cstdio>
 #include <cstring>
 #include <thread>
@@ -500,7 +502,12 @@ using ChunkReader = std::function<bool(size_t off, size_t n, uint8_t *dst)>;
 
 // Pageable bytes (or a reader's) -> pinned chunks -> `landing`, on the copy stream.  Several threads fill the chunks piece by
 // piece while the copy engine drains the finished ones; the calling thread enqueues chunks in order, hands freed buffers out
-// again, and copies pieces itself in between.  Pageable 99 MB: 8.4 ms with one thread, 2.35 ms here, 1.95 ms from pinned memory; 5 MB: 0.36, 0.24, 0.12 ms.  (16 MB of chunks: with 8 MB the 99 MB took 3.1 ms, with 32 MB 2.85.)
+// again, and copies pieces itself in between.  Pageable 99 MB: 8.4 ms with one thread, 2.35 ms here, 1.95 ms from pinned memory;
+// 5 MB: 0.36, 0.24, 0.12 ms.  (16 MB of chunks: with 8 MB the 99 MB took 3.1 ms, with 32 MB 2.85.)
+// While the copy engine is at work a chunk is on its way for 40 us, and everybody stays awake; when it has not freed a buffer for
+// AWAKE (it waits for a layer, say), the workers sleep until it does and the caller between looks.  (Events of the sleeping
+// kind, an interrupt for every chunk, cost every admission 7 %.)
+constexpr std::chrono::microseconds AWAKE(100);
 int upload_staged(mer_backend *b, uint32_t id, uint8_t *landing, const uint8_t *src, const ChunkReader *reader) {
   const uint32_t layer = 0, expert = id;
   const size_t bytes = b->expert_bytes;
@@ -511,6 +518,8 @@ int upload_staged(mer_backend *b, uint32_t id, uint8_t *landing, const uint8_t *
     std::vector<std::atomic<uint32_t>> done;
     std::atomic<size_t> next{0}, open{0};  // next piece to take; chunks whose buffer is free to be filled
     std::atomic<bool> failed{false};
+    std::mutex mu;  // workers that sleep until `open` or `next` moves on
+    std::condition_variable moved;
     explicit State(size_t n) : done(n) {}
   };
   const auto st = std::make_shared<State>(n_chunks);
@@ -531,44 +540,78 @@ int upload_staged(mer_backend *b, uint32_t id, uint8_t *landing, const uint8_t *
       if (st->next.compare_exchange_weak(p, p + 1, std::memory_order_relaxed)) return *piece = p, true;
     return false;
   };
+  using Clock = std::chrono::steady_clock;
   const bool pool = n_pieces >= 4;
   if (pool) {
     if (!b->copy_pool) b->copy_pool.reset(new (std::nothrow) CopyPool());
     if (b->copy_pool)
-      b->copy_pool->start(std::make_shared<const std::function<void()>>([st, take, copy_piece, n_pieces] {
+      b->copy_pool->start(std::make_shared<const std::function<void()>>([st, take, copy_piece, n_pieces, per_chunk] {
+        auto since = Clock::now();  // when a buffer was last opened
+        size_t open = 0;
         while (st->next.load(std::memory_order_relaxed) < n_pieces) {
           size_t piece;
-          if (take(&piece))
+          if (const size_t o = st->open.load(std::memory_order_relaxed); o != open) open = o, since = Clock::now();
+          if (take(&piece)) {
             copy_piece(piece);
-          else
+          } else if (Clock::now() - since < AWAKE) {
             std::this_thread::yield();
+          } else {
+            std::unique_lock<std::mutex> l(st->mu);
+            st->moved.wait(l, [&] {
+              const size_t n = st->next.load();
+              return n >= n_pieces || n / per_chunk < st->open.load();
+            });
+            since = Clock::now();
+          }
         }
       }));
   }
   cudaError_t e = cudaSuccess;
   size_t c = 0;  // chunks enqueued
+  auto since = Clock::now();  // the last step forward
   while (c < n_chunks && e == cudaSuccess && !st->failed.load(std::memory_order_relaxed)) {
     const uint32_t pieces = (uint32_t)std::min(per_chunk, n_pieces - c * per_chunk);
     if (st->done[c].load(std::memory_order_acquire) == pieces) {
       e = cudaMemcpyAsync(landing + c * chunk, stage + (c % STAGE_BUFS) * chunk, std::min(chunk, bytes - c * chunk), cudaMemcpyHostToDevice, b->copy);
       if (e == cudaSuccess) e = cudaEventRecord(b->ev_stage[c % STAGE_BUFS], b->copy);
-      c++;
+      c++, since = Clock::now();
       continue;
     }
     const size_t ready = st->open.load(std::memory_order_relaxed);
     if (ready < n_chunks && ready < c + STAGE_BUFS) {  // has the buffer's previous chunk (of this or an earlier admission) left it?
       const cudaError_t q = cudaEventQuery(b->ev_stage[ready % STAGE_BUFS]);
-      if (q == cudaSuccess)
-        st->open.store(ready + 1, std::memory_order_release);
-      else if (q != cudaErrorNotReady)
+      if (q == cudaSuccess) {
+        {
+          std::lock_guard<std::mutex> l(st->mu);
+          st->open.store(ready + 1, std::memory_order_release);
+        }
+        st->moved.notify_all();
+        since = Clock::now();
+        continue;
+      }
+      if (q != cudaErrorNotReady) {
         e = q;
-      if (q == cudaSuccess) continue;
+      } else if (ready == c && Clock::now() - since > AWAKE) {  // all open chunks are enqueued: only the copy engine can go on
+        std::this_thread::sleep_for(AWAKE / 2);
+        continue;
+      }
     }
     size_t piece;
-    if (take(&piece)) copy_piece(piece);
+    if (take(&piece)) {
+      copy_piece(piece);
+      since = Clock::now();
+    } else if (ready > c && Clock::now() - since > AWAKE) {  // workers are at the last pieces of a chunk (out of a slow file)
+      std::this_thread::sleep_for(AWAKE / 2);
+    }
   }
   // on an early end: nothing more is taken, and what has been taken is copied to its end before the source may go away
-  for (size_t taken = st->next.exchange(n_pieces), k = 0; c < n_chunks && k < n_chunks; k++) {
+  size_t taken;
+  {
+    std::lock_guard<std::mutex> l(st->mu);
+    taken = st->next.exchange(n_pieces);
+  }
+  st->moved.notify_all();
+  for (size_t k = 0; c < n_chunks && k < n_chunks; k++) {
     const size_t first = k * per_chunk, last = std::min(std::min(first + per_chunk, n_pieces), taken);
     while (first < last && st->done[k].load(std::memory_order_acquire) < last - first) std::this_thread::yield();
   }

@@ -176,3 +176,37 @@ def test_admission_does_not_wait_for_work_enqueued_on_the_default_stream_behind_
         torch.cuda.synchronize()
         assert overlapped, "the uploads waited for work behind the layer"
         assert rel_rms_err(out.cpu().numpy(), ref) <= 1e-3
+
+
+def test_an_admission_that_waits_for_a_layer_leaves_the_processor_to_others():
+    # a pageable payload larger than the staging memory, behind a layer that cannot start for a third of a second: the
+    # calling thread and its helpers sleep meanwhile
+    torch = pytest.importorskip("torch")
+    import time
+    dtype, D, F, B = oracle.Q8_0, 2048, 8192, 2
+    blob = np.zeros(mer_b200.expert_bytes(dtype, D, F), np.uint8)
+    W = synth.make_router(2, D, 66)
+    x = torch.from_numpy(synth.make_activations(B, D, 66)).cuda()
+    out = torch.empty(B, D, device="cuda")
+    side = torch.cuda.Stream()
+    with make_backend(dtype, D, F, slots=2, max_tokens=B, max_top_k=2) as b:
+        for e in (0, 1):
+            b.admit(e, 1, blob)
+        mer_b200.LinearGate(W, 2, D, 1).bind(b, 0)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(1000)
+        b.moe_layer_forward_device(0, x.data_ptr(), B, out.data_ptr(), side.cuda_stream)
+        torch.cuda.synchronize()
+        free = time.perf_counter()
+        b.admit(1, 2, blob, wait=False)
+        b.synchronize()
+        free = time.perf_counter() - free
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(700_000_000)
+        b.moe_layer_forward_device(0, x.data_ptr(), B, out.data_ptr(), side.cuda_stream)
+        wall, cpu = time.perf_counter(), time.process_time()
+        b.admit(1, 3, blob, wait=False)
+        wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+        b.synchronize()
+    # one thread awake all the time would spend `wall`; seven threads may be busy while the payload itself moves
+    assert wall > 0.15 and cpu <= 0.5 * (wall - free) + 7 * free, (wall, cpu, free)
