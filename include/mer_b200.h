@@ -421,12 +421,22 @@ int mer_qualification_matvec(mer_backend *b, int32_t dtype, const void *weights,
  * process exits), so: sizes beyond the maxima below are refused with MER_ERR_VALIDATION_DISPATCH and a
  * message in `err`; all calls on one GPU share that array, so two calls that overlap on the GPU (two
  * streams, two threads) race - serialise them; the first call on a device looks the array's address
- * up, so make that first call outside any stream capture.  Runs the generic fp32 kernels. */
+ * up, so make that first call outside any stream capture.  Rows of whole 32-value blocks (both dimensions, blob and d_x on
+ * 16-byte boundaries) run in one cooperative launch with one grid-wide wait of at most two seconds, everything else in the generic fp32
+ * kernels, which wait for nothing.  Should that wait run out, the output holds NaN where it was not computed and
+ * mer_expert_noalloc_check reports it. */
 #define MER_NOALLOC_MAX_TOKENS 8
 #define MER_NOALLOC_MAX_DIM 16384
 int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint64_t d_ff, const void *d_expert_blob,
                                const float *d_x, size_t n_tokens, float *d_out, float swiglu_limit,
                                void *stream, char *err, size_t err_len);
+/* The same with the limit of the wait chosen by the caller (nanoseconds, 0 = two seconds). */
+int mer_expert_forward_noalloc_bounded(int32_t dtype, uint64_t d_model, uint64_t d_ff, const void *d_expert_blob,
+                                       const float *d_x, size_t n_tokens, float *d_out, float swiglu_limit,
+                                       uint64_t wait_ns, void *stream, char *err, size_t err_len);
+/* Synchronises `stream` (the one the calls were enqueued on) of the current device, reads and clears the status that the
+ * no-allocation calls on this GPU have left: MER_OK or MER_ERR_TIMEOUT.  Allocates nothing.  (mer_stream_check's counterpart.) */
+int mer_expert_noalloc_check(void *stream, char *err, size_t err_len);
 
 /* ---- pipelined host entry: mer_moe_layer_forward for callers that keep several independent token batches in
  * flight (a serving loop over micro-batches; the reference's engine overlaps SSD reads with compute the same way,

@@ -10,7 +10,8 @@ CUDA device is present, calls raise.
 from .capi import (ABI_SYMBOLS, DTYPE_Q4_0, DTYPE_Q8_0, EXPERT_NONE, LIB_PATH, SCORE_SIGMOID, SCORE_SOFTMAX,
                    MerCounters, MerErrorInfo, load_library)
 from .backend import (Backend, GpuExpertBatchDispatchOutcome, GpuExpertDispatchError, GpuExpertDispatchErrorKind,
-                      expert_bytes, expert_forward_noalloc, routed_expert_gpu_compatibility)
+                      expert_bytes, expert_forward_noalloc, expert_forward_noalloc_bounded, expert_noalloc_check,
+                      routed_expert_gpu_compatibility)
 from .expert_cache import (GpuAdmission, GpuDemandAdmissionError, GpuDemandAdmissionPreflight, GpuExpertCache,
                            GpuHotPromotionOutcome, GpuLookup)
 from .gating import LinearGate, RoutingDecision, ScoringFunc
@@ -20,6 +21,7 @@ __all__ = [
     "GpuAdmission", "GpuDemandAdmissionError", "GpuDemandAdmissionPreflight", "GpuExpertCache",
     "GpuExpertDispatchError", "GpuExpertDispatchErrorKind", "GpuHotPromotionOutcome", "GpuLookup", "LIB_PATH", "LinearGate", "MerCounters", "MerErrorInfo",
     "RoutingDecision", "SCORE_SIGMOID", "SCORE_SOFTMAX", "ScoringFunc", "expert_bytes", "expert_forward_noalloc",
+    "expert_forward_noalloc_bounded", "expert_noalloc_check",
     "load_library",
     "routed_expert_gpu_compatibility",
 ]

@@ -289,12 +289,27 @@ class Backend:
 NOALLOC_MAX_TOKENS, NOALLOC_MAX_DIM = 8, 16384
 
 
+def _check_noalloc(rc, msg):
+    if rc != 0:
+        raise GpuExpertDispatchError(0, capi.EXPERT_NONE, rc, msg.value.decode(errors="replace"))
+
+
 def expert_forward_noalloc(dtype, d_model, d_ff, d_expert_blob, d_x, n_tokens, d_out, swiglu_limit=0.0, stream=0):
     """mer_expert_forward_noalloc: device pointers (ints) in and out, nothing allocated, asynchronous on
     `stream` of the current device.  All calls on a GPU share one fixed scratch array inside the library,
     so the caller must not let two of them overlap."""
+    expert_forward_noalloc_bounded(dtype, d_model, d_ff, d_expert_blob, d_x, n_tokens, d_out, swiglu_limit, 0, stream)
+
+
+def expert_forward_noalloc_bounded(dtype, d_model, d_ff, d_expert_blob, d_x, n_tokens, d_out, swiglu_limit=0.0, wait_ns=0, stream=0):
+    """The same; `wait_ns` limits the call's one device-side wait (0 = two seconds)."""
     msg = C.create_string_buffer(256)
-    rc = capi.load_library().mer_expert_forward_noalloc(dtype, d_model, d_ff, C.c_void_p(d_expert_blob), C.c_void_p(d_x),
-                                                        n_tokens, C.c_void_p(d_out), swiglu_limit, C.c_void_p(stream), msg, 256)
-    if rc != 0:
-        raise GpuExpertDispatchError(0, capi.EXPERT_NONE, rc, msg.value.decode(errors="replace"))
+    _check_noalloc(capi.load_library().mer_expert_forward_noalloc_bounded(
+        dtype, d_model, d_ff, C.c_void_p(d_expert_blob), C.c_void_p(d_x), n_tokens, C.c_void_p(d_out), swiglu_limit, wait_ns,
+        C.c_void_p(stream), msg, 256), msg)
+
+
+def expert_noalloc_check(stream=0):
+    """Synchronises `stream` and raises the typed error that no-allocation calls on this GPU have left, if any, once."""
+    msg = C.create_string_buffer(256)
+    _check_noalloc(capi.load_library().mer_expert_noalloc_check(C.c_void_p(stream), msg, 256), msg)

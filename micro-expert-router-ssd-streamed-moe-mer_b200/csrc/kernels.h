@@ -197,7 +197,7 @@ cudaError_t launch_reduce_parts(const MoeDispatch &d, cudaStream_t s, int *launc
 // kernels_flat.cu: one expert on the flat block stream (up to eight tokens), in one cooperative launch.
 bool flat_expert_supported(const void *expert, const void *x, uint32_t D, uint32_t F, uint32_t n_tokens);
 cudaError_t launch_flat_expert(int dtype, const uint8_t *expert, const float *x, float *h, float *out, uint32_t D, uint32_t F, uint32_t n_tokens, float limit,
-                               uint32_t *bar, uint32_t *status, int sm_count, cudaStream_t s);
+                               uint64_t wait_ns, uint32_t *bar, uint32_t *status, int sm_count, cudaStream_t s);
 
 // kernels_gemm.cu: tcgen05 / TMEM grouped GEMM for groups of a dozen tokens and more.
 bool gemm_ffn_supported(int dtype, uint32_t D, uint32_t F);

@@ -18,14 +18,9 @@
 // MER_DEVSTAT_TIMEOUT and carries on without the peer's data (the host then fails the call).
 #include "../../include/mer_b200.h"
 #include "kernels.h"
+#include "ptx.cuh"
 
 namespace {
-
-__device__ __forceinline__ uint64_t global_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
 
 __device__ __forceinline__ uint32_t ld_flag(const uint32_t *p) {
   uint32_t v;

@@ -11,6 +11,8 @@
 //     for another one's fragments.  Integer weights become A fragments as in kernels_stream.cu; two adjacent blocks (36 or 68
 //     bytes) are loaded as aligned 32-bit words and shifted by the two bytes of the first scale.
 //   * An epilogue warp adds the sixteen partial tiles, and at the last range applies SiLU(gate) * up or stores the output.
+//   * Every wait is bounded.  A CTA whose wait ran out latches MER_DEVSTAT_TIMEOUT and stores NaN for what it has not computed: the
+//     call is asynchronous, and a caller that does not ask for the status must not take the rest for a result.
 // One warp per weight row with byte loads, as before, took 620 us for a 4096 x 14336 Q4_0 expert and four tokens.
 #include <algorithm>
 
@@ -47,6 +49,7 @@ struct FlatParams {
   float *h, *out;
   uint32_t D, F, n_tokens;
   float limit;
+  uint64_t wait_ns;        // limit of the wait between the projections
   uint32_t *bar, *status;  // bar[0]: arrivals, bar[1]: exits; both zero between launches
 };
 
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
         const uint32_t nb = min(S::RANGE, kbt - kb0);
 #pragma unroll 1
         for (uint32_t tile = t0; tile < t1; tile++) {
-          if (round > 0) ok = mbar_wait(&empty[stage], (round - 1) & 1);
+          if (round > 0) ok = mbar_wait(&empty[stage], (round - 1) & 1, s_abort);
           if (*s_abort) ok = false;
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
@@ -169,8 +172,10 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
     }
     if (!ok) {
       if (lane == 0) *s_abort = 1;
-      // copies already in flight get a bounded chance to land before the CTA's memory is released
-      for (uint32_t s = 0; s < S::STAGES; s++) (void)mbar_wait(&full[s], 0), (void)mbar_wait(&full[s], 1);
+      // copies in flight get a bounded chance to land before the CTA's memory is released: the last phase of every stage
+      // issued to (which stays open, to the limit, only if the other producer stopped before it)
+      for (uint32_t s = 0; s < S::STAGES; s++)
+        if (s < stage || round > 0) mbar_drain(&full[s], (s < stage ? round : round - 1) & 1, 10000000ull);
     }
   } else if (warp < FC_WARPS) {
     // ------------------------------------------------------------------------------------------------------ consumers
@@ -336,13 +341,21 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
         }
       }
       __syncwarp();
+      if (!ok) {  // fail closed: NaN rows of h make every output NaN
+        const float nan = __uint_as_float(0x7fc00000u);
+        const uint32_t rows = ph == 0 ? 8 : 16, len = ph == 0 ? p.F : p.D;
+        float *dst = ph == 0 ? p.h : p.out;
+        for (uint32_t i = lane; i < (t1 - t0) * rows * p.n_tokens; i += 32)
+          dst[(size_t)(i / ((t1 - t0) * rows)) * len + t0 * rows + i % ((t1 - t0) * rows)] = nan;
+        __syncwarp();
+      }
       if (ph == 0) {  // h is exchanged between all CTAs
         if (lane == 0) {
           __threadfence();
           atomicAdd(p.bar, 1u);
           const uint64_t since = global_ns();
           while (*(volatile uint32_t *)p.bar < gridDim.x && ok)
-            if (global_ns() - since > 2000000000ull) ok = false;
+            if (global_ns() - since > p.wait_ns) ok = false;
           __threadfence();
         }
         ok = __all_sync(0xffffffffu, ok);
@@ -388,7 +401,7 @@ bool flat_expert_supported(const void *expert, const void *x, uint32_t D, uint32
 }
 
 cudaError_t launch_flat_expert(int dtype, const uint8_t *expert, const float *x, float *h, float *out, uint32_t D, uint32_t F, uint32_t n_tokens, float limit,
-                               uint32_t *bar, uint32_t *status, int sm_count, cudaStream_t s) {
-  const FlatParams p{expert, x, h, out, D, F, n_tokens, limit, bar, status};
+                               uint64_t wait_ns, uint32_t *bar, uint32_t *status, int sm_count, cudaStream_t s) {
+  const FlatParams p{expert, x, h, out, D, F, n_tokens, limit, wait_ns, bar, status};
   return dtype == MER_DTYPE_Q4_0 ? launch_flat_dt<MER_DTYPE_Q4_0>(p, sm_count, s) : launch_flat_dt<MER_DTYPE_Q8_0>(p, sm_count, s);
 }

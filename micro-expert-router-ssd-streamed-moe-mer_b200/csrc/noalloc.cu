@@ -33,11 +33,11 @@ constexpr size_t OFF_OFFSETS = H_BYTES + 128;      // uint32 [2]
 constexpr size_t OFF_PERM = H_BYTES + 192;         // uint32 [MAX_TOKENS]
 constexpr size_t OFF_PAIR_EXPERT = H_BYTES + 320;  // uint32 [MAX_TOKENS]
 constexpr size_t OFF_PAIR_WEIGHT = H_BYTES + 448;  // float  [MAX_TOKENS]
-constexpr size_t OFF_STATUS = H_BYTES + 576;       // uint32 [1]
+constexpr size_t OFF_STATUS = H_BYTES + 576;       // uint32 [1], kept until mer_expert_noalloc_check reads it
 constexpr size_t OFF_BAR = H_BYTES + 640;          // uint32 [2], zero between calls
 
 // Device code may name the array directly.  Everything a call depends on is rewritten here, because
-// the array still holds whatever the previous call left in it.
+// the array still holds whatever the previous call left in it.  (Not the status word: an earlier call's timeout is still to be read.)
 __global__ void k_noalloc_setup(const uint8_t *expert, uint32_t n_tokens) {
   unsigned char *s = g_noalloc_scratch;
   if (threadIdx.x == 0) {
@@ -45,7 +45,6 @@ __global__ void k_noalloc_setup(const uint8_t *expert, uint32_t n_tokens) {
     *reinterpret_cast<uint32_t *>(s + OFF_GROUP) = 0;  // the one group runs "expert id" 0 of a 1-entry table
     reinterpret_cast<uint32_t *>(s + OFF_OFFSETS)[0] = 0;
     reinterpret_cast<uint32_t *>(s + OFF_OFFSETS)[1] = n_tokens;
-    *reinterpret_cast<uint32_t *>(s + OFF_STATUS) = 0;
   }
   if (threadIdx.x < MER_NOALLOC_MAX_TOKENS) {
     reinterpret_cast<uint32_t *>(s + OFF_PERM)[threadIdx.x] = threadIdx.x;
@@ -54,6 +53,7 @@ __global__ void k_noalloc_setup(const uint8_t *expert, uint32_t n_tokens) {
   }
 }
 
+constexpr uint64_t DEFAULT_WAIT_NS = 2000000000ull;
 constexpr int MAX_DEVICES = 64;
 std::mutex g_mu;
 unsigned char *g_scratch_ptr[MAX_DEVICES] = {};
@@ -63,11 +63,43 @@ void set_err(char *err, size_t err_len, const char *msg) {
   if (err && err_len) snprintf(err, err_len, "%s", msg);
 }
 
+// Device address of the static array on the current device, and the device's SM count.
+int device_scratch(unsigned char **scratch, int *sm_count, char *err, size_t err_len) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
+    cudaGetLastError();
+    set_err(err, err_len, "no current CUDA device");
+    return MER_ERR_DEVICE_LOST;
+  }
+  // First call on this device: resolve the device address of the static array (no allocation).
+  std::lock_guard<std::mutex> lock(g_mu);
+  if (!g_scratch_ptr[dev]) {
+    unsigned char *p = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_noalloc_scratch);
+    if (e != cudaSuccess || !p) {
+      if (err && err_len) snprintf(err, err_len, "cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
+      cudaGetLastError();
+      return MER_ERR_RUNTIME_INVARIANT;
+    }
+    if (cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sm_count[dev] = 0;
+    g_scratch_ptr[dev] = p;
+  }
+  *scratch = g_scratch_ptr[dev];
+  *sm_count = g_sm_count[dev];
+  return MER_OK;
+}
+
 }  // namespace
 
 MER_EXPORT int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint64_t d_ff, const void *d_expert_blob,
                                           const float *d_x, size_t n_tokens, float *d_out, float swiglu_limit, void *stream,
                                           char *err, size_t err_len) {
+  return mer_expert_forward_noalloc_bounded(dtype, d_model, d_ff, d_expert_blob, d_x, n_tokens, d_out, swiglu_limit, 0, stream, err, err_len);
+}
+
+MER_EXPORT int mer_expert_forward_noalloc_bounded(int32_t dtype, uint64_t d_model, uint64_t d_ff, const void *d_expert_blob,
+                                                  const float *d_x, size_t n_tokens, float *d_out, float swiglu_limit,
+                                                  uint64_t wait_ns, void *stream, char *err, size_t err_len) {
   if (dtype != MER_DTYPE_Q4_0 && dtype != MER_DTYPE_Q8_0) {
     set_err(err, err_len, "unknown dtype");
     return MER_ERR_INVALID_ARGUMENT;
@@ -85,36 +117,15 @@ MER_EXPORT int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint6
                n_tokens, MER_NOALLOC_MAX_TOKENS, (unsigned long long)d_model, (unsigned long long)d_ff, MER_NOALLOC_MAX_DIM);
     return MER_ERR_VALIDATION_DISPATCH;
   }
-  int dev = -1;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) {
-    cudaGetLastError();
-    set_err(err, err_len, "no current CUDA device");
-    return MER_ERR_DEVICE_LOST;
-  }
   unsigned char *scratch;
   int sm_count;
-  {
-    // First call on this device: resolve the device address of the static array (no allocation).
-    std::lock_guard<std::mutex> lock(g_mu);
-    if (!g_scratch_ptr[dev]) {
-      unsigned char *p = nullptr;
-      cudaError_t e = cudaGetSymbolAddress(reinterpret_cast<void **>(&p), g_noalloc_scratch);
-      if (e != cudaSuccess || !p) {
-        if (err && err_len) snprintf(err, err_len, "cudaGetSymbolAddress failed: %s", cudaGetErrorString(e));
-        cudaGetLastError();
-        return MER_ERR_RUNTIME_INVARIANT;
-      }
-      if (cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) g_sm_count[dev] = 0;
-      g_scratch_ptr[dev] = p;
-    }
-    scratch = g_scratch_ptr[dev];
-    sm_count = g_sm_count[dev];
-  }
+  const int rc = device_scratch(&scratch, &sm_count, err, err_len);
+  if (rc != MER_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (sm_count > 0 && flat_expert_supported(d_expert_blob, d_x, (uint32_t)d_model, (uint32_t)d_ff, (uint32_t)n_tokens)) {
     cudaError_t e = launch_flat_expert(dtype, static_cast<const uint8_t *>(d_expert_blob), d_x, reinterpret_cast<float *>(scratch), d_out, (uint32_t)d_model,
-                                       (uint32_t)d_ff, (uint32_t)n_tokens, swiglu_limit, reinterpret_cast<uint32_t *>(scratch + OFF_BAR),
-                                       reinterpret_cast<uint32_t *>(scratch + OFF_STATUS), sm_count, s);
+                                       (uint32_t)d_ff, (uint32_t)n_tokens, swiglu_limit, wait_ns ? wait_ns : DEFAULT_WAIT_NS,
+                                       reinterpret_cast<uint32_t *>(scratch + OFF_BAR), reinterpret_cast<uint32_t *>(scratch + OFF_STATUS), sm_count, s);
     if (e == cudaSuccess) return MER_OK;
     cudaGetLastError();  // no cooperative launch to be had: the kernels for any shape below
   }
@@ -145,6 +156,28 @@ MER_EXPORT int mer_expert_forward_noalloc(int32_t dtype, uint64_t d_model, uint6
   if (e != cudaSuccess) {
     if (err && err_len) snprintf(err, err_len, "kernel launch failed: %s", cudaGetErrorString(e));
     return MER_ERR_SUBMISSION;
+  }
+  return MER_OK;
+}
+
+MER_EXPORT int mer_expert_noalloc_check(void *stream, char *err, size_t err_len) {
+  unsigned char *scratch;
+  int sm_count;
+  const int rc = device_scratch(&scratch, &sm_count, err, err_len);
+  if (rc != MER_OK) return rc;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  uint32_t status = 0;
+  cudaError_t e = cudaMemcpyAsync(&status, scratch + OFF_STATUS, 4, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && status) e = cudaMemsetAsync(scratch + OFF_STATUS, 0, 4, s);
+  if (e == cudaSuccess && status) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) {
+    if (err && err_len) snprintf(err, err_len, "reading the status word: %s", cudaGetErrorString(e));
+    return MER_ERR_READBACK_MAP;
+  }
+  if (status & MER_DEVSTAT_TIMEOUT) {
+    set_err(err, err_len, "a bounded device-side wait of an earlier call on this GPU expired; its output holds NaN");
+    return MER_ERR_TIMEOUT;
   }
   return MER_OK;
 }

@@ -36,19 +36,37 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// Bounded wait: false when the phase did not complete within SPIN_LIMIT polls.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t addr = smem_u32(bar);
+__device__ __forceinline__ uint64_t global_ns() {
+  uint64_t t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Whether the phase with this parity is complete; suspends for a while if not.
+__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(addr), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait: false when the phase did not complete within SPIN_LIMIT polls, or (with `abort`) once *abort is set.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, const volatile uint32_t *abort = nullptr) {
+  const uint32_t addr = smem_u32(bar);
   for (uint32_t i = 0; i < SPIN_LIMIT; i++) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    if (ok) return true;
+    if (mbar_try(addr, parity)) return true;
+    if (abort && *abort) return false;
   }
   return false;
+}
+// The same, bounded by time: for the way out after an error.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity, uint64_t ns) {
+  const uint32_t addr = smem_u32(bar);
+  const uint64_t since = global_ns();
+  while (!mbar_try(addr, parity) && global_ns() - since < ns) {
+  }
 }
 // The same for a barrier that other CTAs of the cluster arrive on.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t *bar, uint32_t parity) {

@@ -31,3 +31,26 @@ def test_flat_expert_matches_the_oracle(dtype, D, F, n):
     for t in range(n):
         ref = oracle.expert_forward(dtype, blob, x[t], D, F)
         assert np.abs(got[t] - ref).max() <= 1e-3 * np.sqrt(np.mean(ref.astype(np.float64) ** 2))
+
+
+@pytest.mark.parametrize("dtype,D,F,n", [(mer_b200.DTYPE_Q4_0, 2048, 4096, 3), (mer_b200.DTYPE_Q8_0, 4096, 1408, 8)])
+def test_a_wait_that_runs_out_is_reported_once_and_leaves_nan(dtype, D, F, n):
+    # a limit of one nanosecond: the CTAs that arrive first give up on the others
+    import torch
+    blob = synth.make_expert_blob(dtype, D, F, 92, 0, 0)
+    x = synth.make_activations(n, D, 92)
+    d_blob, d_x = torch.from_numpy(blob).cuda(), torch.from_numpy(x).cuda()
+    d_out = torch.zeros((n, D), device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    args = (dtype, D, F, d_blob.data_ptr(), d_x.data_ptr(), n, d_out.data_ptr(), 0.0)
+    mer_b200.expert_noalloc_check(stream)  # nothing is pending
+    mer_b200.expert_forward_noalloc_bounded(*args, 1, stream)
+    with pytest.raises(mer_b200.GpuExpertDispatchError) as e:
+        mer_b200.expert_noalloc_check(stream)
+    assert e.value.kind == mer_b200.GpuExpertDispatchErrorKind.Timeout
+    assert np.isnan(d_out.cpu().numpy()).any(axis=1).all()  # in every row
+    mer_b200.expert_noalloc_check(stream)  # reported once
+    mer_b200.expert_forward_noalloc(*args, stream)  # and the next call is whole
+    mer_b200.expert_noalloc_check(stream)
+    ref = np.stack([oracle.expert_forward(dtype, blob, r, D, F) for r in x])
+    assert np.abs(d_out.cpu().numpy() - ref).max() <= 1e-3 * np.sqrt(np.mean(ref.astype(np.float64) ** 2))
