@@ -105,9 +105,6 @@ __device__ __forceinline__ uint32_t leader_addr(const void *p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
-__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 // The box of `map` at (column x, row r) of the activation matrix into this CTA's shared memory (128-byte rows, swizzled);
 // the bytes are counted on a barrier of the pair's first CTA.
 __device__ __forceinline__ void tile_g2s(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t r, uint32_t bar) {
@@ -282,7 +279,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, pg++) {
         if (pg >= p.n_b) {
           const uint32_t sp = pg - p.n_b;
-          ok = mbar_wait(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
+          ok = mbar_wait_cluster(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
         }
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
@@ -324,9 +321,9 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       const uint32_t d_tmem = tmem_base + buf * 128;
       for (uint32_t st = 0; st < p.kb_total && ok; st += GROUP, grp++) {
         const uint32_t ag = grp % A_RING;
-        if (st == 0 && use > 0) ok = mbar_wait_cluster(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
+        if (st == 0 && use > 0) ok = mbar_wait_tmem(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
         if (ok) ok = mbar_wait_cluster(&b_full[rb.stage], rb.round & 1);
-        if (ok) ok = mbar_wait_cluster(&a_full[ag], (grp / A_RING) & 1);
+        if (ok) ok = mbar_wait_tmem(&a_full[ag], (grp / A_RING) & 1);
         ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the vote also tells the compiler so
         if (!ok) break;
         tc_fence_after();
@@ -463,7 +460,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         if (grp >= A_RING && ok) {
           // the group's A stages were last read by the MMAs of the group A_RING before it
           const uint32_t sp = grp - A_RING;
-          ok = mbar_wait(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
+          ok = mbar_wait_tmem(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
         }
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -472,7 +469,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(leader_addr(&a_full[grp % A_RING]));
+        if (lane == 0) mbar_arrive_tmem(leader_addr(&a_full[grp % A_RING]));
       }
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
@@ -510,7 +507,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         asm volatile("bar.sync %0, 128;" ::"r"(1 + buf) : "memory");
       }
       if (resident && !dead) {
-        ok = mbar_wait(&acc_full[buf], used & 1);
+        ok = mbar_wait_tmem(&acc_full[buf], used & 1);
         used++;
         if (*s_abort) ok = false;
         if (!__all_sync(0xffffffffu, ok)) dead = true;
@@ -574,7 +571,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       if (resident && !dead) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) arrive_cluster(leader_addr(&acc_empty[buf]));
+        if (lane == 0) mbar_arrive_tmem(leader_addr(&acc_empty[buf]));
       }
     }
     if (dead && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);

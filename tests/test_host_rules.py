@@ -2,6 +2,7 @@
 compiler into a small library and called here."""
 import ctypes as C
 import os
+import re
 import subprocess
 
 import pytest
@@ -120,3 +121,20 @@ def test_the_passes_of_a_group_share_its_pairs_evenly(rules, tpp):
         elif k:
             widths = [(c + 15) // 16 for c in got]  # of an MMA, in units of 16 columns
             assert max(widths) - min(widths) <= 1 and sum(widths) == -(-n // 16), (n, got)
+
+
+def test_barriers_between_the_ctas_of_a_pair_name_their_scope():
+    # an mbarrier operation without one orders memory within its own CTA only; the pair's barriers are signalled by both
+    ptx, gemm = (open(os.path.join(CSRC, f)).read() for f in ("ptx.cuh", "kernels_gemm.cu"))
+    for arrive in re.findall(r"mbarrier\.arrive[^ ]*shared::cluster[^ ]*", ptx + gemm):
+        assert re.match(r"mbarrier\.arrive\.(relaxed|release)\.cluster\.", arrive), arrive
+    for name, sem in (("mbar_wait_tmem", "relaxed"), ("mbar_wait_cluster", "acquire")):
+        body = ptx[ptx.index(f"bool {name}("):]
+        assert f"mbarrier.try_wait.parity.{sem}.cluster." in body[:body.index("\n}\n")]
+    kernel = gemm[gemm.index("k_ffn_gemm("):]
+    waits = re.findall(r"ok = (mbar_wait\w*)\(&(\w+)\[", kernel)
+    crossing = {"a_full": "tmem", "acc_empty": "tmem", "acc_full": "tmem", "b_full": "cluster"}
+    assert {b for _, b in waits} == {*crossing, "done", "raw_full", "raw_empty"}
+    for wait, barrier in waits:
+        assert wait in ({"mbar_wait_tmem", "mbar_wait_cluster"} if barrier == "done" else
+                        {"mbar_wait_" + crossing[barrier]} if barrier in crossing else {"mbar_wait"}), (wait, barrier)
