@@ -653,8 +653,10 @@ int admit_impl(mer_backend *b, uint32_t id, uint64_t generation, const void *blo
   uint8_t *landing = b->packed ? b->d_raw_stage : payload;  // packed slots: land flat bytes in staging, then permute
   const uint8_t *src = static_cast<const uint8_t *>(blob);
   if (from_device) {
-    if (b->packed)
-      landing = const_cast<uint8_t *>(src);  // permute straight out of the caller's device buffer
+    if (b->packed && reinterpret_cast<uintptr_t>(src) % 2 == 0)
+      landing = const_cast<uint8_t *>(src);  // permute straight out of the caller's device buffer (16 bits at a time)
+    else if (b->packed)
+      CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(D2D)", cudaMemcpyAsync(landing, src, b->expert_bytes, cudaMemcpyDeviceToDevice, b->copy));
     else
       CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(D2D)", cudaMemcpyAsync(payload, src, b->expert_bytes, cudaMemcpyDeviceToDevice, b->copy));
   } else {
@@ -1304,6 +1306,15 @@ MER_EXPORT int mer_layer_install(mer_backend *b, uint32_t layer, const mer_layer
 }
 
 namespace {
+// The kernels read and write rows 16 bytes at a time; a caller's rows may start on any float.
+bool row_aligned(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+// Device rows that kernels can read: the caller's, or a copy of them in the workspace.
+cudaError_t readable_rows(mer_backend *b, const float *&rows, size_t n_tokens, cudaStream_t s) {
+  if (row_aligned(rows)) return cudaSuccess;
+  const cudaError_t e = cudaMemcpyAsync(b->d_x, rows, n_tokens * b->cfg.d_model * 4, cudaMemcpyDeviceToDevice, s);
+  rows = b->d_x;
+  return e;
+}
 // Enqueues router (+ optional FFN + combine) for device-resident x on stream s.
 int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens, float *d_out, bool run_ffn_too,
                   cudaStream_t s, int *launches, MoeDispatch *out_d, bool capturing = false, bool status_cleared = false) {
@@ -1320,8 +1331,9 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   d.max_group_tokens = d.n_tokens;  // a token reaches an expert at most once
   d.active_groups_hint = std::min(d.n_groups, d.n_tokens * d.slots);
   if (run_ffn_too) bind_ffn(b, d);
+  CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(unaligned x)", readable_rows(b, d_x, n_tokens, s));
   d.x = d_x;
-  d.out = d_out;
+  d.out = row_aligned(d_out) ? d_out : b->d_out;
   if (!status_cleared && (!run_ffn_too || !router_sets_status(d))) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
   if (!capturing) CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
   cudaEvent_t *ev = (run_ffn_too && !capturing) ? next_timing_set(b) : nullptr;
@@ -1347,6 +1359,8 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
     if (ev) cudaEventRecord(ev[3], s);
     CU(MER_ERR_SUBMISSION, "combine kernel", launch_combine(d, s, launches));
     if (ev) cudaEventRecord(ev[4], s);
+    if (d.out != d_out)
+      CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(unaligned out)", cudaMemcpyAsync(d_out, d.out, n_tokens * d.D * 4, cudaMemcpyDeviceToDevice, s));
   }
   if (out_d) *out_d = d;
   return MER_OK;
@@ -1984,8 +1998,9 @@ MER_EXPORT int mer_ep_local_experts_forward_device(mer_backend *b, uint32_t laye
   ep.top_k = r.top_k, ep.id_base = r.id_base, ep.tokens_per_rank = (uint32_t)tokens_per_rank;
   MoeDispatch d = base_dispatch(b);
   d.n_tokens = (uint32_t)n_tokens_all;
+  CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(unaligned x)", readable_rows(b, d_x_all, n_tokens_all, s));
   d.x = d_x_all;
-  d.out = d_out_partial;
+  d.out = row_aligned(d_out_partial) ? d_out_partial : b->d_out;
   const uint32_t slots = r.top_k + (r.shared_expert_id != MER_NONE ? 1u : 0u);
   CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
   CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
@@ -1994,6 +2009,8 @@ MER_EXPORT int mer_ep_local_experts_forward_device(mer_backend *b, uint32_t laye
   int rc = ep_run_local_experts(b, layer, r, d, s, &launches);
   if (rc) return rc;
   CU(MER_ERR_SUBMISSION, "combine kernel", launch_combine(d, s, &launches));
+  if (d.out != d_out_partial)
+    CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(unaligned out)", cudaMemcpyAsync(d_out_partial, d.out, n_tokens_all * d.D * 4, cudaMemcpyDeviceToDevice, s));
   CU(MER_ERR_SUBMISSION, "cudaEventRecord(stream use)", note_stream_use(b, s));
   b->ctr.kernel_launches += (uint64_t)launches;
   return MER_OK;
@@ -2021,6 +2038,8 @@ int ep_enqueue(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens
   if (n_tokens == 0 || n_tokens > b->ep_cfg.max_tokens_per_rank)
     return fail(b, MER_ERR_VALIDATION_DISPATCH, layer, expert, "n_tokens %zu outside 1..=%u per rank", n_tokens, b->ep_cfg.max_tokens_per_rank);
   if ((b->cfg.d_model & 3) != 0) return fail(b, MER_ERR_INELIGIBLE, layer, expert, "d_model must be a multiple of 4");
+  if (!row_aligned(d_out) || (!row_aligned(d_x) && (it->second.layer_flags & MER_LAYER_RESIDUAL)))
+    return fail(b, MER_ERR_INVALID_ARGUMENT, layer, expert, "the output rows, and input rows that are added to them, must start on 16 bytes");
   CU(MER_ERR_SUBMISSION, "cudaSetDevice", cudaSetDevice(b->cfg.device));
   int launches = 0;
   const size_t D = b->cfg.d_model;

@@ -125,3 +125,48 @@ def test_repeated_host_calls_read_new_rows(B):
             out, ids, _ = b.moe_layer_forward(0, x)
             assert (ids == rids).all() and rel_rms_err(out, ref) <= FFN_TOL
             assert rel_rms_err(b.moe_step_weighted_into(0, x[0], rids[0], rw[0]), ref[0]) <= FFN_TOL
+
+
+@pytest.mark.parametrize("D,F,E,k,B,path", [(96, 160, 4, 2, 3, 0), (1024, 32, 8, 2, 5, 0), (256, 128, 4, 2, 300, 0), (45, 37, 4, 2, 3, 0),
+                                            (256, 256, 4, 2, 40, 3), (64, 96, 4, 2, 7, 1)])
+@pytest.mark.parametrize("block", [False, True])
+def test_device_rows_may_start_on_any_float(D, F, E, k, B, path, block):
+    import torch
+    dtype = oracle.Q8_0
+    x = synth.make_activations(B, D, 98)
+    with backend(dtype, D, F, E, max_tokens=B, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, synth.make_expert_blob(dtype, D, F, 98, 0, e))
+        mer_b200.LinearGate(synth.make_router(E, D, 98), E, D, k).bind(b, 0)
+        if block:
+            b.install_layer(0, np.linspace(0.5, 1.5, D, dtype=np.float32), 1e-6, residual=True)
+        b.set_kernel_path(path)
+        results = []
+        for shift in (0, 1, 2, 3):
+            d_x = torch.zeros(B * D + 4, device="cuda")[shift:shift + B * D]
+            d_out = torch.zeros(B * D + 4, device="cuda")
+            d_x.copy_(torch.from_numpy(x.reshape(-1)))
+            for rep in range(4):  # plain launches, the capture, a replay
+                d_out.fill_(7.0)
+                b.moe_layer_forward_device(0, d_x.data_ptr(), B, d_out.data_ptr() + 4 * shift, torch.cuda.current_stream().cuda_stream)
+                b.stream_check(0, torch.cuda.current_stream().cuda_stream)
+                got = d_out.cpu().numpy()
+                assert (got[:shift] == 7.0).all() and (got[shift + B * D:] == 7.0).all()
+                results.append(got[shift:shift + B * D])
+        assert np.isfinite(results[0]).all() and all(np.array_equal(results[0], r) for r in results)
+
+
+@pytest.mark.parametrize("dtype,D,F", [(oracle.Q8_0, 96, 32), (oracle.Q4_0, 256, 256), (oracle.Q4_0, 45, 37)])
+def test_a_device_payload_may_start_on_any_byte(dtype, D, F):
+    import torch
+    blob = synth.make_expert_blob(dtype, D, F, 99, 0, 0)
+    x = synth.make_activations(2, D, 99)
+    with backend(dtype, D, F, 4, max_tokens=2) as b:
+        for shift in range(4):
+            buf = torch.zeros(blob.size + 4, dtype=torch.uint8, device="cuda")
+            buf[shift:shift + blob.size].copy_(torch.from_numpy(blob))
+            torch.cuda.synchronize()
+            b.admit_device(shift, 1, buf.data_ptr() + shift, blob.size)
+        got = [b.expert_forward_f32(0, e, x) for e in range(4)]
+    ref = np.stack([oracle.expert_forward(dtype, blob, r, D, F) for r in x])
+    assert rel_rms_err(got[0], ref) <= FFN_TOL and all(np.array_equal(got[0], g) for g in got)
