@@ -358,11 +358,11 @@ constexpr uint32_t MID_PAIRS = 2048, MID_GROUPS = 512;
 // `s_pair` [P]: group (16 bits) and rank of every pair.  Loops stay rolled: the code runs once, cold.
 __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint32_t *s_pair) {
   constexpr uint32_t PER_G = MID_GROUPS / 256;
-  __shared__ uint32_t s_cnt[MID_GROUPS], s_cum[MID_PAIRS / 8 + MID_GROUPS + 1];
+  __shared__ uint32_t s_cnt[MID_GROUPS], s_cum[MID_PAIRS / 8 + MID_GROUPS + 1];  // s_cum: passes of eight
   __shared__ uint64_t s_part[8];
   const uint32_t P = d.n_tokens * d.slots, G = d.n_groups, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t tpp = d.tokens_per_pass, shift = 31 - __clz(tpp);
-  const bool bounds = d.item_bounds != nullptr;
+  const bool bounds = d.item_bounds != nullptr, weighted = bounds && tpp == 8;  // (passes of four can be more than s_cum holds)
   for (uint32_t i = tid; i < MID_GROUPS; i += 256) s_cnt[i] = 0;
   __syncthreads();
 #pragma unroll 1
@@ -416,7 +416,7 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
         const uint32_t cnt = cut.count(j, n - st);
         d.pass_group[pass] = g, d.pass_start[pass] = beg + st, d.pass_count[pass] = cnt;
         st += cnt;
-        if (bounds) s_cum[pass] = cum, cum += cnt > 4 ? 13 : 10;
+        if (weighted) s_cum[pass] = cum, cum += cnt > 4 ? 13 : 10;
       }
     }
     base += mine[i];
@@ -425,7 +425,7 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
     d.offsets[G] = (uint32_t)total & 0xFFFFF;
     d.n_passes[0] = n_passes;
     d.n_passes[1] = d.n_passes[2] = 0;
-    if (bounds) s_cum[n_passes] = (uint32_t)(total >> 40);
+    if (weighted) s_cum[n_passes] = (uint32_t)(total >> 40);
   }
   __syncthreads();
 #pragma unroll 1
@@ -433,7 +433,7 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
     const uint32_t v = s_pair[p];
     if (v != MER_NONE) d.perm[s_cnt[v >> 16] + (v & 0xFFFF)] = p;
   }
-  if (bounds) build_item_bounds(d, n_passes, tpp == 8 ? s_cum : nullptr);
+  if (bounds) build_item_bounds(d, n_passes, weighted ? s_cum : nullptr);
 }
 
 // Runs in one CTA after every token has been routed: groups pairs by expert.

@@ -25,6 +25,7 @@ def backend(dtype, D, F, n_experts, **kw):
     (8, 2, 16, 64, 32), (8, 2, 17, 64, 32),        # 32 pairs are grouped in one warp, more in a block
     (4, 1, 2048, 64, 32), (4, 1, 2049, 64, 32),    # the block's largest number of pairs
     (512, 1, 40, 64, 32), (513, 1, 40, 64, 32),    # and of groups
+    (512, 32, 4, 64, 32), (64, 16, 3, 64, 32),     # the same with passes of four
     (3, 1, 1, 1024, 32), (100, 2, 5, 1024, 32),    # one and two expert rows per router CTA
     (16, 1, 300, 1024, 32), (17, 1, 300, 1024, 32),  # logits of a large batch: direct, in small tiles,
     (128, 1, 1921, 512, 32),                       # in large ones
