@@ -392,10 +392,12 @@ int mer_moe_layer_forward(mer_backend *b, uint32_t layer, const float *x, size_t
                           float *out, uint32_t *ids, float *weights);
 
 /* ---- compute, device buffers, asynchronous on `stream` (a cudaStream_t) ----
- * The launch sequence of a call is captured into a CUDA graph the first time a (layer, n_tokens,
- * pointers, stream) combination is seen and replayed afterwards (one cudaGraphLaunch per call), so
- * the first call with new arguments must not itself be inside a stream capture.  The backend's
- * workspace is shared: calls on different streams must not overlap. */
+ * The launch sequence of a call is captured into a CUDA graph (on a stream of the backend's own) when the same
+ * layer, n_tokens and pointers come for the third time, and replayed from then on into whatever stream the call
+ * names (one cudaGraphLaunch per call).  A call on a stream that the caller is capturing becomes plain launches
+ * of that capture.  Rows may start on any float; off a 16-byte boundary they cost one copy through the workspace
+ * (the mer_ep_* calls refuse such output rows).  The backend's workspace is shared: calls on different streams
+ * must not overlap. */
 int mer_moe_layer_forward_device(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tokens,
                                  float *d_out, uint32_t *d_ids, float *d_weights, void *stream);
 
@@ -545,7 +547,8 @@ int mer_last_error(mer_backend *b, mer_error_info *out);
 int mer_snapshot(mer_backend *b, mer_counters *out);
 /* Selects the kernel family: 0 = automatic (streaming kernels for a few tokens per expert, the
  * tcgen05 GEMM kernels from a mean of 12 tokens per expert), 1 = generic fp32 kernels (any shape),
- * 2 = streaming tensor-core kernels, 3 = tcgen05 GEMM kernels (2 and 3: block-aligned shapes).
+ * 2 = streaming tensor-core kernels (d_model and d_ff multiples of 32), 3 = tcgen05 GEMM kernels (multiples of
+ * 128, a backend of at least 12 tokens).
  * For qualification runs. */
 int mer_set_kernel_path(mer_backend *b, int path);
 

@@ -1,4 +1,5 @@
 // Device helpers shared by the decode kernels (kernels_stream.cu, kernels_flat.cu): integer weights as f16 subnormals, mma.sync.
+// (kernels_gemm.cu: h2_bits.)
 #pragma once
 
 #include <cuda_fp16.h>

@@ -133,7 +133,6 @@ cudaError_t launch_a2a_combine(uint32_t n_tokens, uint32_t D, uint32_t slots, ui
 // `counted`: the pairs per group are already in d.group_count (only honoured when groups_layer_on_grid(d)).
 bool groups_layer_on_grid(const MoeDispatch &d);
 cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaStream_t s, int *launches, bool counted = false);
-// group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
 // Launches `kern` so that it may start while its predecessor in the stream still runs (the kernel waits for it itself).  Between the
 // three or four short kernels of a decode layer this hides launch and set-up, 1 to 2 us each.
 template <typename... P, typename... A>
@@ -149,9 +148,12 @@ inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, unsigned blo
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// Pinned host memory <-> device inside a call's own sequence, a few KB (launch_host_out: `rows` rows of `words` words, `stride` apart,
+// packed; `done`, if not null, receives ++*count last).
 cudaError_t launch_host_in(const void *src, void *dst, size_t words, uint32_t *status, cudaStream_t s, int *launches);
 cudaError_t launch_host_out(const void *src, size_t stride, size_t rows, size_t words, void *dst, uint32_t *count, uint32_t *done, cudaStream_t s, int *launches);
 bool router_sets_status(const MoeDispatch &d);
+// group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s, int *launches,
                           bool group = true);
 cudaError_t launch_groups_from_pairs(const MoeDispatch &d, cudaStream_t s, int *launches);
@@ -164,7 +166,6 @@ cudaError_t launch_pre_moe(const float *x, uint32_t n_tokens, uint32_t D, const 
 cudaError_t launch_dequant(int dtype, const uint8_t *src, float *dst, size_t n_weights, cudaStream_t s);
 // Dequantises projection `matrix` (0 gate, 1 up, 2 down) of a packed expert into row-major f32.
 cudaError_t launch_dequant_packed(int dtype, const uint8_t *expert, int matrix, uint32_t D, uint32_t F, float *dst, cudaStream_t s);
-// Flat gate||up||down block stream -> tile-major fragment layout (same bytes, permuted).
 // What an admission leaves beside the payload: the slot's header and the expert's table entry (slot null: only the entry).
 struct SlotHeader {  // at the start of every occupied slot
   uint64_t epoch;
@@ -180,6 +181,7 @@ struct SlotWrite {
   uint32_t expert_id, dtype;
   uint64_t payload_bytes;
 };
+// Flat gate||up||down block stream -> tile-major fragment layout (same bytes, permuted); then writes the slot.
 cudaError_t launch_repack(int dtype, const uint8_t *flat, uint8_t *packed, uint32_t D, uint32_t F, const SlotWrite &sw, cudaStream_t s);
 cudaError_t launch_slot_write(const SlotWrite &sw, cudaStream_t s);
 cudaError_t launch_raw_matvec(int dtype, const uint8_t *w, const float *x, float *y, size_t rows, size_t cols, cudaStream_t s);

@@ -20,10 +20,12 @@
 //     predicated instructions; every operand is computed in uniform registers) and TMEM owner, 2..9 = epilogue (two groups
 //     of four, one per accumulator buffer), 10..25 = dequantisers (four per quarter of the rows, a block of every weight
 //     stage each), 26 = producer of the weight stages (lanes 0..7 copy one packed tile each).
-// What bounds it: full-width passes run the tensor pipe with the chip at its power limit (2048 tokens on 128 experts of
-// 2048 x 768: 990 W at 1.64 GHz, tensor pipe 63 % active, 345 us for gate/up against 416 us with single CTAs, two 66 KB activation stages
-// and eight dequantiser warps; 4096 tokens on 256 experts of 7168 x 2048: 5.7 ms, 6.6 ms before); passes of a few tokens are bound
-// by reading the weights and by their instructions.  Sorting the passes by width, widest first, changed neither.
+// What bounds it: the MMAs and the way of A through tensor memory, which overlap only in part, and on full-width passes the power
+// limit.  2048 tokens on 128 experts of 2048 x 768, gate/up with the split of its rows: 348 us in a run through 48 layers (902 to 990 W, 1.64
+// to 1.67 GHz; 416 us with single CTAs, two 66 KB activation stages and eight dequantiser warps), 309 us at burst clocks, of which
+// leaving out the second and third product saves 50, the stores to tensor memory 37, both 104, the conversion arithmetic 4; tensor
+// pipe 62 % active.  4096 tokens on 256 experts of 7168 x 2048: 5.7 ms, 6.6 ms before.  Passes of a few tokens are bound by reading the
+// weights and by their instructions.  Sorting the passes by width, widest first, changed neither.
 // Every wait is bounded; on expiry the CTA latches MER_DEVSTAT_TIMEOUT, stops issuing work, waits
 // (bounded) for its copies and MMAs in flight, frees its TMEM and returns.
 #include <cuda.h>
@@ -32,6 +34,7 @@
 #include <type_traits>
 
 #include "../../include/mer_b200.h"
+#include "decode.cuh"
 #include "kernels.h"
 #include "layout.cuh"
 #include "ptx.cuh"
@@ -150,7 +153,6 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }
 __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 
 // Two integers held as the f16 values 1024 + b (b in the low mantissa bits) -> hi = f16(d * (b - zp)),

@@ -2,8 +2,8 @@
 //
 // Data flow per projection phase (gate/up, then down):
 //   * Experts are resident in the tile-major fragment layout of layout.cuh (the reference's bytes,
-//     permuted at admission).  A stage of the ring is two contiguous 16-row tile chunks, each moved
-//     global -> shared memory by ONE bulk async copy (cp.async.bulk, completion on an mbarrier):
+//     permuted at admission).  A stage of the ring is one chunk of each of an item's sixteen 16-row tiles, each chunk
+//     moved global -> shared memory by ONE bulk async copy (cp.async.bulk, completion on an mbarrier):
 //     every byte of an expert is read from HBM once, as a linear stream.
 //   * Warps unpack the integer part of the weights straight into f16 mma.sync A fragments.  A
 //     4-bit or 8-bit field masked into the low mantissa bits of an f16 IS the subnormal value
@@ -20,11 +20,12 @@
 // a CTA owns one 16-row tile of the item over the item's K range: no warp ever waits for another
 // one's partial sums (an earlier version split K across warps and lost a third of its time at the
 // hand-off barrier).  Load balance comes from splitting K across CTAs instead: partial sums go to
-// scratch and the next kernel adds them (k_h_finalize applies SiLU(gate)*up, the combine kernel sums
-// the down partials), always in the same order, so results are deterministic.  Each persistent CTA
-// takes a contiguous item range and rebuilds activation fragments only when its (pass, K split)
-// changes; no atomics on data, no inter-CTA waits.  Every mbarrier wait is bounded: on expiry the
-// warp stops computing, the CTA latches MER_DEVSTAT_TIMEOUT, drains its copies in flight and returns.
+// scratch and the launch's tail adds them behind a grid-wide barrier (SiLU(gate)*up, or the weighted combine
+// of the down partials; kernels of their own where a cooperative launch is refused), always in the same
+// order, so results are deterministic.  Each persistent CTA takes a contiguous item range and rebuilds
+// activation fragments only when its (pass, K split) changes; no atomics on data, and that barrier is the only
+// wait between CTAs.  Every wait is bounded: on expiry the warp stops computing, the CTA latches
+// MER_DEVSTAT_TIMEOUT, drains its copies in flight and returns.
 //
 // What bounds it: the consumers' instructions.  Weights are waited for a tenth of the time; a block of 16 rows takes a warp about
 // 30 instructions (40 with the zero point as every block's accumulator start) at one issue in two cycles of a scheduler's four
@@ -719,18 +720,17 @@ struct Plan {
 constexpr size_t SMEM_LIMIT = 226 * 1024;  // 227 KB per CTA less the kernel's static shared memory
 constexpr uint32_t MAX_KSPLIT = 64;
 
-// Shapes one phase.  An item is 16 tiles (one per warp) over one K split.
-//  * K split: the largest split (whole K, K/2, K/4, ... in multiples of 8 blocks, at least 16 blocks)
-//    that still leaves about eight items per CTA for the expected number of active experts, within
-//    `max_ksplit` (what the partial-sum scratch can hold);
-//  * a stage holds 8 (Q4_0) or 4 block pairs per warp if at least three stages then fit, else half of that, and so on (8: 2 % on one token);
-//  * fragment arrays are sized by the most tokens any group can hold in this dispatch.
 // Shared memory of a plan without its ring.
 size_t fixed_smem(uint32_t kb_split, uint32_t nt, uint32_t max_group_tokens) {
   const uint32_t tp = 4 * nt, frag_cols = 2 * (max_group_tokens < tp ? max_group_tokens : tp);
   return HEADER_BYTES + (size_t)seed_words(kb_split) * 2 * tp * 4 + 128 + (size_t)frag_cols * (kb_split * 64 + 64);
 }
 
+// Shapes one phase.  An item is 16 tiles (one per warp) over one K split.
+//  * K split: multiples of 8 blocks, at least 16, within `max_ksplit` splits (what the partial-sum scratch can hold): the one with
+//    the smallest estimated time of the busiest CTA (below);
+//  * a stage holds 8 (Q4_0) or 4 block pairs per warp if at least three stages then fit, else half of that, and so on (8: 2 % on one token);
+//  * fragment arrays are sized by the most tokens any group can hold in this dispatch.
 Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt, uint32_t max_group_tokens,
                uint32_t active_groups, int n_ctas, uint32_t max_ksplit) {
   const uint32_t bb = dtype == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
@@ -743,7 +743,7 @@ Plan make_plan(int dtype, uint32_t kb_total, uint32_t packed_tiles, uint32_t nt,
   // Pick the K split that minimises the busiest CTA's estimated time, in units of one block step (16 tiles x one
   // block of K).  A CTA gets ceil(items / CTAs) items of kb_split block steps each, pays a fixed cost per item
   // (epilogue) and one activation-fragment rebuild per (pass, K split) unit its contiguous range touches; a rebuild
-  // measures about 4 us, i.e. ~10 block steps of Q8_0 or ~20 of Q4_0 at the rate one SM streams.
+  // measures about 3 us, i.e. ~10 block steps of Q8_0 or ~20 of Q4_0 at the rate one SM streams.
   {
     const double rebuild = dtype == MER_DTYPE_Q4_0 ? 20.0 : 10.0, per_item = 6.0;
     double best = 1e30;

@@ -256,9 +256,11 @@ bool use_stream_path(mer_backend *b, const MoeDispatch &d) {
   return stream_ffn_supported(d.dtype, d.D, d.F) && b->d_stream_scratch != nullptr;
 }
 
-constexpr uint32_t GEMM_MIN_MEAN_TOKENS = 12;  // mean tokens per expert from which the tcgen05 GEMM path takes over (measured:
-                                               // at a mean of 8-9 the streaming kernels are level or ahead, at 16 the GEMM kernels
-                                               // win by 5 % on Mixtral-sized and by 50 % on Qwen3-sized experts)
+// Mean tokens per expert from which the tcgen05 GEMM path takes over: one line between the formats' own.  Us a layer, streaming / GEMM,
+// at means of 8, 12, 16, 20: Q8_0, 128 experts of 2048 x 768: 242 / 256, 311 / 266, 375 / 264, 469 / 283, and 64 of 2048 x 1408: 213 / 227, 266 / 229,
+// 328 / 238, 397 / 242 (they cross at 9); Q4_0, 8 of 4096 x 14336: 307 / 522, 403 / 524, 471 / 526, 594 / 526, and 64 of 7168 x 2048: 582 / 946,
+// 750 / 948, 936 / 952, 1131 / 971 (they cross at 17).
+constexpr uint32_t GEMM_MIN_MEAN_TOKENS = 12;
 
 // Chooses the kernel family of a dispatch and binds its scratch (call before the grouping kernel, which
 // cuts the groups into passes of d.tokens_per_pass).
