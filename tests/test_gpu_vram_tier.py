@@ -167,15 +167,22 @@ def test_admission_does_not_wait_for_work_enqueued_on_the_default_stream_behind_
         for _ in range(4):  # plain launches, the capture, a replay
             b.moe_layer_forward_device(0, xd.data_ptr(), B, out.data_ptr(), 0)
         torch.cuda.synchronize()
-        b.moe_layer_forward_device(0, xd.data_ptr(), B, out.data_ptr(), 0)
-        torch.cuda._sleep(1_000_000_000)  # half a second
-        behind.record()
-        for e in range(E):
-            b.admit(e, 2, other)  # returns when the payload is in its slot
-        overlapped = not behind.query()
-        torch.cuda.synchronize()
+        gen, overlapped = 1, False
+        for _ in range(3):  # a host that stalls for half a second in between proves nothing
+            for e in range(E):
+                b.admit(e, gen + 1, blobs[e])
+            gen += 2
+            b.moe_layer_forward_device(0, xd.data_ptr(), B, out.data_ptr(), 0)
+            torch.cuda._sleep(1_000_000_000)  # half a second
+            behind.record()
+            for e in range(E):
+                b.admit(e, gen, other)  # returns when the payload is in its slot
+            overlapped = not behind.query()
+            torch.cuda.synchronize()
+            assert rel_rms_err(out.cpu().numpy(), ref) <= 1e-3
+            if overlapped:
+                break
         assert overlapped, "the uploads waited for work behind the layer"
-        assert rel_rms_err(out.cpu().numpy(), ref) <= 1e-3
 
 
 def test_an_admission_that_waits_for_a_layer_leaves_the_processor_to_others():
@@ -197,16 +204,23 @@ def test_an_admission_that_waits_for_a_layer_leaves_the_processor_to_others():
             torch.cuda._sleep(1000)
         b.moe_layer_forward_device(0, x.data_ptr(), B, out.data_ptr(), side.cuda_stream)
         torch.cuda.synchronize()
-        free = time.perf_counter()
-        b.admit(1, 2, blob, wait=False)
-        b.synchronize()
-        free = time.perf_counter() - free
-        with torch.cuda.stream(side):
-            torch.cuda._sleep(700_000_000)
-        b.moe_layer_forward_device(0, x.data_ptr(), B, out.data_ptr(), side.cuda_stream)
-        wall, cpu = time.perf_counter(), time.process_time()
-        b.admit(1, 3, blob, wait=False)
-        wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
-        b.synchronize()
-    # one thread awake all the time would spend `wall`; seven threads may be busy while the payload itself moves
-    assert wall > 0.15 and cpu <= 0.5 * (wall - free) + 7 * free, (wall, cpu, free)
+        gen = 1
+
+        def admit_timed():
+            nonlocal gen
+            gen += 1
+            wall, cpu = time.perf_counter(), time.process_time()
+            b.admit(1, gen, blob, wait=False)
+            wall, cpu = time.perf_counter() - wall, time.process_time() - cpu
+            b.synchronize()
+            return wall, cpu
+
+        _, busy = admit_timed()  # copying alone
+        for _ in range(3):  # a host that stalls in front of the admission proves nothing
+            with torch.cuda.stream(side):
+                torch.cuda._sleep(700_000_000)
+            b.moe_layer_forward_device(0, x.data_ptr(), B, out.data_ptr(), side.cuda_stream)
+            wall, cpu = admit_timed()
+            if wall > 0.15 and cpu - busy <= 0.5 * wall:
+                break
+    assert wall > 0.15 and cpu - busy <= 0.5 * wall, (wall, cpu, busy)  # one thread awake all the time would spend `wall`
