@@ -46,6 +46,11 @@ __device__ __forceinline__ void unpack_q8(uint32_t lo, uint32_t hi, uint32_t (&r
   r[2] = (hi ^ 0x80808080u) & 0x00FF00FFu;
   r[3] = ((hi >> 8) ^ 0x00808080u) & 0x00FF00FFu;
 }
+// The same for bytes that are stored as q + 128 (layout.cuh): four instructions for eight weights instead of six.
+__device__ __forceinline__ void unpack_q8_biased(uint32_t lo, uint32_t hi, uint32_t (&r)[4]) {
+  r[0] = lo & 0x00FF00FFu, r[1] = __byte_perm(lo, 0u, 0x4341);
+  r[2] = hi & 0x00FF00FFu, r[3] = __byte_perm(hi, 0u, 0x4341);
+}
 __device__ __forceinline__ float2 h2_to_f2(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2 *>(&v)); }
 
 __device__ __forceinline__ uint32_t h2_bits(__half2 v) { return *reinterpret_cast<uint32_t *>(&v); }

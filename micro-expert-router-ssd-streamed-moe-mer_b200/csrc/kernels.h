@@ -27,6 +27,17 @@ struct RouterDev {
 
 #define MER_EP_MAX_WORLD 16
 
+// A token pass of the streaming kernels: at most tokens_per_pass (4 or 8) pairs of one expert.  All that a CTA needs to know of it in
+// one round trip to L2.
+struct __align__(64) PassDesc {
+  const uint8_t *base;  // the expert's payload, null = not resident
+  uint32_t count, pad;
+  uint32_t pair[8];
+};
+
+// Zero-point terms of a row of K values: a run of this many for the hi parts, then one for the lo parts.
+__host__ __device__ inline uint32_t image_seed_stride(uint32_t K) { return (K / 32 + 3) & ~3u; }
+
 // One MoE dispatch: P = n_tokens * slots pairs (token, slot); pair p belongs to token p / slots.
 // Pairs are grouped by expert: group g covers perm[offsets[g] .. offsets[g+1]) and runs expert
 // group_expert[g].
@@ -56,8 +67,15 @@ struct MoeDispatch {
   uint32_t active_groups_hint;  // expected number of non-empty groups (shapes the work split)
   uint32_t expected_pairs;      // expected number of pairs that reach a group (0 = all of them; fewer under expert parallelism)
   // token passes of the streaming FFN (null when the generic kernels run): groups cut into runs of at most
-  // tokens_per_pass pairs, built by the grouping kernels; amax = per-pair max |h| cell, zeroed there too
-  uint32_t *pass_group, *pass_start, *pass_count, *n_passes, *amax;
+  // tokens_per_pass pairs, built by the grouping kernels
+  uint32_t *pass_group, *pass_start, *pass_count, *n_passes;
+  PassDesc *pass_desc;      // the same for the streaming kernels (null: the GEMM path), which find the first pass of a group in pass_group
+  uint64_t *taken;          // [2][MER_MAX_CTAS1] items taken from either end of every CTA's range, zeroed by the grouping kernels
+  uint32_t *amax;           // [2][scratch_pairs] max |gate| and max |up| over a pair's partial sums (float bits), zeroed by the grouping kernels
+  // Activation images of the streaming kernels (act_image.cuh).  The tokens' lie where the outputs of the down projection go later,
+  // the hidden rows' in `h`; both share the seeds.  Null: nobody multiplies them.
+  void *x_rows;
+  float *act_seeds, *x_un, *h_un;  // *_un: 2^24 / scale of every row
   uint32_t tokens_per_pass;
   // Work split of the streaming kernels, built with the passes: item_bounds[phase * MER_MAX_CTAS1 + b] = first item of
   // CTA b in that phase (b = 0 .. n_ctas), items weighted by the tokens of their pass (null: the GEMM path).
@@ -192,9 +210,11 @@ cudaError_t launch_f32_to_f16(const float *src, uint16_t *dst, size_t n, cudaStr
 bool stream_ffn_supported(int dtype, uint32_t D, uint32_t F);
 size_t stream_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F);
 cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid);
-// Points d.pass_* / d.amax into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
+// Points d.pass_*, d.amax and the activation images into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
 void stream_bind(MoeDispatch &d, void *scratch, int sm_count);
 cudaError_t launch_reduce_parts(const MoeDispatch &d, cudaStream_t s, int *launches);
+// Images of all of the dispatch's tokens, where neither router nor grouping made them on the way.
+cudaError_t launch_x_images(const MoeDispatch &d, cudaStream_t s, int *launches);
 
 // kernels_flat.cu: one expert on the flat block stream (up to eight tokens), in one cooperative launch.
 bool flat_expert_supported(const void *expert, const void *x, uint32_t D, uint32_t F, uint32_t n_tokens);

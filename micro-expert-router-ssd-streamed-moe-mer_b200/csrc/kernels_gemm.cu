@@ -431,11 +431,10 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
 #pragma unroll
           for (int t = 0; t < 4; t++) {  // values 8t .. 8t+7
             const uint2 w = lds64(src + packed_piece(g, t) * 16 + half * 8);
-            const uint32_t w0 = w.x ^ 0x80808080u, w1 = w.y ^ 0x80808080u;
-            dq2(__byte_perm(w0, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
-            dq2(__byte_perm(w0, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
-            dq2(__byte_perm(w1, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
-            dq2(__byte_perm(w1, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
+            dq2(__byte_perm(w.x, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
+            dq2(__byte_perm(w.x, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
+            dq2(__byte_perm(w.y, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
+            dq2(__byte_perm(w.y, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
           }
         } else {
           // block-pair record: 16 bytes per (g, t) = words (slot g, blk 0), (slot g+8, blk 0), (slot g, blk 1), (slot g+8, blk 1);
@@ -715,6 +714,7 @@ void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) 
   stream_bind(d, stream_scratch, sm_count);  // pass tables live in the streaming scratch
   d.tokens_per_pass = bn;
   d.item_bounds = nullptr;  // items are dealt round-robin
+  d.pass_desc = nullptr, d.x_rows = nullptr, d.taken = nullptr;
 }
 
 cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid) {

@@ -9,6 +9,7 @@
 
 #include <cuda_fp16.h>
 #include "../../include/mer_b200.h"
+#include "act_image.cuh"
 #include "layout.cuh"
 #include "passes.cuh"
 #include "route.cuh"
@@ -44,7 +45,7 @@ __device__ __forceinline__ float weight_at(const MoeDispatch &d, const uint8_t *
     PackedAddr a = packed_locate<DT>(d.D, d.F, matrix, row, col);
     float sc = f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(base + a.scale));
     uint32_t byte = base[a.quant];
-    int q = DT == MER_DTYPE_Q8_0 ? (int)(int8_t)byte : (int)((col & 16u) ? (byte >> 4) : (byte & 15u)) - 8;
+    int q = DT == MER_DTYPE_Q8_0 ? (int)byte - 128 : (int)((col & 16u) ? (byte >> 4) : (byte & 15u)) - 8;
     return __fmul_rn(sc, (float)q);
   }
   const size_t bb = DT == MER_DTYPE_Q8_0 ? MER_Q8_BLOCK_BYTES : MER_Q4_BLOCK_BYTES;
@@ -122,15 +123,33 @@ __device__ void build_item_bounds(const MoeDispatch &d, uint32_t n_passes, const
   }
 }
 
+// Entry of the pass table.
+__device__ __forceinline__ void put_pass(const MoeDispatch &d, uint32_t pass, uint32_t g, const uint8_t *base, uint32_t start, uint32_t count) {
+  if (d.pass_desc) {
+    d.pass_desc[pass].base = base, d.pass_desc[pass].count = count;
+  } else {
+    d.pass_group[pass] = g, d.pass_start[pass] = start, d.pass_count[pass] = count;
+  }
+}
+__device__ __forceinline__ const uint8_t *expert_payload(const MoeDispatch &d, uint32_t eid) { return eid < d.max_experts ? d.expert_ptr[eid] : nullptr; }
+__device__ __forceinline__ void clear_maxima(const MoeDispatch &d, uint32_t pair) {
+  if (d.pass_desc) d.amax[pair] = 0, d.amax[d.scratch_pairs + pair] = 0;
+}
+__device__ __forceinline__ void clear_taken(const MoeDispatch &d) {  // by a CTA of 256 threads
+  if (d.taken && threadIdx.x < d.n_ctas) d.taken[threadIdx.x] = 0, d.taken[MER_MAX_CTAS1 + threadIdx.x] = 0;
+}
+
 // Cuts every group into passes of at most d.tokens_per_pass pairs (the unit the streaming FFN works
 // on) and clears the per-pair max cells.  One CTA of 256 threads; `off` = the group offsets.
-__device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
+// `perm_ready`: the pairs are in d.perm, else k_group_scatter puts them into the passes.
+__device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off, bool perm_ready) {
   __shared__ uint32_t s_pcnt[257];
   __shared__ uint8_t s_cost[1024];  // cost of each of the first 1024 passes (the weighted work split below)
   const uint32_t tpp = d.tokens_per_pass, P = d.n_tokens * d.slots;
   const uint32_t tpp_shift = 31 - __clz(tpp);  // tokens per pass is a power of two (4 or 8; 16 .. 128 for the GEMM kernels)
 #pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < P; i += 256) d.amax[i] = 0;
+  for (uint32_t i = threadIdx.x; i < P; i += 256) clear_maxima(d, i);
+  clear_taken(d);
   const uint32_t per = (d.n_groups + 255) / 256;
   const uint32_t g0 = threadIdx.x * per, g1 = min(g0 + per, d.n_groups);
   uint32_t mine = 0;
@@ -159,21 +178,21 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off) {
   for (uint32_t g = g0; g < g1; g++) {
     const uint32_t beg = off[g], end = off[g + 1];
     const PassCut cut(end - beg, tpp, tpp_shift);
+    const uint8_t *base = d.pass_desc && cut.passes ? expert_payload(d, d.group_expert[g]) : nullptr;
     uint32_t st = beg;
+    if (d.pass_desc) d.pass_group[g] = np;
 #pragma unroll 1
     for (uint32_t i = 0; i < cut.passes; i++) {
       const uint32_t cnt = cut.count(i, end - st);
-      d.pass_group[np] = g;
-      d.pass_start[np] = st;
-      d.pass_count[np] = cnt;
+      put_pass(d, np, g, base, st, cnt);
+      if (d.pass_desc && perm_ready)
+#pragma unroll 1
+        for (uint32_t j = 0; j < cnt; j++) d.pass_desc[np].pair[j] = d.perm[st + j];
       if (np < 1024) s_cost[np] = cnt > 4 ? 13 : 10;
       np++, st += cnt;
     }
   }
-  if (threadIdx.x == 0) {
-    d.n_passes[0] = s_pcnt[256];
-    d.n_passes[1] = d.n_passes[2] = 0;  // arrival counters of the streaming kernels' grid-wide barriers
-  }
+  if (threadIdx.x == 0) d.n_passes[0] = s_pcnt[256];
   if (!d.item_bounds) return;
   __shared__ uint32_t s_cum[1025];
   const uint32_t n_passes = s_pcnt[256];
@@ -286,13 +305,16 @@ __global__ void __launch_bounds__(256) k_group_scan(RouterDev r, MoeDispatch d) 
   if (threadIdx.x == 0) d.offsets[G] = s_run;
   __threadfence_block();
   __syncthreads();
-  if (d.pass_group) build_passes_block(d, d.offsets);
+  if (d.pass_group) build_passes_block(d, d.offsets, false);
 }
 __global__ void __launch_bounds__(256) k_group_scatter(RouterDev r, MoeDispatch d) {
   const uint32_t P = d.n_tokens * d.slots;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
     const uint32_t k = pair_group_key(r, d, p);
-    if (k != MER_NONE) d.perm[d.offsets[k] + atomicAdd(d.group_cursor + k, 1u)] = p;
+    if (k == MER_NONE) continue;
+    const uint32_t rank = atomicAdd(d.group_cursor + k, 1u);
+    d.perm[d.offsets[k] + rank] = p;
+    if (d.pass_desc) d.pass_desc[d.pass_group[k] + rank / d.tokens_per_pass].pair[rank % d.tokens_per_pass] = p;
   }
 }
 // The same for at most 32 pairs of the streaming kernels, in registers of one warp: sorted position of every pair, the pairs
@@ -300,11 +322,13 @@ __global__ void __launch_bounds__(256) k_group_scatter(RouterDev r, MoeDispatch 
 // as the kernels that follow need for the weights of half of them.
 __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
   __shared__ uint32_t s_np, s_cum[33];
+  clear_taken(d);
   const uint32_t P = d.n_tokens * d.slots, tpp = d.tokens_per_pass;
   const bool weighted = tpp == 8;
   if (threadIdx.x < 32) {
     const uint32_t p = threadIdx.x, before = (1u << p) - 1;
     const uint32_t eid = p < P ? __ldcg(d.pair_expert + p) : MER_NONE;
+    const uint8_t *base = expert_payload(d, eid);
     uint32_t key = eid;  // group index; unfilled slots sort last
     if (eid != MER_NONE) key = p % d.slots >= r.top_k || eid == r.shared_expert_id ? r.num_experts : eid - r.id_base;
     const uint32_t same = __match_any_sync(0xffffffffu, key), rank = __popc(same & before);
@@ -319,12 +343,12 @@ __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
       if (rank == 0) d.group_expert[key] = eid;
     }
     const uint32_t count = min(tpp, __popc(same) - rank), pass = __popc(starters & ((1u << pos) - 1));
-    if (starts) d.pass_group[pass] = key, d.pass_start[pass] = pos, d.pass_count[pass] = count;
-    if (p < P) d.amax[p] = 0;
+    if (starts) put_pass(d, pass, key, base, pos, count);
+    if (valid) d.pass_desc[__popc(starters & ((2u << pos) - 1)) - 1].pair[rank % tpp] = p;
+    if (p < P) clear_maxima(d, p);
     if (p == 0) {
       d.offsets[d.n_groups] = n_valid;  // all of the offsets that anyone reads after the streaming kernels
       d.n_passes[0] = s_np = np;
-      d.n_passes[1] = d.n_passes[2] = 0;
     }
     if (weighted) {
       if (starts) s_cum[pass + 1] = count > 4 ? 13 : 10;
@@ -359,16 +383,17 @@ constexpr uint32_t MID_PAIRS = 2048, MID_GROUPS = 512;
 // `s_pair` [P]: group (16 bits) and rank of every pair.  Loops stay rolled: the code runs once, cold.
 __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint32_t *s_pair) {
   constexpr uint32_t PER_G = MID_GROUPS / 256;
-  __shared__ uint32_t s_cnt[MID_GROUPS], s_cum[MID_PAIRS / 8 + MID_GROUPS + 1];  // s_cum: passes of eight
+  __shared__ uint32_t s_cnt[MID_GROUPS], s_pass[MID_GROUPS], s_cum[MID_PAIRS / 8 + MID_GROUPS + 1];  // s_cum: passes of eight
   __shared__ uint64_t s_part[8];
   const uint32_t P = d.n_tokens * d.slots, G = d.n_groups, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t tpp = d.tokens_per_pass, shift = 31 - __clz(tpp);
   const bool bounds = d.item_bounds != nullptr, weighted = bounds && tpp == 8;  // (passes of four can be more than s_cum holds)
   for (uint32_t i = tid; i < MID_GROUPS; i += 256) s_cnt[i] = 0;
+  clear_taken(d);
   __syncthreads();
 #pragma unroll 1
   for (uint32_t p = tid; p < P; p += 256) {
-    d.amax[p] = 0;
+    clear_maxima(d, p);
     const uint32_t eid = __ldcg(d.pair_expert + p);
     uint32_t v = MER_NONE;
     if (eid != MER_NONE) {
@@ -406,16 +431,18 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
   for (uint32_t i = 0; i < PER_G; i++) {
     const uint32_t g = tid * PER_G + i, n = (uint32_t)mine[i] & 0xFFFFF, beg = (uint32_t)base & 0xFFFFF;
     uint32_t pass = (uint32_t)(base >> 20) & 0xFFFFF, cum = (uint32_t)(base >> 40);
-    s_cnt[g] = beg;
+    s_cnt[g] = beg, s_pass[g] = pass;
     if (g < G) {
-      d.group_expert[g] = g < r.num_experts ? r.id_base + g : r.shared_expert_id;
+      const uint32_t eid = g < r.num_experts ? r.id_base + g : r.shared_expert_id;
+      const uint8_t *payload = d.pass_desc && n ? expert_payload(d, eid) : nullptr;
+      d.group_expert[g] = eid;
       d.offsets[g] = beg;
       const PassCut cut(n, tpp, shift);
       uint32_t st = 0;
 #pragma unroll 1
       for (uint32_t j = 0; j < cut.passes; j++, pass++) {
         const uint32_t cnt = cut.count(j, n - st);
-        d.pass_group[pass] = g, d.pass_start[pass] = beg + st, d.pass_count[pass] = cnt;
+        put_pass(d, pass, g, payload, beg + st, cnt);
         st += cnt;
         if (weighted) s_cum[pass] = cum, cum += cnt > 4 ? 13 : 10;
       }
@@ -425,14 +452,16 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
   if (tid == 0) {
     d.offsets[G] = (uint32_t)total & 0xFFFFF;
     d.n_passes[0] = n_passes;
-    d.n_passes[1] = d.n_passes[2] = 0;
     if (weighted) s_cum[n_passes] = (uint32_t)(total >> 40);
   }
   __syncthreads();
 #pragma unroll 1
   for (uint32_t p = tid; p < P; p += 256) {
     const uint32_t v = s_pair[p];
-    if (v != MER_NONE) d.perm[s_cnt[v >> 16] + (v & 0xFFFF)] = p;
+    if (v == MER_NONE) continue;
+    const uint32_t g = v >> 16, rank = v & 0xFFFF;
+    d.perm[s_cnt[g] + rank] = p;
+    if (d.pass_desc) d.pass_desc[s_pass[g] + (rank >> shift)].pair[rank & (tpp - 1)] = p;
   }
   if (bounds) build_item_bounds(d, n_passes, weighted ? s_cum : nullptr);
 }
@@ -553,7 +582,7 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
   __syncthreads();
 #pragma unroll 1
   for (uint32_t g = tid; g <= G; g += nt) d.offsets[g] = s_off[g];
-  if (d.pass_group) build_passes_block(d, s_off);
+  if (d.pass_group) build_passes_block(d, s_off, true);
 }
 
 // Router logits of a large batch as a tiled fp32 GEMM: logits[t][e] = x[t] . w[e].  A CTA computes TT tokens x TE experts; K
@@ -661,7 +690,7 @@ __global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r,
 }
 
 template <int ROWS>
-__global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int pre, int group_here) {
+__global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int pre, int group_here, uint32_t logit_ctas) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t E = r.num_experts, D = d.D;
   const uint32_t tile = blockIdx.y, t0 = tile * ROUTER_TT;
@@ -670,12 +699,27 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   const uint32_t e0 = blockIdx.x * ROWS;
   __shared__ float s_part[ROWS][ROUTER_TT][ROUTER_WARPS + 1];  // [row][token][warp]
   __shared__ float s_logit[ROUTER_TT][ROWS];                  // used when one CTA covers all experts
-  const bool single = gridDim.x == 1 && !pre;
+  const bool single = logit_ctas == 1 && !pre;
   // With the grouping done here, status bits gather in a scratch word, which the last CTA publishes: no launch clears them.
   uint32_t *const status = group_here == 1 ? d.counters + max_tokens + 1 : d.status;
+  // What the steps behind the logits read once a layer, and the layers in between have long pushed out of L2: a miss each, on their
+  // critical path.
+  if (tile == 0 && warp == 1) {
+    const uint32_t line = 128 / 4 * (blockIdx.x * 32 + lane);  // a CTA covers 32 lines
+    if (line < E) {
+      if (r.logit_bias) prefetch_l2(r.logit_bias + line);
+      if (r.correction_bias) prefetch_l2(r.correction_bias + line);
+    }
+    if (d.pass_desc && line / 2 < E && r.id_base + line / 2 < d.max_experts) prefetch_l2(d.expert_ptr + r.id_base + line / 2);
+  }
   grid_dep_wait();
   grid_dep_launch();
 
+  if (blockIdx.x >= logit_ctas) {  // CTAs beside the logits' make the activation images of the tile's tokens
+    const uint32_t tt = blockIdx.x - logit_ctas;
+    if (tt < n_here) build_x_image(d, t0 + tt, threadIdx.x, ROUTER_THREADS, &s_part[0][0][0]);
+    return;
+  }
   if (pre) {
     // logits are already in d.logits (k_router_logits_tiled)
   } else if ((D & 1023u) == 0) {
@@ -750,7 +794,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   if (!single && !pre) {
     if (threadIdx.x == 0) {
       const uint32_t prev = arrive_acq_rel(&d.counters[tile]);
-      s_flag = (prev == gridDim.x - 1);
+      s_flag = (prev == logit_ctas - 1);
       if (s_flag) d.counters[tile] = 0;  // re-arm for the next launch
     }
     __syncthreads();
@@ -811,7 +855,13 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_groups_layer(RouterDev r, Mo
 }
 
 // Routing supplied by the caller: mode 0 = every pair is its own group, mode 1 = one group.
-__global__ void k_groups_from_pairs(MoeDispatch d, int single_group) {
+// The first CTA; the others make the tokens' activation images.
+__global__ void __launch_bounds__(256) k_groups_from_pairs(MoeDispatch d, int single_group) {
+  if (blockIdx.x > 0) {
+    __shared__ float s_max[8];
+    build_x_image(d, blockIdx.x - 1, threadIdx.x, 256, s_max);
+    return;
+  }
   const uint32_t P = d.n_tokens * d.slots;
   for (uint32_t p = threadIdx.x; p < P; p += blockDim.x) {
     d.perm[p] = p;
@@ -832,7 +882,7 @@ __global__ void k_groups_from_pairs(MoeDispatch d, int single_group) {
   }
   if (d.pass_group) {
     __syncthreads();  // the offsets written above are read back by the whole block
-    build_passes_block(d, d.offsets);
+    build_passes_block(d, d.offsets, true);
   }
 }
 
@@ -1106,7 +1156,7 @@ __global__ void k_dequant_packed(const uint8_t *__restrict__ expert, int matrix,
     PackedAddr a = packed_locate<DT>(D, F, matrix, row, col);
     float sc = f16_bits_to_f32(*reinterpret_cast<const uint16_t *>(expert + a.scale));
     uint32_t byte = expert[a.quant];
-    int q = DT == MER_DTYPE_Q8_0 ? (int)(int8_t)byte : (int)((col & 16u) ? (byte >> 4) : (byte & 15u)) - 8;
+    int q = DT == MER_DTYPE_Q8_0 ? (int)byte - 128 : (int)((col & 16u) ? (byte >> 4) : (byte & 15u)) - 8;
     dst[i] = __fmul_rn(sc, (float)q);
   }
 }
@@ -1145,6 +1195,7 @@ __global__ void k_repack(const uint8_t *__restrict__ flat, uint8_t *__restrict__
         uint2 v;
         v.x = (uint32_t)src[1 + 4 * t] | ((uint32_t)src[2 + 4 * t] << 16);
         v.y = (uint32_t)src[3 + 4 * t] | ((uint32_t)src[4 + 4 * t] << 16);
+        v.x ^= 0x80808080u, v.y ^= 0x80808080u;  // q + 128
         *reinterpret_cast<uint2 *>(packed + a.quant) = v;
       }
     }
@@ -1219,14 +1270,15 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
   uint32_t rows = 8;
   while (!tiled && rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
-  const dim3 grid(tiled ? 1 : (E + rows - 1) / rows, tiles);
+  const uint32_t logit_ctas = tiled ? 1 : (E + rows - 1) / rows;
+  const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
   const bool grid_grouping = group && P >= GRID_GROUPING_PAIRS && d.group_count != nullptr;
   auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0);
+  cudaError_t e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0, logit_ctas);
   if (e != cudaSuccess) return e;
   if (launches) (*launches)++;
   if (grid_grouping) {  // the router has counted the pairs per group
@@ -1242,6 +1294,8 @@ bool groups_layer_on_grid(const MoeDispatch &d) { return d.n_tokens * d.slots >=
 
 cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaStream_t s, int *launches, bool counted) {
   const uint32_t G = d.n_groups, P = d.n_tokens * d.slots;
+  const cudaError_t ei = launch_x_images(d, s, launches);
+  if (ei != cudaSuccess) return ei;
   if (groups_layer_on_grid(d)) {  // a large dispatch: count / scan / scatter over the grid
     const unsigned blocks = (P + 1023) / 1024;
     if (!counted) k_group_count<<<blocks, 256, 0, s>>>(r, d);
@@ -1262,7 +1316,7 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
 }
 
 cudaError_t launch_groups_from_pairs(const MoeDispatch &d, cudaStream_t s, int *launches) {
-  k_groups_from_pairs<<<1, 256, 0, s>>>(d, d.n_groups == 1);
+  k_groups_from_pairs<<<d.x_rows ? 1 + d.n_tokens : 1, 256, 0, s>>>(d, d.n_groups == 1);
   if (launches) (*launches)++;
   return cudaGetLastError();
 }

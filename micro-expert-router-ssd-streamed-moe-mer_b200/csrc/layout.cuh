@@ -1,8 +1,8 @@
 // Resident (HBM slot) layout of an expert: "tile-major fragment order".
 //
-// The bytes of the reference's gate||up||down block stream are kept one for one (same scales,
-// same quants, same total size); only their order changes at admission so that the streaming
-// kernels read every operand with aligned 128-bit shared-memory loads:
+// The blocks of the reference's gate||up||down stream are kept one for one (same scales, same quants, same total size); their
+// order changes at admission so that the streaming kernels read every operand with aligned 128-bit shared-memory loads, and
+// a Q8_0 quant q is stored as the byte q + 128, which is what the kernels make f16 integers of:
 //
 //   region 0, gate/up: F/8 tiles.  Tile tt holds 16 row slots: slots 0..7 = gate rows 8tt..8tt+7,
 //                      slots 8..15 = up rows 8tt..8tt+7 (so SiLU(gate)*up pairs up inside a thread).

@@ -9,9 +9,9 @@ namespace {
 constexpr uint32_t SPIN_LIMIT = 1u << 16;  // polls per bounded wait; a poll suspends for tens of microseconds
 
 // Arrival counters between CTAs: what the CTA wrote before (a __syncthreads() in front) is visible to whoever acquires the count.
-__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t *counter) {
+__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t *counter, uint32_t by = 1) {
   uint32_t v;
-  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(v) : "l"(counter) : "memory");
+  asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], %2;" : "=r"(v) : "l"(counter), "r"(by) : "memory");
   return v;
 }
 __device__ __forceinline__ uint32_t load_acquire(const uint32_t *p) {
@@ -24,6 +24,8 @@ __device__ __forceinline__ uint32_t load_acquire(const uint32_t *p) {
 // it touches anything the predecessor reads or writes; without the attribute both are no-ops.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -49,6 +51,16 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
       "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
       : "r"(addr), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same without suspending.
+__device__ __forceinline__ bool mbar_test(const uint64_t *bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
 }

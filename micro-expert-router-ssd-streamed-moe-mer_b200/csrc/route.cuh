@@ -98,11 +98,8 @@ __device__ Pick route_token_reg(const RouterDev &r, float *s_score, float *s_sel
       if (g < ng) {
 #pragma unroll 4
         for (uint32_t i = lane % per; i < gs; i += per) {
-          const float s = s_sel[g * gs + i];
-          if (s > top1)
-            top2 = top1, top1 = s;
-          else if (s > top2)
-            top2 = s;
+          const float v = s_sel[g * gs + i], s = v == v ? v : -CUDART_INF_F;
+          top2 = fmaxf(top2, fminf(top1, s)), top1 = fmaxf(top1, s);
         }
       }
 #pragma unroll 1
@@ -125,32 +122,43 @@ __device__ Pick route_token_reg(const RouterDev &r, float *s_score, float *s_sel
         else gkey[1] = INT_MIN;
       }
     }
+    const uint32_t inv = (65536 + gs - 1) / gs;  // i / gs = i * inv >> 16 as i * gs < 65536
 #pragma unroll
     for (int j = 0; j < EJ; j++) {
       const uint32_t i = lane + 32 * j;
-      if (i < E && !(taken >> (i / gs) & 1)) keys[j] = INT_MIN;
+      if (i < E && !(taken >> (i * inv >> 16) & 1)) keys[j] = INT_MIN;
     }
   }
-  // top-k by (selection desc, id asc), non-finite skipped (gating.rs:315-333, 429-441)
+  // top-k by (selection desc, id asc), non-finite skipped (gating.rs:315-333, 429-441).  Every lane sorts its own keys first
+  // (neighbours change places while the later one is larger: equal keys keep their order), so that a pick is one warp maximum over the
+  // lanes' first ones, a vote and a shift in the lane that wins.
+  uint32_t ord[EJ];  // j of the key
+#pragma unroll
+  for (int j = 0; j < EJ; j++) ord[j] = j;
+#pragma unroll
+  for (int round = 0; round < EJ; round++) {
+#pragma unroll
+    for (int j = round & 1; j + 1 < EJ; j += 2) {
+      const bool swap = keys[j + 1] > keys[j];
+      const int ka = keys[j], kb = keys[j + 1];
+      const uint32_t oa = ord[j], ob = ord[j + 1];
+      keys[j] = swap ? kb : ka, keys[j + 1] = swap ? ka : kb, ord[j] = swap ? ob : oa, ord[j + 1] = swap ? oa : ob;
+    }
+  }
   uint32_t my_id = MER_NONE, n_sel = 0;
 #pragma unroll 1
   for (uint32_t n = 0; n < k; n++) {
-    int bk = INT_MIN;
-    uint32_t bj = 0;
-#pragma unroll
-    for (int j = 0; j < EJ; j++)
-      if (keys[j] > bk) bk = keys[j], bj = j;  // ascending j keeps the lowest id on ties
-    const int top_key = __reduce_max_sync(0xffffffffu, bk);
+    const int top_key = __reduce_max_sync(0xffffffffu, keys[0]);
     if (top_key == INT_MIN) break;  // nothing left to pick
-    const uint32_t tied = __ballot_sync(0xffffffffu, bk == top_key);
+    const uint32_t tied = __ballot_sync(0xffffffffu, keys[0] == top_key);
     uint32_t top_lane = __ffs(tied) - 1;
     if (tied & (tied - 1))  // equal keys in several lanes: the lowest id wins
-      top_lane = __reduce_min_sync(0xffffffffu, bk == top_key ? lane + 32 * bj : MER_NONE) & 31u;
-    const uint32_t top_j = __shfl_sync(0xffffffffu, bj, top_lane);
+      top_lane = __reduce_min_sync(0xffffffffu, keys[0] == top_key ? lane + 32 * ord[0] : MER_NONE) & 31u;
+    const uint32_t top_j = __shfl_sync(0xffffffffu, ord[0], top_lane);
     if (lane == top_lane) {
 #pragma unroll
-      for (int j = 0; j < EJ; j++)
-        if ((uint32_t)j == bj) keys[j] = INT_MIN;
+      for (int j = 0; j + 1 < EJ; j++) keys[j] = keys[j + 1], ord[j] = ord[j + 1];
+      keys[EJ - 1] = INT_MIN;
     }
     if (lane == (n & 31)) my_id = top_lane + 32 * top_j;
     n_sel++;
