@@ -31,6 +31,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "../../include/mer_b200.h"
@@ -55,8 +56,11 @@ constexpr uint32_t MAX_RING = 8;
 // copies), issues the group's MMAs and commits done[] in both CTAs, which releases all of it.
 constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16;
 constexpr uint32_t CHUNK_K = 64, CHUNKS = GROUP * 32 / CHUNK_K;  // a row's piece of a chunk is 128 bytes, the swizzle span
-constexpr uint32_t PASS_TOKENS = 128;    // tokens of a pass at most: N of one MMA, and the columns of an accumulator buffer
-constexpr uint32_t PART_BYTES = PASS_TOKENS / PAIR * 128, CHUNK_BYTES = 2 * PART_BYTES, B_STAGE = CHUNKS * CHUNK_BYTES;  // hi rows, then lo rows
+constexpr uint32_t PASS_TOKENS = 256;    // tokens of a pass at most: N of one MMA
+// A pass of up to BUF_TOKENS takes one of the two accumulator buffers and one activation stage a group; a wider one takes both buffers (its MMAs then
+// wait for the epilogue of the item before) and two stages: what it saves is a second conversion of the weights.
+constexpr uint32_t BUF_TOKENS = 128;
+constexpr uint32_t PART_BYTES = BUF_TOKENS / PAIR * 128, CHUNK_BYTES = 2 * PART_BYTES, B_STAGE = CHUNKS * CHUNK_BYTES;  // hi rows, then lo rows
 static_assert(RAW_BLOCKS % GROUP == 0 && DQ_WARPS == 4 * RAW_BLOCKS && A_STAGES % RAW_BLOCKS == 0, "a block of a weight stage for each of a quarter's warps");
 constexpr float POW2_SCALE_TARGET = 9;   // activations are scaled so that the row maximum lies in [256, 512)
 
@@ -171,13 +175,29 @@ __host__ __device__ constexpr uint32_t pass_width(uint32_t count) { return (coun
 // rule looks at the group, not at the pass, so that the order of a token's additions depends only on how many tokens its
 // expert received, never on which pass it landed in: results stay bit-identical from run to run although large
 // dispatches are grouped with atomics.
-constexpr uint32_t SPLIT_TOKENS = PASS_TOKENS / 2;
+constexpr uint32_t SPLIT_TOKENS = BUF_TOKENS / 2;
 
 struct Ring {
   uint32_t stage = 0, round = 0, n;
   __device__ explicit Ring(uint32_t n_) : n(n_) {}
   __device__ void advance() {
     if (++stage == n) stage = 0, round++;
+  }
+};
+
+// The ring of activation stages (an even number of at most eight) as its producer and the issuer count it: a group of blocks takes one stage, or
+// two adjacent ones from an even one on.
+struct StageRing {
+  uint32_t n, at = 0, phases = 0;  // bit i of phases: parity of the next use of stage i's barrier
+  __device__ explicit StageRing(uint32_t n_) : n(n_) {}
+  __device__ __forceinline__ uint32_t take(bool wide, uint32_t &parity) {
+    if (wide) at = (at + 1) & ~1u;
+    if (at >= n) at = 0;
+    const uint32_t st = at;
+    parity = phases >> st & 1;
+    phases ^= 1u << st;
+    at += wide ? 2 : 1;
+    return st;
   }
 };
 
@@ -271,27 +291,32 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // one stage = one group of blocks of K of this CTA's half of the pass's rows; lane l copies chunk l / 2, the hi parts
     // (even l) or the lo parts.  A stage is free again when the MMAs of the group that used it have run: the
     // issuer's done[] commit says so.
-    Ring rb(p.n_b);
+    StageRing rb(p.n_b);
+    uint32_t holder = 0;  // lane i: 1 + the group that took stage i last
     uint32_t pg = 0;  // groups issued so far, over all items (the issuer counts the same way)
     const uint32_t chunk = lane >> 1, part = lane & 1, K = p.kb_total * 32;
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
       if (!next_item(item, pstart, pcount)) continue;
       const uint32_t width = pass_width(pcount), row = pstart + rank * (width / PAIR);
       const CUtensorMap *map = &maps.m[width / 16 - 1];
+      const bool wide = width > BUF_TOKENS;
+      const uint32_t part_bytes = wide ? 2 * PART_BYTES : PART_BYTES;
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, pg++) {
-        if (pg >= p.n_b) {
-          const uint32_t sp = pg - p.n_b;
-          ok = mbar_wait_cluster(&done[sp % DONE_RING], (sp / DONE_RING) & 1);
-        }
+        uint32_t parity;
+        const uint32_t stage = rb.take(wide, parity);
+        // 1 + the newest group that has had one of these stages
+        const bool mine = lane == stage || (wide && lane == stage + 1);
+        const uint32_t busy = __reduce_max_sync(0xffffffffu, mine ? holder : 0u);
+        if (mine) holder = pg + 1;
+        if (busy) ok = mbar_wait_cluster(&done[(busy - 1) % DONE_RING], ((busy - 1) / DONE_RING) & 1);
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (rank == 0 && lane == 0) mbar_expect_tx(&b_full[rb.stage], CHUNKS * width * 2 * 128);  // both CTAs' bytes
+        if (rank == 0 && lane == 0) mbar_expect_tx(&b_full[stage], CHUNKS * width * 2 * 128);  // both CTAs' bytes
         __syncwarp();
         if (lane < 2 * CHUNKS)
-          tile_g2s(smem_u32(s_b) + rb.stage * B_STAGE + chunk * CHUNK_BYTES + part * PART_BYTES, map,
-                   part * K + (gi * CHUNKS + chunk) * CHUNK_K, row, leader_addr(&b_full[rb.stage]));
-        rb.advance();
+          tile_g2s(smem_u32(s_b) + stage * B_STAGE + (chunk * 2 + part) * part_bytes, map, part * K + (gi * CHUNKS + chunk) * CHUNK_K, row,
+                   leader_addr(&b_full[stage]));
       }
     }
     if (!ok) {
@@ -305,9 +330,9 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     if (rank == 0) {
     // The whole warp walks the loops and waits (every value it computes is warp-uniform); the elected lane issues.
     // one step = one 32-value block of K: two instructions of 16 values for each of the three operand pairings
-    Ring rb(p.n_b);
+    StageRing rb(p.n_b);
     const uint32_t leader = elect_one();  // the warp is converged here; the same lane issues from now on
-    uint32_t n_done = 0;  // items issued so far: accumulator buffer = n_done & 1, its k-th use has k = n_done >> 1
+    uint32_t next_buf = 0, uses0 = 0, uses1 = 0;  // accumulator buffer of the next item that takes one; items that have used either
     uint32_t grp = 0;     // groups of GROUP blocks issued so far, over all items; A-stage half = grp & 1
     // B descriptors differ only in their start-address field: one base, then 64-bit adds of (byte offset >> 4).
     // (The ring lies well inside the 256 KB the 14-bit field spans, so the adds never carry out of it.)
@@ -319,12 +344,19 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     auto run_item = [&](auto width_tag, auto split_tag) {
       constexpr uint32_t LO = decltype(split_tag)::value ? SPLIT_TOKENS : 0;  // columns of the small products
       constexpr uint32_t idesc = instr_desc(decltype(width_tag)::value);
-      const uint32_t buf = n_done & 1, use = n_done >> 1;
+      constexpr bool WIDE = decltype(width_tag)::value > BUF_TOKENS;
+      constexpr uint32_t PART = WIDE ? 2 * PART_BYTES : PART_BYTES;
+      const uint32_t buf = WIDE ? 0 : next_buf;
       const uint32_t d_tmem = tmem_base + buf * 128;
       for (uint32_t st = 0; st < p.kb_total && ok; st += GROUP, grp++) {
         const uint32_t ag = grp % A_RING;
-        if (st == 0 && use > 0) ok = mbar_wait_tmem(&acc_empty[buf], (use - 1) & 1);  // the buffer's previous item has been drained
-        if (ok) ok = mbar_wait_cluster(&b_full[rb.stage], rb.round & 1);
+        uint32_t parity;
+        const uint32_t stage = rb.take(WIDE, parity);
+        if (st == 0) {  // the previous item of the buffer (of both) has been drained
+          if ((WIDE || buf == 0) && uses0 > 0) ok = mbar_wait_tmem(&acc_empty[0], (uses0 - 1) & 1);
+          if ((WIDE || buf == 1) && uses1 > 0) ok = mbar_wait_tmem(&acc_empty[1], (uses1 - 1) & 1) && ok;
+        }
+        if (ok) ok = mbar_wait_cluster(&b_full[stage], parity);
         if (ok) ok = mbar_wait_tmem(&a_full[ag], (grp / A_RING) & 1);
         ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the vote also tells the compiler so
         if (!ok) break;
@@ -332,21 +364,25 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
 #pragma unroll
         for (uint32_t b4 = 0; b4 < GROUP; b4++) {
           const uint32_t a_hi = tmem_base + TMEM_A0 + (ag * GROUP + b4) * A_STAGE_COLS, a_lo = a_hi + 16;
-          const uint64_t b_blk = b_desc0 + (uint64_t)((rb.stage * B_STAGE + (b4 >> 1) * CHUNK_BYTES + (b4 & 1) * 64) >> 4);
+          const uint64_t b_blk = b_desc0 + (uint64_t)((stage * B_STAGE + (b4 >> 1) * 2 * PART + (b4 & 1) * 64) >> 4);
 #pragma unroll
           for (uint32_t j = 0; j < 2; j++) {  // 16 values of K per instruction: 8 TMEM columns of A, 32 bytes of a row of B
-            const uint64_t dbh = b_blk + (uint64_t)(j * 2), dbl = dbh + (PART_BYTES >> 4);
+            const uint64_t dbh = b_blk + (uint64_t)(j * 2), dbl = dbh + (PART >> 4);
             const uint32_t acc = (b4 == 0 && j == 0) ? (st != 0) : 1u;  // the item's first MMA overwrites the accumulator
             tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc, acc);
             tc_mma_ts(leader, d_tmem + LO, a_hi + j * 8, dbl, idesc, LO ? acc : 1u);
             tc_mma_ts_acc(leader, d_tmem + LO, a_lo + j * 8, dbh, idesc);
           }
         }
-        rb.advance();
         tc_commit(leader, &done[grp % DONE_RING]);  // frees the group's A stages and its activation stage, in both CTAs
-        if (st + GROUP >= p.kb_total) tc_commit(leader, &acc_full[buf]);
+        if (st + GROUP >= p.kb_total) {
+          tc_commit(leader, &acc_full[buf]);
+          if (WIDE) tc_commit(leader, &acc_full[1]);
+        }
       }
-      n_done++;
+      if (WIDE || buf == 0) uses0++;
+      if (WIDE || buf == 1) uses1++;
+      next_buf = WIDE ? 0 : buf ^ 1;
     };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
       if (!next_item(item, pstart, pcount, &split)) continue;
@@ -370,7 +406,15 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
           case 5: run_item(std::integral_constant<uint32_t, 80>{}, F{}); break;
           case 6: run_item(std::integral_constant<uint32_t, 96>{}, F{}); break;
           case 7: run_item(std::integral_constant<uint32_t, 112>{}, F{}); break;
-          default: run_item(std::integral_constant<uint32_t, 128>{}, F{}); break;
+          case 8: run_item(std::integral_constant<uint32_t, 128>{}, F{}); break;
+          case 9: run_item(std::integral_constant<uint32_t, 144>{}, F{}); break;
+          case 10: run_item(std::integral_constant<uint32_t, 160>{}, F{}); break;
+          case 11: run_item(std::integral_constant<uint32_t, 176>{}, F{}); break;
+          case 12: run_item(std::integral_constant<uint32_t, 192>{}, F{}); break;
+          case 13: run_item(std::integral_constant<uint32_t, 208>{}, F{}); break;
+          case 14: run_item(std::integral_constant<uint32_t, 224>{}, F{}); break;
+          case 15: run_item(std::integral_constant<uint32_t, 240>{}, F{}); break;
+          default: run_item(std::integral_constant<uint32_t, 256>{}, F{}); break;
         }
       }
     }
@@ -483,28 +527,33 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     const uint32_t buf = (warp - W_EPI0) >> 2, gw = (warp - W_EPI0) & 3;  // group, warp within the group
     float *s_un = reinterpret_cast<float *>(smem + 1024 + buf * 2048 + 512);
     float **s_row = reinterpret_cast<float **>(smem + 1024 + buf * 2048 + 1024);  // down phase: each token's output row
-    uint32_t n_item = 0, used = 0;  // resident items seen by the CTA; uses of this group's buffer
+    uint32_t next_buf = 0, used = 0;  // buffer of the next resident item that takes one; uses of this group's
     // A group whose bounded wait expired goes "dead": it stops touching TMEM and waiting but keeps walking the items, so
     // that the group's named barriers always see all four warps.
     bool dead = false;
     for (uint32_t item = item_beg; item < n_items; item += item_step) {
       const uint32_t mt = (item % m_pairs) * PAIR + rank;
       const bool resident = next_item(item, pstart, pcount, &split) != nullptr;
+      // A wide item fills both buffers, and each group drains its own.
+      const bool wide = pcount > BUF_TOKENS;
+      const uint32_t col0 = wide ? buf * BUF_TOKENS : 0, cols = min(pcount - col0, BUF_TOKENS);  // this group's columns of the pass
       if (resident) {
-        if ((n_item++ & 1) != buf) continue;  // the other group's item
-      } else if (buf != 0) {
-        continue;  // items of missing experts are zero-filled by group 0
+        const uint32_t which = next_buf;
+        next_buf = wide ? 0 : which ^ 1;
+        if (!wide && which != buf) continue;  // the other group's item
+      } else if (!wide && buf != 0) {
+        continue;  // narrow items of missing experts are zero-filled by group 0
       }
       // The pass's pair indices and un-scale factors go to shared memory (one column per thread of the group), fetched
       // before the accumulator is waited for so that their latency hides behind the item's MMAs; the column loop then
       // reads them as broadcasts.
       {
         const uint32_t c = gw * 32 + lane;
-        const bool have = c < pcount;
-        const float un = have ? __ldg(p.unscale + pstart + c) : 0.0f;
+        const bool have = c < cols;
+        const float un = have ? __ldg(p.unscale + pstart + col0 + c) : 0.0f;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + buf) : "memory");  // the group has finished reading the previous item's tables
         s_un[c] = un;
-        if (p.phase == 1) s_row[c] = have ? pair_output_row(d, p.out, __ldg(d.perm + pstart + c)) : nullptr;
+        if (p.phase == 1) s_row[c] = have ? pair_output_row(d, p.out, __ldg(d.perm + pstart + col0 + c)) : nullptr;
         asm volatile("bar.sync %0, 128;" ::"r"(1 + buf) : "memory");
       }
       if (resident && !dead) {
@@ -520,7 +569,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
       const bool is_gate = (lane & 8) == 0;
       const bool clamp = d.swiglu_limit > 0.0f && isfinite(d.swiglu_limit);
       constexpr int EC = 16;  // columns (tokens) at a time
-      for (uint32_t cbase = 0; cbase < pcount && mt < m_tiles; cbase += EC) {
+      for (uint32_t cbase = 0; cbase < cols && mt < m_tiles; cbase += EC) {
         float val[EC];
         if (resident && !dead) {
           uint32_t v[EC];
@@ -558,15 +607,15 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
           }
           // h in the order of the groups: its rows are then the rows of the down phase's passes
           const uint32_t col = cbase + (is_gate ? 0 : EC / 2);
-          float *dst = p.out + (size_t)(pstart + col) * d.F + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
+          float *dst = p.out + (size_t)(pstart + col0 + col) * d.F + (mt * 8 + (row >> 4)) * 8 + (lane & 7);
 #pragma unroll
           for (int i = 0; i < EC / 2; i++)
-            if (col + i < pcount) dst[(size_t)i * d.F] = h[i];
+            if (col + i < cols) dst[(size_t)i * d.F] = h[i];
         } else {
           const uint32_t off = mt * 128 + row;
 #pragma unroll
           for (int i = 0; i < EC; i++)
-            if (cbase + i < pcount) s_row[cbase + i][off] = val[i];
+            if (cbase + i < cols) s_row[cbase + i][off] = val[i];
         }
       }
       if (resident && !dead) {
@@ -707,7 +756,13 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
   const uint64_t P = (uint64_t)d.n_tokens * d.slots;
   const uint32_t groups = d.active_groups_hint ? d.active_groups_hint : 1;
   const uint64_t mean = (d.expected_pairs ? d.expected_pairs : P) / groups;
-  return mean < min_mean_tokens || P > d.scratch_pairs ? 0 : PASS_TOKENS;
+  if (mean < min_mean_tokens || P > d.scratch_pairs) return 0;
+  // Passes of up to 256 tokens instead of 128 save conversions of the weights (129 to 256 tokens of an expert: half of them) and leave the MMAs idle while
+  // an item's epilogue drains both buffers, some 5000 cycles.  That pays where an item's K is long and where there are enough items to
+  // share out evenly.  Us a pass, 128 / 256: 4096 tokens on 256 experts of 7168 x 2048 9516 / 8827; 2048 on 128 of 2048 x 768 (24 blocks of K
+  // in the down phase) 658 / 705; 256 on 8 of 4096 x 14336 (two items a pair of CTAs in the down phase) 690 / 720.
+  const bool long_k = d.D / 32 >= 128 && d.F / 32 >= 64, many = (uint64_t)groups * (std::min(2 * d.F, d.D) / 256) >= 8 * 74;
+  return long_k && many ? PASS_TOKENS : BUF_TOKENS;
 }
 
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) {
