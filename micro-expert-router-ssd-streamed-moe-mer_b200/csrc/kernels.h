@@ -14,6 +14,8 @@
 // Router parameters resident on the device (one per installed layer).
 struct RouterDev {
   const float *w;                // [E x D]
+  const uint8_t *w_split;        // the same in f16 parts and fragment order (kernels_logits.cu), or null: rows or values that it does not take
+  const float *w_unscale;        // [E rounded up to 8] of its rows
   const float *correction_bias;  // [E] or null
   const float *logit_bias;       // [E] or null
   uint32_t num_experts, top_k;
@@ -53,6 +55,7 @@ struct MoeDispatch {
   uint32_t *group_expert;   // [n_groups]
   uint32_t *offsets;        // [n_groups + 1]
   uint32_t *perm;           // [P]
+  uint32_t *pos;            // [P] place of every pair in perm, MER_NONE for a pair without a group (null: the streaming kernels)
   uint32_t *group_count;    // [n_groups] zero between dispatches: per-group pair counts of the grid-wide grouping,
   uint32_t *group_cursor;   //   and its scatter cursors (both null: always group in one CTA)
   float *h;                 // [P x F]   silu(gate) * up
@@ -170,8 +173,12 @@ inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, unsigned blo
 // packed; `done`, if not null, receives ++*count last).
 cudaError_t launch_host_in(const void *src, void *dst, size_t words, uint32_t *status, cudaStream_t s, int *launches);
 cudaError_t launch_host_out(const void *src, size_t stride, size_t rows, size_t words, void *dst, uint32_t *count, uint32_t *done, cudaStream_t s, int *launches);
-bool router_sets_status(const MoeDispatch &d);
-// group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
+// kernels_logits.cu: router logits of a few hundred tokens and more on the tensor cores.  `sets`: partial sums of K that the logits scratch then holds.
+bool router_split_supported(uint32_t D);
+size_t router_split_bytes(uint32_t E, uint32_t D);
+cudaError_t launch_split_router(const float *w, uint32_t E, uint32_t D, uint8_t *out, float *unscale, cudaStream_t s);
+cudaError_t launch_router_logits(const RouterDev &r, const MoeDispatch &d, uint32_t *status, uint32_t *sets, cudaStream_t s);
+// With `group` it leaves d.status written: no need to clear it first.  group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s, int *launches,
                           bool group = true);
 cudaError_t launch_groups_from_pairs(const MoeDispatch &d, cudaStream_t s, int *launches);
@@ -211,7 +218,7 @@ bool stream_ffn_supported(int dtype, uint32_t D, uint32_t F);
 size_t stream_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F);
 cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid);
 // Points d.pass_*, d.amax and the activation images into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
-void stream_bind(MoeDispatch &d, void *scratch, int sm_count);
+void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm = false);
 cudaError_t launch_reduce_parts(const MoeDispatch &d, cudaStream_t s, int *launches);
 // Images of all of the dispatch's tokens, where neither router nor grouping made them on the way.
 cudaError_t launch_x_images(const MoeDispatch &d, cudaStream_t s, int *launches);

@@ -636,19 +636,29 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
   }
 }
 
+// Four values of a row -> their hi and lo parts.
+__device__ __forceinline__ void split_values(float4 v, float sc, uint2 &hi, uint2 &lo) {
+  const float a = v.x * sc, b = v.y * sc, c = v.z * sc, e = v.w * sc;
+  const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, e);
+  const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+  hi = make_uint2(h2_bits(h0), h2_bits(h1));
+  lo = make_uint2(h2_bits(__floats2half2_rn(a - f0.x, b - f0.y)), h2_bits(__floats2half2_rn(c - f1.x, e - f1.y)));
+}
+
 // Rows of activations -> rows of their f16 hi parts and lo parts, [hi K | lo K], after an exact power-of-two scaling of the
 // row, and its inverse.  Row i of the output belongs to the i-th pair in group order, so that a pass is a run of rows and
-// one copy fetches a chunk of all of them; its source is row i of h, or with `perm` row perm[i] / slots of the tokens
-// (a token that eight experts share is converted eight times; rows picked by the GEMM's own copies instead,
-// four per gather, took 80 cycles per four rows and doubled the GEMM's time).  TPR threads per row.
-template <int TPR>
-__global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ act, uint32_t K, const uint32_t *__restrict__ perm,
+// one copy fetches a chunk of all of them.  The source is row i of h, or with `pos` the tokens' rows: a row is then read and converted once and
+// written to the places of all of its `slots` pairs (rows picked by the GEMM's own copies instead, four per gather, took 80 cycles per four
+// rows and doubled the GEMM's time).  TPR threads per row.  What bounds it is writing the rows.  With a row of x read and converted by each of
+// its pairs: 4096 tokens of 7168 for nine experts each 299 us.
+template <int TPR, bool TOKENS>
+__global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ act, uint32_t n_rows, uint32_t K, const uint32_t *__restrict__ pos,
                                                     uint32_t slots, const uint32_t *__restrict__ n_grouped, uint16_t *__restrict__ out,
                                                     float *__restrict__ unscale) {
   const uint32_t i = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, t = threadIdx.x % TPR;
-  const bool have = i < *n_grouped;  // fewer than the pairs of the dispatch under expert parallelism
+  const bool have = TOKENS ? i < n_rows : i < *n_grouped;  // fewer than the pairs of the dispatch under expert parallelism
   if (TPR <= 32 && !have) return;
-  const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)(have && perm ? perm[i] / slots : i) * K);
+  const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)(have ? i : 0) * K);
   float mx = 0.0f;
   bool nan = false;
   if (have) {
@@ -678,26 +688,50 @@ __global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ ac
   } else if (mx != mx || isinf(mx)) {
     sc = mx;  // non-finite activations poison the row, as they would in fp32
   }
-  if (t == 0) unscale[i] = 1.0f / sc;
-  uint2 *hi = reinterpret_cast<uint2 *>(out + (size_t)i * 2 * K), *lo = hi + K / 4;
+  if (!TOKENS) {
+    if (t == 0) unscale[i] = 1.0f / sc;
+    uint2 *hi = reinterpret_cast<uint2 *>(out + (size_t)i * 2 * K), *lo = hi + K / 4;
 #pragma unroll 4
-  for (uint32_t k = t; k < K / 4; k += TPR) {
-    const float4 v = __ldg(src + k);
-    const float a = v.x * sc, b = v.y * sc, c = v.z * sc, e = v.w * sc;
-    const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(c, e);
-    const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-    hi[k] = make_uint2(h2_bits(h0), h2_bits(h1));
-    lo[k] = make_uint2(h2_bits(__floats2half2_rn(a - f0.x, b - f0.y)), h2_bits(__floats2half2_rn(c - f1.x, e - f1.y)));
+    for (uint32_t k = t; k < K / 4; k += TPR) split_values(__ldg(src + k), sc, hi[k], lo[k]);
+    return;
+  }
+  constexpr uint32_t S = 9, U = 4;  // places a pass over the row writes to; steps of it in flight
+#pragma unroll 1
+  for (uint32_t s0 = 0; s0 < slots; s0 += S) {
+    uint32_t at[S];
+#pragma unroll
+    for (uint32_t j = 0; j < S; j++) {
+      at[j] = s0 + j < slots ? __ldg(pos + (size_t)i * slots + s0 + j) : MER_NONE;
+      if (t == 0 && at[j] != MER_NONE) unscale[at[j]] = 1.0f / sc;
+    }
+#pragma unroll 1
+    for (uint32_t k0 = t; k0 < K / 4; k0 += U * TPR) {
+      float4 v[U];
+#pragma unroll
+      for (uint32_t u = 0; u < U; u++) v[u] = k0 + u * TPR < K / 4 ? __ldg(src + k0 + u * TPR) : make_float4(0, 0, 0, 0);
+#pragma unroll
+      for (uint32_t u = 0; u < U; u++) {
+        const uint32_t k = k0 + u * TPR;
+        if (k >= K / 4) break;
+        uint2 hi, lo;
+        split_values(v[u], sc, hi, lo);
+#pragma unroll
+        for (uint32_t j = 0; j < S; j++) {
+          if (at[j] == MER_NONE) continue;
+          uint2 *dst = reinterpret_cast<uint2 *>(out + (size_t)at[j] * 2 * K);
+          dst[k] = hi, dst[K / 4 + k] = lo;
+        }
+      }
+    }
   }
 }
 
-void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *perm, uint32_t slots, const uint32_t *n_grouped,
+void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *pos, uint32_t slots, const uint32_t *n_grouped,
                        uint16_t *out, float *unscale, cudaStream_t s) {
   // a warp per row keeps short rows of large batches cheap; long rows, and few of them, want more loads in flight
-  if (K <= 2048 && n_rows >= 2048)
-    k_split_rows<32><<<(n_rows + 7) / 8, 256, 0, s>>>(act, K, perm, slots, n_grouped, out, unscale);
-  else
-    k_split_rows<256><<<n_rows, 256, 0, s>>>(act, K, perm, slots, n_grouped, out, unscale);
+  const bool warps = K <= 2048 && n_rows >= 2048;
+  auto kern = pos ? (warps ? k_split_rows<32, true> : k_split_rows<256, true>) : (warps ? k_split_rows<32, false> : k_split_rows<256, false>);
+  kern<<<warps ? (n_rows + 7) / 8 : n_rows, 256, 0, s>>>(act, n_rows, K, pos, slots, n_grouped, out, unscale);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -766,7 +800,7 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
 }
 
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn) {
-  stream_bind(d, stream_scratch, sm_count);  // pass tables live in the streaming scratch
+  stream_bind(d, stream_scratch, sm_count, true);  // pass tables live in the streaming scratch
   d.tokens_per_pass = bn;
   d.item_bounds = nullptr;  // items are dealt round-robin
   d.pass_desc = nullptr, d.x_rows = nullptr, d.taken = nullptr;
@@ -785,7 +819,7 @@ cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes,
 
   for (int phase = 0; phase < 2; phase++) {
     const uint32_t K = phase == 0 ? d.D : d.F;
-    launch_split_rows(phase == 0 ? d.x : d.h, P, K, phase == 0 ? d.perm : nullptr, d.slots, d.offsets + d.n_groups, rows, unscale, s);
+    launch_split_rows(phase == 0 ? d.x : d.h, phase == 0 ? d.n_tokens : P, K, phase == 0 ? d.pos : nullptr, d.slots, d.offsets + d.n_groups, rows, unscale, s);
     ActMaps maps;
     if (!activation_maps(&maps, rows, P, K)) return cudaErrorNotSupported;
     GemmParams p{};

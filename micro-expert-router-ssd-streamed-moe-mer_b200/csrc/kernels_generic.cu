@@ -8,6 +8,9 @@
 #include "ptx.cuh"
 
 #include <cuda_fp16.h>
+
+#include <algorithm>
+
 #include "../../include/mer_b200.h"
 #include "act_image.cuh"
 #include "layout.cuh"
@@ -135,6 +138,10 @@ __device__ __forceinline__ const uint8_t *expert_payload(const MoeDispatch &d, u
 __device__ __forceinline__ void clear_maxima(const MoeDispatch &d, uint32_t pair) {
   if (d.pass_desc) d.amax[pair] = 0, d.amax[d.scratch_pairs + pair] = 0;
 }
+__device__ __forceinline__ void put_pair(const MoeDispatch &d, uint32_t at, uint32_t pair) {
+  d.perm[at] = pair;
+  if (d.pos) d.pos[pair] = at;
+}
 __device__ __forceinline__ void clear_taken(const MoeDispatch &d) {  // by a CTA of 256 threads
   if (d.taken && threadIdx.x < d.n_ctas) d.taken[threadIdx.x] = 0, d.taken[MER_MAX_CTAS1 + threadIdx.x] = 0;
 }
@@ -254,7 +261,9 @@ __global__ void __launch_bounds__(256) k_group_count(RouterDev r, MoeDispatch d)
     if (k != MER_NONE) atomicAdd(d.group_count + k, 1u);
   }
 }
-__global__ void __launch_bounds__(256) k_group_scan(RouterDev r, MoeDispatch d) {
+// `status`: where the router has left its bits, to be published (null: nothing to do).
+__global__ void __launch_bounds__(256) k_group_scan(RouterDev r, MoeDispatch d, uint32_t *status) {
+  if (status && threadIdx.x == 0) *d.status = atomicExch(status, 0u);
   const uint32_t G = d.n_groups;
   for (uint32_t g = threadIdx.x; g < G; g += blockDim.x) {
     d.group_expert[g] = (g < r.num_experts) ? r.id_base + g : r.shared_expert_id;
@@ -311,9 +320,12 @@ __global__ void __launch_bounds__(256) k_group_scatter(RouterDev r, MoeDispatch 
   const uint32_t P = d.n_tokens * d.slots;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
     const uint32_t k = pair_group_key(r, d, p);
-    if (k == MER_NONE) continue;
+    if (k == MER_NONE) {
+      if (d.pos) d.pos[p] = MER_NONE;
+      continue;
+    }
     const uint32_t rank = atomicAdd(d.group_cursor + k, 1u);
-    d.perm[d.offsets[k] + rank] = p;
+    put_pair(d, d.offsets[k] + rank, p);
     if (d.pass_desc) d.pass_desc[d.pass_group[k] + rank / d.tokens_per_pass].pair[rank % d.tokens_per_pass] = p;
   }
 }
@@ -458,9 +470,12 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
 #pragma unroll 1
   for (uint32_t p = tid; p < P; p += 256) {
     const uint32_t v = s_pair[p];
-    if (v == MER_NONE) continue;
+    if (v == MER_NONE) {
+      if (d.pos) d.pos[p] = MER_NONE;
+      continue;
+    }
     const uint32_t g = v >> 16, rank = v & 0xFFFF;
-    d.perm[s_cnt[g] + rank] = p;
+    put_pair(d, s_cnt[g] + rank, p);
     if (d.pass_desc) d.pass_desc[s_pass[g] + (rank >> shift)].pair[rank & (tpp - 1)] = p;
   }
   if (bounds) build_item_bounds(d, n_passes, weighted ? s_cum : nullptr);
@@ -549,7 +564,9 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
       const uint32_t same = __match_any_sync(0xffffffffu, k);
       if (k != MER_NONE) {
         const uint32_t rank = __popc(same & ((1u << lane) - 1));
-        d.perm[s_off[k] + s_cnt[warp * G + k] + rank] = p;
+        put_pair(d, s_off[k] + s_cnt[warp * G + k] + rank, p);
+      } else if (d.pos && p < p1) {
+        d.pos[p] = MER_NONE;
       }
       __syncwarp();
       if (k != MER_NONE && (same & ((1u << lane) - 1)) == 0) s_cnt[warp * G + k] += __popc(same);
@@ -576,7 +593,8 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
 #pragma unroll 1
     for (uint32_t p = tid; p < P; p += nt) {
       uint32_t k = key_of(p);
-      if (k != MER_NONE) d.perm[s_off[k] + atomicAdd(&s_cnt[k], 1u)] = p;
+      if (k != MER_NONE) put_pair(d, s_off[k] + atomicAdd(&s_cnt[k], 1u), p);
+      else if (d.pos) d.pos[p] = MER_NONE;
     }
   }
   __syncthreads();
@@ -585,112 +603,81 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
   if (d.pass_group) build_passes_block(d, s_off, true);
 }
 
-// Router logits of a large batch as a tiled fp32 GEMM: logits[t][e] = x[t] . w[e].  A CTA computes TT tokens x TE experts; K
-// runs in chunks of KC values that cp.async double-buffers in shared memory.  A warp owns 32 tokens x 64 experts over a
-// slice of every chunk; a thread holds 8 tokens x 8 experts (rows ty + 4 i and tx + 8 j: neighbouring lanes read neighbouring
-// rows, whose stride of 4 mod 32 floats keeps every 128-bit load conflict-free), i.e. 16 shared 128-bit loads per 256 FMAs.
-// The slices' partial sums are added at the end in warp order.  k_router then runs with `pre` set and only scores / selects.
-// What bounds it is reading operand rows from L2: the 64 x 128 tile reads half as much per FMA as 32 x 64
-// (4096 x 256 x 7168 with selection and grouping: 710 us before, 614 now).
-constexpr int RL_WARPS = 8, RL_THREADS = 32 * RL_WARPS;
-template <int TT, int TE, int KC>
-struct LogitsTile {
-  static constexpr int SPATIAL = TT / 32 * (TE / 64), SLICES = RL_WARPS / SPATIAL, SLICE_K = KC / SLICES, LD = KC + 4;
-  static constexpr size_t BUF = (size_t)(TT + TE) * LD, SMEM = 2 * BUF * 4;  // floats per buffer; bytes
-};
-template <int TT, int TE, int KC>
-__global__ void __launch_bounds__(RL_THREADS) k_router_logits_tiled(RouterDev r, MoeDispatch d, uint32_t ksplit) {
-  using S = LogitsTile<TT, TE, KC>;
-  constexpr int RL_TT = TT, RL_TE = TE, RL_KC = KC, RL_LD = S::LD, PIECES = KC / 4, STEP = RL_THREADS / PIECES;
-  constexpr size_t RL_BUF = S::BUF;
-  extern __shared__ __align__(16) float sm[];
-  const uint32_t E = r.num_experts, D = d.D, T = d.n_tokens;
-  const uint32_t t0 = blockIdx.y * RL_TT, e0 = blockIdx.x * RL_TE;
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t where = warp % S::SPATIAL, slice = warp / S::SPATIAL;
-  const uint32_t ty = where % (TT / 32) * 32 + (lane >> 3), tx = where / (TT / 32) * 64 + (lane & 7);
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; i++)
-#pragma unroll
-    for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
-  // global -> shared: a thread copies one 16-byte piece of every STEP-th row
-  const uint32_t lr = tid / PIECES, lc = tid % PIECES * 4;
-  auto issue_chunk = [&](uint32_t k0, uint32_t buf) {
-    float *xs = sm + buf * RL_BUF, *ws = xs + RL_TT * RL_LD;
-#pragma unroll
-    for (int i = 0; i < RL_TT / STEP; i++) {
-      const uint32_t row = STEP * i + lr;
-      const float *src = d.x + (size_t)min(t0 + row, T - 1) * D + k0 + lc;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(xs + row * RL_LD + lc)), "l"(src) : "memory");
+// Selection for the TT tokens from t0 on, whose logits are there, one warp per token; the last of `n_tiles` CTAs that get here groups all pairs.
+// `direct`: the logits [TT][stride] in shared memory, or null: `sets` partial sums of them in d.logits ([sets][T][E], added in order).
+template <int TT>
+__device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispatch &d, uint32_t t0, uint32_t n_tiles, const float *direct, uint32_t stride, uint32_t sets,
+                                              bool recheck, uint8_t *smem_raw, uint32_t *status, uint32_t max_tokens, int group_here) {
+  const uint32_t E = r.num_experts, D = d.D, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ uint32_t s_last;
+  __shared__ uint32_t s_groups[TT][64];
+  __shared__ float s_gscore[TT][64];
+  uint32_t picked = MER_NONE;
+  if (warp < min((uint32_t)TT, d.n_tokens - t0)) {
+    float *s_score = reinterpret_cast<float *>(smem_raw) + (size_t)warp * 2 * E;  // [E] scores (become mixing weights)
+    float *s_sel = s_score + E;                                                    // [E] selection scores
+    uint8_t *s_ok = smem_raw + (size_t)TT * 2 * E * 4 + (size_t)warp * E;          // [E] allowed & not yet taken
+    const uint32_t token = t0 + warp;
+    bool nan = false;
+    for (uint32_t i = lane; i < E; i += 32) {
+      float v = direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
+      for (uint32_t z = 1; z < sets; z++) v += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i);
+      s_score[i] = v;
+      nan |= v != v;
     }
-#pragma unroll
-    for (int j = 0; j < RL_TE / STEP; j++) {
-      const uint32_t row = STEP * j + lr;
-      const float *src = r.w + (size_t)min(e0 + row, E - 1) * D + k0 + lc;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(ws + row * RL_LD + lc)), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  // A batch of a few hundred tokens makes too few tiles for the SMs: blockIdx.z then takes one of `ksplit` slices of K
-  // and writes its partial logits to set z of d.logits ([ksplit][T][E]); k_router adds the sets in order.
-  const uint32_t n_chunks = D / RL_KC / ksplit, c_base = blockIdx.z * n_chunks;
-  issue_chunk(c_base * RL_KC, 0);
-  for (uint32_t c = 0; c < n_chunks; c++) {
-    if (c + 1 < n_chunks) {
-      issue_chunk((c_base + c + 1) * RL_KC, (c + 1) & 1);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");  // chunk c has landed (this thread's pieces)
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();  // ... and everybody else's
-    const float *xs = sm + (c & 1) * RL_BUF, *ws = xs + RL_TT * RL_LD;
-#pragma unroll 2
-    for (int kk = 0; kk < S::SLICE_K; kk += 4) {
-      const int k = slice * S::SLICE_K + kk;
-      float4 a[8], b[8];
-#pragma unroll
-      for (int i = 0; i < 8; i++) a[i] = *reinterpret_cast<const float4 *>(xs + (ty + 4 * i) * RL_LD + k);
-#pragma unroll
-      for (int j = 0; j < 8; j++) b[j] = *reinterpret_cast<const float4 *>(ws + (tx + 8 * j) * RL_LD + k);
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j < 8; j++) {
-          acc[i][j] = fmaf(a[i].x, b[j].x, acc[i][j]);
-          acc[i][j] = fmaf(a[i].y, b[j].y, acc[i][j]);
-          acc[i][j] = fmaf(a[i].z, b[j].z, acc[i][j]);
-          acc[i][j] = fmaf(a[i].w, b[j].w, acc[i][j]);
-        }
-    }
-    __syncthreads();  // the buffer may be refilled two iterations from now
-  }
-  // partial sums of slices 1.. through shared memory (the operand buffers are done with), added to slice 0's in order
-  float *red = sm;  // [SLICES - 1][RL_TT * RL_TE]
-  static_assert((S::SLICES - 1) * RL_TT * RL_TE <= 2 * RL_BUF, "the partial sums fit the operand buffers");
-  if (slice > 0) {
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int j = 0; j < 8; j++) red[(slice - 1) * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j] = acc[i][j];
-  }
-  __syncthreads();
-  if (slice == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-      for (int j = 0; j < 8; j++) {
-        float v = acc[i][j];
-#pragma unroll
-        for (int g = 0; g < S::SLICES - 1; g++) v += red[g * RL_TT * RL_TE + (ty + 4 * i) * RL_TE + tx + 8 * j];
-        const uint32_t t = t0 + ty + 4 * i, e = e0 + tx + 8 * j;
-        if (t < T && e < E) d.logits[((size_t)blockIdx.z * T + t) * E + e] = v;
+    // Non-finite values do not survive the split into parts (kernels_logits.cu): such a token's logits are made again in fp32.
+    if (recheck && __any_sync(0xffffffffu, nan))
+#pragma unroll 1
+      for (uint32_t e = 0; e < E; e++) {
+        float v = 0.0f;
+        for (uint32_t i = lane; i < D; i += 32) v = fmaf(__ldg(r.w + (size_t)e * D + i), __ldg(d.x + (size_t)token * D + i), v);
+        v = warp_sum(v);
+        if (lane == 0) s_score[e] = v;
       }
+    __syncwarp();
+    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], status);
+    const size_t p0 = (size_t)token * d.slots;
+    if (lane < r.top_k) picked = pick.id;
+    if (lane < r.top_k) {
+      d.pair_expert[p0 + lane] = pick.id == MER_NONE ? MER_NONE : r.id_base + pick.id;
+      d.pair_weight[p0 + lane] = pick.weight;
+    }
+    if (lane == 0 && d.slots > r.top_k) {
+      d.pair_expert[p0 + r.top_k] = r.shared_expert_id;
+      d.pair_weight[p0 + r.top_k] = r.shared_scale ? r.shared_scale[token] : 1.0f;
+    }
   }
+  if (group_here == 2) {
+    // A large dispatch is grouped by the grid-wide kernels that follow; their count step is done here, over the CTA's tokens first (an atomic
+    // per pick: all of a batch's on a few cache lines, 2048 tokens 16 us of selection).
+    uint32_t *s_hist = reinterpret_cast<uint32_t *>(smem_raw);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS) s_hist[i] = 0;
+    __syncthreads();
+    if (picked != MER_NONE) atomicAdd(&s_hist[picked], 1u);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS)
+      if (s_hist[i]) atomicAdd(d.group_count + i, s_hist[i]);
+    if (threadIdx.x == 0 && d.slots > r.top_k) atomicAdd(d.group_count + E, min((uint32_t)TT, d.n_tokens - t0));
+    return;
+  }
+  if (group_here != 1) return;
+  __syncthreads();
+  if (n_tiles > 1) {
+    if (threadIdx.x == 0) {
+      const uint32_t prev = arrive_acq_rel(&d.counters[max_tokens]);
+      s_last = (prev == n_tiles - 1);
+      if (s_last) d.counters[max_tokens] = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+  }
+  if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
+  build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
 }
 
 template <int ROWS>
-__global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int pre, int group_here, uint32_t logit_ctas) {
+__global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int group_here, uint32_t logit_ctas) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t E = r.num_experts, D = d.D;
   const uint32_t tile = blockIdx.y, t0 = tile * ROUTER_TT;
@@ -699,9 +686,9 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   const uint32_t e0 = blockIdx.x * ROWS;
   __shared__ float s_part[ROWS][ROUTER_TT][ROUTER_WARPS + 1];  // [row][token][warp]
   __shared__ float s_logit[ROUTER_TT][ROWS];                  // used when one CTA covers all experts
-  const bool single = logit_ctas == 1 && !pre;
-  // With the grouping done here, status bits gather in a scratch word, which the last CTA publishes: no launch clears them.
-  uint32_t *const status = group_here == 1 ? d.counters + max_tokens + 1 : d.status;
+  const bool single = logit_ctas == 1;
+  // Status bits gather in a scratch word, which the grouping publishes: no launch clears them.
+  uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
   // What the steps behind the logits read once a layer, and the layers in between have long pushed out of L2: a miss each, on their
   // critical path.
   if (tile == 0 && warp == 1) {
@@ -720,9 +707,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     if (tt < n_here) build_x_image(d, t0 + tt, threadIdx.x, ROUTER_THREADS, &s_part[0][0][0]);
     return;
   }
-  if (pre) {
-    // logits are already in d.logits (k_router_logits_tiled)
-  } else if ((D & 1023u) == 0) {
+  if ((D & 1023u) == 0) {
     const uint32_t slice4 = D / 4 / ROUTER_WARPS;  // float4 per warp slice
     float acc[ROWS][ROUTER_TT];
 #pragma unroll
@@ -791,7 +776,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   }
   __shared__ uint32_t s_flag;
   __syncthreads();
-  if (!single && !pre) {
+  if (!single) {
     if (threadIdx.x == 0) {
       const uint32_t prev = arrive_acq_rel(&d.counters[tile]);
       s_flag = (prev == logit_ctas - 1);
@@ -801,51 +786,21 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     if (!s_flag) return;
   }
 
-  // ---- this CTA holds the last logits of the token tile: one warp routes one token ----
-  __shared__ uint32_t s_groups[ROUTER_TT][64];
-  __shared__ float s_gscore[ROUTER_TT][64];
-  if (warp < n_here) {
-    float *s_score = reinterpret_cast<float *>(smem_raw) + (size_t)warp * 2 * E;  // [E] scores (become mixing weights)
-    float *s_sel = s_score + E;                                                    // [E] selection scores
-    uint8_t *s_ok = smem_raw + (size_t)ROUTER_TT * 2 * E * 4 + (size_t)warp * E;    // [E] allowed & not yet taken
-    const uint32_t token = t0 + warp;
-    if (pre > 1) {  // the logits kernel split K: add its partial sets in order
-      for (uint32_t i = lane; i < E; i += 32) {
-        float v = __ldcg(d.logits + (size_t)token * E + i);
-        for (int z = 1; z < pre; z++) v += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i);
-        s_score[i] = v;
-      }
-    } else {
-      for (uint32_t i = lane; i < E; i += 32) s_score[i] = single ? s_logit[warp][i] : __ldcg(d.logits + (size_t)token * E + i);
-    }
-    __syncwarp();
-    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], status);
-    const size_t p0 = (size_t)token * d.slots;
-    if (lane < r.top_k) {
-      d.pair_expert[p0 + lane] = pick.id == MER_NONE ? MER_NONE : r.id_base + pick.id;
-      d.pair_weight[p0 + lane] = pick.weight;
-      if (group_here == 2 && pick.id != MER_NONE) atomicAdd(d.group_count + pick.id, 1u);  // the grid-wide grouping's count step, done here
-    }
-    if (lane == 0 && d.slots > r.top_k) {
-      if (group_here == 2) atomicAdd(d.group_count + E, 1u);
-      d.pair_expert[p0 + r.top_k] = r.shared_expert_id;
-      d.pair_weight[p0 + r.top_k] = r.shared_scale ? r.shared_scale[token] : 1.0f;
-    }
+  // ---- this CTA holds the last logits of the token tile
+  finish_tokens<ROUTER_TT>(r, d, t0, gridDim.y, single ? &s_logit[0][0] : nullptr, ROWS, 1, false, smem_raw, status, max_tokens, group_here);
+}
+
+// The same behind the logits kernel of a large batch: every warp has a token.  (In the kernel above, whose registers leave room for two CTAs on an SM,
+// 4096 tokens of 256 experts took 47 us.)
+__global__ void __launch_bounds__(ROUTER_THREADS) k_router_select(const __grid_constant__ RouterDev r, const __grid_constant__ MoeDispatch d, uint32_t max_tokens, uint32_t sets,
+                                                                  int group_here, uint32_t select_ctas) {
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  if (blockIdx.x >= select_ctas) {  // activation images of the tokens
+    build_x_image(d, blockIdx.x - select_ctas, threadIdx.x, ROUTER_THREADS, reinterpret_cast<float *>(smem_raw));
+    return;
   }
-  if (group_here != 1) return;  // a large dispatch is grouped by the grid-wide kernels that follow (2: their count step is done above)
-  __syncthreads();
-  const uint32_t n_tiles = gridDim.y;
-  if (n_tiles > 1) {
-    if (threadIdx.x == 0) {
-      const uint32_t prev = arrive_acq_rel(&d.counters[max_tokens]);
-      s_flag = (prev == n_tiles - 1);
-      if (s_flag) d.counters[max_tokens] = 0;
-    }
-    __syncthreads();
-    if (!s_flag) return;
-  }
-  if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
-  build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
+  uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
+  finish_tokens<ROUTER_WARPS>(r, d, blockIdx.x * ROUTER_WARPS, select_ctas, nullptr, 0, sets, true, smem_raw, status, max_tokens, group_here);
 }
 
 // Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.
@@ -864,7 +819,7 @@ __global__ void __launch_bounds__(256) k_groups_from_pairs(MoeDispatch d, int si
   }
   const uint32_t P = d.n_tokens * d.slots;
   for (uint32_t p = threadIdx.x; p < P; p += blockDim.x) {
-    d.perm[p] = p;
+    put_pair(d, p, p);
     if (!single_group) {
       d.group_expert[p] = d.pair_expert[p];
       d.offsets[p] = p;
@@ -1226,64 +1181,47 @@ __global__ void k_f32_to_f16(const float *__restrict__ src, uint16_t *__restrict
 
 }  // namespace
 
-// Whether launch_router leaves d.status written by itself (it groups in its last CTA): no need to clear it first.
-bool router_sets_status(const MoeDispatch &d) { return d.n_tokens * d.slots < GRID_GROUPING_PAIRS || d.group_count == nullptr; }
 
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s,
                           int *launches, bool group) {
   const uint32_t E = r.num_experts, G = d.n_groups;
   const uint32_t P = d.n_tokens * d.slots;
-  size_t smem_topk = (size_t)ROUTER_TT * E * 9;
-  size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
-  size_t smem = smem_topk > smem_grp ? smem_topk : smem_grp;
-  smem = (smem + 15) & ~(size_t)15;
-  // From a few hundred tokens the logits are a tiled GEMM of their own, unless the experts are so few that most of a tile would be
-  // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel).
-  const bool tiled = d.n_tokens >= 256 && d.D % 256 == 0 && (E > 16 || d.D % 1024 != 0);
-  uint32_t ksplit = 1;
-  if (tiled) {
-    // split K over blockIdx.z while the tiles alone leave SMs idle (the partial sets must fit the logits scratch,
-    // which holds max_tokens x 4096 floats, and a slice is a whole number of chunks)
-    auto plan = [&](uint32_t tt, uint32_t te, uint32_t kc, dim3 &grid) {
-      grid = dim3((E + te - 1) / te, (d.n_tokens + tt - 1) / tt);
-      const uint32_t n_chunks = d.D / kc, tiles = grid.x * grid.y;
-      for (uint32_t ks = 2; ks <= 8 && ks <= n_chunks; ks++)
-        if (n_chunks % ks == 0 && tiles * ks <= 160 && (size_t)ks * E <= 4096) grid.z = ks;
-    };
-    auto run = [&](auto kern, size_t bytes, dim3 grid) {
-      ksplit = grid.z;
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-      if (e == cudaSuccess) kern<<<grid, RL_THREADS, bytes, s>>>(r, d, ksplit);
-      return e;
-    };
-    // the large tile where it fills the chip and the experts fill it
-    dim3 big, small;
-    plan(64, 128, 128, big), plan(32, 64, 256, small);
-    const bool use_big = E > 64 && (E % 128 == 0 || E > 512) && big.x * big.y * big.z >= 120;
-    const cudaError_t e = use_big ? run(k_router_logits_tiled<64, 128, 128>, LogitsTile<64, 128, 128>::SMEM, big)
-                                  : run(k_router_logits_tiled<32, 64, 256>, LogitsTile<32, 64, 256>::SMEM, small);
-    if (e != cudaSuccess) return e;
-    if (launches) (*launches)++;
-  }
-  // Expert rows per CTA: eight share the loads of x best, but a small call wants its few rows on as many SMs as there are
-  // (one token, 128 experts of 2048: 13.4 us with a row per CTA, 16.6 us with eight).
-  const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
-  uint32_t rows = 8;
-  while (!tiled && rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
-  const uint32_t logit_ctas = tiled ? 1 : (E + rows - 1) / rows;
-  const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
+  const size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   const bool grid_grouping = group && P >= GRID_GROUPING_PAIRS && d.group_count != nullptr;
-  auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+  const int group_here = grid_grouping ? 2 : group ? 1 : 0;
+  auto room = [&](auto kern, uint32_t tokens, size_t &smem) -> cudaError_t {
+    smem = (std::max((size_t)tokens * E * 9, group_here == 1 ? smem_grp : (size_t)0) + 15) & ~(size_t)15;
+    return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+  };
+  size_t smem;
+  cudaError_t e;
+  // From a few hundred tokens the logits are a GEMM of their own, unless the experts are so few that most of a tile would be
+  // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel) or so many that a CTA's tokens do not fit shared memory.
+  if (d.n_tokens >= 256 && r.w_split && E <= 2048 && (E > 16 || d.D % 1024 != 0)) {
+    uint32_t sets = 1;
+    if ((e = launch_router_logits(r, d, group_here ? d.counters + max_tokens + 1 : d.status, &sets, s)) != cudaSuccess) return e;
+    if ((e = room(k_router_select, ROUTER_WARPS, smem)) != cudaSuccess) return e;
+    const uint32_t ctas = (d.n_tokens + ROUTER_WARPS - 1) / ROUTER_WARPS;
+    k_router_select<<<ctas + (d.x_rows ? d.n_tokens : 0), ROUTER_THREADS, smem, s>>>(r, d, max_tokens, sets, group_here, ctas);
+    e = cudaGetLastError();
+    if (launches) (*launches)++;
+  } else {
+    // Expert rows per CTA: eight share the loads of x best, but a small call wants its few rows on as many SMs as there are
+    // (one token, 128 experts of 2048: 13.4 us with a row per CTA, 16.6 us with eight).
+    const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
+    uint32_t rows = 8;
+    while (rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
+    const uint32_t logit_ctas = (E + rows - 1) / rows;
+    const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
+    auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
+    if ((e = room(kern, ROUTER_TT, smem)) != cudaSuccess) return e;
+    e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, group_here, logit_ctas);
   }
-  cudaError_t e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, tiled ? (int)ksplit : 0, grid_grouping ? 2 : group ? 1 : 0, logit_ctas);
   if (e != cudaSuccess) return e;
   if (launches) (*launches)++;
   if (grid_grouping) {  // the router has counted the pairs per group
     const unsigned blocks = (P + 1023) / 1024;
-    k_group_scan<<<1, 256, 0, s>>>(r, d);
+    k_group_scan<<<1, 256, 0, s>>>(r, d, d.counters + max_tokens + 1);
     k_group_scatter<<<blocks, 256, 0, s>>>(r, d);
     if (launches) (*launches) += 2;
   }
@@ -1299,7 +1237,7 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
   if (groups_layer_on_grid(d)) {  // a large dispatch: count / scan / scatter over the grid
     const unsigned blocks = (P + 1023) / 1024;
     if (!counted) k_group_count<<<blocks, 256, 0, s>>>(r, d);
-    k_group_scan<<<1, 256, 0, s>>>(r, d);
+    k_group_scan<<<1, 256, 0, s>>>(r, d, nullptr);
     k_group_scatter<<<blocks, 256, 0, s>>>(r, d);
     if (launches) (*launches) += counted ? 2 : 3;
     return cudaGetLastError();

@@ -911,7 +911,7 @@ Plan make_plan(int dtype, uint32_t D, uint32_t F, uint32_t nt, uint32_t max_grou
 }
 
 struct ScratchLayout {
-  size_t bar, amax, npass, pgroup, pstart, pcount, pdesc, taken, bounds, seeds, x_un, h_un, parts, parts_bytes, total;
+  size_t bar, amax, pos, npass, pgroup, pstart, pcount, pdesc, taken, bounds, seeds, x_un, h_un, parts, parts_bytes, total;
 };
 
 // `parts` holds the partial sums of whichever phase is running: gate/up partials [n_ksplit][P][2][F], then (after they have become hidden
@@ -926,6 +926,7 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
   };
   L.bar = take(N_BARRIERS * 4);
   L.amax = take((size_t)2 * max_pairs * 4);
+  L.pos = take((size_t)max_pairs * 4);
   L.npass = take(256);
   L.pgroup = take(((size_t)std::max(max_pairs, 4096u) + 2) * 4);
   L.pstart = take((size_t)max_pairs * 4);
@@ -986,7 +987,7 @@ Plan plan_dispatch(const MoeDispatch &d, int sm_count) {
 }
 }  // namespace
 
-void stream_bind(MoeDispatch &d, void *scratch, int sm_count) {
+void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm) {
   if (sm_count > MER_MAX_CTAS1 - 1) sm_count = MER_MAX_CTAS1 - 1;
   uint8_t *base = static_cast<uint8_t *>(scratch);
   const ScratchLayout L = scratch_layout(d.scratch_pairs, d.D, d.F);
@@ -997,6 +998,7 @@ void stream_bind(MoeDispatch &d, void *scratch, int sm_count) {
   d.pass_desc = reinterpret_cast<PassDesc *>(base + L.pdesc);
   d.taken = reinterpret_cast<uint64_t *>(base + L.taken);
   d.amax = reinterpret_cast<uint32_t *>(base + L.amax);
+  d.pos = for_gemm ? reinterpret_cast<uint32_t *>(base + L.pos) : nullptr;
   d.x_rows = d.y;  // [n_tokens x D] fp32 in size, and free until the down phase
   d.act_seeds = reinterpret_cast<float *>(base + L.seeds);
   d.x_un = reinterpret_cast<float *>(base + L.x_un);

@@ -42,7 +42,8 @@ struct Slot {
 
 struct RouterEntry {
   RouterDev dev{};
-  float *d_w = nullptr, *d_cbias = nullptr, *d_lbias = nullptr;
+  float *d_w = nullptr, *d_cbias = nullptr, *d_lbias = nullptr, *d_w_unscale = nullptr;
+  uint8_t *d_w_split = nullptr;
   // steps either side of the MoE block (mer_layer_install)
   float *d_rms_w = nullptr, *d_shared_gate = nullptr;
   float rms_eps = 0.0f;
@@ -424,6 +425,8 @@ void free_all(mer_backend *b) {
     F(kv.second.d_w);
     F(kv.second.d_cbias);
     F(kv.second.d_lbias);
+    F(kv.second.d_w_split);
+    F(kv.second.d_w_unscale);
     F(kv.second.d_rms_w);
     F(kv.second.d_shared_gate);
   }
@@ -1250,6 +1253,8 @@ MER_EXPORT int mer_router_install(mer_backend *b, uint32_t layer, const float *h
   if (r.d_w) cudaFree(r.d_w), r.d_w = nullptr;
   if (r.d_cbias) cudaFree(r.d_cbias), r.d_cbias = nullptr;
   if (r.d_lbias) cudaFree(r.d_lbias), r.d_lbias = nullptr;
+  if (r.d_w_split) cudaFree(r.d_w_split), r.d_w_split = nullptr;
+  if (r.d_w_unscale) cudaFree(r.d_w_unscale), r.d_w_unscale = nullptr;
   size_t wbytes = (size_t)cfg->num_experts * b->cfg.d_model * 4, ebytes = (size_t)cfg->num_experts * 4;
   CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(router)", cudaMalloc((void **)&r.d_w, wbytes));
   CU(MER_ERR_UPLOAD, "cudaMemcpy(router)", cudaMemcpy(r.d_w, host_weights, wbytes, cudaMemcpyHostToDevice));
@@ -1261,7 +1266,17 @@ MER_EXPORT int mer_router_install(mer_backend *b, uint32_t layer, const float *h
     CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(bias)", cudaMalloc((void **)&r.d_lbias, ebytes));
     CU(MER_ERR_UPLOAD, "cudaMemcpy(bias)", cudaMemcpy(r.d_lbias, cfg->logit_bias, ebytes, cudaMemcpyHostToDevice));
   }
+  // for batches of 256 tokens and more: the weights in parts, beside the fp32 rows (finite weights only)
+  const uint32_t E = cfg->num_experts, D = (uint32_t)b->cfg.d_model;
+  if (b->cfg.max_tokens >= 256 && router_split_supported(D) &&
+      std::all_of(host_weights, host_weights + (size_t)E * D, [](float v) { return std::isfinite(v); })) {
+    CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(router parts)", cudaMalloc((void **)&r.d_w_split, router_split_bytes(E, D)));
+    CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(router scales)", cudaMalloc((void **)&r.d_w_unscale, ((size_t)E + 7) / 8 * 8 * 4));
+    CU(MER_ERR_UPLOAD, "router parts", launch_split_router(r.d_w, E, D, r.d_w_split, r.d_w_unscale, b->compute));
+    CU(MER_ERR_UPLOAD, "cudaStreamSynchronize", cudaStreamSynchronize(b->compute));
+  }
   r.dev.w = r.d_w;
+  r.dev.w_split = r.d_w_split, r.dev.w_unscale = r.d_w_unscale;
   r.dev.correction_bias = r.d_cbias;
   r.dev.logit_bias = r.d_lbias;
   r.dev.num_experts = cfg->num_experts;
@@ -1336,7 +1351,7 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   CU(MER_ERR_SUBMISSION, "cudaMemcpyAsync(unaligned x)", readable_rows(b, d_x, n_tokens, s));
   d.x = d_x;
   d.out = row_aligned(d_out) ? d_out : b->d_out;
-  if (!status_cleared && (!run_ffn_too || !router_sets_status(d))) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
+  if (!status_cleared && !run_ffn_too) CU(MER_ERR_SUBMISSION, "cudaMemsetAsync(status)", cudaMemsetAsync(b->d_status, 0, 4, s));
   if (!capturing) CU(MER_ERR_SUBMISSION, "wait for uploads", order_after_copies(b, s));
   cudaEvent_t *ev = (run_ffn_too && !capturing) ? next_timing_set(b) : nullptr;
   if (ev) cudaEventRecord(ev[0], s);
