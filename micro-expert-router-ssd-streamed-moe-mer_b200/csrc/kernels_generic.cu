@@ -603,9 +603,25 @@ __device__ void build_groups_layer(const RouterDev &r, const MoeDispatch &d, uin
   if (d.pass_group) build_passes_block(d, s_off, true);
 }
 
+// A large dispatch is grouped by grid-wide kernels; their count step is done here, over the CTA's tokens first (an atomic per pick: all of a
+// batch's on a few cache lines, 2048 tokens 16 us of selection instead of 13).  Out of line: small calls run past it cold.
+__device__ __noinline__ void count_picks(const RouterDev &r, const MoeDispatch &d, uint32_t picked, uint32_t tokens, uint32_t *s_hist) {
+  const uint32_t E = r.num_experts;
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS) s_hist[i] = 0;
+  __syncthreads();
+  if (picked != MER_NONE) atomicAdd(&s_hist[picked], 1u);
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS)
+    if (s_hist[i]) atomicAdd(d.group_count + i, s_hist[i]);
+  if (threadIdx.x == 0 && d.slots > r.top_k) atomicAdd(d.group_count + E, tokens);
+}
+
 // Selection for the TT tokens from t0 on, whose logits are there, one warp per token; the last of `n_tiles` CTAs that get here groups all pairs.
 // `direct`: the logits [TT][stride] in shared memory, or null: `sets` partial sums of them in d.logits ([sets][T][E], added in order).
-template <int TT>
+// EJ > 0: at most 32 EJ experts and 32 pairs of the streaming kernels, with no other code in the kernel: it runs once a layer, cold, and what a call of one
+// token waits for is its instructions (one token on 128 experts of 2048 x 768: 1 us a layer).
+template <int TT, int EJ>
 __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispatch &d, uint32_t t0, uint32_t n_tiles, const float *direct, uint32_t stride, uint32_t sets,
                                               bool recheck, uint8_t *smem_raw, uint32_t *status, uint32_t max_tokens, int group_here) {
   const uint32_t E = r.num_experts, D = d.D, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -635,7 +651,11 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
         if (lane == 0) s_score[e] = v;
       }
     __syncwarp();
-    const Pick pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], status);
+    Pick pick;
+    if constexpr (EJ > 0)
+      pick = route_token_reg<EJ>(r, s_score, s_sel, status);
+    else
+      pick = route_token(r, s_score, s_sel, s_ok, s_groups[warp], s_gscore[warp], status);
     const size_t p0 = (size_t)token * d.slots;
     if (lane < r.top_k) picked = pick.id;
     if (lane < r.top_k) {
@@ -647,20 +667,7 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
       d.pair_weight[p0 + r.top_k] = r.shared_scale ? r.shared_scale[token] : 1.0f;
     }
   }
-  if (group_here == 2) {
-    // A large dispatch is grouped by the grid-wide kernels that follow; their count step is done here, over the CTA's tokens first (an atomic
-    // per pick: all of a batch's on a few cache lines, 2048 tokens 16 us of selection).
-    uint32_t *s_hist = reinterpret_cast<uint32_t *>(smem_raw);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS) s_hist[i] = 0;
-    __syncthreads();
-    if (picked != MER_NONE) atomicAdd(&s_hist[picked], 1u);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < E; i += ROUTER_THREADS)
-      if (s_hist[i]) atomicAdd(d.group_count + i, s_hist[i]);
-    if (threadIdx.x == 0 && d.slots > r.top_k) atomicAdd(d.group_count + E, min((uint32_t)TT, d.n_tokens - t0));
-    return;
-  }
+  if (EJ == 0 && group_here == 2) return count_picks(r, d, picked, min((uint32_t)TT, d.n_tokens - t0), reinterpret_cast<uint32_t *>(smem_raw));
   if (group_here != 1) return;
   __syncthreads();
   if (n_tiles > 1) {
@@ -673,10 +680,13 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     if (!s_last) return;
   }
   if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
-  build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
+  if constexpr (EJ > 0)
+    build_groups_small(r, d);
+  else
+    build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
 }
 
-template <int ROWS>
+template <int ROWS, int EJ>
 __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispatch d, uint32_t max_tokens, int group_here, uint32_t logit_ctas) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   const uint32_t E = r.num_experts, D = d.D;
@@ -787,7 +797,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   }
 
   // ---- this CTA holds the last logits of the token tile
-  finish_tokens<ROUTER_TT>(r, d, t0, gridDim.y, single ? &s_logit[0][0] : nullptr, ROWS, 1, false, smem_raw, status, max_tokens, group_here);
+  finish_tokens<ROUTER_TT, EJ>(r, d, t0, gridDim.y, single ? &s_logit[0][0] : nullptr, ROWS, 1, false, smem_raw, status, max_tokens, group_here);
 }
 
 // The same behind the logits kernel of a large batch: every warp has a token.  (In the kernel above, whose registers leave room for two CTAs on an SM,
@@ -800,7 +810,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router_select(const __grid_c
     return;
   }
   uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
-  finish_tokens<ROUTER_WARPS>(r, d, blockIdx.x * ROUTER_WARPS, select_ctas, nullptr, 0, sets, true, smem_raw, status, max_tokens, group_here);
+  finish_tokens<ROUTER_WARPS, 0>(r, d, blockIdx.x * ROUTER_WARPS, select_ctas, nullptr, 0, sets, true, smem_raw, status, max_tokens, group_here);
 }
 
 // Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.
@@ -1213,7 +1223,10 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     while (rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
     const uint32_t logit_ctas = (E + rows - 1) / rows;
     const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
-    auto kern = rows == 1 ? k_router<1> : rows == 2 ? k_router<2> : rows == 4 ? k_router<4> : k_router<8>;
+    auto kern = rows == 1 ? k_router<1, 0> : rows == 2 ? k_router<2, 0> : rows == 4 ? k_router<4, 0> : k_router<8, 0>;
+    if (group_here == 1 && P <= 32 && d.item_bounds && E <= 256)
+      kern = E <= 128 ? (rows == 1 ? k_router<1, 4> : rows == 2 ? k_router<2, 4> : rows == 4 ? k_router<4, 4> : k_router<8, 4>)
+                      : (rows == 1 ? k_router<1, 8> : rows == 2 ? k_router<2, 8> : rows == 4 ? k_router<4, 8> : k_router<8, 8>);
     if ((e = room(kern, ROUTER_TT, smem)) != cudaSuccess) return e;
     e = launch_overlapped(kern, grid, ROUTER_THREADS, smem, s, false, r, d, max_tokens, group_here, logit_ctas);
   }
