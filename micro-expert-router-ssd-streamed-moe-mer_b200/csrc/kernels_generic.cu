@@ -329,6 +329,16 @@ __global__ void __launch_bounds__(256) k_group_scatter(RouterDev r, MoeDispatch 
     if (d.pass_desc) d.pass_desc[d.pass_group[k] + rank / d.tokens_per_pass].pair[rank % d.tokens_per_pass] = p;
   }
 }
+// Work split over passes of equal cost.
+__device__ __forceinline__ void even_bounds(const MoeDispatch &d, uint32_t n_passes) {
+  const uint32_t G = d.n_ctas, n0 = n_passes * d.items_per_pass[0], n1 = n_passes * d.items_per_pass[1];
+  if (threadIdx.x <= G && (uint64_t)max(n0, n1) * G <= 0xFFFFFFFFull && G < 256) {
+    d.item_bounds[threadIdx.x] = n0 * threadIdx.x / G;
+    d.item_bounds[MER_MAX_CTAS1 + threadIdx.x] = n1 * threadIdx.x / G;
+  } else if ((uint64_t)max(n0, n1) * G > 0xFFFFFFFFull || G >= 256) {
+    build_item_bounds(d, n_passes, nullptr);
+  }
+}
 // The same for at most 32 pairs of the streaming kernels, in registers of one warp: sorted position of every pair, the pairs
 // that start a pass, their order.  The general form's dozen block-wide steps took 4 us on B200 for one token's eight pairs, as long
 // as the kernels that follow need for the weights of half of them.
@@ -377,14 +387,25 @@ __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
   }
   __syncthreads();
   if (weighted) return build_item_bounds(d, s_np, s_cum);
-  const uint32_t G = d.n_ctas;  // passes of equal cost
-  const uint32_t n0 = s_np * d.items_per_pass[0], n1 = s_np * d.items_per_pass[1];
-  if (threadIdx.x <= G && (uint64_t)max(n0, n1) * G <= 0xFFFFFFFFull && G < 256) {
-    d.item_bounds[threadIdx.x] = n0 * threadIdx.x / G;
-    d.item_bounds[MER_MAX_CTAS1 + threadIdx.x] = n1 * threadIdx.x / G;
-  } else if ((uint64_t)max(n0, n1) * G > 0xFFFFFFFFull || G >= 256) {
-    build_item_bounds(d, s_np, nullptr);
+  even_bounds(d, s_np);
+}
+// The same for the pairs of one token, at most 32: every pair that has an expert is a pass of its own.  `eid`: expert of pair threadIdx.x (first warp).
+__device__ __forceinline__ void build_groups_token(const MoeDispatch &d, uint32_t eid) {
+  __shared__ uint32_t s_np;
+  clear_taken(d);
+  if (threadIdx.x < 32) {
+    const uint32_t p = threadIdx.x, P = d.slots;
+    const uint32_t valid = __ballot_sync(0xffffffffu, eid != MER_NONE), pass = __popc(valid & ((1u << p) - 1));
+    if (p < P) clear_maxima(d, p);
+    if (eid != MER_NONE) {
+      put_pass(d, pass, 0, expert_payload(d, eid), pass, 1);
+      d.pass_desc[pass].pair[0] = p;
+      d.perm[pass] = p;
+    }
+    if (p == 0) d.offsets[d.n_groups] = d.n_passes[0] = s_np = __popc(valid);
   }
+  __syncthreads();
+  even_bounds(d, s_np);
 }
 
 // The same for a batch of decode size (at most 2048 pairs, 512 groups): the counting atomics hand out the pairs' ranks, and
@@ -402,6 +423,13 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
   const bool bounds = d.item_bounds != nullptr, weighted = bounds && tpp == 8;  // (passes of four can be more than s_cum holds)
   for (uint32_t i = tid; i < MID_GROUPS; i += 256) s_cnt[i] = 0;
   clear_taken(d);
+  // the payloads of the thread's groups: a round trip that passes while the pairs are counted
+  const uint8_t *payload[PER_G];
+#pragma unroll
+  for (uint32_t i = 0; i < PER_G; i++) {
+    const uint32_t g = tid * PER_G + i;
+    payload[i] = d.pass_desc && g < G ? expert_payload(d, g < r.num_experts ? r.id_base + g : r.shared_expert_id) : nullptr;
+  }
   __syncthreads();
 #pragma unroll 1
   for (uint32_t p = tid; p < P; p += 256) {
@@ -446,7 +474,6 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
     s_cnt[g] = beg, s_pass[g] = pass;
     if (g < G) {
       const uint32_t eid = g < r.num_experts ? r.id_base + g : r.shared_expert_id;
-      const uint8_t *payload = d.pass_desc && n ? expert_payload(d, eid) : nullptr;
       d.group_expert[g] = eid;
       d.offsets[g] = beg;
       const PassCut cut(n, tpp, shift);
@@ -454,7 +481,7 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
 #pragma unroll 1
       for (uint32_t j = 0; j < cut.passes; j++, pass++) {
         const uint32_t cnt = cut.count(j, n - st);
-        put_pass(d, pass, g, payload, beg + st, cnt);
+        put_pass(d, pass, g, payload[i], beg + st, cnt);
         st += cnt;
         if (weighted) s_cum[pass] = cum, cum += cnt > 4 ? 13 : 10;
       }
@@ -680,9 +707,13 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     if (!s_last) return;
   }
   if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
-  if constexpr (EJ > 0)
+  if constexpr (EJ > 0) {
+    if (d.n_tokens == 1) {  // the picks are still in the first warp's registers
+      const uint32_t eid = threadIdx.x < r.top_k ? (picked == MER_NONE ? MER_NONE : r.id_base + picked) : threadIdx.x < d.slots ? r.shared_expert_id : MER_NONE;
+      return build_groups_token(d, eid);
+    }
     build_groups_small(r, d);
-  else
+  } else
     build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
 }
 
@@ -821,13 +852,20 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_groups_layer(RouterDev r, Mo
 
 // Routing supplied by the caller: mode 0 = every pair is its own group, mode 1 = one group.
 // The first CTA; the others make the tokens' activation images.
-__global__ void __launch_bounds__(256) k_groups_from_pairs(MoeDispatch d, int single_group) {
+__global__ void __launch_bounds__(256) k_groups_from_pairs(const __grid_constant__ MoeDispatch d, int single_group) {
+  grid_dep_wait();
+  grid_dep_launch();
   if (blockIdx.x > 0) {
     __shared__ float s_max[8];
     build_x_image(d, blockIdx.x - 1, threadIdx.x, 256, s_max);
     return;
   }
   const uint32_t P = d.n_tokens * d.slots;
+  if (!single_group && d.pass_desc && d.n_tokens == 1) {
+    if (threadIdx.x == 0) *d.status = 0;
+    build_groups_token(d, threadIdx.x < P ? d.pair_expert[threadIdx.x] : MER_NONE);
+    return;
+  }
   for (uint32_t p = threadIdx.x; p < P; p += blockDim.x) {
     put_pair(d, p, p);
     if (!single_group) {
@@ -1267,9 +1305,9 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
 }
 
 cudaError_t launch_groups_from_pairs(const MoeDispatch &d, cudaStream_t s, int *launches) {
-  k_groups_from_pairs<<<d.x_rows ? 1 + d.n_tokens : 1, 256, 0, s>>>(d, d.n_groups == 1);
+  const cudaError_t e = launch_overlapped(k_groups_from_pairs, dim3(d.x_rows ? 1 + d.n_tokens : 1), 256, 0, s, false, d, d.n_groups == 1);
   if (launches) (*launches)++;
-  return cudaGetLastError();
+  return e;
 }
 
 cudaError_t launch_ffn_generic(const MoeDispatch &d, cudaStream_t s, int *launches, cudaEvent_t ev_mid) {
