@@ -79,6 +79,9 @@ struct MoeDispatch {
   // the hidden rows' in `h`; both share the seeds.  Null: nobody multiplies them.
   void *x_rows;
   float *act_seeds, *x_un, *h_un;  // *_un: 2^24 / scale of every row
+  // One token: the router kernel leaves the logits only, and every CTA of the streaming kernel selects the experts itself, by this router.
+  int route_here;
+  RouterDev route;
   uint32_t tokens_per_pass;
   // Work split of the streaming kernels, built with the passes: item_bounds[phase * MER_MAX_CTAS1 + b] = first item of
   // CTA b in that phase (b = 0 .. n_ctas), items weighted by the tokens of their pass (null: the GEMM path).
@@ -219,6 +222,8 @@ size_t stream_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F);
 cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid);
 // Points d.pass_*, d.amax and the activation images into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
 void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm = false);
+// Whether launch_ffn_stream can route this (bound) dispatch itself: d.route_here.
+bool route_in_stream(const MoeDispatch &d, const RouterDev &r);
 cudaError_t launch_reduce_parts(const MoeDispatch &d, cudaStream_t s, int *launches);
 // Images of all of the dispatch's tokens, where neither router nor grouping made them on the way.
 cudaError_t launch_x_images(const MoeDispatch &d, cudaStream_t s, int *launches);

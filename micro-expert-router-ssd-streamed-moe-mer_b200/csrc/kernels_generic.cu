@@ -82,6 +82,7 @@ constexpr int ROUTER_TT = 4;                      // tokens per CTA
 constexpr uint32_t ROUTER_CTAS = 240;             // rows per CTA are halved while there are fewer CTAs than this
 constexpr uint32_t SMALL_P = 4096;                // pair keys staged in shared memory below this many pairs
 constexpr uint32_t STABLE_G = 512;                // (token, slot)-ordered grouping up to this many groups
+constexpr int ROUTE_LATER = 3;                    // `group_here`: selection and grouping are the streaming kernel's
 constexpr uint32_t GRID_GROUPING_PAIRS = 8192;    // from this many pairs the grouping runs grid-wide (count / scan / scatter)
 
 // 64-bit divisions cost a few hundred cycles and much code, and this sits on the critical path of every decode layer: they are
@@ -727,7 +728,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   const uint32_t e0 = blockIdx.x * ROWS;
   __shared__ float s_part[ROWS][ROUTER_TT][ROUTER_WARPS + 1];  // [row][token][warp]
   __shared__ float s_logit[ROUTER_TT][ROWS];                  // used when one CTA covers all experts
-  const bool single = logit_ctas == 1;
+  const bool single = logit_ctas == 1 && group_here != ROUTE_LATER;
   // Status bits gather in a scratch word, which the grouping publishes: no launch clears them.
   uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
   // What the steps behind the logits read once a layer, and the layers in between have long pushed out of L2: a miss each, on their
@@ -745,6 +746,11 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
 
   if (blockIdx.x >= logit_ctas) {  // CTAs beside the logits' make the activation images of the tile's tokens
     const uint32_t tt = blockIdx.x - logit_ctas;
+    if (group_here == ROUTE_LATER && tt == 0) {  // what the grouping would clear
+      if (threadIdx.x == 0) *d.status = 0;
+      if (threadIdx.x < d.slots) clear_maxima(d, threadIdx.x);
+      clear_taken(d);
+    }
     if (tt < n_here) build_x_image(d, t0 + tt, threadIdx.x, ROUTER_THREADS, &s_part[0][0][0]);
     return;
   }
@@ -815,6 +821,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
       }
     }
   }
+  if (group_here == ROUTE_LATER) return;
   __shared__ uint32_t s_flag;
   __syncthreads();
   if (!single) {
@@ -1236,7 +1243,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   const uint32_t P = d.n_tokens * d.slots;
   const size_t smem_grp = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   const bool grid_grouping = group && P >= GRID_GROUPING_PAIRS && d.group_count != nullptr;
-  const int group_here = grid_grouping ? 2 : group ? 1 : 0;
+  const int group_here = group && d.route_here ? ROUTE_LATER : grid_grouping ? 2 : group ? 1 : 0;
   auto room = [&](auto kern, uint32_t tokens, size_t &smem) -> cudaError_t {
     smem = (std::max((size_t)tokens * E * 9, group_here == 1 ? smem_grp : (size_t)0) + 15) & ~(size_t)15;
     return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
@@ -1262,7 +1269,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     const uint32_t logit_ctas = (E + rows - 1) / rows;
     const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
     auto kern = rows == 1 ? k_router<1, 0> : rows == 2 ? k_router<2, 0> : rows == 4 ? k_router<4, 0> : k_router<8, 0>;
-    if (group_here == 1 && P <= 32 && d.item_bounds && E <= 256)
+    if ((group_here == 1 || group_here == ROUTE_LATER) && P <= 32 && d.item_bounds && E <= 256)
       kern = E <= 128 ? (rows == 1 ? k_router<1, 4> : rows == 2 ? k_router<2, 4> : rows == 4 ? k_router<4, 4> : k_router<8, 4>)
                       : (rows == 1 ? k_router<1, 8> : rows == 2 ? k_router<2, 8> : rows == 4 ? k_router<4, 8> : k_router<8, 8>);
     if ((e = room(kern, ROUTER_TT, smem)) != cudaSuccess) return e;

@@ -44,6 +44,7 @@
 #include "decode.cuh"
 #include "layout.cuh"
 #include "ptx.cuh"
+#include "route.cuh"
 
 namespace {
 
@@ -79,9 +80,7 @@ struct StreamParams {
   uint32_t frag_cols;        // fragment arrays of a buffer: 2 * min(4 * NT, most tokens of any group)
   uint32_t frag_bytes;       // bytes of a buffer
   float *parts;              // gate/up partials [n_ksplit][P][2][F]
-  float *down_parts;         // with K split, down partials [n_ksplit][P x D]: the same place, except with `local`
-  int local;                 // at most one down item a CTA: every CTA makes the hidden values that its own item wants, in shared memory (no
-                             // hidden rows in memory, no second barrier between the phases, no copy: 2.5 of 23 us for one token on 128 x 8 experts)
+  float *down_parts;         // with K split, down partials [n_ksplit][P x D]: the same place, except with LOCAL
   int sync;                  // cooperative launch: the grid-wide steps below run here (0: kernels of their own follow)
   int tail;                  // after the down phase, by the whole grid after a grid-wide barrier:
                              // TAIL_COMBINE: out[token] = weighted sum of its pairs' outputs in slot order;
@@ -261,14 +260,16 @@ struct __align__(16) Item {
 struct Claims {
   const uint32_t *bounds;
   uint64_t *taken;  // low half: from the front, high half: from the back; the first item of a range is its owner's
-  uint32_t beg, n_own, n_items, lane;
+  uint32_t beg, n_own, n_items, per, more, lane;  // per, more: without a table of bounds, the first `more` CTAs have per + 1 items, the others per
   bool first = true, own = true;
   __device__ Claims(const StreamParams &p, int phase, uint32_t n_passes, uint32_t lane_) : lane(lane_) {
     const PhaseParams &f = p.ph[phase];
     n_items = n_passes * f.n_ksplit * ((f.packed_tiles + ITEM_TILES - 1) / ITEM_TILES);
-    bounds = p.d.item_bounds + phase * MER_MAX_CTAS1, taken = p.d.taken + phase * MER_MAX_CTAS1;
-    beg = min(n_items, bounds[blockIdx.x]), n_own = min(n_items, bounds[blockIdx.x + 1]) - beg;
+    bounds = p.d.route_here ? nullptr : p.d.item_bounds + phase * MER_MAX_CTAS1, taken = p.d.taken + phase * MER_MAX_CTAS1;
+    per = n_items / gridDim.x, more = n_items - per * gridDim.x;
+    beg = bound(blockIdx.x), n_own = bound(blockIdx.x + 1) - beg;
   }
+  __device__ uint32_t bound(uint32_t cta) const { return bounds ? min(n_items, bounds[cta]) : per * cta + min(cta, more); }
   // Next item, or MER_NONE.
   __device__ uint32_t next() {
     if (own) {
@@ -287,7 +288,7 @@ struct Claims {
 #pragma unroll 1
       for (uint32_t c = lane; c < gridDim.x; c += 32) {
         const uint64_t v = *(volatile uint64_t *)(taken + c);
-        const uint32_t b = min(n_items, bounds[c]), e = min(n_items, bounds[c + 1]), gone = (uint32_t)v + (uint32_t)(v >> 32) + 1;
+        const uint32_t b = bound(c), e = bound(c + 1), gone = (uint32_t)v + (uint32_t)(v >> 32) + 1;
         if (e - b > gone && e - b - gone > best) best = e - b - gone, from = c, end = e;
       }
       const uint32_t most = __reduce_max_sync(0xffffffffu, best);
@@ -296,7 +297,7 @@ struct Claims {
       uint32_t item = MER_NONE;
       if (lane == who) {
         const uint64_t old = atomicAdd(reinterpret_cast<unsigned long long *>(taken + from), 1ull << 32);
-        const uint32_t n = end - min(n_items, bounds[from]);
+        const uint32_t n = end - bound(from);
         if ((uint32_t)old + (uint32_t)(old >> 32) + 1 < n) item = end - 1 - (uint32_t)(old >> 32);
       }
       item = __shfl_sync(0xffffffffu, item, who);
@@ -305,8 +306,34 @@ struct Claims {
   }
 };
 
+// Routing of a dispatch of one token by the scheduler of every CTA, from the router kernel's logits: passes of one pair each, in slot order.  All
+// CTAs come to the same selection; the first one writes it down.  What it saves is the router's last CTA: arrivals, its tables' way through L2 and a
+// round trip for them.  `scratch`: 2 x 256 floats, `word`: where the other CTAs' status bits go.  Returns the number of passes.
+__device__ __forceinline__ uint32_t route_token_here(const MoeDispatch &d, float *scratch, const uint8_t **s_base, uint32_t *s_slot, uint32_t *word, uint32_t lane) {
+  const RouterDev &r = d.route;
+  for (uint32_t i = lane; i < r.num_experts; i += 32) scratch[i] = __ldcg(d.logits + i);
+  __syncwarp();
+  uint32_t *status = blockIdx.x == 0 ? d.status : word;
+  const Pick pick = r.num_experts <= 128 ? route_token_reg<4>(r, scratch, scratch + 256, status) : route_token_reg<8>(r, scratch, scratch + 256, status);
+  const bool routed = lane < r.top_k;
+  const uint32_t eid = routed ? (pick.id == MER_NONE ? MER_NONE : r.id_base + pick.id) : lane < d.slots ? r.shared_expert_id : MER_NONE;
+  const uint32_t valid = __ballot_sync(0xffffffffu, eid != MER_NONE), pass = __popc(valid & ((1u << lane) - 1)), n = __popc(valid);
+  if (eid != MER_NONE) s_base[pass] = eid < d.max_experts ? d.expert_ptr[eid] : nullptr, s_slot[pass] = lane;
+  if (blockIdx.x == 0) {
+    if (lane < d.slots) d.pair_expert[lane] = eid, d.pair_weight[lane] = routed ? pick.weight : r.shared_scale ? *r.shared_scale : 1.0f;
+    if (eid != MER_NONE) d.perm[pass] = lane;
+    if (lane == 0) d.offsets[d.n_groups] = d.n_passes[0] = n;
+  }
+  __syncwarp();
+  fence_async();  // the scratch is a stage of the ring
+  return n;
+}
+
 // RAGGED: the last group of 16 tiles is not full, or K or a stage is no multiple of four blocks (the checks cost the even shapes 1 to 3 %).
-template <int DT, int NT, bool RAGGED>
+// ROUTE: the scheduler selects the experts of the only token.  LOCAL: at most one down item a CTA, which makes the hidden values that the item wants in
+// its own shared memory: no hidden rows in memory, no second barrier between the phases, no copy.  (Parameters and not branches: the code of either
+// beside the loops cost 16 tokens on 8 experts of 4096 x 14336 4 %.)
+template <int DT, int NT, bool RAGGED, bool ROUTE, bool LOCAL>
 __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   extern __shared__ __align__(128) uint8_t smem[];
   constexpr uint32_t BB = BlockBytes<DT>::value;
@@ -319,6 +346,8 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   uint64_t *built = full + 21;                                  // the item's hidden values are in shared memory (`local`)
   uint64_t *q_full = full + 56, *q_empty = q_full + QUEUE;      // [QUEUE] each
   Item *s_item = reinterpret_cast<Item *>(smem + 512);          // [QUEUE]
+  const uint8_t **s_base = reinterpret_cast<const uint8_t **>(smem + 640);  // [32] payload of every pass, where the scheduler routes
+  uint32_t *s_slot = reinterpret_cast<uint32_t *>(smem + 896);  // [32] its slot
   uint32_t *s_abort = reinterpret_cast<uint32_t *>(smem + 176), *s_ok = s_abort + 1;
   uint32_t *s_info = reinterpret_cast<uint32_t *>(smem + 184);  // [2] tokens of the unit's pass
   uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 192);  // [2][8] pair index of each of them
@@ -419,7 +448,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   if (warp == SCHED_WARP) {
     // ------------------------------ scheduler: claims items, and for each new unit, i.e. (pass, K split), fetches the activations: lane l
     // copies part l % 4 (hi fragments, lo fragments, their zero-point terms) of the pass's token l / 4.
-    const uint32_t n_passes = *d.n_passes;
+    const uint32_t n_passes = ROUTE ? route_token_here(d, reinterpret_cast<float *>(s_stage), s_base, s_slot, s_abort + 108, lane) : *d.n_passes;
     uint32_t unit = 0, slot = 0, round = 0;
     bool ok = true;
     const uint32_t tok = lane >> 2, part = lane & 3;
@@ -447,9 +476,13 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         const uint32_t tile = item % n_tiles, ks = (item / n_tiles) % f.n_ksplit, pp = item / n_tiles / f.n_ksplit;
         const bool new_unit = more && (pp != cur_pp || ks != cur_ks);
         if (new_unit && pp != cur_pp) {
-          const PassDesc &pass = d.pass_desc[pp];
-          base = pass.base, count = pass.count;
-          pair = pass.pair[tok];
+          if (ROUTE) {
+            base = s_base[pp], count = 1, pair = s_slot[pp];
+          } else {
+            const PassDesc &pass = d.pass_desc[pp];
+            base = pass.base, count = pass.count;
+            pair = pass.pair[tok];
+          }
           if (tok < count) {
             const ImageRow row(phase == 0 ? d.x_rows : d.h, d.act_seeds, phase == 0 ? pair / d.slots : pair, K);
             src = part == 0 ? row.hi : part == 1 ? row.lo : reinterpret_cast<const uint8_t *>(part == 2 ? row.seed_hi : row.seed_lo);
@@ -479,7 +512,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         const uint32_t kb0 = ks * f.kb_split, kbn = min(f.kb_split, f.kb_total - kb0), seed_bytes = ((kbn + 3) & ~3u) * 4;
         if (phase == 0 && use > 0 && lane < 16) flush_maxima(buf, lane);
         __syncwarp();
-        const bool copies = !(phase == 1 && p.local);
+        const bool copies = !(LOCAL && phase == 1);
         if (lane == 0) mbar_expect_tx(&frag_full[buf], copies ? count * 2 * (kbn * 64 + seed_bytes) : 0);
         __syncwarp();
         if (tok < count && !copies) {
@@ -569,7 +602,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       dead = !__all_sync(0xffffffffu, mbar_wait(&frag_full[buf], use & 1));
       if (dead) break;
       pcount = *(volatile uint32_t *)&s_info[buf];
-      if (phase == 1 && p.local) {
+      if (LOCAL && phase == 1) {
         uint8_t *frag = s_frag + buf * p.frag_bytes;
         float *seeds = reinterpret_cast<float *>(frag + p.frag_cols * stride);
         const uint32_t chunks = (kbn + 3) / 4;
@@ -808,12 +841,14 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     *(volatile uint32_t *)s_abort = 1;
     atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
   }
+  if (phase == 0) {  // the maxima of the units that are still in the buffers
+    consumer_sync();
+    if (threadIdx.x < 32) flush_maxima(threadIdx.x >> 4, threadIdx.x & 15);
+  }
   if (!p.sync) continue;
   if (phase == 0) {
     // all partial sums, then all hidden rows
-    consumer_sync();
-    if (threadIdx.x < 32) flush_maxima(threadIdx.x >> 4, threadIdx.x & 15);
-    if (p.local) {
+    if (LOCAL) {
       if (!grid_barrier(p.bar + 1, s_ok, d.status)) dead = true;
       if (threadIdx.x == 0) mbar_arrive(hidden);
       continue;
@@ -835,9 +870,9 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   }
 }
 
-template <int DT, int NT, bool RAGGED>
+template <int DT, int NT, bool RAGGED, bool ROUTE, bool LOCAL>
 __global__ void __launch_bounds__(THREADS, 1) k_ffn_stream(const __grid_constant__ StreamParams p) {
-  ffn_stream_body<DT, NT, RAGGED>(p);
+  ffn_stream_body<DT, NT, RAGGED, ROUTE, LOCAL>(p);
 }
 
 // The step between the phases as a kernel of its own, where a cooperative launch is refused.  A warp per unit.
@@ -986,11 +1021,17 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
 }
 
 template <int DT>
-cudaError_t launch_stream(const StreamParams &p, uint32_t nt, size_t smem, int grid, cudaStream_t s) {
+cudaError_t launch_stream(const StreamParams &p, uint32_t nt, bool local, size_t smem, int grid, cudaStream_t s) {
   bool ragged = p.kc % 4 != 0;
   for (const PhaseParams &ph : p.ph) ragged = ragged || ph.packed_tiles % ITEM_TILES != 0 || ph.kb_total % 4 != 0;
-  void (*kern)(StreamParams) = ragged ? (nt == 2 ? k_ffn_stream<DT, 2, true> : k_ffn_stream<DT, 1, true>)
-                                      : (nt == 2 ? k_ffn_stream<DT, 2, false> : k_ffn_stream<DT, 1, false>);
+  auto one = [&](auto route, auto local) -> void (*)(StreamParams) {
+    return ragged ? k_ffn_stream<DT, 1, true, decltype(route)::value, decltype(local)::value> : k_ffn_stream<DT, 1, false, decltype(route)::value, decltype(local)::value>;
+  };
+  using T = std::true_type;
+  using F = std::false_type;
+  void (*kern)(StreamParams) = nt == 2          ? (ragged ? k_ffn_stream<DT, 2, true, false, false> : k_ffn_stream<DT, 2, false, false, false>)
+                               : p.d.route_here ? (local ? one(T{}, T{}) : one(T{}, F{}))
+                                                : (local ? one(F{}, T{}) : one(F{}, F{}));
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   // the grid-wide steps wait for every CTA: a cooperative launch guarantees that they are all resident
@@ -1020,7 +1061,20 @@ Plan plan_dispatch(const MoeDispatch &d, int sm_count) {
   if (pl.nt == 2 && pl.n_stages < 3) pl = make_plan(d.dtype, d.D, d.F, 1, mgt, act, sm_count, cap_gu, cap_dn);  // eight tokens per pass do not fit: four
   return pl;
 }
+// At most one down item a CTA, of no more than one round of its warps (28 units, 3.5 rounds: one token on 8 experts of 4096 x 14336 209 us for
+// 201), and room for both phases' partial sums: the kernels with LOCAL (one token on 128 experts of 2048 x 768 268 us for 284).
+bool one_down_item(const MoeDispatch &d, const Plan &pl, size_t parts_bytes) {
+  const uint64_t P = (uint64_t)d.n_tokens * d.slots;
+  return pl.nt == 1 && P * d.items_per_pass[1] <= d.n_ctas && pl.frag_cols / 2 * ((pl.ph[1].kb_split + 3) / 4) <= CONSUMER_WARPS &&
+         (pl.ph[0].n_ksplit * P * 2 * d.F + pl.ph[1].n_ksplit * P * d.D) * 4 <= parts_bytes;
+}
 }  // namespace
+
+// (248 us for 268.  Where the weights of an item are longer it loses: one token on 8 experts of 4096 x 14336 208 us for 201.)
+bool route_in_stream(const MoeDispatch &d, const RouterDev &r) {
+  return d.pass_desc && d.x_rows && d.n_tokens == 1 && r.num_experts <= 256 && d.slots <= 32 &&
+         one_down_item(d, plan_dispatch(d, (int)d.n_ctas), scratch_layout(d.scratch_pairs, d.D, d.F).parts_bytes);
+}
 
 void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm) {
   if (sm_count > MER_MAX_CTAS1 - 1) sm_count = MER_MAX_CTAS1 - 1;
@@ -1060,19 +1114,17 @@ cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaS
   p.n_frag = pl.n_frag, p.frag_cols = pl.frag_cols, p.frag_bytes = pl.frag_bytes;
   p.parts = reinterpret_cast<float *>(base + L.parts);
   p.bar = reinterpret_cast<uint32_t *>(base + L.bar);
-  // at most one down item a CTA, of no more than one round of its warps (28 units, 3.5 rounds: one token on 8 x 2 experts of 4096 x 14336 209 us for 201), and room for both phases' partial sums
-  const size_t gate_up_floats = (size_t)pl.ph[0].n_ksplit * P * 2 * d.F, down_floats = (size_t)pl.ph[1].n_ksplit * P * d.D;
-  const bool local = pl.nt == 1 && (uint64_t)P * d.items_per_pass[1] <= (uint64_t)sm_count && pl.frag_cols / 2 * ((pl.ph[1].kb_split + 3) / 4) <= CONSUMER_WARPS &&
-                     (gate_up_floats + down_floats) * 4 <= L.parts_bytes;
+  const bool local = one_down_item(d, pl, L.parts_bytes);
   // the weighted combine of the layer rides on the same launch when the caller asked for it
   const int tail = d.fuse_combine ? TAIL_COMBINE : (d.fuse_reduce && pl.ph[1].n_ksplit > 1) ? TAIL_REDUCE : TAIL_NONE;
   cudaError_t e;
   int n = 0;
   auto launch = [&](uint32_t phases, bool sync) {
-    p.local = phases == 3 && sync && local, p.down_parts = p.local ? p.parts + gate_up_floats : p.parts;
+    const bool here = phases == 3 && sync && local;
+    p.down_parts = here ? p.parts + (size_t)pl.ph[0].n_ksplit * P * 2 * d.F : p.parts;
     p.phases = phases, p.sync = sync ? 1 : 0, p.tail = sync && (phases & 2) ? tail : TAIL_NONE;
     n++;
-    e = d.dtype == MER_DTYPE_Q4_0 ? launch_stream<MER_DTYPE_Q4_0>(p, pl.nt, pl.smem, sm_count, s) : launch_stream<MER_DTYPE_Q8_0>(p, pl.nt, pl.smem, sm_count, s);
+    e = d.dtype == MER_DTYPE_Q4_0 ? launch_stream<MER_DTYPE_Q4_0>(p, pl.nt, here, pl.smem, sm_count, s) : launch_stream<MER_DTYPE_Q8_0>(p, pl.nt, here, pl.smem, sm_count, s);
     return e == cudaSuccess;
   };
   bool whole = true;  // the grid-wide steps ran

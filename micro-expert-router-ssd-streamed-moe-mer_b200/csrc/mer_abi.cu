@@ -1368,6 +1368,8 @@ int enqueue_layer(mer_backend *b, uint32_t layer, const float *d_x, size_t n_tok
   }
   if (re.layer_flags & MER_LAYER_RESIDUAL) d.residual = d_x, d.routed_slots = r.top_k;
   const RouterDev &r2 = rl;
+  d.route_here = run_ffn_too && route_in_stream(d, rl);
+  d.route = rl;
   CU(MER_ERR_SUBMISSION, "router kernel", launch_router(r2, d, b->cfg.max_tokens, s, launches, run_ffn_too));
   if (run_ffn_too) {
     if (ev) cudaEventRecord(ev[1], s);
