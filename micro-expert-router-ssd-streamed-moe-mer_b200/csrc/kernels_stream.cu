@@ -1,37 +1,36 @@
-// Streaming expert FFN for decode-sized token groups (a few tokens per expert): HBM-bound.
+// Streaming expert FFN for decode-sized token groups (a few tokens per expert).
 //
-// Data flow per projection phase (gate/up, then down):
-//   * Experts are resident in the tile-major fragment layout of layout.cuh (the reference's bytes,
-//     permuted at admission).  A stage of the ring is one chunk of each of an item's sixteen 16-row tiles, each chunk
-//     moved global -> shared memory by ONE bulk async copy (cp.async.bulk, completion on an mbarrier):
-//     every byte of an expert is read from HBM once, as a linear stream.
-//   * Warps unpack the integer part of the weights straight into f16 mma.sync A fragments.  A
-//     4-bit or 8-bit field masked into the low mantissa bits of an f16 IS the subnormal value
-//     q * 2^-24 (q * 2^-20 for a field at bits 4..7), so unpacking is one LOP3 per two weights and
-//     the integers are exact.  The zero point (8 for Q4_0, 128 for the sign-flipped Q8_0 byte) is
-//     added four blocks at a time as the product of the blocks' scales and -zp * sum(x_block).
-//   * Activations are pre-split into f16 hi + lo parts (22+ significant bits) after an exact
-//     power-of-two per-token scaling; hi and lo are two columns of the n=8 MMA tile, so one tile
-//     carries 4 tokens.  Products are exact, accumulation is fp32 in the tensor core.
-//   * The per-block f16 scale d is applied in fp32 when a block's partial is folded into the row
-//     accumulator: acc += d * partial (the ordering of matmul_q4_0.wgsl:65-85 in the reference).
+// One cooperative launch runs a layer's gate/up phase, the hidden values, the down phase and the weighted combine:
+//   * Experts are resident in the tile-major fragment layout of layout.cuh (the reference's blocks, permuted at admission).  A stage
+//     of the ring is one chunk of each of an item's sixteen 16-row tiles, each chunk moved global -> shared memory by ONE bulk async
+//     copy (cp.async.bulk, completion on an mbarrier): every byte of an expert is read from HBM once, as a linear stream.  The
+//     copies run on into the down phase while the grid finishes the gate/up phase.
+//   * Warps unpack the integer part of the weights straight into f16 mma.sync A fragments.  A 4-bit or 8-bit field masked into the
+//     low mantissa bits of an f16 IS the subnormal value q * 2^-24 (q * 2^-20 for a field at bits 4..7), so unpacking is one ALU
+//     instruction per two weights and the integers are exact.  The zero point (8 for Q4_0, 128 for the biased Q8_0 byte) is added
+//     four blocks at a time as the product of the blocks' scales and -zp * sum(x_block).
+//   * Activations come as images (act_image.cuh): f16 hi + lo parts (22 significant bits) after an exact power-of-two scaling of
+//     the row; hi and lo are two columns of the n=8 MMA tile, so one tile carries 4 tokens.  Products are exact, accumulation is
+//     fp32 in the tensor core.  A CTA copies those of the unit, i.e. (pass, K split), that comes next while it multiplies the present
+//     one; warps meet at no barrier when units change.
+//   * The per-block f16 scale d is applied in fp32 when a block's partial is folded into the row accumulator: acc += d * partial
+//     (the ordering of matmul_q4_0.wgsl:65-85 in the reference).
 //
-// Work is cut into items (token pass, K split, group of 16 tiles).  Each of the 16 consumer warps of
-// a CTA owns one 16-row tile of the item over the item's K range: no warp ever waits for another
-// one's partial sums (an earlier version split K across warps and lost a third of its time at the
-// hand-off barrier).  Load balance comes from splitting K across CTAs instead: partial sums go to
-// scratch and the launch's tail adds them behind a grid-wide barrier (SiLU(gate)*up, or the weighted combine
-// of the down partials; kernels of their own where a cooperative launch is refused), always in the same
-// order, so results are deterministic.  Each persistent CTA takes a contiguous item range and rebuilds
-// activation fragments only when its (pass, K split) changes; no atomics on data, and that barrier is the only
-// wait between CTAs.  Every wait is bounded: on expiry the warp stops computing, the CTA latches
-// MER_DEVSTAT_TIMEOUT, drains its copies in flight and returns.
+// Work is cut into items (token pass, K split, group of 16 tiles), which a scheduler warp claims for its CTA; each of the eight
+// consumer warps owns two tiles of the item over its K range, so no warp ever waits for another one's partial sums.  Load balance
+// comes from splitting K across CTAs and from taking over items: partial sums go to scratch and are added behind grid-wide barriers
+// (SiLU(gate) * up between the phases, the weighted combine at the end; kernels of their own where a cooperative launch is
+// refused), always in the same order, so results are deterministic; no atomics on data.  Every wait is bounded: on expiry the warp
+// stops computing, the CTA latches MER_DEVSTAT_TIMEOUT, drains its copies in flight and returns.
 //
-// What bounds it: the consumers' instructions.  Weights are waited for a tenth of the time; a block of 16 rows takes a warp about
-// 30 instructions (40 with the zero point as every block's accumulator start) at one issue in two cycles of a scheduler's four
-// warps, 38 GB/s per SM of the 44 that HBM gives.  Around the multiplication: first fragments 3 to 5 us, a rebuild 3, the grid
-// barrier 1.5 and its tail 0.5 to 4.  Measured, gate/up and down together: 64 tokens on 128 experts of 2048 x 768 (Q8_0) 172 -> 154 us;
-// 16 tokens on 8 of 4096 x 14336 (Q4_0) 285 -> 229; 16 on 256 of 7168 x 2048 589 -> 490; 1 on 8 of 4096 x 14336 76 -> 69.
+// What bounds it: instructions of the consumers, next to HBM.  On sm_100 an m16n8k16 holds a scheduler's FMA pipe for 8 cycles, and an ALU
+// operation half a warp-instruction slot: a block of 16 rows costs 2.25 MMAs, 4 FMAs and 10 (Q4_0) or 8 (Q8_0) ALU operations at up to
+// four tokens.  With the copies left out the gate/up phase of 64 tokens on 128 experts of 2048 x 768 took 74 us of 79, with the
+// products left out 65; 16 tokens on 8 of 4096 x 14336 122 of 128, and 91.  Q8_0 bytes with the sign bit to flip (12 ALU operations
+// a block) took 10 % more of the whole layer, and one tile a warp in sixteen warps 6 % more on 16 tokens of 256 x 7168 x 2048
+// (even elsewhere).  Around the loops: barriers 1.3 us each, hidden values 2 to 3, combine 3 to 5, first activations 3 to 4.  FFN of a layer, two launches
+// before and one now: 64 tokens on 128 experts of 2048 x 768 146 -> 129 us, 16 on 256 of 7168 x 2048 500 -> 470, one on 128 of
+// 2048 x 768 (with its routing) 37 -> 28.
 #include "kernels.h"
 
 #include <cuda_fp16.h>
@@ -48,9 +47,6 @@
 
 namespace {
 
-// A consumer warp multiplies two tiles by every activation fragment that it loads.  What bounds these loops is shared memory: with one
-// tile per warp (sixteen warps) sixteen tiles read a block's fragments sixteen times, 13 wavefronts a tile and block of Q8_0 and 11 of Q4_0 at
-// eight tokens, of which 8 are fragments, beside the 4 or 2 with which the copies write it.
 constexpr int ITEM_TILES = 16, WARP_TILES = 2, CONSUMER_WARPS = ITEM_TILES / WARP_TILES, CONSUMERS = CONSUMER_WARPS * 32;
 constexpr int PRODUCER_WARPS = 2;  // each issues the bulk copies of half a stage's tiles: one warp alone was busy ~90 % of the time
 constexpr int SCHED_WARP = CONSUMER_WARPS + PRODUCER_WARPS;  // claims the CTA's items and fetches their activations
