@@ -122,30 +122,38 @@ __device__ bool grid_barrier(uint32_t *counter, uint32_t *s_ok, uint32_t *status
 // Four hidden values of a pair, from f0 on: h = SiLU(sum of gate partials) * (sum of up partials), partials added in K-split order, times the
 // row's scale.  That comes from a bound, (splits * max |gate partial|) * (splits * max |up partial|) >= max |h|, which is known before any h
 // is: it puts the row below 2^15, and a bound 2^8 too large still leaves every value within 2^-9 of the row's maximum its full 22 bits.
-__device__ __forceinline__ float4 hidden_values(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t pair, uint32_t f0, bool inside, float &sc) {
+struct HiddenSums {
+  float4 g, up;
+  float gm, um;  // bounds of the row's gate and up sums
+};
+__device__ __forceinline__ HiddenSums hidden_sums(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t pair, uint32_t f0, bool inside) {
   const uint32_t P = d.n_tokens * d.slots, F = d.F;
-  float4 g = make_float4(0, 0, 0, 0), up = make_float4(0, 0, 0, 0);
-  float gm = __uint_as_float(__ldcg(d.amax + pair)) * (float)n_ksplit, um = __uint_as_float(__ldcg(d.amax + d.scratch_pairs + pair)) * (float)n_ksplit;
+  HiddenSums v;
+  v.g = v.up = make_float4(0, 0, 0, 0);
+  v.gm = __uint_as_float(__ldcg(d.amax + pair)) * (float)n_ksplit, v.um = __uint_as_float(__ldcg(d.amax + d.scratch_pairs + pair)) * (float)n_ksplit;
   if (inside) {
 #pragma unroll 4
     for (uint32_t k = 0; k < n_ksplit; k++) {  // loads of several splits in flight, added in order
       const float *base = parts + ((size_t)k * P + pair) * 2 * F;
       const float4 a = __ldcg(reinterpret_cast<const float4 *>(base + f0)), b = __ldcg(reinterpret_cast<const float4 *>(base + F + f0));
-      g.x += a.x, g.y += a.y, g.z += a.z, g.w += a.w;
-      up.x += b.x, up.y += b.y, up.z += b.z, up.w += b.w;
+      v.g.x += a.x, v.g.y += a.y, v.g.z += a.z, v.g.w += a.w;
+      v.up.x += b.x, v.up.y += b.y, v.up.z += b.z, v.up.w += b.w;
     }
   }
+  return v;
+}
+__device__ __forceinline__ float4 hidden_finish(const MoeDispatch &d, HiddenSums v, float &sc) {
   const bool clamp = d.swiglu_limit > 0.0f && isfinite(d.swiglu_limit);
-  if (clamp && gm == gm) gm = fminf(gm, d.swiglu_limit);
+  if (clamp && v.gm == v.gm) v.gm = fminf(v.gm, d.swiglu_limit);
   sc = 1.0f;
-  if (!isfinite(gm) || !isfinite(um)) {
+  if (!isfinite(v.gm) || !isfinite(v.um)) {
     sc = __int_as_float(0x7fc00000);  // non-finite values poison the row, as they would in fp32
-  } else if (gm > 0.0f && um > 0.0f) {
+  } else if (v.gm > 0.0f && v.um > 0.0f) {
     int eg, eu;
-    frexpf(gm, &eg), frexpf(um, &eu);  // |h| < 2^(eg + eu), and < 2^128 if it is finite
+    frexpf(v.gm, &eg), frexpf(v.um, &eu);  // |h| < 2^(eg + eu), and < 2^128 if it is finite
     sc = ldexpf(1.0f, max(-113, min(127, 15 - (eg + eu))));
   }
-  const float gv[4] = {g.x, g.y, g.z, g.w}, uv[4] = {up.x, up.y, up.z, up.w};
+  const float gv[4] = {v.g.x, v.g.y, v.g.z, v.g.w}, uv[4] = {v.up.x, v.up.y, v.up.z, v.up.w};
   float hv[4];
 #pragma unroll
   for (int i = 0; i < 4; i++) {
@@ -155,15 +163,26 @@ __device__ __forceinline__ float4 hidden_values(const MoeDispatch &d, const floa
   }
   return make_float4(hv[0], hv[1], hv[2], hv[3]);
 }
-// A warp's share of the step between the phases: 128 consecutive hidden values of one pair into the activation image of the down phase.
-__device__ __forceinline__ void hidden_unit(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t unit, uint32_t lane) {
-  const uint32_t fchunks = (d.F + 127) / 128, pair = unit / fchunks, q = (unit % fchunks) * 32 + lane;
-  const bool inside = q * 4 < d.F;
-  float sc;
-  const float4 v = hidden_values(d, parts, n_ksplit, pair, q * 4, inside, sc);
-  if (q == 0) d.h_un[pair] = POW2_24 / sc;
-  const ImageRow row(d.h, d.act_seeds, pair, d.F);
-  image_store4(d.dtype, v, q, inside, row.hi, row.lo, row.seed_hi, row.seed_lo);
+// A warp's share of the step between the phases: units first, first + step, ... of 128 consecutive hidden values of one pair, into the activation
+// image of the down phase.  What bounds it is the round trip of a unit's loads, so the next unit's are in flight while one is finished
+// (43 tokens on 96 experts of 1792 x 6656, 15 units a warp: 381 -> 376 us a layer; 16 on 8 of 4096 x 14336, three: 232 -> 228).
+__device__ __forceinline__ void hidden_units(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t first, uint32_t step, uint32_t lane) {
+  const uint32_t fchunks = (d.F + 127) / 128, units = d.n_tokens * d.slots * fchunks;
+  if (first >= units) return;
+  uint32_t pair = first / fchunks, q = (first % fchunks) * 32 + lane;
+  HiddenSums v = hidden_sums(d, parts, n_ksplit, pair, q * 4, q * 4 < d.F);
+#pragma unroll 1
+  for (uint32_t u = first; u < units; u += step) {
+    const uint32_t next = u + step, pair1 = next / fchunks, q1 = (next % fchunks) * 32 + lane;
+    HiddenSums v1 = v;
+    if (next < units) v1 = hidden_sums(d, parts, n_ksplit, pair1, q1 * 4, q1 * 4 < d.F);
+    float sc;
+    const float4 h = hidden_finish(d, v, sc);
+    if (q == 0) d.h_un[pair] = POW2_24 / sc;
+    const ImageRow row(d.h, d.act_seeds, pair, d.F);
+    image_store4(d.dtype, h, q, q * 4 < d.F, row.hi, row.lo, row.seed_hi, row.seed_lo);
+    pair = pair1, q = q1, v = v1;
+  }
 }
 
 // After all CTAs have left their outputs of the down phase: the arithmetic of k_combine / k_reduce_ksplit, spread over the consumers of the grid.
@@ -607,7 +626,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
           const uint32_t tok = u / chunks, q = (u % chunks) * 32 + lane;
           const bool inside = q < kbn * 8;
           float sc;
-          const float4 v = hidden_values(d, p.parts, p.ph[0].n_ksplit, s_pair[buf * 8 + tok], (it.ks * kb_split * 8 + q) * 4, inside, sc);
+          const float4 v = hidden_finish(d, hidden_sums(d, p.parts, p.ph[0].n_ksplit, s_pair[buf * 8 + tok], (it.ks * kb_split * 8 + q) * 4, inside), sc);
           image_store4(DT, v, q, inside, frag + 2 * tok * stride, frag + (2 * tok + 1) * stride, seeds + 2 * tok * words, seeds + (2 * tok + 1) * words);
           if (q == 0) s_un[buf * 8 + tok] = POW2_24 / sc;
         }
@@ -850,9 +869,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       continue;
     }
     if (grid_barrier(p.bar + 1, s_ok, d.status)) {
-      const uint32_t units = (uint32_t)n_pairs * ((d.F + 127) / 128);
-#pragma unroll 1
-      for (uint32_t u = blockIdx.x * CONSUMER_WARPS + warp; u < units; u += gridDim.x * CONSUMER_WARPS) hidden_unit(d, p.parts, p.ph[0].n_ksplit, u, lane);
+      hidden_units(d, p.parts, p.ph[0].n_ksplit, blockIdx.x * CONSUMER_WARPS + warp, gridDim.x * CONSUMER_WARPS, lane);
     } else {
       dead = true;
     }
@@ -873,8 +890,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_ffn_stream(const __grid_constant
 
 // The step between the phases as a kernel of its own, where a cooperative launch is refused.  A warp per unit.
 __global__ void __launch_bounds__(256) k_hidden(const __grid_constant__ MoeDispatch d, const float *parts, uint32_t n_ksplit) {
-  const uint32_t unit = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (unit < d.n_tokens * d.slots * ((d.F + 127) / 128)) hidden_unit(d, parts, n_ksplit, unit, threadIdx.x & 31);
+  hidden_units(d, parts, n_ksplit, blockIdx.x * 8 + (threadIdx.x >> 5), gridDim.x * 8, threadIdx.x & 31);
 }
 
 __global__ void __launch_bounds__(256) k_x_images(const __grid_constant__ MoeDispatch d) {
