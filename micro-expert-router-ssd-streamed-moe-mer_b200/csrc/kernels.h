@@ -74,11 +74,10 @@ struct MoeDispatch {
   uint32_t *pass_group, *pass_start, *pass_count, *n_passes;
   PassDesc *pass_desc;      // the same for the streaming kernels (null: the GEMM path), which find the first pass of a group in pass_group
   uint64_t *taken;          // [2][MER_MAX_CTAS1] items taken from either end of every CTA's range, zeroed by the grouping kernels
-  uint32_t *amax;           // [2][scratch_pairs] max |gate| and max |up| over a pair's partial sums (float bits), zeroed by the grouping kernels
   // Activation images of the streaming kernels (act_image.cuh).  The tokens' lie where the outputs of the down projection go later,
   // the hidden rows' in `h`; both share the seeds.  Null: nobody multiplies them.
   void *x_rows;
-  float *act_seeds, *x_un, *h_un;  // *_un: 2^24 / scale of every row
+  float *act_seeds, *x_un, *h_un;  // *_un: 2^24 / scale of every row, of hidden rows in every K split
   // One token: the router kernel leaves the logits only, and every CTA of the streaming kernel selects the experts itself, by this router.
   int route_here;
   RouterDev route;
@@ -220,7 +219,7 @@ cudaError_t launch_f32_to_f16(const float *src, uint16_t *dst, size_t n, cudaStr
 bool stream_ffn_supported(int dtype, uint32_t D, uint32_t F);
 size_t stream_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F);
 cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaStream_t s, int *launches, cudaEvent_t ev_mid);
-// Points d.pass_*, d.amax and the activation images into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
+// Points d.pass_* and the activation images into the scratch and picks tokens_per_pass for this dispatch (call before grouping).
 void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm = false);
 // Whether launch_ffn_stream can route this (bound) dispatch itself: d.route_here.
 bool route_in_stream(const MoeDispatch &d, const RouterDev &r);

@@ -136,9 +136,6 @@ __device__ __forceinline__ void put_pass(const MoeDispatch &d, uint32_t pass, ui
   }
 }
 __device__ __forceinline__ const uint8_t *expert_payload(const MoeDispatch &d, uint32_t eid) { return eid < d.max_experts ? d.expert_ptr[eid] : nullptr; }
-__device__ __forceinline__ void clear_maxima(const MoeDispatch &d, uint32_t pair) {
-  if (d.pass_desc) d.amax[pair] = 0, d.amax[d.scratch_pairs + pair] = 0;
-}
 __device__ __forceinline__ void put_pair(const MoeDispatch &d, uint32_t at, uint32_t pair) {
   d.perm[at] = pair;
   if (d.pos) d.pos[pair] = at;
@@ -148,15 +145,13 @@ __device__ __forceinline__ void clear_taken(const MoeDispatch &d) {  // by a CTA
 }
 
 // Cuts every group into passes of at most d.tokens_per_pass pairs (the unit the streaming FFN works
-// on) and clears the per-pair max cells.  One CTA of 256 threads; `off` = the group offsets.
+// on).  One CTA of 256 threads; `off` = the group offsets.
 // `perm_ready`: the pairs are in d.perm, else k_group_scatter puts them into the passes.
 __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off, bool perm_ready) {
   __shared__ uint32_t s_pcnt[257];
   __shared__ uint8_t s_cost[1024];  // cost of each of the first 1024 passes (the weighted work split below)
-  const uint32_t tpp = d.tokens_per_pass, P = d.n_tokens * d.slots;
+  const uint32_t tpp = d.tokens_per_pass;
   const uint32_t tpp_shift = 31 - __clz(tpp);  // tokens per pass is a power of two (4 or 8; 16 .. 128 for the GEMM kernels)
-#pragma unroll 1
-  for (uint32_t i = threadIdx.x; i < P; i += 256) clear_maxima(d, i);
   clear_taken(d);
   const uint32_t per = (d.n_groups + 255) / 256;
   const uint32_t g0 = threadIdx.x * per, g1 = min(g0 + per, d.n_groups);
@@ -368,7 +363,6 @@ __device__ void build_groups_small(const RouterDev &r, const MoeDispatch &d) {
     const uint32_t count = min(tpp, __popc(same) - rank), pass = __popc(starters & ((1u << pos) - 1));
     if (starts) put_pass(d, pass, key, base, pos, count);
     if (valid) d.pass_desc[__popc(starters & ((2u << pos) - 1)) - 1].pair[rank % tpp] = p;
-    if (p < P) clear_maxima(d, p);
     if (p == 0) {
       d.offsets[d.n_groups] = n_valid;  // all of the offsets that anyone reads after the streaming kernels
       d.n_passes[0] = s_np = np;
@@ -395,9 +389,8 @@ __device__ __forceinline__ void build_groups_token(const MoeDispatch &d, uint32_
   __shared__ uint32_t s_np;
   clear_taken(d);
   if (threadIdx.x < 32) {
-    const uint32_t p = threadIdx.x, P = d.slots;
+    const uint32_t p = threadIdx.x;
     const uint32_t valid = __ballot_sync(0xffffffffu, eid != MER_NONE), pass = __popc(valid & ((1u << p) - 1));
-    if (p < P) clear_maxima(d, p);
     if (eid != MER_NONE) {
       put_pass(d, pass, 0, expert_payload(d, eid), pass, 1);
       d.pass_desc[pass].pair[0] = p;
@@ -434,7 +427,6 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
   __syncthreads();
 #pragma unroll 1
   for (uint32_t p = tid; p < P; p += 256) {
-    clear_maxima(d, p);
     const uint32_t eid = __ldcg(d.pair_expert + p);
     uint32_t v = MER_NONE;
     if (eid != MER_NONE) {
@@ -748,7 +740,6 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     const uint32_t tt = blockIdx.x - logit_ctas;
     if (group_here == ROUTE_LATER && tt == 0) {  // what the grouping would clear
       if (threadIdx.x == 0) *d.status = 0;
-      if (threadIdx.x < d.slots) clear_maxima(d, threadIdx.x);
       clear_taken(d);
     }
     if (tt < n_here) build_x_image(d, t0 + tt, threadIdx.x, ROUTER_THREADS, &s_part[0][0][0]);

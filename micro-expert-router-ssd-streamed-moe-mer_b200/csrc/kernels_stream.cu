@@ -119,69 +119,96 @@ __device__ bool grid_barrier(uint32_t *counter, uint32_t *s_ok, uint32_t *status
   return *(volatile uint32_t *)s_ok != 0;
 }
 
-// Four hidden values of a pair, from f0 on: h = SiLU(sum of gate partials) * (sum of up partials), partials added in K-split order, times the
-// row's scale.  That comes from a bound, (splits * max |gate partial|) * (splits * max |up partial|) >= max |h|, which is known before any h
-// is: it puts the row below 2^15, and a bound 2^8 too large still leaves every value within 2^-9 of the row's maximum its full 22 bits.
-struct HiddenSums {
-  float4 g, up;
-  float gm, um;  // bounds of the row's gate and up sums
-};
-__device__ __forceinline__ HiddenSums hidden_sums(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t pair, uint32_t f0, bool inside) {
-  const uint32_t P = d.n_tokens * d.slots, F = d.F;
-  HiddenSums v;
-  v.g = v.up = make_float4(0, 0, 0, 0);
-  v.gm = __uint_as_float(__ldcg(d.amax + pair)) * (float)n_ksplit, v.um = __uint_as_float(__ldcg(d.amax + d.scratch_pairs + pair)) * (float)n_ksplit;
-  if (inside) {
-#pragma unroll 4
-    for (uint32_t k = 0; k < n_ksplit; k++) {  // loads of several splits in flight, added in order
-      const float *base = parts + ((size_t)k * P + pair) * 2 * F;
-      const float4 a = __ldcg(reinterpret_cast<const float4 *>(base + f0)), b = __ldcg(reinterpret_cast<const float4 *>(base + F + f0));
-      v.g.x += a.x, v.g.y += a.y, v.g.z += a.z, v.g.w += a.w;
-      v.up.x += b.x, v.up.y += b.y, v.up.z += b.z, v.up.w += b.w;
+// Four hidden values of a pair from each of `R` places: h = SiLU(sum of gate partials) * (sum of up partials), partials added in K-split order.  Place r
+// is f0 + r * step; zeros from f_end on.
+template <int R>
+__device__ __forceinline__ void hidden_values(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t pair, uint32_t f0, uint32_t step, uint32_t f_end, float4 (&h)[R]) {
+  const uint32_t F = d.F;
+  const float *base = parts + (size_t)pair * 2 * F + f0;
+  const size_t part = (size_t)d.n_tokens * d.slots * 2 * F;
+  float4 up[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) h[r] = up[r] = make_float4(0, 0, 0, 0);
+#pragma unroll (8 / R)
+  for (uint32_t k = 0; k < n_ksplit; k++, base += part) {  // loads of several splits in flight, added in order
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+      if (f0 + r * step >= f_end) continue;
+      const float4 a = __ldcg(reinterpret_cast<const float4 *>(base + r * step)), b = __ldcg(reinterpret_cast<const float4 *>(base + F + r * step));
+      h[r].x += a.x, h[r].y += a.y, h[r].z += a.z, h[r].w += a.w;
+      up[r].x += b.x, up[r].y += b.y, up[r].z += b.z, up[r].w += b.w;
     }
   }
-  return v;
-}
-__device__ __forceinline__ float4 hidden_finish(const MoeDispatch &d, HiddenSums v, float &sc) {
   const bool clamp = d.swiglu_limit > 0.0f && isfinite(d.swiglu_limit);
-  if (clamp && v.gm == v.gm) v.gm = fminf(v.gm, d.swiglu_limit);
-  sc = 1.0f;
-  if (!isfinite(v.gm) || !isfinite(v.um)) {
-    sc = __int_as_float(0x7fc00000);  // non-finite values poison the row, as they would in fp32
-  } else if (v.gm > 0.0f && v.um > 0.0f) {
-    int eg, eu;
-    frexpf(v.gm, &eg), frexpf(v.um, &eu);  // |h| < 2^(eg + eu), and < 2^128 if it is finite
-    sc = ldexpf(1.0f, max(-113, min(127, 15 - (eg + eu))));
-  }
-  const float gv[4] = {v.g.x, v.g.y, v.g.z, v.g.w}, uv[4] = {v.up.x, v.up.y, v.up.z, v.up.w};
-  float hv[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    float gate = gv[i];
+  auto one = [&](float gate, float u) {
     if (clamp && gate == gate) gate = fminf(fmaxf(gate, -d.swiglu_limit), d.swiglu_limit);
-    hv[i] = __fdividef(gate, 1.0f + __expf(-gate)) * uv[i] * sc;
-  }
-  return make_float4(hv[0], hv[1], hv[2], hv[3]);
+    return __fdividef(gate, 1.0f + __expf(-gate)) * u;
+  };
+#pragma unroll
+  for (int r = 0; r < R; r++) h[r] = make_float4(one(h[r].x, up[r].x), one(h[r].y, up[r].y), one(h[r].z, up[r].z), one(h[r].w, up[r].w));
 }
-// A warp's share of the step between the phases: units first, first + step, ... of 128 consecutive hidden values of one pair, into the activation
-// image of the down phase.  What bounds it is the round trip of a unit's loads, so the next unit's are in flight while one is finished
-// (43 tokens on 96 experts of 1792 x 6656, 15 units a warp: 381 -> 376 us a layer; 16 on 8 of 4096 x 14336, three: 232 -> 228).
-__device__ __forceinline__ void hidden_units(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, uint32_t first, uint32_t step, uint32_t lane) {
-  const uint32_t fchunks = (d.F + 127) / 128, units = d.n_tokens * d.slots * fchunks;
-  if (first >= units) return;
-  uint32_t pair = first / fchunks, q = (first % fchunks) * 32 + lane;
-  HiddenSums v = hidden_sums(d, parts, n_ksplit, pair, q * 4, q * 4 < d.F);
+// Largest magnitude of a warp's values, as float bits: a NaN sorts above all numbers.
+__device__ __forceinline__ uint32_t abs_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ uint32_t max_bits(uint32_t m, float4 v) { return max(max(max(max(m, abs_bits(v.x)), abs_bits(v.y)), abs_bits(v.z)), abs_bits(v.w)); }
+// Power of two that brings a largest magnitude into [2^14, 2^15): f16 hi + lo parts then have 22 bits for all values within 2^-16 of it (2^-12 in
+// the upper nibbles' places of Q4_0), and an error of 2^-39 (2^-35) of it below.  It has to be that of the values themselves: a bound made of
+// max |gate| and max |up| is too large by e^20 where an expert's gates lie near -20.
+__device__ __forceinline__ float hidden_scale(uint32_t bits) {
+  const float mx = __uint_as_float(bits);
+  if (mx == 0.0f) return 1.0f;
+  if (!isfinite(mx)) return __int_as_float(0x7fc00000);  // non-finite values poison the row, as they would in fp32
+  int e;
+  frexpf(mx, &e);
+  return ldexpf(1.0f, min(127, 15 - e));
+}
+// The step between the phases: the hidden values into the activation images of the down phase.  A unit is what one down item multiplies, the values of a pair in
+// one K split, with a scale of its own: `chunks` runs of 128 values, by a team of so many of the CTA's warps that each has HIDDEN_RUNS of them in
+// registers, or of more while no warp has to take a second unit.  A team of eight keeps the rest of longer units in `stash` (kb_split x 128 bytes).
+// What bounds it is the round trip of a unit's loads.  Us a layer, with a scale per row from a bound, 128 values a unit, / this: 64 tokens on 128 experts of
+// 2048 x 768 154 / 153; 43 on 96 of 1792 x 6656 378 / 368; 16 on 8 of 4096 x 14336 216 / 213; one on those (eight units of 3584 values) 67.0 / 67.4.
+// Four runs in registers spill: the first 155.
+constexpr int HIDDEN_RUNS = 2;
+__device__ __forceinline__ void hidden_units(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, const PhaseParams &down, uint32_t cta, uint32_t n_ctas, uint32_t warp,
+                                             uint32_t lane, uint32_t *s_red, float4 *stash) {
+  const uint32_t chunks = (down.kb_split + 3) / 4, units = d.n_tokens * d.slots * down.n_ksplit;
+  uint32_t W = 1, log_w = 0;
+  while (W < CONSUMER_WARPS && W < chunks && (W * HIDDEN_RUNS < chunks || units * W < n_ctas * (CONSUMER_WARPS / 2))) W *= 2, log_w++;
+  const uint32_t teams = CONSUMER_WARPS >> log_w, team = warp >> log_w, member = warp & (W - 1), span = W * HIDDEN_RUNS * 32;
+  uint32_t *red = s_red + team * W;
 #pragma unroll 1
-  for (uint32_t u = first; u < units; u += step) {
-    const uint32_t next = u + step, pair1 = next / fchunks, q1 = (next % fchunks) * 32 + lane;
-    HiddenSums v1 = v;
-    if (next < units) v1 = hidden_sums(d, parts, n_ksplit, pair1, q1 * 4, q1 * 4 < d.F);
-    float sc;
-    const float4 h = hidden_finish(d, v, sc);
-    if (q == 0) d.h_un[pair] = POW2_24 / sc;
+  for (uint32_t u = cta * teams + team, odd = 0; u < units; u += n_ctas * teams, odd ^= CONSUMER_WARPS) {
+    const uint32_t pair = u / down.n_ksplit, ks = u % down.n_ksplit, kb0 = ks * down.kb_split, n4 = min(down.kb_split, down.kb_total - kb0) * 8;
+    const uint32_t turns = (n4 + span - 1) / span;
+    float4 h[HIDDEN_RUNS];
+    uint32_t m = 0;
+#pragma unroll 1
+    for (uint32_t turn = 0; turn < turns; turn++) {
+      hidden_values<HIDDEN_RUNS>(d, parts, n_ksplit, pair, (kb0 * 8 + turn * span + member * 32 + lane) * 4, W * 128, (kb0 * 8 + n4) * 4, h);
+#pragma unroll
+      for (int r = 0; r < HIDDEN_RUNS; r++) {
+        m = max_bits(m, h[r]);
+        if (turn + 1 < turns) stash[turn * span + (r * W + member) * 32 + lane] = h[r];
+      }
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    if (W > 1) {  // (two sets of words in turn: one barrier a unit)
+      if (lane == 0) red[odd + member] = m;
+      asm volatile("bar.sync %0, %1;" ::"r"(2 + team), "r"(W * 32) : "memory");
+      m = __reduce_max_sync(0xffffffffu, lane < W ? red[odd + lane] : 0u);
+    }
+    const float sc = hidden_scale(m);
+    if (member == 0 && lane == 0) d.h_un[u] = POW2_24 / sc;
     const ImageRow row(d.h, d.act_seeds, pair, d.F);
-    image_store4(d.dtype, h, q, q * 4 < d.F, row.hi, row.lo, row.seed_hi, row.seed_lo);
-    pair = pair1, q = q1, v = v1;
+#pragma unroll 1
+    for (uint32_t turn = turns; turn-- > 0;) {  // the last one's values are still there
+#pragma unroll
+      for (int r = 0; r < HIDDEN_RUNS; r++) {
+        const uint32_t q = turn * span + (r * W + member) * 32 + lane;
+        if (turn + 1 < turns) h[r] = stash[q];
+        const float4 v = make_float4(h[r].x * sc, h[r].y * sc, h[r].z * sc, h[r].w * sc);
+        image_store4(d.dtype, v, kb0 * 8 + q, q < n4, row.hi, row.lo, row.seed_hi, row.seed_lo);
+      }
+    }
   }
 }
 
@@ -367,12 +394,11 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   uint32_t *s_info = reinterpret_cast<uint32_t *>(smem + 184);  // [2] tokens of the unit's pass
   uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 192);  // [2][8] pair index of each of them
   float *s_un = reinterpret_cast<float *>(smem + 256);          // [2][8] its 2^24 / scale
-  uint32_t *s_max = reinterpret_cast<uint32_t *>(smem + 320);   // [2][max |gate|, max |up|][8] over this CTA's tiles of the unit, float bits
+  uint32_t *s_red = reinterpret_cast<uint32_t *>(smem + 320);   // [2][CONSUMER_WARPS] the warps' maxima in the making of hidden values
   uint8_t *s_frag = smem + HEADER_BYTES;                        // [n_frag] x {fragments [frag_cols][frag_stride], zero-point terms [frag_cols][seed_words]}
   uint8_t *s_stage = s_frag + (size_t)p.n_frag * p.frag_bytes;  // [n_stages][16 tiles][chunk_stride]
   const uint32_t stage_bytes = ITEM_TILES * p.chunk_stride;
 
-  if (threadIdx.x < 32) s_max[threadIdx.x] = 0;
   if (threadIdx.x < 2) s_info[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     for (uint32_t s = 0; s < p.n_stages; s++) {
@@ -388,13 +414,6 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   grid_dep_wait();
   grid_dep_launch();
   __syncthreads();
-
-  // Lane l < 16: adds the CTA's maxima of the unit that buffer `buf` holds to its pairs'.
-  auto flush_maxima = [&](uint32_t buf, uint32_t l) {
-    const uint32_t tok = l & 7, m = s_max[buf * 16 + l];
-    if (tok < s_info[buf] && m) atomicMax(d.amax + (l >> 3) * d.scratch_pairs + s_pair[buf * 8 + tok], m);
-    s_max[buf * 16 + l] = 0;
-  };
 
   // The CTA's next item as every warp but the scheduler's sees it; a slot is free again when all have read it.
   uint32_t q_slot = 0, q_round = 0;
@@ -525,8 +544,6 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         const uint32_t kb0 = ks * f.kb_split, kbn = min(f.kb_split, f.kb_total - kb0), seed_bytes = ((kbn + 3) & ~3u) * 4;
-        if (phase == 0 && use > 0 && lane < 16) flush_maxima(buf, lane);
-        __syncwarp();
         const bool copies = !(LOCAL && phase == 1);
         if (lane == 0) mbar_expect_tx(&frag_full[buf], copies ? count * 2 * (kbn * 64 + seed_bytes) : 0);
         __syncwarp();
@@ -539,7 +556,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
             bulk_g2s(dst + col * stride, src + (size_t)kb0 * 64, kbn * 64, &frag_full[buf]);
           else
             bulk_g2s(dst + p.frag_cols * stride + col * words * 4, src + (size_t)kb0 * 4, seed_bytes, &frag_full[buf]);
-          if (part == 0) s_pair[buf * 8 + tok] = pair, s_un[buf * 8 + tok] = __ldcg(phase == 0 ? d.x_un + pair / d.slots : d.h_un + pair);
+          if (part == 0) s_pair[buf * 8 + tok] = pair, s_un[buf * 8 + tok] = __ldcg(phase == 0 ? d.x_un + pair / d.slots : d.h_un + pair * f.n_ksplit + ks);
         }
         if (lane == 0) s_info[buf] = count;
         __syncwarp();
@@ -577,25 +594,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   const uint32_t kb_split = p.ph[phase].kb_split, kb_total = p.ph[phase].kb_total;
   uint32_t cur_unit = 0, pcount = 1, buf = 0;  // units count from 1
   uint32_t fa[NT], ia[NT];  // where column g / token t of each N-tile lives
-  // Largest |gate| and |up| that this lane has seen in the unit, as float bits (NaN sorts above all): they go to the CTA's maxima when
-  // the warp leaves the unit and to the pair's when its last warp has left.  (An atomic per tile and token instead: all of a batch's on
-  // two cache lines, 16 tokens on 8 experts of 4096 x 14336 269 us a layer for 224.)
-  uint32_t gate_max[NT], up_max[NT];
-#pragma unroll
-  for (int n = 0; n < NT; n++) gate_max[n] = up_max[n] = 0;
   auto leave_unit = [&]() {
-    if (phase == 0) {
-#pragma unroll
-      for (int n = 0; n < NT; n++) {
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {  // over the 8 rows held by the lanes that share t
-          gate_max[n] = max(gate_max[n], __shfl_xor_sync(0xffffffffu, gate_max[n], o));
-          up_max[n] = max(up_max[n], __shfl_xor_sync(0xffffffffu, up_max[n], o));
-        }
-        if (g < 2) atomicMax(&s_max[buf * 16 + g * 8 + n * 4 + t], g == 0 ? gate_max[n] : up_max[n]);
-        gate_max[n] = up_max[n] = 0;
-      }
-    }
     __syncwarp();
     if (lane == 0) mbar_arrive(&frag_empty[buf]);
   };
@@ -620,19 +619,28 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       if (LOCAL && phase == 1) {
         uint8_t *frag = s_frag + buf * p.frag_bytes;
         float *seeds = reinterpret_cast<float *>(frag + p.frag_cols * stride);
-        const uint32_t chunks = (kbn + 3) / 4;
-#pragma unroll 1
-        for (uint32_t u = warp; u < pcount * chunks; u += CONSUMER_WARPS) {
-          const uint32_t tok = u / chunks, q = (u % chunks) * 32 + lane;
-          const bool inside = q < kbn * 8;
-          float sc;
-          const float4 v = hidden_finish(d, hidden_sums(d, p.parts, p.ph[0].n_ksplit, s_pair[buf * 8 + tok], (it.ks * kb_split * 8 + q) * 4, inside), sc);
+        // a run of 128 values a warp at most (one_down_item)
+        const uint32_t chunks = (kbn + 3) / 4, tok = warp / chunks, q = warp % chunks * 32 + lane;
+        const bool mine = tok < pcount, inside = mine && q < kbn * 8;
+        auto meet = [&]() {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(built);
+          dead = dead || !__all_sync(0xffffffffu, mbar_wait(built, builds++ & 1));
+        };
+        const uint32_t f0 = it.ks * kb_split * 32;
+        float4 h[1];
+        hidden_values<1>(d, p.parts, p.ph[0].n_ksplit, s_pair[buf * 8 + (mine ? tok : 0)], f0 + q * 4, 0, mine ? f0 + kbn * 32 : 0, h);
+        float4 &v = h[0];
+        const uint32_t most = __reduce_max_sync(0xffffffffu, max_bits(0, v));
+        if (lane == 0) s_red[warp] = most;
+        meet();
+        if (mine) {
+          const float sc = hidden_scale(__reduce_max_sync(0xffffffffu, lane < chunks ? s_red[tok * chunks + lane] : 0u));
+          v.x *= sc, v.y *= sc, v.z *= sc, v.w *= sc;
           image_store4(DT, v, q, inside, frag + 2 * tok * stride, frag + (2 * tok + 1) * stride, seeds + 2 * tok * words, seeds + (2 * tok + 1) * words);
           if (q == 0) s_un[buf * 8 + tok] = POW2_24 / sc;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(built);
-        dead = !__all_sync(0xffffffffu, mbar_wait(built, builds++ & 1));
+        meet();
         if (dead) break;
       }
       // an MMA output column depends on its own B column only, and the columns of absent tokens are never written out: they
@@ -841,7 +849,6 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
               gp[0] = r_lo;
               gp[d.F] = r_hi;
             }
-            gate_max[n] = max(gate_max[n], __float_as_uint(fabsf(r_lo))), up_max[n] = max(up_max[n], __float_as_uint(fabsf(r_hi)));
           } else if (valid) {
             float *yo = (k_is_split ? p.down_parts : d.y) + row * d.D + ptile * 16;
             yo[g] = r_lo;
@@ -856,10 +863,6 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
     *(volatile uint32_t *)s_abort = 1;
     atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
   }
-  if (phase == 0) {  // the maxima of the units that are still in the buffers
-    consumer_sync();
-    if (threadIdx.x < 32) flush_maxima(threadIdx.x >> 4, threadIdx.x & 15);
-  }
   if (!p.sync) continue;
   if (phase == 0) {
     // all partial sums, then all hidden rows
@@ -869,7 +872,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
       continue;
     }
     if (grid_barrier(p.bar + 1, s_ok, d.status)) {
-      hidden_units(d, p.parts, p.ph[0].n_ksplit, blockIdx.x * CONSUMER_WARPS + warp, gridDim.x * CONSUMER_WARPS, lane);
+      hidden_units(d, p.parts, p.ph[0].n_ksplit, p.ph[1], blockIdx.x, gridDim.x, warp, lane, s_red, reinterpret_cast<float4 *>(s_frag));
     } else {
       dead = true;
     }
@@ -888,9 +891,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_ffn_stream(const __grid_constant
   ffn_stream_body<DT, NT, RAGGED, ROUTE, LOCAL>(p);
 }
 
-// The step between the phases as a kernel of its own, where a cooperative launch is refused.  A warp per unit.
-__global__ void __launch_bounds__(256) k_hidden(const __grid_constant__ MoeDispatch d, const float *parts, uint32_t n_ksplit) {
-  hidden_units(d, parts, n_ksplit, blockIdx.x * 8 + (threadIdx.x >> 5), gridDim.x * 8, threadIdx.x & 31);
+// The step between the phases as a kernel of its own, where a cooperative launch is refused.
+__global__ void __launch_bounds__(CONSUMERS) k_hidden(const __grid_constant__ MoeDispatch d, const float *parts, uint32_t n_ksplit, const __grid_constant__ PhaseParams down) {
+  extern __shared__ __align__(128) uint8_t smem[];  // 2 * CONSUMER_WARPS words, then the stash
+  hidden_units(d, parts, n_ksplit, down, blockIdx.x, gridDim.x, threadIdx.x >> 5, threadIdx.x & 31, reinterpret_cast<uint32_t *>(smem), reinterpret_cast<float4 *>(smem + 128));
 }
 
 __global__ void __launch_bounds__(256) k_x_images(const __grid_constant__ MoeDispatch d) {
@@ -993,7 +997,7 @@ Plan make_plan(int dtype, uint32_t D, uint32_t F, uint32_t nt, uint32_t max_grou
 }
 
 struct ScratchLayout {
-  size_t bar, amax, pos, npass, pgroup, pstart, pcount, pdesc, taken, bounds, seeds, x_un, h_un, parts, parts_bytes, total;
+  size_t bar, pos, npass, pgroup, pstart, pcount, pdesc, taken, bounds, seeds, x_un, h_un, parts, parts_bytes, total;
 };
 
 // `parts` holds the partial sums of whichever phase is running: gate/up partials [n_ksplit][P][2][F], then (after they have become hidden
@@ -1007,7 +1011,6 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
     return o;
   };
   L.bar = take(N_BARRIERS * 4);
-  L.amax = take((size_t)2 * max_pairs * 4);
   L.pos = take((size_t)max_pairs * 4);
   L.npass = take(256);
   L.pgroup = take(((size_t)std::max(max_pairs, 4096u) + 2) * 4);
@@ -1018,7 +1021,6 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
   L.bounds = take((size_t)2 * MER_MAX_CTAS1 * 4);
   L.seeds = take((size_t)max_pairs * 2 * image_seed_stride(std::max(D, F)) * 4);
   L.x_un = take((size_t)max_pairs * 4);
-  L.h_un = take((size_t)max_pairs * 4);
   // room for 8 splits of the largest batch, but never less than 64 splits of an 8-pair dispatch, capped at 1 GiB
   const size_t per_pair = (size_t)(2 * F > D ? 2 * F : D) * 4;
   size_t want = (size_t)8 * max_pairs * per_pair;
@@ -1027,6 +1029,7 @@ ScratchLayout scratch_layout(uint32_t max_pairs, uint32_t D, uint32_t F) {
   if (want > ((size_t)1 << 30)) want = (size_t)1 << 30;
   if (want < (size_t)max_pairs * per_pair) want = (size_t)max_pairs * per_pair;
   L.parts_bytes = want;
+  L.h_un = take(std::max<size_t>(max_pairs, std::min((size_t)MAX_KSPLIT * max_pairs, want / ((size_t)D * 4))) * 4);  // of every pair and K split that the scratch can hold
   L.parts = take(want);
   L.total = off;
   return L;
@@ -1098,7 +1101,6 @@ void stream_bind(MoeDispatch &d, void *scratch, int sm_count, bool for_gemm) {
   d.pass_count = reinterpret_cast<uint32_t *>(base + L.pcount);
   d.pass_desc = reinterpret_cast<PassDesc *>(base + L.pdesc);
   d.taken = reinterpret_cast<uint64_t *>(base + L.taken);
-  d.amax = reinterpret_cast<uint32_t *>(base + L.amax);
   d.pos = for_gemm ? reinterpret_cast<uint32_t *>(base + L.pos) : nullptr;
   d.x_rows = d.y;  // [n_tokens x D] fp32 in size, and free until the down phase
   d.act_seeds = reinterpret_cast<float *>(base + L.seeds);
@@ -1149,7 +1151,9 @@ cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaS
     cudaGetLastError();
     whole = false, n = 0;
     if (!launch(1, false)) return e;
-    k_hidden<<<(P * ((d.F + 127) / 128) + 7) / 8, 256, 0, s>>>(d, p.parts, pl.ph[0].n_ksplit);
+    const uint32_t smem = 128 + pl.ph[1].kb_split * 128;
+    if ((e = cudaFuncSetAttribute(k_hidden, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    k_hidden<<<std::min(P * pl.ph[1].n_ksplit, 8u * (uint32_t)sm_count), CONSUMERS, smem, s>>>(d, p.parts, pl.ph[0].n_ksplit, pl.ph[1]);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     n++;
     if (!launch(2, false)) return e;
