@@ -106,5 +106,11 @@ __device__ __forceinline__ void build_x_image(const MoeDispatch &d, uint32_t tok
     }
   }
 }
+// The same by a CTA of 256 threads for a token that may have none of its experts here (expert parallelism).
+__device__ __forceinline__ void build_wanted_image(const MoeDispatch &d, uint32_t token, float *s_max) {
+  bool wanted = false;
+  for (uint32_t i = threadIdx.x; i < d.slots; i += 256) wanted |= d.pair_expert[(size_t)token * d.slots + i] != MER_NONE;
+  if (__syncthreads_or(wanted)) build_x_image(d, token, threadIdx.x, 256, s_max);
+}
 
 }  // namespace

@@ -647,18 +647,18 @@ __device__ __forceinline__ void split_values(float4 v, float sc, uint2 &hi, uint
 
 // Rows of activations -> rows of their f16 hi parts and lo parts, [hi K | lo K], after an exact power-of-two scaling of the
 // row, and its inverse.  Row i of the output belongs to the i-th pair in group order, so that a pass is a run of rows and
-// one copy fetches a chunk of all of them.  The source is row i of h, or with `pos` the tokens' rows: a row is then read and converted once and
-// written to the places of all of its `slots` pairs (rows picked by the GEMM's own copies instead, four per gather, took 80 cycles per four
+// one copy fetches a chunk of all of them.  The source is row i of h, the row of pair i's token with `perm`, or with `pos` the tokens' rows: a row is then read and
+// converted once and written to the places of all of its `slots` pairs (rows picked by the GEMM's own copies instead, four per gather, took 80 cycles per four
 // rows and doubled the GEMM's time).  TPR threads per row.  What bounds it is writing the rows.  With a row of x read and converted by each of
 // its pairs: 4096 tokens of 7168 for nine experts each 299 us.
 template <int TPR, bool TOKENS>
 __global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ act, uint32_t n_rows, uint32_t K, const uint32_t *__restrict__ pos,
-                                                    uint32_t slots, const uint32_t *__restrict__ n_grouped, uint16_t *__restrict__ out,
+                                                    const uint32_t *__restrict__ perm, uint32_t slots, const uint32_t *__restrict__ n_grouped, uint16_t *__restrict__ out,
                                                     float *__restrict__ unscale) {
   const uint32_t i = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, t = threadIdx.x % TPR;
   const bool have = TOKENS ? i < n_rows : i < *n_grouped;  // fewer than the pairs of the dispatch under expert parallelism
   if (TPR <= 32 && !have) return;
-  const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)(have ? i : 0) * K);
+  const float4 *src = reinterpret_cast<const float4 *>(act + (size_t)(!have ? 0 : !TOKENS && perm ? __ldg(perm + i) / slots : i) * K);
   float mx = 0.0f;
   bool nan = false;
   if (have) {
@@ -726,12 +726,12 @@ __global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ ac
   }
 }
 
-void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *pos, uint32_t slots, const uint32_t *n_grouped,
+void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *pos, const uint32_t *perm, uint32_t slots, const uint32_t *n_grouped,
                        uint16_t *out, float *unscale, cudaStream_t s) {
   // a warp per row keeps short rows of large batches cheap; long rows, and few of them, want more loads in flight
   const bool warps = K <= 2048 && n_rows >= 2048;
   auto kern = pos ? (warps ? k_split_rows<32, true> : k_split_rows<256, true>) : (warps ? k_split_rows<32, false> : k_split_rows<256, false>);
-  kern<<<warps ? (n_rows + 7) / 8 : n_rows, 256, 0, s>>>(act, n_rows, K, pos, slots, n_grouped, out, unscale);
+  kern<<<warps ? (n_rows + 7) / 8 : n_rows, 256, 0, s>>>(act, n_rows, K, pos, perm, slots, n_grouped, out, unscale);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -819,7 +819,11 @@ cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes,
 
   for (int phase = 0; phase < 2; phase++) {
     const uint32_t K = phase == 0 ? d.D : d.F;
-    launch_split_rows(phase == 0 ? d.x : d.h, phase == 0 ? d.n_tokens : P, K, phase == 0 ? d.pos : nullptr, d.slots, d.offsets + d.n_groups, rows, unscale, s);
+    // Under expert parallelism few of a token's pairs are here, of many tokens none: each pair's row by itself (512 tokens from each of 16 ranks, 16 of 256 experts of
+    // 4096 x 1536 here: 274 us a layer by token).
+    const bool by_token = phase == 0 && d.expected_pairs == 0;
+    launch_split_rows(phase == 0 ? d.x : d.h, by_token ? d.n_tokens : P, K, by_token ? d.pos : nullptr, phase == 0 ? d.perm : nullptr, d.slots, d.offsets + d.n_groups, rows,
+                      unscale, s);
     ActMaps maps;
     if (!activation_maps(&maps, rows, P, K)) return cudaErrorNotSupported;
     GemmParams p{};

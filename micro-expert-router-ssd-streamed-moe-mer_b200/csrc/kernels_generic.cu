@@ -842,9 +842,13 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router_select(const __grid_c
   finish_tokens<ROUTER_WARPS, 0>(r, d, blockIdx.x * ROUTER_WARPS, select_ctas, nullptr, 0, sets, true, smem_raw, status, max_tokens, group_here);
 }
 
-// Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.
+// Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.  The first CTA; the others make the activation images.
 __global__ void __launch_bounds__(ROUTER_THREADS) k_groups_layer(RouterDev r, MoeDispatch d) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
+  if (blockIdx.x > 0) {
+    __shared__ float s_max[ROUTER_WARPS];
+    return build_wanted_image(d, blockIdx.x - 1, s_max);
+  }
   build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
 }
 
@@ -1281,15 +1285,13 @@ bool groups_layer_on_grid(const MoeDispatch &d) { return d.n_tokens * d.slots >=
 
 cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaStream_t s, int *launches, bool counted) {
   const uint32_t G = d.n_groups, P = d.n_tokens * d.slots;
-  const cudaError_t ei = launch_x_images(d, s, launches);
-  if (ei != cudaSuccess) return ei;
   if (groups_layer_on_grid(d)) {  // a large dispatch: count / scan / scatter over the grid
     const unsigned blocks = (P + 1023) / 1024;
     if (!counted) k_group_count<<<blocks, 256, 0, s>>>(r, d);
     k_group_scan<<<1, 256, 0, s>>>(r, d, nullptr);
     k_group_scatter<<<blocks, 256, 0, s>>>(r, d);
     if (launches) (*launches) += counted ? 2 : 3;
-    return cudaGetLastError();
+    return launch_x_images(d, s, launches);
   }
   size_t smem = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   smem = (smem + 15) & ~(size_t)15;
@@ -1297,7 +1299,7 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
     cudaError_t e = cudaFuncSetAttribute(k_groups_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k_groups_layer<<<1, ROUTER_THREADS, smem, s>>>(r, d);
+  k_groups_layer<<<d.x_rows ? 1 + d.n_tokens : 1, ROUTER_THREADS, smem, s>>>(r, d);
   if (launches) (*launches)++;
   return cudaGetLastError();
 }

@@ -170,14 +170,15 @@ __device__ __forceinline__ float hidden_scale(uint32_t bits) {
 constexpr int HIDDEN_RUNS = 2;
 __device__ __forceinline__ void hidden_units(const MoeDispatch &d, const float *parts, uint32_t n_ksplit, const PhaseParams &down, uint32_t cta, uint32_t n_ctas, uint32_t warp,
                                              uint32_t lane, uint32_t *s_red, float4 *stash) {
-  const uint32_t chunks = (down.kb_split + 3) / 4, units = d.n_tokens * d.slots * down.n_ksplit;
+  const bool some = d.expected_pairs != 0;  // under expert parallelism a fraction of all pairs is here
+  const uint32_t chunks = (down.kb_split + 3) / 4, units = (some ? __ldcg(d.offsets + d.n_groups) : d.n_tokens * d.slots) * down.n_ksplit;
   uint32_t W = 1, log_w = 0;
   while (W < CONSUMER_WARPS && W < chunks && (W * HIDDEN_RUNS < chunks || units * W < n_ctas * (CONSUMER_WARPS / 2))) W *= 2, log_w++;
   const uint32_t teams = CONSUMER_WARPS >> log_w, team = warp >> log_w, member = warp & (W - 1), span = W * HIDDEN_RUNS * 32;
   uint32_t *red = s_red + team * W;
 #pragma unroll 1
   for (uint32_t u = cta * teams + team, odd = 0; u < units; u += n_ctas * teams, odd ^= CONSUMER_WARPS) {
-    const uint32_t pair = u / down.n_ksplit, ks = u % down.n_ksplit, kb0 = ks * down.kb_split, n4 = min(down.kb_split, down.kb_total - kb0) * 8;
+    const uint32_t i = u / down.n_ksplit, ks = u % down.n_ksplit, pair = some ? __ldcg(d.perm + i) : i, kb0 = ks * down.kb_split, n4 = min(down.kb_split, down.kb_total - kb0) * 8;
     const uint32_t turns = (n4 + span - 1) / span;
     float4 h[HIDDEN_RUNS];
     uint32_t m = 0;
@@ -197,7 +198,7 @@ __device__ __forceinline__ void hidden_units(const MoeDispatch &d, const float *
       m = __reduce_max_sync(0xffffffffu, lane < W ? red[odd + lane] : 0u);
     }
     const float sc = hidden_scale(m);
-    if (member == 0 && lane == 0) d.h_un[u] = POW2_24 / sc;
+    if (member == 0 && lane == 0) d.h_un[pair * down.n_ksplit + ks] = POW2_24 / sc;
     const ImageRow row(d.h, d.act_seeds, pair, d.F);
 #pragma unroll 1
     for (uint32_t turn = turns; turn-- > 0;) {  // the last one's values are still there
@@ -899,7 +900,7 @@ __global__ void __launch_bounds__(CONSUMERS) k_hidden(const __grid_constant__ Mo
 
 __global__ void __launch_bounds__(256) k_x_images(const __grid_constant__ MoeDispatch d) {
   __shared__ float s_max[8];
-  build_x_image(d, blockIdx.x, threadIdx.x, 256, s_max);
+  build_wanted_image(d, blockIdx.x, s_max);
 }
 
 __global__ void k_reduce_ksplit(const float *__restrict__ part, float *__restrict__ y, size_t n, uint32_t n_ksplit) {

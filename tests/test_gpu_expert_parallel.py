@@ -109,6 +109,43 @@ def test_collective_mode_ranks_in_turn_match_the_oracle(world, case, placement):
     assert rel_rms_err(got, ref) <= FFN_TOL
 
 
+# Tokens with none, one or all of their experts on the rank, through both kernel families and each form of grouping (32 pairs, a few
+# hundred, from 8192 on): rows without an expert here get no activations made, and zeros.
+@pytest.mark.parametrize("path", [2, 3])
+@pytest.mark.parametrize("B", [1, 20, 512])
+def test_tokens_without_a_local_expert(B, path):
+    import ctypes as C
+    dtype, E, D, F, k, world, rank = oracle.Q8_0, 16, 256, 128, 2, 8, 5
+    T = B * world
+    blobs = [synth.make_expert_blob(dtype, D, F, 66, 0, e) for e in range(E)]
+    b, ep = make_rank(dtype, E, D, F, k, world, rank, blobs, synth.make_router(E, D, 66), max(B, 2), 0)
+    rng = np.random.default_rng(66)
+    ids = np.stack([rng.permutation(E)[:k] for _ in range(T)])
+    mine = list(local_expert_range(rank, world, E))
+    ids[T // 2], ids[0] = mine[::-1], [0, 1]
+    w = rng.uniform(0.2, 0.8, (T, k)).astype(np.float32)
+    x = rng.standard_normal((T, D)).astype(np.float32)
+    try:
+        b.set_kernel_path(path)
+        dev = torch.device("cuda:0")
+        xd, wd, idd = torch.from_numpy(x).to(dev), torch.from_numpy(w).to(dev), torch.from_numpy(ids.astype(np.int32)).to(dev)
+        out = torch.full((T, D), float("nan"), device=dev)
+        for _ in range(2):
+            b._check(b.lib.mer_ep_local_experts_forward_device(b.h, 0, C.c_void_p(xd.data_ptr()), C.c_void_p(idd.data_ptr()), C.c_void_p(wd.data_ptr()),
+                                                               T, B, C.c_void_p(out.data_ptr()), C.c_void_p(0)))
+            ep.check(0)
+        got = out.cpu().numpy()
+    finally:
+        b.close()
+    here = np.isin(ids, mine)
+    assert (got[~here.any(1)] == 0).all()
+    some = np.flatnonzero(here.any(1))
+    assert T // 2 in some and here[T // 2].all()
+    for t in set(some[:6]) | set(some[-6:]) | {T // 2}:
+        ref = sum(np.float64(w[t, j]) * oracle.expert_forward(dtype, blobs[ids[t, j]], x[t], D, F) for j in range(k) if here[t, j])
+        assert rel_rms_err(got[t], ref) <= FFN_TOL, t
+
+
 def test_peer_mode_world_of_one_equals_the_single_gpu_entry_point():
     dtype, E, D, F, k, B, layer = oracle.Q8_0, 16, 256, 512, 4, 7, 0
     blobs = [synth.make_expert_blob(dtype, D, F, 62, 0, e) for e in range(E)]
