@@ -337,7 +337,10 @@ int mer_dataset_metadata_parse(const char *json, size_t len, mer_dataset_info *o
 int mer_expert_admit_file(mer_backend *b, uint32_t expert_id, uint64_t generation, const char *path, size_t block_align,
                           uint32_t flags);
 
-/* ---- router: LinearGate::new / with_routing (gating.rs:149-238). ---- */
+/* ---- router: LinearGate::new / with_routing (gating.rs:149-238).
+ * With max_tokens >= 256 and d_model a multiple of 256 the weights lie in device memory twice (fp32, and f16 parts for batches of that size: another
+ * 4 bytes a weight); where the second copy finds no room, or its parts do not hold the weights, such batches run in fp32.  Waits for the
+ * backend's own stream.  ---- */
 int mer_router_install(mer_backend *b, uint32_t layer, const float *host_weights /*[E x D]*/,
                        const mer_router_cfg *cfg);
 /* ---- the steps either side of the MoE block, per layer (optional; install after the layer's router):

@@ -14,7 +14,7 @@
 // Router parameters resident on the device (one per installed layer).
 struct RouterDev {
   const float *w;                // [E x D]
-  const uint8_t *w_split;        // the same in f16 parts and fragment order (kernels_logits.cu), or null: rows or values that it does not take
+  const uint8_t *w_split;        // the same in f16 parts and fragment order (kernels_logits.cu), or null: rows or values that these do not hold
   const float *w_unscale;        // [E rounded up to 8] of its rows
   const float *correction_bias;  // [E] or null
   const float *logit_bias;       // [E] or null
@@ -175,11 +175,13 @@ inline cudaError_t launch_overlapped(void (*kern)(P...), dim3 grid, unsigned blo
 // packed; `done`, if not null, receives ++*count last).
 cudaError_t launch_host_in(const void *src, void *dst, size_t words, uint32_t *status, cudaStream_t s, int *launches);
 cudaError_t launch_host_out(const void *src, size_t stride, size_t rows, size_t words, void *dst, uint32_t *count, uint32_t *done, cudaStream_t s, int *launches);
-// kernels_logits.cu: router logits of a few hundred tokens and more on the tensor cores.  `sets`: partial sums of K that the logits scratch then holds.
+// kernels_logits.cu: router logits of a few hundred tokens and more.  `unfit`: device word, nonzero if the parts do not hold the weights
+// (non-finite ones, or too far apart).  `sets`: partial sums of K that the logits scratch then holds.
 bool router_split_supported(uint32_t D);
 size_t router_split_bytes(uint32_t E, uint32_t D);
-cudaError_t launch_split_router(const float *w, uint32_t E, uint32_t D, uint8_t *out, float *unscale, cudaStream_t s);
-cudaError_t launch_router_logits(const RouterDev &r, const MoeDispatch &d, uint32_t *status, uint32_t *sets, cudaStream_t s);
+cudaError_t launch_split_router(const float *w, uint32_t E, uint32_t D, uint8_t *out, float *unscale, uint32_t *unfit, cudaStream_t s);
+// `in_parts`: tokens whose logits come out non-finite are to be looked at again.
+cudaError_t launch_router_logits(const RouterDev &r, const MoeDispatch &d, uint32_t *status, uint32_t *sets, bool *in_parts, cudaStream_t s);
 // With `group` it leaves d.status written: no need to clear it first.  group = false: route only (the caller groups later, e.g. after gathering other ranks' tokens)
 cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max_tokens, cudaStream_t s, int *launches,
                           bool group = true);

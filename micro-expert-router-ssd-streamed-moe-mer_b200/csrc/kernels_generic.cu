@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cfloat>
 
 #include "../../include/mer_b200.h"
 #include "act_image.cuh"
@@ -654,15 +655,15 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     float *s_sel = s_score + E;                                                    // [E] selection scores
     uint8_t *s_ok = smem_raw + (size_t)TT * 2 * E * 4 + (size_t)warp * E;          // [E] allowed & not yet taken
     const uint32_t token = t0 + warp;
-    bool nan = false;
+    bool bad = false;
     for (uint32_t i = lane; i < E; i += 32) {
       float v = direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
       for (uint32_t z = 1; z < sets; z++) v += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i);
       s_score[i] = v;
-      nan |= v != v;
+      bad |= !(fabsf(v) <= FLT_MAX);
     }
     // Non-finite values do not survive the split into parts (kernels_logits.cu): such a token's logits are made again in fp32.
-    if (recheck && __any_sync(0xffffffffu, nan))
+    if (recheck && __any_sync(0xffffffffu, bad))
 #pragma unroll 1
       for (uint32_t e = 0; e < E; e++) {
         float v = 0.0f;
@@ -831,15 +832,16 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
 
 // The same behind the logits kernel of a large batch: every warp has a token.  (In the kernel above, whose registers leave room for two CTAs on an SM,
 // 4096 tokens of 256 experts took 47 us.)
+template <int TT>
 __global__ void __launch_bounds__(ROUTER_THREADS) k_router_select(const __grid_constant__ RouterDev r, const __grid_constant__ MoeDispatch d, uint32_t max_tokens, uint32_t sets,
-                                                                  int group_here, uint32_t select_ctas) {
+                                                                  int recheck, int group_here, uint32_t select_ctas) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   if (blockIdx.x >= select_ctas) {  // activation images of the tokens
     build_x_image(d, blockIdx.x - select_ctas, threadIdx.x, ROUTER_THREADS, reinterpret_cast<float *>(smem_raw));
     return;
   }
   uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
-  finish_tokens<ROUTER_WARPS, 0>(r, d, blockIdx.x * ROUTER_WARPS, select_ctas, nullptr, 0, sets, true, smem_raw, status, max_tokens, group_here);
+  finish_tokens<TT, 0>(r, d, blockIdx.x * TT, select_ctas, nullptr, 0, sets, recheck != 0, smem_raw, status, max_tokens, group_here);
 }
 
 // Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.  The first CTA; the others make the activation images.
@@ -1246,13 +1248,16 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   size_t smem;
   cudaError_t e;
   // From a few hundred tokens the logits are a GEMM of their own, unless the experts are so few that most of a tile would be
-  // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel) or so many that a CTA's tokens do not fit shared memory.
-  if (d.n_tokens >= 256 && r.w_split && E <= 2048 && (E > 16 || d.D % 1024 != 0)) {
+  // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel).
+  if (d.n_tokens >= 256 && d.D % 256 == 0 && (E > 16 || d.D % 1024 != 0)) {
     uint32_t sets = 1;
-    if ((e = launch_router_logits(r, d, group_here ? d.counters + max_tokens + 1 : d.status, &sets, s)) != cudaSuccess) return e;
-    if ((e = room(k_router_select, ROUTER_WARPS, smem)) != cudaSuccess) return e;
-    const uint32_t ctas = (d.n_tokens + ROUTER_WARPS - 1) / ROUTER_WARPS;
-    k_router_select<<<ctas + (d.x_rows ? d.n_tokens : 0), ROUTER_THREADS, smem, s>>>(r, d, max_tokens, sets, group_here, ctas);
+    bool in_parts = false;
+    if ((e = launch_router_logits(r, d, group_here ? d.counters + max_tokens + 1 : d.status, &sets, &in_parts, s)) != cudaSuccess) return e;
+    const uint32_t tokens = E <= 2048 ? ROUTER_WARPS : ROUTER_WARPS / 2;  // what fits shared memory
+    auto kern = E <= 2048 ? k_router_select<ROUTER_WARPS> : k_router_select<ROUTER_WARPS / 2>;
+    if ((e = room(kern, tokens, smem)) != cudaSuccess) return e;
+    const uint32_t ctas = (d.n_tokens + tokens - 1) / tokens;
+    kern<<<ctas + (d.x_rows ? d.n_tokens : 0), ROUTER_THREADS, smem, s>>>(r, d, max_tokens, sets, in_parts ? 1 : 0, group_here, ctas);
     e = cudaGetLastError();
     if (launches) (*launches)++;
   } else {

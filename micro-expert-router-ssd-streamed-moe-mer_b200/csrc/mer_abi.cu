@@ -1266,14 +1266,24 @@ MER_EXPORT int mer_router_install(mer_backend *b, uint32_t layer, const float *h
     CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(bias)", cudaMalloc((void **)&r.d_lbias, ebytes));
     CU(MER_ERR_UPLOAD, "cudaMemcpy(bias)", cudaMemcpy(r.d_lbias, cfg->logit_bias, ebytes, cudaMemcpyHostToDevice));
   }
-  // for batches of 256 tokens and more: the weights in parts, beside the fp32 rows (finite weights only)
+  // For batches of 256 tokens and more: the weights in parts, beside the fp32 rows.  Without them, for lack of memory or as the parts do not hold them, such
+  // batches run the kernel of smaller ones.
   const uint32_t E = cfg->num_experts, D = (uint32_t)b->cfg.d_model;
-  if (b->cfg.max_tokens >= 256 && router_split_supported(D) &&
-      std::all_of(host_weights, host_weights + (size_t)E * D, [](float v) { return std::isfinite(v); })) {
-    CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(router parts)", cudaMalloc((void **)&r.d_w_split, router_split_bytes(E, D)));
-    CU(MER_ERR_PHYSICAL_CAPACITY, "cudaMalloc(router scales)", cudaMalloc((void **)&r.d_w_unscale, ((size_t)E + 7) / 8 * 8 * 4));
-    CU(MER_ERR_UPLOAD, "router parts", launch_split_router(r.d_w, E, D, r.d_w_split, r.d_w_unscale, b->compute));
-    CU(MER_ERR_UPLOAD, "cudaStreamSynchronize", cudaStreamSynchronize(b->compute));
+  if (b->cfg.max_tokens >= 256 && router_split_supported(D)) {
+    const size_t rows = ((size_t)E + 7) / 8 * 8;
+    uint32_t unfit = 1;
+    if (cudaMalloc((void **)&r.d_w_split, router_split_bytes(E, D)) == cudaSuccess && cudaMalloc((void **)&r.d_w_unscale, (rows + 1) * 4) == cudaSuccess) {
+      uint32_t *d_unfit = reinterpret_cast<uint32_t *>(r.d_w_unscale + rows);
+      CU(MER_ERR_UPLOAD, "router parts", launch_split_router(r.d_w, E, D, r.d_w_split, r.d_w_unscale, d_unfit, b->compute));
+      CU(MER_ERR_UPLOAD, "cudaMemcpyAsync(router parts)", cudaMemcpyAsync(&unfit, d_unfit, 4, cudaMemcpyDeviceToHost, b->compute));
+      CU(MER_ERR_UPLOAD, "cudaStreamSynchronize", cudaStreamSynchronize(b->compute));
+    } else {
+      cudaGetLastError();
+    }
+    if (unfit) {
+      if (r.d_w_split) cudaFree(r.d_w_split), r.d_w_split = nullptr;
+      if (r.d_w_unscale) cudaFree(r.d_w_unscale), r.d_w_unscale = nullptr;
+    }
   }
   r.dev.w = r.d_w;
   r.dev.w_split = r.d_w_split, r.dev.w_unscale = r.d_w_unscale;

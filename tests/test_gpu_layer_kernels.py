@@ -134,9 +134,10 @@ def test_passes_of_two_accumulator_buffers(dtype):
     assert np.max(np.abs(out - other) / rms) <= FFN_TOL  # the two kernel families, every row
 
 
-# partial expert tiles (8 a fragment tile, 64 and 128 a CTA), partial token tiles of 128, slices of K, one chunk of a slice
+# partial expert tiles (8 a fragment tile, 64 and 128 a CTA), partial token tiles of 128, slices of K, one chunk of a slice; both sides of the rule that takes
+# fp32 tiles, those of 32 x 64 and of 64 x 128; tokens that are selected four a CTA
 @pytest.mark.parametrize("E,k,T,D", [(17, 2, 256, 256), (60, 6, 257, 512), (64, 8, 383, 2304), (65, 4, 300, 1024), (128, 8, 385, 2048), (129, 8, 256, 7168),
-                                     (256, 8, 511, 1280)])
+                                     (256, 8, 511, 1280), (128, 8, 320, 2048), (128, 8, 321, 2048), (128, 4, 1600, 256), (2050, 8, 256, 256)])
 def test_router_logits_of_large_batches(E, k, T, D):
     F, dtype = 32, oracle.Q8_0
     rng = np.random.default_rng(E)
@@ -159,6 +160,36 @@ def test_router_logits_of_large_batches(E, k, T, D):
     ref = p / p.sum(1, keepdims=True)
     # an error d of a logit is one of d, relatively, of its weight
     assert (np.abs(w - ref) <= ref * (4 * noise[:, None] + 1e-6)).all()
+
+
+# Values far above the rest of their router row (at columns where the tokens are zero) or of their token (where the router is): the logits come from the
+# small ones alone, and are as good as without the large ones.
+@pytest.mark.parametrize("where,power", [("router", 10), ("router", 15), ("router", 20), ("router", 26), ("router", 40), ("token", 10), ("token", 20), ("token", 26)])
+def test_router_logits_beside_values_far_above_the_others(where, power):
+    E, k, T, D, F, dtype = 64, 8, 700, 2048, 32, oracle.Q8_0  # (the parts: what a thread of the fp32 tiles would add is long enough)
+    rng = np.random.default_rng(power)
+    W = (rng.standard_normal((E, D)) * 0.05).astype(np.float32)
+    x = rng.standard_normal((T, D)).astype(np.float32)
+    far = rng.permutation(D)[:16]  # one of 64 neighbours, or a few
+    W[:, far], x[:, far] = 0.0, 0.0
+    if where == "router":
+        W[:, far] = 0.05 * 2.0 ** power * rng.choice([-1.0, 1.0], (E, 16))
+    else:
+        x[:, far] = 2.0 ** power
+    blob = np.zeros(mer_b200.expert_bytes(dtype, D, F), np.uint8)
+    with backend(dtype, D, F, E, max_tokens=T, max_top_k=k) as b:
+        for e in range(E):
+            b.admit(e, 1, blob, wait=e == E - 1)
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        ids, w = b.route(0, x)
+    s = x.astype(np.float64) @ W.astype(np.float64).T
+    # fp32 sums of D terms are good to about 1e-6 of the terms' root sum of squares, softmax scores to a few units of 2^-24
+    noise = 1e-6 * np.sqrt(D) * 0.05 + 5e-7
+    picked = np.take_along_axis(s, ids.astype(np.int64), 1)
+    assert (picked >= -np.sort(-s, axis=1)[:, k - 1:k] - noise).all() and all(len(set(r)) == k for r in ids.tolist())
+    p = np.exp(picked - picked.max(1, keepdims=True))
+    ref = p / p.sum(1, keepdims=True)
+    assert (np.abs(w - ref) <= ref * (4 * noise + 1e-6)).all()
 
 
 def test_router_logits_of_tokens_that_are_not_finite():
