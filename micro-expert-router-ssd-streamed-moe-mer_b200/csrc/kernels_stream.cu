@@ -52,7 +52,7 @@ constexpr int PRODUCER_WARPS = 2;  // each issues the bulk copies of half a stag
 constexpr int SCHED_WARP = CONSUMER_WARPS + PRODUCER_WARPS;  // claims the CTA's items and fetches their activations
 constexpr int THREADS = (SCHED_WARP + 1) * 32;
 constexpr uint32_t QUEUE = 3;
-constexpr uint32_t HEADER_BYTES = 1024;  // mbarriers and the token tables of two units at the start of shared memory
+constexpr uint32_t HEADER_BYTES = 1024;  // of `Header`
 constexpr uint32_t N_BARRIERS = 4;       // grid-wide barriers of a launch, one counter each
 
 constexpr int TAIL_NONE = 0, TAIL_COMBINE = 1, TAIL_REDUCE = 2;
@@ -296,6 +296,25 @@ struct __align__(16) Item {
   const uint8_t *base;  // the expert's payload, null = not resident
 };
 
+// The start of shared memory.
+struct Header {
+  uint64_t full[8], empty[8];             // [n_stages] the ring's stages
+  uint64_t frag_full[2], frag_empty[2];   // [n_frag] the activation buffers
+  uint64_t hidden;                        // the hidden rows are there
+  uint64_t built;                         // LOCAL: the item's hidden values are in shared memory
+  uint64_t q_full[QUEUE], q_empty[QUEUE]; // the item queue
+  uint32_t abort, ok;
+  uint32_t other_status;                  // ROUTE: where CTAs but the first leave the router's status bits
+  uint32_t info[2];                       // tokens of the unit's pass
+  uint32_t pair[2 * 8];                   // pair index of each of them
+  float un[2 * 8];                        // its 2^24 / scale
+  uint32_t red[2 * CONSUMER_WARPS];       // the warps' maxima in the making of hidden values
+  Item item[QUEUE];
+  const uint8_t *base[32];                // ROUTE: payload of every pass,
+  uint32_t slot[32];                      //   its slot
+};
+static_assert(sizeof(Header) <= HEADER_BYTES, "");
+
 // Claims items for a CTA.  The grouping kernel cut the phase's items, ordered (pass, K split, tile), into one contiguous range per CTA,
 // balanced by the tokens of the passes.  A CTA takes its own from the front and, when they are used up, those of the CTA that has most
 // left from the back: SMs reach HBM at different speeds, and the slowest of them finished 10 to 17 us behind the others
@@ -383,19 +402,14 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   const MoeDispatch &d = p.d;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  // shared memory carve-up
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + 8;   // [n_stages <= 8] each
-  uint64_t *frag_full = full + 16, *frag_empty = full + 18, *hidden = full + 20;  // [n_frag] each; the hidden rows are there
-  uint64_t *built = full + 21;                                  // the item's hidden values are in shared memory (`local`)
-  uint64_t *q_full = full + 56, *q_empty = q_full + QUEUE;      // [QUEUE] each
-  Item *s_item = reinterpret_cast<Item *>(smem + 512);          // [QUEUE]
-  const uint8_t **s_base = reinterpret_cast<const uint8_t **>(smem + 640);  // [32] payload of every pass, where the scheduler routes
-  uint32_t *s_slot = reinterpret_cast<uint32_t *>(smem + 896);  // [32] its slot
-  uint32_t *s_abort = reinterpret_cast<uint32_t *>(smem + 176), *s_ok = s_abort + 1;
-  uint32_t *s_info = reinterpret_cast<uint32_t *>(smem + 184);  // [2] tokens of the unit's pass
-  uint32_t *s_pair = reinterpret_cast<uint32_t *>(smem + 192);  // [2][8] pair index of each of them
-  float *s_un = reinterpret_cast<float *>(smem + 256);          // [2][8] its 2^24 / scale
-  uint32_t *s_red = reinterpret_cast<uint32_t *>(smem + 320);   // [2][CONSUMER_WARPS] the warps' maxima in the making of hidden values
+  Header &hd = *reinterpret_cast<Header *>(smem);
+  uint64_t *const full = hd.full, *const empty = hd.empty, *const frag_full = hd.frag_full, *const frag_empty = hd.frag_empty;
+  uint64_t *const hidden = &hd.hidden, *const built = &hd.built, *const q_full = hd.q_full, *const q_empty = hd.q_empty;
+  uint32_t *const s_abort = &hd.abort, *const s_ok = &hd.ok, *const s_info = hd.info, *const s_pair = hd.pair, *const s_red = hd.red;
+  float *const s_un = hd.un;
+  Item *const s_item = hd.item;
+  const uint8_t **const s_base = hd.base;
+  uint32_t *const s_slot = hd.slot;
   uint8_t *s_frag = smem + HEADER_BYTES;                        // [n_frag] x {fragments [frag_cols][frag_stride], zero-point terms [frag_cols][seed_words]}
   uint8_t *s_stage = s_frag + (size_t)p.n_frag * p.frag_bytes;  // [n_stages][16 tiles][chunk_stride]
   const uint32_t stage_bytes = ITEM_TILES * p.chunk_stride;
@@ -483,7 +497,7 @@ __device__ __forceinline__ void ffn_stream_body(const StreamParams &p) {
   if (warp == SCHED_WARP) {
     // ------------------------------ scheduler: claims items, and for each new unit, i.e. (pass, K split), fetches the activations: lane l
     // copies part l % 4 (hi fragments, lo fragments, their zero-point terms) of the pass's token l / 4.
-    const uint32_t n_passes = ROUTE ? route_token_here(d, reinterpret_cast<float *>(s_stage), s_base, s_slot, s_abort + 108, lane) : *d.n_passes;
+    const uint32_t n_passes = ROUTE ? route_token_here(d, reinterpret_cast<float *>(s_stage), s_base, s_slot, &hd.other_status, lane) : *d.n_passes;
     uint32_t unit = 0, slot = 0, round = 0;
     bool ok = true;
     const uint32_t tok = lane >> 2, part = lane & 3;
