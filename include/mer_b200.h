@@ -551,7 +551,8 @@ int mer_snapshot(mer_backend *b, mer_counters *out);
 /* Selects the kernel family: 0 = automatic (streaming kernels for a few tokens per expert, the
  * tcgen05 GEMM kernels from a mean of 12 tokens per expert), 1 = generic fp32 kernels (any shape),
  * 2 = streaming tensor-core kernels (d_model and d_ff multiples of 32), 3 = tcgen05 GEMM kernels (multiples of
- * 128, a backend of at least 12 tokens).
+ * 128, a backend of at least 12 tokens), 4 = as 2, as it runs where the device refuses cooperative launches (a kernel for
+ * every step).
  * For qualification runs. */
 int mer_set_kernel_path(mer_backend *b, int path);
 

@@ -91,6 +91,7 @@ struct MoeDispatch {
   uint32_t y_nparts;        //   or null / 1 when `y` already holds them
   int fuse_combine;         // in: a weighted combine into `out` follows the expert FFN; the FFN launch may do it itself
   int combined;             // out: it did (launch_combine then does nothing)
+  int steps_apart;          // in: the streaming FFN runs as if cooperative launches were refused
   int fuse_reduce;          // in: the caller wants final per-pair outputs in `y` for the grouped pairs (no K-split partials left)
   uint32_t gemm_bn;         // > 0: the tcgen05 GEMM path runs this dispatch with passes of gemm_bn tokens
   int packed;               // 1: slots hold the tile-major fragment layout (layout.cuh), 0: the flat block stream

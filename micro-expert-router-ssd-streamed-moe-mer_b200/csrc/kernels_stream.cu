@@ -1161,7 +1161,7 @@ cudaError_t launch_ffn_stream(MoeDispatch &d, void *scratch, int sm_count, cudaS
     if (!launch(1, true)) return e;
     cudaEventRecord(ev_mid, s);
     if (!launch(2, true)) return e;
-  } else if (!launch(3, true)) {
+  } else if (d.steps_apart || !launch(3, true)) {
     // a cooperative launch is refused: the steps between and behind the phases are kernels of their own
     cudaGetLastError();
     whole = false, n = 0;

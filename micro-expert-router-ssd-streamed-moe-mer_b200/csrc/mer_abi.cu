@@ -268,7 +268,7 @@ constexpr uint32_t GEMM_MIN_MEAN_TOKENS = 12;
 void bind_ffn(mer_backend *b, MoeDispatch &d) {
   d.gemm_bn = 0;
   if (!use_stream_path(b, d)) return;
-  if (b->d_gemm_scratch && b->kernel_path != 2) {
+  if (b->d_gemm_scratch && b->kernel_path != 2 && b->kernel_path != 4) {
     const uint32_t bn = gemm_pick_bn(d, b->kernel_path == 3 ? 1u : GEMM_MIN_MEAN_TOKENS);
     if (bn) {
       gemm_bind(d, b->d_stream_scratch, b->sm_count, bn);
@@ -277,6 +277,7 @@ void bind_ffn(mer_backend *b, MoeDispatch &d) {
     }
   }
   stream_bind(d, b->d_stream_scratch, b->sm_count);
+  d.steps_apart = b->kernel_path == 4;
 }
 
 cudaError_t run_ffn(mer_backend *b, MoeDispatch &d, cudaStream_t s, int *launches, cudaEvent_t ev_mid = nullptr) {
@@ -2268,9 +2269,9 @@ MER_EXPORT int mer_snapshot(mer_backend *b, mer_counters *out) {
 }
 
 MER_EXPORT int mer_set_kernel_path(mer_backend *b, int path) {
-  if (!b || path < 0 || path > 3) return MER_ERR_INVALID_ARGUMENT;
+  if (!b || path < 0 || path > 4) return MER_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(b->mu);
-  if (path == 2 && !b->d_stream_scratch)
+  if ((path == 2 || path == 4) && !b->d_stream_scratch)
     return fail(b, MER_ERR_INELIGIBLE, 0, MER_NONE, "streaming kernels need d_model and d_ff to be multiples of 32");
   if (path == 3 && !b->d_gemm_scratch)
     return fail(b, MER_ERR_INELIGIBLE, 0, MER_NONE,

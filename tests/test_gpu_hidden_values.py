@@ -97,3 +97,31 @@ def test_hidden_values_that_are_not_finite(dtype, n_tokens):
     assert not np.isfinite(got[0]).any()
     for t in range(1, n_tokens):
         assert rel_rms_err(got[t], oracle.expert_forward(dtype, blob, x[t], D, F)) <= FFN_TOL
+
+
+# Where the device refuses cooperative launches every step is a kernel of its own: the same values, added in the same order.
+@pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
+@pytest.mark.parametrize("D,F,E,k,n_tokens,shared", [
+    (2048, 768, 24, 8, 1, False), (4096, 288, 9, 2, 1, True), (512, 14336, 4, 2, 3, False), (256, 2048, 40, 4, 9, True), (288, 96, 12, 3, 70, False)])
+def test_steps_in_kernels_of_their_own(dtype, D, F, E, k, n_tokens, shared):
+    blobs = [synth.make_expert_blob(dtype, D, F, 60, 0, e) for e in range(3)]
+    W = synth.make_router(E, D, 61)
+    x = synth.make_activations(n_tokens, D, 61)
+    with backend(dtype, D, F, E + 1, max_tokens=n_tokens, max_top_k=k + 1) as b:
+        for e in range(E + 1):
+            b.admit(e, 1, blobs[e % 3], wait=e == E)
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0, *([E] if shared else []))
+        results = []
+        for path in (2, 4):
+            b.set_kernel_path(path)
+            results += [b.moe_layer_forward(0, x) for _ in range(4)]  # plain launches, then replayed ones
+            one = b.moe_step_weighted_into(0, x[0], results[0][1][0], results[0][2][0])
+            results[-1] += (one,)
+    for out, ids, w, *_ in results:
+        assert np.array_equal(out, results[0][0]) and np.array_equal(ids, results[0][1]) and np.array_equal(w, results[0][2])
+    assert np.array_equal(results[3][3], results[7][3])
+    for t in {0, n_tokens // 2, n_tokens - 1}:
+        ref = sum(np.float64(wi) * oracle.expert_forward(dtype, blobs[i % 3], x[t], D, F) for i, wi in zip(results[0][1][t], results[0][2][t]))
+        if shared:
+            ref = ref + oracle.expert_forward(dtype, blobs[E % 3], x[t], D, F)
+        assert rel_rms_err(results[4][0][t], ref) <= FFN_TOL
