@@ -238,8 +238,8 @@ cudaError_t launch_flat_expert(int dtype, const uint8_t *expert, const float *x,
 // kernels_gemm.cu: tcgen05 / TMEM grouped GEMM for groups of a dozen tokens and more.
 bool gemm_ffn_supported(int dtype, uint32_t D, uint32_t F);
 size_t gemm_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F);
-// Tokens per pass (16..128) for this dispatch, or 0 when its groups are too small for the GEMM path.
-uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens);
+// Tokens per pass at most (128 or 256) for this dispatch, or 0 when its groups are too small for the GEMM path.
+uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens, int sm_count);
 void gemm_bind(MoeDispatch &d, void *stream_scratch, int sm_count, uint32_t bn);
 cudaError_t launch_ffn_gemm(MoeDispatch &d, void *gemm_scratch, size_t gemm_scratch_bytes, int sm_count,
                             cudaStream_t s, int *launches, cudaEvent_t ev_mid);

@@ -786,7 +786,7 @@ size_t gemm_ffn_scratch_bytes(uint32_t max_pairs, uint32_t D, uint32_t F) {
 }
 
 // Tokens per pass at most, or 0 when the dispatch is better served by the streaming kernels.
-uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
+uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens, int sm_count) {
   const uint64_t P = (uint64_t)d.n_tokens * d.slots;
   const uint32_t groups = d.active_groups_hint ? d.active_groups_hint : 1;
   const uint64_t mean = (d.expected_pairs ? d.expected_pairs : P) / groups;
@@ -794,8 +794,10 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens) {
   // Passes of up to 256 tokens instead of 128 save conversions of the weights (129 to 256 tokens of an expert: half of them) and leave the MMAs idle while
   // an item's epilogue drains both buffers, some 5000 cycles.  That pays where an item's K is long and where there are enough items to
   // share out evenly.  Us a pass, 128 / 256: 4096 tokens on 256 experts of 7168 x 2048 9516 / 8827; 2048 on 128 of 2048 x 768 (24 blocks of K
-  // in the down phase) 658 / 705; 256 on 8 of 4096 x 14336 (two items a pair of CTAs in the down phase) 690 / 720.
-  const bool long_k = d.D / 32 >= 128 && d.F / 32 >= 64, many = (uint64_t)groups * (std::min(2 * d.F, d.D) / 256) >= 8 * 74;
+  // in the down phase) 658 / 705; 256 on 8 of 4096 x 14336 (two items a pair of CTAs in the down phase) 690 / 720.  Beside the line of K, mean of 163 to 256 tokens: 64 experts
+  // of 4096 x 1536 1477 / 1518, of 2048 x 1536 808 / 880, 128 of 3072 x 2048 3198 / 3256, of 2048 x 2048 1611 / 1580.  Below the line of items (five to seven a pair) it
+  // depends on how the experts' tokens fill passes: 32 of 4096 x 2048, 200 tokens each, 787 / 769, with Zipf(1) routing 830 / 866; 32 of 4096 x 8192, 162 each, 2859 / 2376.
+  const bool long_k = d.D / 32 >= 128 && d.F / 32 >= 64, many = (uint64_t)groups * (std::min(2 * d.F, d.D) / 256) >= 8 * (uint64_t)(sm_count / PAIR);
   return long_k && many ? PASS_TOKENS : BUF_TOKENS;
 }
 

@@ -269,7 +269,7 @@ void bind_ffn(mer_backend *b, MoeDispatch &d) {
   d.gemm_bn = 0;
   if (!use_stream_path(b, d)) return;
   if (b->d_gemm_scratch && b->kernel_path != 2 && b->kernel_path != 4) {
-    const uint32_t bn = gemm_pick_bn(d, b->kernel_path == 3 ? 1u : GEMM_MIN_MEAN_TOKENS);
+    const uint32_t bn = gemm_pick_bn(d, b->kernel_path == 3 ? 1u : GEMM_MIN_MEAN_TOKENS, b->sm_count);
     if (bn) {
       gemm_bind(d, b->d_stream_scratch, b->sm_count, bn);
       d.gemm_bn = bn;
