@@ -54,6 +54,7 @@ SWEEP = [  # (workload, batches) measured after the headline at N = 1; cfg1 / cf
 ]
 DTYPE_NAME = {0: "q4_0", 1: "q8_0"}
 GEMM_MEAN_TOKENS = 12  # mean tokens per expert from which the library's automatic selection runs the tcgen05 GEMM kernels
+APART = "launches of the stage-timed layers, one for each phase, the hidden values in the first; the layers timed for the value run both phases in one launch"
 PARITY_TOKENS = 4
 PARITY_BAR = 1e-3      # max-abs error of a token's output relative to the RMS of the oracle's output
 PARALLELISM_NOTE = {
@@ -358,7 +359,7 @@ def measure_point(stack, name, zipf_s, B, layers, passes, warm, peaks, x_seed_ba
         ach = kb / (gu_ms * 1e-3) / 1e9 if gu_ms > 0 else None
         roof = {"bound": "hbm", "kernel": "expert_gate_up (gate/up dequant-matvec + SiLU*mul)", "achieved": ach, "peak": hbm_peak,
                 "unit": "GB/s", "frac": ach / hbm_peak if ach else None, "peak_source": f"of {kind}",
-                "frac_of_8tbs": ach / 8000.0 if ach else None, "algorithmic_bytes_per_launch": kb, "avg_launch_ms": gu_ms}
+                "frac_of_8tbs": ach / 8000.0 if ach else None, "algorithmic_bytes_per_launch": kb, "avg_launch_ms": gu_ms, "note": APART}
     layer_gbs = layer_bytes / (per_layer_ms * 1e-3) / 1e9
     entry = {"workload": name, "batch": B, "layers_rotated": len(layers), "passes": passes, "tokens_per_s": B / (per_layer_ms * 1e-3),
              "ms_per_layer": per_layer_ms, "roofline": roof,
@@ -891,7 +892,7 @@ def main():
             roofline = {"bound": "hbm", "kernel": "expert_gate_up (gate/up dequant-matvec + SiLU*mul)", "achieved": achieved, "peak": hbm_peak,
                         "unit": "GB/s", "frac": achieved / hbm_peak if achieved else None, "peak_source": f"of {peak_kind}",
                         "traffic": traffic, "algorithmic_bytes_per_launch": kernel_bytes, "avg_launch_ms": gu_ms,
-                        "frac_of_8tbs": achieved / 8000.0 if achieved else None}
+                        "frac_of_8tbs": achieved / 8000.0 if achieved else None, "note": APART}
     elif gemm:
         # expert-parallel step: no per-stage timers; rank 0's share of the layer's algorithmic FLOPs over its whole layer pass
         flops = 2.0 * tokens_global * slots * 3 * cfg.d_model * cfg.d_ff / world
