@@ -152,7 +152,7 @@ __device__ void build_passes_block(const MoeDispatch &d, const uint32_t *off, bo
   __shared__ uint32_t s_pcnt[257];
   __shared__ uint8_t s_cost[1024];  // cost of each of the first 1024 passes (the weighted work split below)
   const uint32_t tpp = d.tokens_per_pass;
-  const uint32_t tpp_shift = 31 - __clz(tpp);  // tokens per pass is a power of two (4 or 8; 16 .. 128 for the GEMM kernels)
+  const uint32_t tpp_shift = 31 - __clz(tpp);  // tokens per pass is a power of two (4 or 8; 128 or 256 for the GEMM kernels)
   clear_taken(d);
   const uint32_t per = (d.n_groups + 255) / 256;
   const uint32_t g0 = threadIdx.x * per, g1 = min(g0 + per, d.n_groups);

@@ -1,5 +1,5 @@
-"""One token routed inside the FFN kernel, passes of the GEMM kernels wider than an accumulator buffer, router logits on the tensor
-cores, hidden rows scaled by a bound: sizes and values at which each changes its way, against the CPU oracle."""
+"""One token routed inside the FFN kernel, passes of the GEMM kernels wider than an accumulator buffer, router logits of large
+batches, hidden rows of any size: sizes and values at which each changes its way, against the CPU oracle."""
 import numpy as np
 import pytest
 
@@ -84,8 +84,8 @@ def test_one_token_with_a_missing_expert_fails_closed_and_the_next_call_works():
                 assert rel_rms_err(out[0], ffn_reference(dtype, [blob] * E, x[t], F, ids[0], w[0])) <= FFN_TOL
 
 
-# Hidden values far apart: the scale comes from bounds of the gate and up sums, the values keep their own precision.  The products of the
-# two largest are 1e8 times the others'; FFN_TOL is relative to the row's RMS, which the large ones set, so the small rows are looked at alone.
+# Tokens of very small and very large values: gate, up and hidden values scale with them (SiLU is linear in its limits).  Values of one row that lie far apart, and rows
+# far below their bounds, are in test_gpu_hidden_values.py.
 @pytest.mark.parametrize("n_tokens", [1, 4, 9])
 @pytest.mark.parametrize("scale", [1e-18, 1.0, 1e15])
 def test_hidden_rows_of_any_magnitude(n_tokens, scale):
