@@ -137,7 +137,7 @@ def test_passes_of_two_accumulator_buffers(dtype):
 # partial expert tiles (8 a fragment tile, 64 and 128 a CTA), partial token tiles of 128, slices of K, one chunk of a slice; both sides of the rule that takes
 # fp32 tiles, those of 32 x 64 and of 64 x 128; tokens that are selected four a CTA
 @pytest.mark.parametrize("E,k,T,D", [(17, 2, 256, 256), (60, 6, 257, 512), (64, 8, 383, 2304), (65, 4, 300, 1024), (128, 8, 385, 2048), (129, 8, 256, 7168),
-                                     (256, 8, 511, 1280), (128, 8, 320, 2048), (128, 8, 321, 2048), (128, 4, 1600, 256), (2050, 8, 256, 256)])
+                                     (256, 8, 511, 1280), (128, 8, 320, 2048), (128, 8, 321, 2048), (128, 4, 1600, 256), (2050, 8, 256, 256), (2050, 4, 300, 512)])
 def test_router_logits_of_large_batches(E, k, T, D):
     F, dtype = 32, oracle.Q8_0
     rng = np.random.default_rng(E)
