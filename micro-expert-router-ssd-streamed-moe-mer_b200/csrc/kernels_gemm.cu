@@ -18,14 +18,16 @@
 //     in fp32 in TMEM, so the result matches the fp32 reference to ~1e-4 of the output RMS instead of f16's 2e-3.
 //   * Warp roles: 0 = producer of the activation stages, 1 = MMA issuer (of the pair's first CTA; one elected lane issues
 //     predicated instructions; every operand is computed in uniform registers) and TMEM owner, 2..9 = epilogue (two groups
-//     of four, one per accumulator buffer), 10..25 = dequantisers (four per quarter of the rows, a block of every weight
-//     stage each), 26 = producer of the weight stages (lanes 0..7 copy one packed tile each).
-// What bounds it: the MMAs and the way of A through tensor memory, which overlap only in part, and on full-width passes the power
-// limit.  2048 tokens on 128 experts of 2048 x 768, gate/up with the split of its rows: 348 us in a run through 48 layers (902 to 990 W, 1.64
-// to 1.67 GHz; 416 us with single CTAs, two 66 KB activation stages and eight dequantiser warps), 309 us at burst clocks, of which
-// leaving out the second and third product saves 50, the stores to tensor memory 37, both 104, the conversion arithmetic 4; tensor
-// pipe 62 % active.  4096 tokens on 256 experts of 7168 x 2048: 5.7 ms, 6.6 ms before.  Passes of a few tokens are bound by reading the
-// weights and by their instructions.  Sorting the passes by width, widest first, changed neither.
+//     of four, one per accumulator buffer), 10..25 = dequantisers (two teams of two per quarter of the rows, two blocks of every second
+//     weight stage each), 26 and 27 = producers of the weight stages (lanes 0..3 copy one packed tile each).
+// What bounds it: the way of A through tensor memory on passes of up to 64 tokens, the MMAs from about 80 on, the power limit on full-width
+// ones.  A group of four blocks takes 1050 cycles on a pass of 32 tokens (1750 before) and 1150 on one of 80; the MMAs of N columns N / 2 each,
+// 24 a group, so 380 and 960 (alone, with A in tensor memory, they run at that rate for every N, whatever else uses tensor or shared memory).  The
+// rest is the cycle MMAs -> done -> store -> arrival at the issuer of the other CTA, 2000 cycles of which two are in flight.
+// Us a pass, before and after uniform operands, one activation copy a group, two weight producers and two teams of dequantisers: 256 tokens on 8
+// experts of 4096 x 14336 594 / 524, 2 layers of 2048 on 128 of 2048 x 768 1097 / 1050, 4096 on 256 of 7168 x 2048 8680 / 8240.
+// Tried without gain: one MMA for hi * [hi | lo] of passes up to 32 tokens, the conversion of both blocks ahead of the wait (spills),
+// commits or groups of two blocks, fewer instructions in the conversion, a look at the issuer's next barrier ahead.
 // Every wait is bounded; on expiry the CTA latches MER_DEVSTAT_TIMEOUT, stops issuing work, waits
 // (bounded) for its copies and MMAs in flight, frees its TMEM and returns.
 #include <cuda.h>
@@ -42,26 +44,26 @@
 
 namespace {
 
-constexpr int G_WARPS = 27, G_THREADS = G_WARPS * 32;
-constexpr int W_PRODUCER = 0, W_MMA = 1, W_EPI0 = 2, W_DQ0 = 10, W_WEIGHTS = 26;
+constexpr int G_WARPS = 28, G_THREADS = G_WARPS * 32;
+constexpr int W_PRODUCER = 0, W_MMA = 1, W_EPI0 = 2, W_DQ0 = 10, W_WEIGHTS = 26, WEIGHT_WARPS = 2;
 constexpr int EPI_WARPS = 4, DQ_WARPS = 16;  // EPI_WARPS per accumulator
 constexpr uint32_t PAIR = 2;             // CTAs of a cluster: they share the B operand, each holding half of its rows
 constexpr uint32_t RAW_BLOCKS = 4;       // blocks of K per weight stage (per packed tile: one bulk copy)
 constexpr uint32_t G_HEADER = 5120;      // mbarriers, TMEM base, and from byte 1024 the epilogue groups' per-pass tables (2 KB each)
 constexpr uint32_t TMEM_COLS = 512;      // [0, 256): two accumulator buffers of up to 128 columns; [256, 512): A stages
 constexpr uint32_t TMEM_A0 = 256, A_STAGES = 8, A_STAGE_COLS = 32;  // a stage = one block: 16 columns hi + 16 columns lo
-constexpr uint32_t MAX_RING = 8;
-// The MMA issuer synchronises with its producers once per GROUP blocks of K: it waits for the group's A stages of both
-// CTAs (a_full: every dequantiser warp of the pair) and for its activation stage (b_full: the bytes of both CTAs'
-// copies), issues the group's MMAs and commits done[] in both CTAs, which releases all of it.
-constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16;
+constexpr uint32_t RAW_STAGES = 4;
+// The MMA issuer synchronises with its producers once per GROUP blocks of K: it waits for the group's activation stage (b_full: the bytes of both
+// CTAs' copies) and for its A stages of both CTAs (a_full: the dequantiser warps of the pair that convert it), issues the group's
+// MMAs and commits done[] in both CTAs, which releases all of it.  The barriers are counted by groups, of which no more than n_b are in flight.
+constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16, FULL_RING = 8;
 constexpr uint32_t CHUNK_K = 64, CHUNKS = GROUP * 32 / CHUNK_K;  // a row's piece of a chunk is 128 bytes, the swizzle span
 constexpr uint32_t PASS_TOKENS = 256;    // tokens of a pass at most: N of one MMA
 // A pass of up to BUF_TOKENS takes one of the two accumulator buffers and one activation stage a group; a wider one takes both buffers (its MMAs then
 // wait for the epilogue of the item before) and two stages: what it saves is a second conversion of the weights.
 constexpr uint32_t BUF_TOKENS = 128;
-constexpr uint32_t PART_BYTES = BUF_TOKENS / PAIR * 128, CHUNK_BYTES = 2 * PART_BYTES, B_STAGE = CHUNKS * CHUNK_BYTES;  // hi rows, then lo rows
-static_assert(RAW_BLOCKS % GROUP == 0 && DQ_WARPS == 4 * RAW_BLOCKS && A_STAGES % RAW_BLOCKS == 0, "a block of a weight stage for each of a quarter's warps");
+constexpr uint32_t B_STAGE = CHUNKS * 2 * (BUF_TOKENS / PAIR) * 128;  // of each chunk the hi rows, then the lo rows
+static_assert(RAW_BLOCKS == GROUP && DQ_WARPS == 4 * RAW_BLOCKS && A_RING == 2, "a weight stage is a group; two of its blocks for each of a quarter's warps of a team");
 constexpr float POW2_SCALE_TARGET = 9;   // activations are scaled so that the row maximum lies in [256, 512)
 
 struct GemmParams {
@@ -70,11 +72,11 @@ struct GemmParams {
   const float *unscale;    // 1 / scale of each activation row
   uint32_t rows;           // F (gate/up) or D (down)
   uint32_t kb_total;       // 32-value blocks per weight row
-  uint32_t n_raw, n_b;     // ring depths (weights, activations)
+  uint32_t n_b;            // stages of the activation ring
   float *out;              // phase 0: h [P x F]; phase 1: y [P x D]
 };
 
-// The activation matrix in boxes of 8, 16 .. 64 rows (half a pass's width) x 64 values.
+// The activation matrix in boxes of 8, 16 .. 128 rows (half a pass's width) x both parts x a group's chunks of 64 values.
 struct ActMaps {
   CUtensorMap m[PASS_TOKENS / 16];
 };
@@ -112,12 +114,12 @@ __device__ __forceinline__ uint32_t leader_addr(const void *p) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
   return a;
 }
-// The box of `map` at (column x, row r) of the activation matrix into this CTA's shared memory (128-byte rows, swizzled);
-// the bytes are counted on a barrier of the pair's first CTA.
-__device__ __forceinline__ void tile_g2s(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t r, uint32_t bar) {
+// The box of `map` at row r and chunk `chunk` of the activation matrix into this CTA's shared memory (128-byte rows, swizzled: the rows' hi parts
+// of the first chunk, their lo parts, the same of the second); the bytes are counted on a barrier of the pair's first CTA.
+__device__ __forceinline__ void group_g2s(uint32_t dst, const CUtensorMap *map, uint32_t r, uint32_t chunk, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(map), "r"(x), "r"(r), "r"(bar)
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes.cta_group::2 [%0], [%1, {%2, %3, %2, %4}], [%5];" ::"r"(dst),
+      "l"(map), "r"(0), "r"(r), "r"(chunk), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void cluster_sync() {
@@ -188,14 +190,12 @@ struct Ring {
 // The ring of activation stages (an even number of at most eight) as its producer and the issuer count it: a group of blocks takes one stage, or
 // two adjacent ones from an even one on.
 struct StageRing {
-  uint32_t n, at = 0, phases = 0;  // bit i of phases: parity of the next use of stage i's barrier
+  uint32_t n, at = 0;
   __device__ explicit StageRing(uint32_t n_) : n(n_) {}
-  __device__ __forceinline__ uint32_t take(bool wide, uint32_t &parity) {
+  __device__ __forceinline__ uint32_t take(bool wide) {
     if (wide) at = (at + 1) & ~1u;
     if (at >= n) at = 0;
     const uint32_t st = at;
-    parity = phases >> st & 1;
-    phases ^= 1u << st;
     at += wide ? 2 : 1;
     return st;
   }
@@ -230,10 +230,9 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
   uint8_t *s_raw = s_b + p.n_b * B_STAGE;
 
   if (threadIdx.x == 0) {
-    for (uint32_t s = 0; s < MAX_RING; s++) {
-      mbar_init(&raw_full[s], 1), mbar_init(&raw_empty[s], DQ_WARPS);  // filled by the weight producer, left by every dequantiser warp
-      mbar_init(&a_full[s], PAIR * 4 * GROUP), mbar_init(&b_full[s], 1);
-    }
+    // filled by the weight producers, left by a team of dequantisers
+    for (uint32_t s = 0; s < RAW_STAGES; s++) mbar_init(&raw_full[s], WEIGHT_WARPS), mbar_init(&raw_empty[s], DQ_WARPS / 2);
+    for (uint32_t s = 0; s < FULL_RING; s++) mbar_init(&a_full[s], PAIR * DQ_WARPS / 2), mbar_init(&b_full[s], 1);
     for (uint32_t s = 0; s < DONE_RING; s++) mbar_init(&done[s], 1);
     for (uint32_t s = 0; s < 2; s++) mbar_init(&acc_full[s], 1), mbar_init(&acc_empty[s], PAIR * EPI_WARPS);
     mbar_init(drain, 1);
@@ -288,22 +287,19 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
 
   if (warp == W_PRODUCER) {
     // ------------------------------------------------------------------------ producer of the activation stages
-    // one stage = one group of blocks of K of this CTA's half of the pass's rows; lane l copies chunk l / 2, the hi parts
-    // (even l) or the lo parts.  A stage is free again when the MMAs of the group that used it have run: the
-    // issuer's done[] commit says so.
+    // one stage = one group of blocks of K of this CTA's half of the pass's rows: one copy.  Four of 64 values and a part each kept this warp busy for
+    // 1000 cycles a group.  A stage is free again when the MMAs of the group that used it have run: the issuer's done[] commit says so.
     StageRing rb(p.n_b);
     uint32_t holder = 0;  // lane i: 1 + the group that took stage i last
     uint32_t pg = 0;  // groups issued so far, over all items (the issuer counts the same way)
-    const uint32_t chunk = lane >> 1, part = lane & 1, K = p.kb_total * 32;
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
       if (!next_item(item, pstart, pcount)) continue;
       const uint32_t width = pass_width(pcount), row = pstart + rank * (width / PAIR);
       const CUtensorMap *map = &maps.m[width / 16 - 1];
       const bool wide = width > BUF_TOKENS;
-      const uint32_t part_bytes = wide ? 2 * PART_BYTES : PART_BYTES;
       for (uint32_t gi = 0; gi < n_groups && ok; gi++, pg++) {
-        uint32_t parity;
-        const uint32_t stage = rb.take(wide, parity);
+        const uint32_t stage = rb.take(wide);
+        uint64_t *bar = &b_full[pg % FULL_RING];
         // 1 + the newest group that has had one of these stages
         const bool mine = lane == stage || (wide && lane == stage + 1);
         const uint32_t busy = __reduce_max_sync(0xffffffffu, mine ? holder : 0u);
@@ -312,18 +308,17 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (rank == 0 && lane == 0) mbar_expect_tx(&b_full[stage], CHUNKS * width * 2 * 128);  // both CTAs' bytes
-        __syncwarp();
-        if (lane < 2 * CHUNKS)
-          tile_g2s(smem_u32(s_b) + stage * B_STAGE + (chunk * 2 + part) * part_bytes, map, part * K + (gi * CHUNKS + chunk) * CHUNK_K, row,
-                   leader_addr(&b_full[stage]));
+        if (lane == 0) {
+          if (rank == 0) mbar_expect_tx(bar, CHUNKS * width * 2 * 128);  // both CTAs' bytes
+          group_g2s(smem_u32(s_b) + stage * B_STAGE, map, row, gi * CHUNKS, leader_addr(bar));
+        }
       }
     }
     if (!ok) {
       if (lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
       // copies already in flight get a bounded chance to land before the pair's shared memory is released
       if (rank == 0)
-        for (uint32_t s = 0; s < p.n_b; s++) (void)mbar_wait(&b_full[s], 0), (void)mbar_wait(&b_full[s], 1);
+        for (uint32_t s = 0; s < FULL_RING; s++) mbar_drain(&b_full[s], 0, 10000000ull), mbar_drain(&b_full[s], 1, 10000000ull);
     }
   } else if (warp == W_MMA) {
     // -------------------------------------------------------------------------- MMA issuer (of the pair: its first CTA)
@@ -342,43 +337,49 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     // constants are computed there directly, values derived from a loaded pass count had to be moved over per
     // instruction (measured: +25 % issue time).
     auto run_item = [&](auto width_tag, auto split_tag) {
+      constexpr uint32_t WIDTH = decltype(width_tag)::value;
       constexpr uint32_t LO = decltype(split_tag)::value ? SPLIT_TOKENS : 0;  // columns of the small products
-      constexpr uint32_t idesc = instr_desc(decltype(width_tag)::value);
-      constexpr bool WIDE = decltype(width_tag)::value > BUF_TOKENS;
-      constexpr uint32_t PART = WIDE ? 2 * PART_BYTES : PART_BYTES;
+      constexpr uint32_t idesc = instr_desc(WIDTH);
+      constexpr bool WIDE = WIDTH > BUF_TOKENS;
+      constexpr uint32_t PART = WIDTH / PAIR * 128;  // bytes of the hi or the lo rows of a chunk
       const uint32_t buf = WIDE ? 0 : next_buf;
-      const uint32_t d_tmem = tmem_base + buf * 128;
-      for (uint32_t st = 0; st < p.kb_total && ok; st += GROUP, grp++) {
-        const uint32_t ag = grp % A_RING;
-        uint32_t parity;
-        const uint32_t stage = rb.take(WIDE, parity);
-        if (st == 0) {  // the previous item of the buffer (of both) has been drained
-          if ((WIDE || buf == 0) && uses0 > 0) ok = mbar_wait_tmem(&acc_empty[0], (uses0 - 1) & 1);
-          if ((WIDE || buf == 1) && uses1 > 0) ok = mbar_wait_tmem(&acc_empty[1], (uses1 - 1) & 1) && ok;
-        }
-        if (ok) ok = mbar_wait_cluster(&b_full[stage], parity);
-        if (ok) ok = mbar_wait_tmem(&a_full[ag], (grp / A_RING) & 1);
-        ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the vote also tells the compiler so
+      // the previous item of the buffer (of both) has been drained
+      if ((WIDE || buf == 0) && uses0 > 0) ok = mbar_wait_tmem(&acc_empty[0], (uses0 - 1) & 1);
+      if ((WIDE || buf == 1) && uses1 > 0) ok = mbar_wait_tmem(&acc_empty[1], (uses1 - 1) & 1) && ok;
+      ok = __all_sync(0xffffffffu, ok);  // warp-uniform by construction; the votes also tell the compiler so
+      uint32_t acc = 0;  // the item's first MMA overwrites the accumulator
+      for (uint32_t left = n_groups; left > 0 && ok; left--) {
+        // A reduction's result sits in a uniform register, and so does all that is computed from it.  Values that the loop over the items carries had to be
+        // moved over for every instruction: 34 cycles to issue one instead of 14.
+        const uint32_t at = __reduce_max_sync(0xffffffffu, rb.take(WIDE) << 2 | (grp % A_RING) << 1 | buf);
+        const uint32_t stage = at >> 2, a_grp = tmem_base + TMEM_A0 + (at >> 1 & 1) * GROUP * A_STAGE_COLS, d_tmem = tmem_base + (at & 1) * 128;
+        // (the activations land well ahead of the A stages: their wait, 200 cycles of which are its acquire at cluster scope, costs nothing)
+        ok = mbar_wait_cluster(&b_full[grp % FULL_RING], (grp / FULL_RING) & 1);
+        if (ok) ok = mbar_wait_tmem(&a_full[grp % FULL_RING], (grp / FULL_RING) & 1);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
+        const uint64_t b_stage = b_desc0 + (uint64_t)(stage * (B_STAGE >> 4));
+        uint64_t *freed = &done[grp % DONE_RING];
+        grp++;
 #pragma unroll
         for (uint32_t b4 = 0; b4 < GROUP; b4++) {
-          const uint32_t a_hi = tmem_base + TMEM_A0 + (ag * GROUP + b4) * A_STAGE_COLS, a_lo = a_hi + 16;
-          const uint64_t b_blk = b_desc0 + (uint64_t)((stage * B_STAGE + (b4 >> 1) * 2 * PART + (b4 & 1) * 64) >> 4);
+          const uint32_t a_hi = a_grp + b4 * A_STAGE_COLS, a_lo = a_hi + 16;
+          const uint64_t b_blk = b_stage + (uint64_t)(((b4 >> 1) * 2 * PART + (b4 & 1) * 64) >> 4);
 #pragma unroll
           for (uint32_t j = 0; j < 2; j++) {  // 16 values of K per instruction: 8 TMEM columns of A, 32 bytes of a row of B
             const uint64_t dbh = b_blk + (uint64_t)(j * 2), dbl = dbh + (PART >> 4);
-            const uint32_t acc = (b4 == 0 && j == 0) ? (st != 0) : 1u;  // the item's first MMA overwrites the accumulator
+            if (b4 > 0 || j > 0) acc = 1;
             tc_mma_ts(leader, d_tmem, a_hi + j * 8, dbh, idesc, acc);
             tc_mma_ts(leader, d_tmem + LO, a_hi + j * 8, dbl, idesc, LO ? acc : 1u);
             tc_mma_ts_acc(leader, d_tmem + LO, a_lo + j * 8, dbh, idesc);
           }
         }
-        tc_commit(leader, &done[grp % DONE_RING]);  // frees the group's A stages and its activation stage, in both CTAs
-        if (st + GROUP >= p.kb_total) {
-          tc_commit(leader, &acc_full[buf]);
-          if (WIDE) tc_commit(leader, &acc_full[1]);
-        }
+        tc_commit(leader, freed);  // frees the group's A stages and its activation stage, in both CTAs
+      }
+      if (ok) {
+        tc_commit(leader, &acc_full[buf]);
+        if (WIDE) tc_commit(leader, &acc_full[1]);
       }
       if (WIDE || buf == 0) uses0++;
       if (WIDE || buf == 1) uses1++;
@@ -425,83 +426,107 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     (void)mbar_wait(drain, 0);
     __syncwarp();
     }
-  } else if (warp == W_WEIGHTS) {
-    // ------------------------------------------------------------------------ producer of the weight stages
-    // one stage = RAW_BLOCKS blocks of K of the item's eight packed tiles; lane m < 8 copies tile m's chunk
-    Ring raw(p.n_raw);
+  } else if (warp >= W_WEIGHTS) {
+    // ------------------------------------------------------------------------ producers of the weight stages
+    // one stage = RAW_BLOCKS blocks of K of the item's eight packed tiles; each of two warps copies the chunks of four, a lane one (a copy takes the
+    // warp some 110 cycles; eight of them, 900 a group, were more than what the MMAs of a narrow pass take)
+    constexpr uint32_t TILES = 8 / WEIGHT_WARPS;
+    const uint32_t tile = (warp - W_WEIGHTS) * TILES + lane % TILES;
+    Ring raw(RAW_STAGES);
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
       const uint8_t *base = next_item(item, pstart, pcount);
       if (!base) continue;
       const uint32_t mt = min((item % m_pairs) * PAIR + rank, m_tiles - 1);
-      const uint8_t *src = base + region + (size_t)(mt * 8 + (lane & 7)) * tile_bytes;
+      const uint8_t *src = base + region + (size_t)(mt * 8 + tile) * tile_bytes;
       for (uint32_t gi = 0; gi < p.kb_total / RAW_BLOCKS && ok; gi++) {
         if (raw.round > 0) ok = mbar_wait(&raw_empty[raw.stage], (raw.round - 1) & 1);  // every dequantiser warp has left the stage
         if (*s_abort) ok = false;
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (lane == 0) mbar_expect_tx(&raw_full[raw.stage], RAW_BYTES);
+        if (lane == 0) mbar_expect_tx(&raw_full[raw.stage], RAW_BYTES / WEIGHT_WARPS);
         __syncwarp();
-        if (lane < 8) bulk_g2s(s_raw + raw.stage * RAW_BYTES + lane * TILE_RAW, src + (size_t)gi * TILE_RAW, TILE_RAW, &raw_full[raw.stage]);
+        if (lane < TILES) bulk_g2s(s_raw + raw.stage * RAW_BYTES + tile * TILE_RAW, src + (size_t)gi * TILE_RAW, TILE_RAW, &raw_full[raw.stage]);
         raw.advance();
       }
     }
     if (!ok) {
       if (lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
       // weight copies already in flight get a bounded chance to land before the CTA's shared memory is released
-      for (uint32_t s = 0; s < p.n_raw; s++) (void)mbar_wait(&raw_full[s], 0), (void)mbar_wait(&raw_full[s], 1);
+      for (uint32_t s = 0; s < RAW_STAGES; s++) (void)mbar_wait(&raw_full[s], 0), (void)mbar_wait(&raw_full[s], 1);
     }
   } else if (warp >= W_DQ0) {
     // ------------------------------------------------------------------------ dequantisers
     // A thread owns one weight row of the item: TMEM lane 32 * (warp % 4) + lane, i.e. packed tile 2q + lane / 16,
     // row slot lane % 16.  Per block it reads the row's 32 quants from the tile chunk in shared memory and stores
-    // 16 columns of hi and 16 of lo.  The four warps of a quarter take one block of a weight stage each.
-    Ring raw(p.n_raw);
-    uint32_t gblk = 0;  // blocks of K seen so far, over all items (A stage = gblk % A_STAGES)
-    const uint32_t q = warp & 3, mine = (warp - W_DQ0) >> 2;  // quarter of the rows; block of every weight stage
+    // 16 columns of hi and 16 of lo.  Two teams of eight warps take the groups in turn, a warp two adjacent blocks of each of its
+    // team's: one team converts while the other waits and stores (256 tokens on 8 experts of 4096 x 14336 535 us, with a block of every group a warp 569).
+    const uint32_t q = warp & 3, team = (warp - W_DQ0) >> 2 & 1, mine = (warp - W_DQ0) >> 3 << 1;  // quarter of the rows; first of the two blocks
     const uint32_t T = 2 * q + (lane >> 4), g = lane & 7, half = (lane >> 3) & 1;
     const __half2 zp = DT == MER_DTYPE_Q4_0 ? __floats2half2_rn(1032.0f, 1032.0f) : __floats2half2_rn(1152.0f, 1152.0f);
+    constexpr int RAW_WORDS = DT == MER_DTYPE_Q4_0 ? 4 : 8;
+    uint32_t groups = 0;  // groups of blocks before this item
+    bool ready = false;   // the weight stage has been seen full
+    const uint32_t tile0 = smem_u32(s_raw) + T * TILE_RAW;
+    const uint32_t a_tmem = tmem_base + ((q * 32u) << 16) + TMEM_A0 + mine * A_STAGE_COLS;
+    // the quants of this thread's row in block `blk` of a stage, and their scale
+    auto load = [&](uint32_t src, uint32_t blk, uint32_t (&w)[RAW_WORDS], uint32_t &scale) {
+      if (DT == MER_DTYPE_Q8_0) {
+        src += blk * 544;
+        scale = lds32(src + 512 + g * 4);
+#pragma unroll
+        for (int t = 0; t < 4; t++) {  // values 8t .. 8t+7
+          const uint2 v = lds64(src + packed_piece(g, t) * 16 + half * 8);
+          w[2 * t] = v.x, w[RAW_WORDS > 4 ? 2 * t + 1 : 0] = v.y;
+        }
+      } else {
+        // block-pair record: 16 bytes per (g, t) = words (slot g, blk 0), (slot g+8, blk 0), (slot g, blk 1), (slot g+8, blk 1);
+        // byte i of a word holds values 4t+i (low nibble) and 16+4t+i (high nibble) of its block
+        src += (blk >> 1) * 576;
+        scale = lds32(src + 512 + g * 8 + (blk & 1) * 4);
+#pragma unroll
+        for (int t = 0; t < 4; t++) w[t] = lds32(src + packed_piece(g, t) * 16 + ((blk & 1) * 2 + half) * 4);
+      }
+    };
+    // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
+    auto convert = [&](const uint32_t (&w)[RAW_WORDS], uint32_t scale, uint32_t (&v)[32]) {
+      const __half2 dd = __half2half2(half ? __high2half(bits_h2(scale)) : __low2half(bits_h2(scale)));
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        if (DT == MER_DTYPE_Q8_0) {
+          const uint32_t a = w[2 * t], b = w[RAW_WORDS > 4 ? 2 * t + 1 : 0];
+          dq2(__byte_perm(a, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
+          dq2(__byte_perm(a, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
+          dq2(__byte_perm(b, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
+          dq2(__byte_perm(b, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
+        } else {
+          const uint32_t lows = w[t] & 0x0F0F0F0Fu, highs = (w[t] >> 4) & 0x0F0F0F0Fu;
+          dq2(__byte_perm(lows, 0x64646464u, 0x4140), zp, dd, v[2 * t + 0], v[16 + 2 * t + 0]);
+          dq2(__byte_perm(lows, 0x64646464u, 0x4342), zp, dd, v[2 * t + 1], v[16 + 2 * t + 1]);
+          dq2(__byte_perm(highs, 0x64646464u, 0x4140), zp, dd, v[8 + 2 * t + 0], v[24 + 2 * t + 0]);
+          dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
+        }
+      }
+    };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
       if (!next_item(item, pstart, pcount)) continue;
-      // One weight stage at a time, of which this warp converts one block.  It waits for the A stage only when the
-      // block is ready in registers: the conversion of the next blocks is then off the cycle of MMAs -> done -> store -> MMAs.
-      for (uint32_t gi = 0; gi < p.kb_total / RAW_BLOCKS && ok; gi++, gblk += RAW_BLOCKS) {
-        ok = mbar_wait(&raw_full[raw.stage], raw.round & 1);
-        const uint32_t tile_src = smem_u32(s_raw) + raw.stage * RAW_BYTES + T * TILE_RAW;
-        uint32_t v[32];  // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
-        if (DT == MER_DTYPE_Q8_0) {
-          const uint32_t src = tile_src + mine * 544;
-          const uint32_t sc2 = lds32(src + 512 + g * 4);
-          const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
-#pragma unroll
-          for (int t = 0; t < 4; t++) {  // values 8t .. 8t+7
-            const uint2 w = lds64(src + packed_piece(g, t) * 16 + half * 8);
-            dq2(__byte_perm(w.x, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
-            dq2(__byte_perm(w.x, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
-            dq2(__byte_perm(w.y, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
-            dq2(__byte_perm(w.y, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
-          }
-        } else {
-          // block-pair record: 16 bytes per (g, t) = words (slot g, blk 0), (slot g+8, blk 0), (slot g, blk 1), (slot g+8, blk 1);
-          // byte i of a word holds values 4t+i (low nibble) and 16+4t+i (high nibble) of its block
-          const uint32_t src = tile_src + (mine >> 1) * 576, blk = mine & 1;
-          const uint32_t sc2 = lds32(src + 512 + g * 8 + blk * 4);
-          const __half2 dd = __half2half2(half ? __high2half(bits_h2(sc2)) : __low2half(bits_h2(sc2)));
-#pragma unroll
-          for (int t = 0; t < 4; t++) {
-            const uint32_t w = lds32(src + packed_piece(g, t) * 16 + (blk * 2 + half) * 4);
-            const uint32_t lows = w & 0x0F0F0F0Fu, highs = (w >> 4) & 0x0F0F0F0Fu;
-            dq2(__byte_perm(lows, 0x64646464u, 0x4140), zp, dd, v[2 * t + 0], v[16 + 2 * t + 0]);
-            dq2(__byte_perm(lows, 0x64646464u, 0x4342), zp, dd, v[2 * t + 1], v[16 + 2 * t + 1]);
-            dq2(__byte_perm(highs, 0x64646464u, 0x4140), zp, dd, v[8 + 2 * t + 0], v[24 + 2 * t + 0]);
-            dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
-          }
-        }
-#pragma unroll
-        for (int i = 0; i < 32; i++) asm volatile("" : "+r"(v[i]));  // the conversion stays ahead of the wait below
+      for (uint32_t grp = groups + ((groups ^ team) & 1); grp < groups + n_groups && ok; grp += 2) {
+        const uint32_t stage = grp % RAW_STAGES;
+        if (!ready) ok = mbar_wait(&raw_full[stage], (grp / RAW_STAGES) & 1);
         __syncwarp();
-        if (lane == 0) mbar_arrive(&raw_empty[raw.stage]);
-        raw.advance();
-        const uint32_t grp = (gblk + mine) / GROUP;
+        uint32_t w[RAW_WORDS], w1[RAW_WORDS], scale, scale1, v[32];
+        load(tile0 + stage * RAW_BYTES, mine, w, scale);
+        load(tile0 + stage * RAW_BYTES, mine + 1, w1, scale1);
+        convert(w, scale, v);
+        // The first block is converted, and the second in registers, ahead of the wait: they are then off the cycle of
+        // MMAs -> done -> store -> MMAs.
+#pragma unroll
+        for (int i = 0; i < 32; i++) asm volatile("" : "+r"(v[i]));
+#pragma unroll
+        for (int i = 0; i < RAW_WORDS; i++) asm volatile("" : "+r"(w1[i]));
+        asm volatile("" : "+r"(scale1));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&raw_empty[stage]);
+        ready = mbar_test(&raw_full[(grp + 2) % RAW_STAGES], ((grp + 2) / RAW_STAGES) & 1);
         if (grp >= A_RING && ok) {
           // the group's A stages were last read by the MMAs of the group A_RING before it
           const uint32_t sp = grp - A_RING;
@@ -510,12 +535,17 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        tc_st32(tmem_base + ((q * 32u) << 16) + TMEM_A0 + ((gblk + mine) % A_STAGES) * A_STAGE_COLS, v);
+        const uint32_t a = a_tmem + grp % A_RING * GROUP * A_STAGE_COLS;
+        tc_st32(a, v);
+        convert(w1, scale1, v);
+        tc_st32(a + A_STAGE_COLS, v);
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_tmem(leader_addr(&a_full[grp % A_RING]));
+        if (lane == 0) mbar_arrive_tmem(leader_addr(&a_full[grp % FULL_RING]));
+        ready = __all_sync(0xffffffffu, ready);
       }
+      groups += n_groups;
     }
     if (!ok && lane == 0) *s_abort = 1, atomicOr(d.status, MER_DEVSTAT_TIMEOUT);
   } else {
@@ -746,29 +776,29 @@ EncodeTiled encode_tiled() {
   }();
   return fn;
 }
-// Rows of [hi K | lo K] f16.  Rows past the end read as zeros.
+// Rows of [hi K | lo K] f16 as (value of a chunk, row, part, chunk).  Rows past the end read as zeros.
 bool activation_maps(ActMaps *maps, void *base, uint32_t rows, uint32_t K) {
   const EncodeTiled fn = encode_tiled();
   bool ok = fn != nullptr;
   for (uint32_t i = 0; i < PASS_TOKENS / 16 && ok; i++) {
-    const cuuint64_t dims[2] = {2ull * K, rows}, strides[1] = {4ull * K};
-    const cuuint32_t box[2] = {CHUNK_K, 8 * (i + 1)}, step[2] = {1, 1};
-    ok = fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint64_t dims[4] = {CHUNK_K, rows, 2, K / CHUNK_K}, strides[3] = {4ull * K, 2ull * K, 2 * CHUNK_K};
+    const cuuint32_t box[4] = {CHUNK_K, 8 * (i + 1), 2, CHUNKS}, step[4] = {1, 1, 1, 1};
+    ok = fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   return ok;
 }
 
 struct GemmPlan {
-  uint32_t n_raw, n_b;
+  uint32_t n_b;
   size_t smem;
 };
 
 GemmPlan gemm_plan(int dtype) {
   const uint32_t tile_raw = RAW_BLOCKS * 16 * (dtype == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES);
   GemmPlan pl{};
-  pl.n_raw = 4, pl.n_b = 4;  // weight stages of four blocks; activation stages of one group
-  pl.smem = G_HEADER + (size_t)pl.n_raw * 8 * tile_raw + (size_t)pl.n_b * B_STAGE;
+  pl.n_b = 4;  // activation stages of one group
+  pl.smem = G_HEADER + (size_t)RAW_STAGES * 8 * tile_raw + (size_t)pl.n_b * B_STAGE;
   return pl;
 }
 
@@ -832,7 +862,7 @@ cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes,
     p.d = d, p.phase = phase, p.unscale = unscale;
     p.rows = phase == 0 ? d.F : d.D;
     p.kb_total = K / 32;
-    p.n_raw = pl.n_raw, p.n_b = pl.n_b;
+    p.n_b = pl.n_b;
     p.out = phase == 0 ? d.h : d.y;
     kern<<<sm_count / PAIR * PAIR, G_THREADS, pl.smem, s>>>(p, maps);
     if (phase == 0 && ev_mid) cudaEventRecord(ev_mid, s);

@@ -42,6 +42,22 @@ def test_one_expert_many_tokens_matches_oracle(dtype, D, F, n_tokens):
     assert rel_rms_err(got, streamed) <= 1e-4  # both kernel families carry ~22-bit operands
 
 
+@pytest.mark.parametrize("dtype", [oracle.Q8_0, oracle.Q4_0])
+@pytest.mark.parametrize("D,F,n_tokens", [(128, 128, 13), (128, 384, 33), (384, 128, 129), (640, 20480, 50)])
+def test_odd_numbers_of_k_groups_and_many_items(dtype, D, F, n_tokens):
+    # items of one, three and five groups of 128 values of K: the dequantisers' teams take groups in turn across the items of a pair of
+    # CTAs (160 items of 640 values on 74 pairs), and the rings of two to sixteen groups wrap at any point of an item
+    blob = synth.make_expert_blob(dtype, D, F, 87, 0, 0)
+    x = synth.make_activations(n_tokens, D, 87)
+    with backend(dtype, D, F, 2, max_tokens=n_tokens) as b:
+        b.admit(0, 1, blob)
+        b.set_kernel_path(3)
+        got, again = b.expert_forward_f32(0, 0, x), b.expert_forward_f32(0, 0, x)
+    assert (got == again).all()
+    for t in (0, n_tokens // 2, n_tokens - 1):
+        assert rel_rms_err(got[t], oracle.expert_forward(dtype, blob, x[t], D, F, oracle.FWD_AUTHORITATIVE)) <= FFN_TOL
+
+
 def test_automatic_selection_takes_the_gemm_path_for_large_groups():
     dtype, E, D, F, k, B = oracle.Q8_0, 8, 512, 256, 2, 160  # 320 pairs over 8 experts: 40 tokens per expert
     blobs = [synth.make_expert_blob(dtype, D, F, 82, 0, e) for e in range(E)]
