@@ -6,14 +6,17 @@
 //   * Two producer warps copy each tile's sixteen row pieces global -> shared with bulk async copies into rows padded so that
 //     the eight rows a fragment load touches start in different banks.  A row piece that does not start on a 16-byte
 //     boundary (rows that are no multiple of 256 values) is copied from the boundary below and read with a byte shift.
-//   * Sixteen consumer warps split the range's blocks: every warp multiplies its few blocks of all tiles with activation
+//   * Sixteen consumer warps split the range's blocks: every warp multiplies its few blocks of all tiles, two tiles at a time, with activation
 //     fragments of its own (mma B fragments, f16 hi + lo after an exact power-of-two scaling of the slice), so no warp waits
-//     for another one's fragments.  Integer weights become A fragments as in kernels_stream.cu; two adjacent blocks (36 or 68
+//     for another one's fragments; the values of the next range are fetched while this one is multiplied.  Integer weights become A fragments as in kernels_stream.cu; two adjacent blocks (36 or 68
 //     bytes) are loaded as aligned 32-bit words and shifted by the two bytes of the first scale.
-//   * An epilogue warp adds the sixteen partial tiles, and at the last range applies SiLU(gate) * up or stores the output.
+//   * An epilogue warp adds the sixteen partial tiles of a step, and at the last range applies SiLU(gate) * up or stores the output.
 //   * Every wait is bounded.  A CTA whose wait ran out latches MER_DEVSTAT_TIMEOUT and stores NaN for what it has not computed: the
 //     call is asynchronous, and a caller that does not ask for the status must not take the rest for a result.
-// One warp per weight row with byte loads, as before, took 620 us for a 4096 x 14336 Q4_0 expert and four tokens.
+// What bounds it: the consumers' instructions, 2100 cycles a tile of 4096 values where HBM takes 1600, and 3 us each of start and grid barrier.  A
+// 4096 x 14336 expert, us a call: Q4_0 and four tokens 43 / 39, Q8_0 and one token 59 / 52, with one tile at a time and fragments made from memory by
+// chained shuffles (2.5 us a range, 1.4 now) / now; one warp per weight row with byte loads took 620.  Four producer warps leave the consumers 80
+// registers: 43.
 #include <algorithm>
 
 #include "../../include/mer_b200.h"
@@ -31,16 +34,17 @@ constexpr size_t F_SMEM = 226 * 1024;
 template <int DT, int NT>
 struct Flat {
   static constexpr uint32_t BB = DT == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
+  static constexpr uint32_t TILES = NT == 1 ? 2 : 1;  // that a warp multiplies at a time (two token tiles leave room for two stages only)
   static constexpr uint32_t RANGE = DT == MER_DTYPE_Q4_0 ? 128 : 64, PER_WARP = RANGE / FC_WARPS;
   static constexpr uint32_t ROW = RANGE * BB + (DT == MER_DTYPE_Q4_0 ? 16 : 32);  // = 4 or 8 words mod 32
   static constexpr uint32_t STAGE = 16 * ROW;
   static constexpr uint32_t SEED_ROW = RANGE + 4;
   static constexpr uint32_t OFF_SEED = 512, OFF_RED = (OFF_SEED + 4 * NT * SEED_ROW * 4 + 127) & ~127u;
-  static constexpr uint32_t OFF_ACC = OFF_RED + FC_WARPS * NT * 256, OFF_FRAG = OFF_ACC + F_MAX_TILES * NT * 256;
+  static constexpr uint32_t OFF_ACC = OFF_RED + FC_WARPS * TILES * NT * 256, OFF_FRAG = OFF_ACC + F_MAX_TILES * NT * 256;
   static constexpr uint32_t OFF_RING = OFF_FRAG + RANGE * NT * 512;
   static constexpr uint32_t FIT = (uint32_t)((F_SMEM - 64 - OFF_RING) / STAGE), STAGES = FIT < F_MAX_STAGES ? FIT : F_MAX_STAGES;
   static constexpr uint32_t SMEM = OFF_RING + STAGES * STAGE + 64;  // a shifted load may look a few bytes past the last row
-  static_assert(STAGES >= 2, "two stages at least");
+  static_assert(STAGES >= 2 * TILES, "two steps' stages at least");
 };
 
 struct FlatParams {
@@ -53,39 +57,50 @@ struct FlatParams {
   uint32_t *bar, *status;  // bar[0]: arrivals, bar[1]: exits; both zero between launches
 };
 
-// B fragments of one n = 8 tile (four tokens) of `n` blocks, and their seeds.  `row`: this lane's token at the lane's first value
-// of the first block (null: zeros).  The two lanes of a token load half of a block's eight values each and swap hi and lo
-// parts.  Returns 2^24 / scale of the token of this lane's accumulator columns.
-template <int DT>
-__device__ __forceinline__ float flat_fragments(const float *row, uint32_t n, uint32_t pairs2, uint8_t *frag, uint32_t stride, float *seed) {
+// B fragments of one n = 8 tile (four tokens) of PW blocks, and their seeds, from v: this lane's half of the eight values that it and the other lane of
+// its token hold of a block (zeros: absent); the two swap hi and lo parts.  Returns 2^24 / scale of the token of this lane's accumulator columns.
+template <int DT, int PW>
+__device__ __forceinline__ float flat_fragments(float4 (&v)[PW], uint8_t *frag, uint32_t stride, float *seed) {
   const uint32_t lane = threadIdx.x & 31, t = lane & 3;
   const bool lo_lane = lane & 4;
-  float mx = 0.0f;
-#pragma unroll 8
-  for (uint32_t j = 0; j < pairs2; j++) {
-    float4 v = make_float4(0, 0, 0, 0);
-    if (row && j < n) v = *reinterpret_cast<const float4 *>(row + j * 32);
-    *reinterpret_cast<float4 *>(frag + j * stride) = v;  // parked where the fragment will be; read back by this lane only
-    mx = nan_max(nan_max(nan_max(nan_max(mx, fabsf(v.x)), fabsf(v.y)), fabsf(v.z)), fabsf(v.w));
-  }
+  uint32_t most = 0;  // of the magnitudes' bits: a NaN's are above an infinity's
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) mx = nan_max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  float sc = 1.0f;
-  if (mx > 0.0f && isfinite(mx)) {
-    int e;
-    frexpf(mx, &e);  // mx = m * 2^e, m in [0.5, 1): scaled to [256, 512)
-    sc = ldexpf(1.0f, min(9 - e, 126));
-  } else if (mx != mx || isinf(mx)) {
-    sc = mx;  // non-finite activations poison the row, as they would in fp32
-  }
-#pragma unroll 2
-  for (uint32_t j = 0; j < pairs2; j++) {
-    const float4 v = *reinterpret_cast<const float4 *>(frag + j * stride);
-    float m[4] = {v.x * sc, v.y * sc, v.z * sc, v.w * sc};  // exact (a power of two)
-    float sum = (m[0] + m[1]) + (m[2] + m[3]);
+  for (int j = 0; j < PW; j++)
+    most = max(max(max(max(most, __float_as_uint(fabsf(v[j].x))), __float_as_uint(fabsf(v[j].y))), __float_as_uint(fabsf(v[j].z))), __float_as_uint(fabsf(v[j].w)));
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((lane & 7) == 0) seed[j] = -(DT == MER_DTYPE_Q4_0 ? 8.0f : 128.0f) / POW2_24 * sum;
+  for (int o = 1; o < 8; o <<= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+  // scaled to [256, 512), by 2^126 at most; non-finite activations poison the row, as they would in fp32
+  const int e = min(135 - (int)(most >> 23), 126);
+  const bool finite = most < 0x7f800000u;
+  const float sc = most == 0 ? 1.0f : finite ? __int_as_float((e + 127) << 23) : __uint_as_float(most);
+  const float un = most == 0 ? POW2_24 : finite ? POW2_24 * __int_as_float((127 - e) << 23) : POW2_24 / sc;
+  float sum[PW];
+#pragma unroll
+  for (int j = 0; j < PW; j++) {
+    v[j].x *= sc, v[j].y *= sc, v[j].z *= sc, v[j].w *= sc;  // exact (a power of two)
+    sum[j] = (v[j].x + v[j].y) + (v[j].z + v[j].w);
+  }
+  // A block's sum over the token's eight lanes: in each step a lane hands on half of its sums, so that it ends with one block's.
+  uint32_t at = 0;
+#pragma unroll
+  for (int o = 1, n = PW; o < 8; o <<= 1) {
+    const bool upper = lane & o;
+    if (n > 1) {
+      n >>= 1;
+#pragma unroll
+      for (int j = 0; j < n; j++) {
+        const float other = __shfl_xor_sync(0xffffffffu, upper ? sum[j] : sum[n + j], o);
+        sum[j] = (upper ? sum[n + j] : sum[j]) + other;
+      }
+      at += upper ? n : 0;
+    } else {
+      sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], o);
+    }
+  }
+  seed[at] = -(DT == MER_DTYPE_Q4_0 ? 8.0f : 128.0f) / POW2_24 * sum[0];
+#pragma unroll
+  for (int j = 0; j < PW; j++) {
+    float m[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
     if (DT == MER_DTYPE_Q4_0 && lo_lane) m[0] *= 0.0625f, m[1] *= 0.0625f, m[2] *= 0.0625f, m[3] *= 0.0625f;  // their nibbles sit 4 bits higher
     const __half2 h0 = __floats2half2_rn(m[0], m[2]), h1 = __floats2half2_rn(m[1], m[3]);
     const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
@@ -95,7 +110,7 @@ __device__ __forceinline__ float flat_fragments(const float *row, uint32_t n, ui
     *reinterpret_cast<uint4 *>(frag + j * stride) = lo_lane ? make_uint4(g0, g1, lb0, lb1) : make_uint4(hb0, hb1, g0, g1);
   }
   __syncwarp();  // the seeds cross lanes
-  return __shfl_sync(0xffffffffu, POW2_24 / sc, t * 8);
+  return __shfl_sync(0xffffffffu, un, t * 8);
 }
 
 // Four bytes at a byte offset that is a multiple of two.
@@ -182,7 +197,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
     uint8_t *s_frag = smem + S::OFF_FRAG + warp * (S::PER_WARP * NT * 512) + lane * 16;
     float *s_seed = reinterpret_cast<float *>(smem + S::OFF_SEED) + warp * S::PER_WARP;
     const uint32_t frags = smem_u32(s_frag), seeds = smem_u32(s_seed) + t * (S::SEED_ROW * 4);
-    float2 *s_red = reinterpret_cast<float2 *>(smem + S::OFF_RED) + warp * (NT * 32) + lane;
+    float2 *s_red = reinterpret_cast<float2 *>(smem + S::OFF_RED) + warp * (S::TILES * NT * 32) + lane;
     const uint32_t lane_value = (DT == MER_DTYPE_Q4_0 ? 4 : 8) * t + ((lane & 4) ? (DT == MER_DTYPE_Q4_0 ? 16 : 4) : 0);
     uint32_t n_red = 0;
 #pragma unroll 1
@@ -196,99 +211,133 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
         if (!ok) break;
       }
       const float *act = ph == 0 ? p.x : p.h;
+      if (t0 == t1) continue;
+      // this warp's blocks of a range, whole pairs
+      auto share = [&](uint32_t kb0, uint32_t &b0) {
+        const uint32_t nb = min(S::RANGE, kbt - kb0), width = ((nb + FC_WARPS - 1) / FC_WARPS + 1) & ~1u;
+        b0 = warp * width;
+        return nb > b0 ? min(width, nb - b0) : 0u;
+      };
+      float4 v[S::PER_WARP];  // this lane's values of a range
+      auto fetch = [&](uint32_t kb0, int n) {
+        uint32_t b0;
+        const uint32_t mine = share(kb0, b0), tok = n * 4 + (g8 >> 1);
+        const float *row = act + (size_t)tok * kbt * 32 + (kb0 + b0) * 32 + lane_value;
+#pragma unroll
+        for (uint32_t j = 0; j < S::PER_WARP; j++)
+          v[j] = tok < p.n_tokens && j < mine ? *reinterpret_cast<const float4 *>(row + j * 32) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      };
+      if (NT == 1) fetch(0, 0);
 #pragma unroll 1
       for (uint32_t kb0 = 0; kb0 < kbt && ok; kb0 += S::RANGE) {
-        const uint32_t nb = min(S::RANGE, kbt - kb0);
-        const uint32_t width = ((nb + FC_WARPS - 1) / FC_WARPS + 1) & ~1u;  // blocks per warp, whole pairs
-        const uint32_t b0 = warp * width, mine = nb > b0 ? min(width, nb - b0) : 0u;
-        if (t0 == t1) break;
+        uint32_t b0;
+        const uint32_t mine = share(kb0, b0);
         float un[NT];
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-          const uint32_t tok = n * 4 + (g8 >> 1);
-          const float *row = tok < p.n_tokens ? act + (size_t)tok * kbt * 32 + (kb0 + b0) * 32 + lane_value : nullptr;
-          un[n] = flat_fragments<DT>(row, mine, (mine + 1) & ~1u, s_frag + n * 512, NT * 512, s_seed + tok * S::SEED_ROW);
+          if (NT > 1) fetch(kb0, n);
+          un[n] = flat_fragments<DT>(v, s_frag + n * 512, NT * 512, s_seed + (n * 4 + (g8 >> 1)) * S::SEED_ROW);
         }
+        if (NT == 1 && kb0 + S::RANGE < kbt) fetch(kb0 + S::RANGE, 0);  // the next range's values arrive while this one is multiplied
 #pragma unroll 1
-        for (uint32_t tile = t0; tile < t1; tile++) {
-          float acc[NT][4];
-#pragma unroll
-          for (int n = 0; n < NT; n++) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+        for (uint32_t tile = t0; tile < t1; tile += S::TILES) {
+          const uint32_t live = min(S::TILES, t1 - tile);
+          float acc[S::TILES][NT][4];
           // row addresses of slots g8 and g8 + 8 (and where their first block starts inside the copied piece)
-          uint32_t r0 = smem_u32(smem) + S::OFF_RING + stage * S::STAGE + g8 * S::ROW, r1 = r0 + 8 * S::ROW;
-          if (!ALIGNED) {
-            r0 += (uint32_t)((size_t)row_ptr(ph, tile, g8, kbt, kb0) & 15u);
-            r1 += (uint32_t)((size_t)row_ptr(ph, tile, g8 + 8, kbt, kb0) & 15u);
+          uint32_t r0[S::TILES], r1[S::TILES];
+#pragma unroll
+          for (uint32_t u = 0; u < S::TILES; u++) {
+#pragma unroll
+            for (int n = 0; n < NT; n++) acc[u][n][0] = acc[u][n][1] = acc[u][n][2] = acc[u][n][3] = 0.0f;
+            if (u > 0 && u >= live) break;
+            r0[u] = smem_u32(smem) + S::OFF_RING + stage * S::STAGE + g8 * S::ROW, r1[u] = r0[u] + 8 * S::ROW;
+            if (!ALIGNED) {
+              r0[u] += (uint32_t)((size_t)row_ptr(ph, tile + u, g8, kbt, kb0) & 15u);
+              r1[u] += (uint32_t)((size_t)row_ptr(ph, tile + u, g8 + 8, kbt, kb0) & 15u);
+            }
+            r0[u] += b0 * S::BB, r1[u] += b0 * S::BB;
+            if (ok) ok = mbar_wait(&full[stage], round & 1);
+            next_stage();
           }
-          r0 += b0 * S::BB, r1 += b0 * S::BB;
-          if (ok) ok = mbar_wait(&full[stage], round & 1);
           ok = __all_sync(0xffffffffu, ok);
           if (ok) {
 #pragma unroll 1
-            for (uint32_t j = 0; j < mine; j += 2, r0 += 2 * S::BB, r1 += 2 * S::BB) {
-              uint32_t a[2][2][4];  // [block][row slot g8, g8 + 8]
-              uint32_t s[2][2];     // f16 scale bits
+            for (uint32_t j = 0; j < mine; j += 2) {
+              uint4 b[NT][2];
+              float sd[NT][2];
 #pragma unroll
-              for (int r = 0; r < 2; r++) {
-                const uint32_t rp = r ? r1 : r0;
-                if (DT == MER_DTYPE_Q4_0) {
-                  uint32_t q0, q1;
-                  if (ALIGNED) {
-                    const uint32_t w0 = lds32(rp + 4 * t), w1 = lds32(rp + 4 * t + 4);
-                    q0 = __funnelshift_r(w0, w1, 16), q1 = lds32(rp + 20 + 4 * t);
-                    s[0][r] = lds32(rp) & 0xffffu, s[1][r] = lds32(rp + 16) >> 16;
-                  } else {
-                    q0 = lds_u16x2(rp + 2 + 4 * t), q1 = lds_u16x2(rp + 20 + 4 * t);
-                    s[0][r] = lds_u16x2(rp) & 0xffffu, s[1][r] = lds_u16x2(rp + 16) >> 16;
-                  }
-                  unpack_q4(q0, a[0][r]), unpack_q4(q1, a[1][r]);
-                } else {
-                  uint32_t l0, h0, l1, h1;
-                  if (ALIGNED) {
-                    const uint32_t w0 = lds32(rp + 8 * t), w1 = lds32(rp + 8 * t + 4), w2 = lds32(rp + 8 * t + 8);
-                    l0 = __funnelshift_r(w0, w1, 16), h0 = __funnelshift_r(w1, w2, 16);
-                    l1 = lds32(rp + 36 + 8 * t), h1 = lds32(rp + 40 + 8 * t);
-                    s[0][r] = lds32(rp) & 0xffffu, s[1][r] = lds32(rp + 32) >> 16;
-                  } else {
-                    l0 = lds_u16x2(rp + 2 + 8 * t), h0 = lds_u16x2(rp + 6 + 8 * t), l1 = lds_u16x2(rp + 36 + 8 * t), h1 = lds_u16x2(rp + 40 + 8 * t);
-                    s[0][r] = lds_u16x2(rp) & 0xffffu, s[1][r] = lds_u16x2(rp + 32) >> 16;
-                  }
-                  unpack_q8(l0, h0, a[0][r]), unpack_q8(l1, h1, a[1][r]);
-                }
-              }
-              if (j + 1 >= mine) s[1][0] = s[1][1] = 0;  // no second block: stale bytes against zero fragments
-#pragma unroll
-              for (int n = 0; n < NT; n++) {
-                float c1[2][4], c2[2][4];
-                uint4 b[2];
+              for (int n = 0; n < NT; n++)
 #pragma unroll
                 for (int i = 0; i < 2; i++) {
-                  b[i] = lds128(frags + ((j + i) * NT + n) * 512);
-                  const float sd = __uint_as_float(lds32(seeds + n * (4 * S::SEED_ROW * 4) + (j + i) * 4));
-                  mma_f16(c1[i], a[i][0][0], a[i][1][0], a[i][0][1], a[i][1][1], b[i].x, b[i].y, sd, 0.0f, sd, 0.0f);
+                  b[n][i] = lds128(frags + ((j + i) * NT + n) * 512);
+                  sd[n][i] = __uint_as_float(lds32(seeds + n * (4 * S::SEED_ROW * 4) + (j + i) * 4));
                 }
 #pragma unroll
-                for (int i = 0; i < 2; i++)
-                  mma_f16(c2[i], a[i][0][2], a[i][1][2], a[i][0][3], a[i][1][3], b[i].z, b[i].w, c1[i][0], c1[i][1], c1[i][2], c1[i][3]);
+              for (uint32_t u = 0; u < S::TILES; u++) {
+                if (u > 0 && u >= live) break;
+                uint32_t a[2][2][4];  // [block][row slot g8, g8 + 8]
+                uint32_t s[2][2];     // f16 scale bits
 #pragma unroll
-                for (int i = 0; i < 2; i++) {
-                  const float d0 = __half2float(__ushort_as_half((unsigned short)s[i][0])), d1 = __half2float(__ushort_as_half((unsigned short)s[i][1]));
-                  acc[n][0] = fmaf(d0, c2[i][0], acc[n][0]);
-                  acc[n][1] = fmaf(d0, c2[i][1], acc[n][1]);
-                  acc[n][2] = fmaf(d1, c2[i][2], acc[n][2]);
-                  acc[n][3] = fmaf(d1, c2[i][3], acc[n][3]);
+                for (int r = 0; r < 2; r++) {
+                  const uint32_t rp = r ? r1[u] : r0[u];
+                  if (DT == MER_DTYPE_Q4_0) {
+                    uint32_t q0, q1;
+                    if (ALIGNED) {
+                      const uint32_t w0 = lds32(rp + 4 * t), w1 = lds32(rp + 4 * t + 4);
+                      q0 = __funnelshift_r(w0, w1, 16), q1 = lds32(rp + 20 + 4 * t);
+                      s[0][r] = lds32(rp) & 0xffffu, s[1][r] = lds32(rp + 16) >> 16;
+                    } else {
+                      q0 = lds_u16x2(rp + 2 + 4 * t), q1 = lds_u16x2(rp + 20 + 4 * t);
+                      s[0][r] = lds_u16x2(rp) & 0xffffu, s[1][r] = lds_u16x2(rp + 16) >> 16;
+                    }
+                    unpack_q4(q0, a[0][r]), unpack_q4(q1, a[1][r]);
+                  } else {
+                    uint32_t l0, h0, l1, h1;
+                    if (ALIGNED) {
+                      const uint32_t w0 = lds32(rp + 8 * t), w1 = lds32(rp + 8 * t + 4), w2 = lds32(rp + 8 * t + 8);
+                      l0 = __funnelshift_r(w0, w1, 16), h0 = __funnelshift_r(w1, w2, 16);
+                      l1 = lds32(rp + 36 + 8 * t), h1 = lds32(rp + 40 + 8 * t);
+                      s[0][r] = lds32(rp) & 0xffffu, s[1][r] = lds32(rp + 32) >> 16;
+                    } else {
+                      l0 = lds_u16x2(rp + 2 + 8 * t), h0 = lds_u16x2(rp + 6 + 8 * t), l1 = lds_u16x2(rp + 36 + 8 * t), h1 = lds_u16x2(rp + 40 + 8 * t);
+                      s[0][r] = lds_u16x2(rp) & 0xffffu, s[1][r] = lds_u16x2(rp + 32) >> 16;
+                    }
+                    unpack_q8(l0, h0, a[0][r]), unpack_q8(l1, h1, a[1][r]);
+                  }
                 }
+                if (j + 1 >= mine) s[1][0] = s[1][1] = 0;  // no second block: stale bytes against zero fragments
+#pragma unroll
+                for (int n = 0; n < NT; n++) {
+                  float c1[2][4], c2[2][4];
+#pragma unroll
+                  for (int i = 0; i < 2; i++)
+                    mma_f16(c1[i], a[i][0][0], a[i][1][0], a[i][0][1], a[i][1][1], b[n][i].x, b[n][i].y, sd[n][i], 0.0f, sd[n][i], 0.0f);
+#pragma unroll
+                  for (int i = 0; i < 2; i++)
+                    mma_f16(c2[i], a[i][0][2], a[i][1][2], a[i][0][3], a[i][1][3], b[n][i].z, b[n][i].w, c1[i][0], c1[i][1], c1[i][2], c1[i][3]);
+#pragma unroll
+                  for (int i = 0; i < 2; i++) {
+                    const float d0 = __half2float(__ushort_as_half((unsigned short)s[i][0])), d1 = __half2float(__ushort_as_half((unsigned short)s[i][1]));
+                    acc[u][n][0] = fmaf(d0, c2[i][0], acc[u][n][0]);
+                    acc[u][n][1] = fmaf(d0, c2[i][1], acc[u][n][1]);
+                    acc[u][n][2] = fmaf(d1, c2[i][2], acc[u][n][2]);
+                    acc[u][n][3] = fmaf(d1, c2[i][3], acc[u][n][3]);
+                  }
+                }
+                r0[u] += 2 * S::BB, r1[u] += 2 * S::BB;
               }
             }
           }
           __syncwarp();
-          if (lane == 0) mbar_arrive(&empty[stage]);
-          next_stage();
+          if (lane < live) mbar_arrive(&empty[stage >= live - lane ? stage - (live - lane) : stage + S::STAGES - (live - lane)]);
           if (ok && n_red > 0) ok = mbar_wait(red_empty, (n_red - 1) & 1);
           ok = __all_sync(0xffffffffu, ok);
           n_red++;
 #pragma unroll
-          for (int n = 0; n < NT; n++) s_red[n * 32] = make_float2((acc[n][0] + acc[n][1]) * un[n], (acc[n][2] + acc[n][3]) * un[n]);
+          for (uint32_t u = 0; u < S::TILES; u++)
+#pragma unroll
+            for (int n = 0; n < NT; n++)
+              s_red[(u * NT + n) * 32] = make_float2((acc[u][n][0] + acc[u][n][1]) * un[n], (acc[u][n][2] + acc[u][n][3]) * un[n]);
           __syncwarp();
           if (lane == 0) mbar_arrive(red_full);
         }
@@ -309,15 +358,17 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
       for (uint32_t kb0 = 0; kb0 < kbt && ok; kb0 += S::RANGE) {
         const bool first = kb0 == 0, last = kb0 + S::RANGE >= kbt;
 #pragma unroll 1
-        for (uint32_t tile = t0; tile < t1 && ok; tile++) {
+        for (uint32_t first_tile = t0; first_tile < t1 && ok; first_tile += S::TILES) {
           ok = mbar_wait(red_full, n_red++ & 1) && !*s_abort;
           ok = __all_sync(0xffffffffu, ok);
 #pragma unroll
-          for (int n = 0; n < NT; n++) {
+          for (uint32_t un = 0; un < S::TILES * NT; un++) {
+            const uint32_t u = un / NT, n = un % NT, tile = first_tile + u;
+            if (tile >= t1) break;
             float2 o = make_float2(0.0f, 0.0f);
 #pragma unroll
             for (int s = 0; s < FC_WARPS; s++) {
-              const float2 v = s_red[(s * NT + n) * 32];
+              const float2 v = s_red[((s * S::TILES + u) * NT + n) * 32];
               o.x += v.x, o.y += v.y;
             }
             float2 &a = s_acc[((tile - t0) * NT + n) * 32];

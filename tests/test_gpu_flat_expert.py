@@ -33,6 +33,14 @@ def test_flat_expert_matches_the_oracle(dtype, D, F, n):
         assert np.abs(got[t] - ref).max() <= 1e-3 * np.sqrt(np.mean(ref.astype(np.float64) ** 2))
 
 
+@pytest.mark.parametrize("dtype,D,F,n", [
+    (mer_b200.DTYPE_Q4_0, 4800, 4896, 4), (mer_b200.DTYPE_Q4_0, 2560, 7168, 1), (mer_b200.DTYPE_Q8_0, 3200, 2080, 2), (mer_b200.DTYPE_Q8_0, 4864, 2560, 4)])
+def test_steps_of_two_tiles_over_several_ranges(dtype, D, F, n):
+    # up to four tokens a warp multiplies two tiles at a time: CTAs with one, two, three and more of them in either phase, ranges whose last one has
+    # a single block (K of 65 blocks) or a few, rows on and off a 16-byte boundary
+    test_flat_expert_matches_the_oracle(dtype, D, F, n)
+
+
 @pytest.mark.parametrize("dtype,D,F,n", [(mer_b200.DTYPE_Q4_0, 2048, 4096, 3), (mer_b200.DTYPE_Q8_0, 4096, 1408, 8)])
 def test_a_wait_that_runs_out_is_reported_once_and_leaves_nan(dtype, D, F, n):
     # a limit of one nanosecond: the CTAs that arrive first give up on the others
