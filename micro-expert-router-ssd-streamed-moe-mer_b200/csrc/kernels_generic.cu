@@ -427,14 +427,21 @@ __device__ void build_groups_mid(const RouterDev &r, const MoeDispatch &d, uint3
   }
   __syncthreads();
 #pragma unroll 1
-  for (uint32_t p = tid; p < P; p += 256) {
-    const uint32_t eid = __ldcg(d.pair_expert + p);
-    uint32_t v = MER_NONE;
-    if (eid != MER_NONE) {
-      const uint32_t key = eid == r.shared_expert_id || p % d.slots >= r.top_k ? r.num_experts : eid - r.id_base;
-      v = key << 16 | atomicAdd(&s_cnt[key], 1u);
+  for (uint32_t p0 = tid; p0 < P; p0 += 512) {  // two loads in flight
+    uint32_t eid[2];
+#pragma unroll
+    for (uint32_t i = 0; i < 2; i++) eid[i] = p0 + i * 256 < P ? __ldcg(d.pair_expert + p0 + i * 256) : MER_NONE;
+#pragma unroll
+    for (uint32_t i = 0; i < 2; i++) {
+      const uint32_t p = p0 + i * 256;
+      if (p >= P) break;
+      uint32_t v = MER_NONE;
+      if (eid[i] != MER_NONE) {
+        const uint32_t key = eid[i] == r.shared_expert_id || p % d.slots >= r.top_k ? r.num_experts : eid[i] - r.id_base;
+        v = key << 16 | atomicAdd(&s_cnt[key], 1u);
+      }
+      s_pair[p] = v;
     }
-    s_pair[p] = v;
   }
   __syncthreads();
   // packed: pairs (20 bits), passes (20 bits), cost; thread t owns groups t * PER_G ..
@@ -656,11 +663,27 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     uint8_t *s_ok = smem_raw + (size_t)TT * 2 * E * 4 + (size_t)warp * E;          // [E] allowed & not yet taken
     const uint32_t token = t0 + warp;
     bool bad = false;
-    for (uint32_t i = lane; i < E; i += 32) {
-      float v = direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
-      for (uint32_t z = 1; z < sets; z++) v += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i);
-      s_score[i] = v;
-      bad |= !(fabsf(v) <= FLT_MAX);
+    // the loads of a row are in flight together (one by one, a round trip to L2 per 32 experts: 3 us of 256)
+    constexpr int BATCH = EJ > 0 ? EJ : 8;
+#pragma unroll 1
+    for (uint32_t i0 = lane; i0 < E; i0 += 32 * BATCH) {
+      float v[BATCH];
+#pragma unroll
+      for (int j = 0; j < BATCH; j++) {
+        const uint32_t i = i0 + 32 * j;
+        v[j] = i >= E ? 0.0f : direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
+      }
+#pragma unroll 1
+      for (uint32_t z = 1; z < sets; z++) {
+#pragma unroll
+        for (int j = 0; j < BATCH; j++)
+          if (i0 + 32 * j < E) v[j] += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i0 + 32 * j);
+      }
+#pragma unroll
+      for (int j = 0; j < BATCH; j++) {
+        if (i0 + 32 * j < E) s_score[i0 + 32 * j] = v[j];
+        bad |= !(fabsf(v[j]) <= FLT_MAX);
+      }
     }
     // Non-finite values do not survive the split into parts (kernels_logits.cu): such a token's logits are made again in fp32.
     if (recheck && __any_sync(0xffffffffu, bad))
@@ -700,15 +723,17 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     __syncthreads();
     if (!s_last) return;
   }
-  if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);
   if constexpr (EJ > 0) {
     if (d.n_tokens == 1) {  // the picks are still in the first warp's registers
       const uint32_t eid = threadIdx.x < r.top_k ? (picked == MER_NONE ? MER_NONE : r.id_base + picked) : threadIdx.x < d.slots ? r.shared_expert_id : MER_NONE;
-      return build_groups_token(d, eid);
+      build_groups_token(d, eid);
+    } else {
+      build_groups_small(r, d);
     }
-    build_groups_small(r, d);
-  } else
+  } else {
     build_groups_layer(r, d, reinterpret_cast<uint32_t *>(smem_raw));
+  }
+  if (threadIdx.x == 0) *d.status = atomicExch(status, 0u);  // (a round trip that nobody waits for here)
 }
 
 template <int ROWS, int EJ>
@@ -733,6 +758,11 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
       if (r.correction_bias) prefetch_l2(r.correction_bias + line);
     }
     if (d.pass_desc && line / 2 < E && r.id_base + line / 2 < d.max_experts) prefetch_l2(d.expert_ptr + r.id_base + line / 2);
+  }
+  // And the router's weights, which nothing before this kernel writes: behind the norm kernel the CTAs wait here for 4 us.
+  if (tile == 0 && blockIdx.x < logit_ctas && e0 < E) {
+    const float *rows = r.w + (size_t)e0 * D;
+    for (uint32_t i = threadIdx.x * 32; i < min((uint32_t)ROWS, E - e0) * D; i += ROUTER_THREADS * 32) prefetch_l2(rows + i);
   }
   grid_dep_wait();
   grid_dep_launch();
@@ -776,14 +806,29 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
           acc[rr][tt] = fmaf(a[rr].w, b[tt].w, acc[rr][tt]);
         }
     }
+    // Sums over the warp: in each step a lane hands on half of its values, so that it ends with the sum of one (31 shuffles for 32 values instead
+    // of 160; the additions are those of warp_sum).
+    constexpr int N = ROWS * ROUTER_TT;
+    float v[N];
 #pragma unroll
-    for (int rr = 0; rr < ROWS; rr++)
+    for (int i = 0; i < N; i++) v[i] = acc[i / ROUTER_TT][i % ROUTER_TT];
+    uint32_t at = 0;
 #pragma unroll
-      for (int tt = 0; tt < ROUTER_TT; tt++) {
-        if ((uint32_t)tt >= n_here) continue;
-        float v = warp_sum(acc[rr][tt]);
-        if (lane == 0) s_part[rr][tt][warp] = v;
-      }
+    for (int step = 0; step < 5; step++) {
+      const int o = 16 >> step, n = N >> (step + 1);
+      const bool upper = lane & o;
+#pragma unroll
+      for (int i = 0; i < N / 2; i++)
+        if (i < n) {
+          const float other = __shfl_xor_sync(0xffffffffu, upper ? v[i] : v[n + i], o);
+          v[i] = (upper ? v[n + i] : v[i]) + other;
+        }
+      if (n > 0)
+        at += upper ? n : 0;
+      else
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+    if ((lane & (32 / N - 1)) == 0) (&s_part[0][0][0])[at * (ROUTER_WARPS + 1) + warp] = v[0];
     __syncthreads();
     if (threadIdx.x < ROWS * ROUTER_TT) {
       const uint32_t rr = threadIdx.x / ROUTER_TT, tt = threadIdx.x % ROUTER_TT;
