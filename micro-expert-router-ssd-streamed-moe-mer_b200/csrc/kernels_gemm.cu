@@ -161,15 +161,6 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 __device__ __forceinline__ __half2 bits_h2(uint32_t v) { return *reinterpret_cast<__half2 *>(&v); }
 
-// Two integers held as the f16 values 1024 + b (b in the low mantissa bits) -> hi = f16(d * (b - zp)),
-// lo = d * (b - zp) - hi.  Every step is exact except the rounding that defines hi.
-__device__ __forceinline__ void dq2(uint32_t biased, __half2 zp1024, __half2 d2, uint32_t &hi, uint32_t &lo) {
-  const __half2 q = __hsub2(bits_h2(biased), zp1024);
-  const __half2 h = __hmul2(d2, q);
-  hi = h2_bits(h);
-  lo = h2_bits(__hfma2(d2, q, __hneg2(h)));
-}
-
 // Token columns of a pass: its count rounded up to 16.
 __host__ __device__ constexpr uint32_t pass_width(uint32_t count) { return (count + 15u) & ~15u; }
 // A group of at most SPLIT_TOKENS tokens (always a single pass) leaves half of its accumulator buffer free: the two small
@@ -487,24 +478,28 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         for (int t = 0; t < 4; t++) w[t] = lds32(src + packed_piece(g, t) * 16 + ((blk & 1) * 2 + half) * 4);
       }
     };
-    // [0, 16): hi, values (2c, 2c+1) of the block in column c; [16, 32): lo
-    auto convert = [&](const uint32_t (&w)[RAW_WORDS], uint32_t scale, uint32_t (&v)[32]) {
-      const __half2 dd = __half2half2(half ? __high2half(bits_h2(scale)) : __low2half(bits_h2(scale)));
+    // The quants as f16 pairs, exact: column c holds values (2c, 2c+1) of the block.
+    auto integers = [&](const uint32_t (&w)[RAW_WORDS], __half2 (&q)[16]) {
 #pragma unroll
       for (int t = 0; t < 4; t++) {
         if (DT == MER_DTYPE_Q8_0) {
           const uint32_t a = w[2 * t], b = w[RAW_WORDS > 4 ? 2 * t + 1 : 0];
-          dq2(__byte_perm(a, 0x64646464u, 0x4140), zp, dd, v[4 * t + 0], v[16 + 4 * t + 0]);
-          dq2(__byte_perm(a, 0x64646464u, 0x4342), zp, dd, v[4 * t + 1], v[16 + 4 * t + 1]);
-          dq2(__byte_perm(b, 0x64646464u, 0x4140), zp, dd, v[4 * t + 2], v[16 + 4 * t + 2]);
-          dq2(__byte_perm(b, 0x64646464u, 0x4342), zp, dd, v[4 * t + 3], v[16 + 4 * t + 3]);
+          q[4 * t + 0] = __hsub2(bits_h2(__byte_perm(a, 0x64646464u, 0x4140)), zp), q[4 * t + 1] = __hsub2(bits_h2(__byte_perm(a, 0x64646464u, 0x4342)), zp);
+          q[4 * t + 2] = __hsub2(bits_h2(__byte_perm(b, 0x64646464u, 0x4140)), zp), q[4 * t + 3] = __hsub2(bits_h2(__byte_perm(b, 0x64646464u, 0x4342)), zp);
         } else {
           const uint32_t lows = w[t] & 0x0F0F0F0Fu, highs = (w[t] >> 4) & 0x0F0F0F0Fu;
-          dq2(__byte_perm(lows, 0x64646464u, 0x4140), zp, dd, v[2 * t + 0], v[16 + 2 * t + 0]);
-          dq2(__byte_perm(lows, 0x64646464u, 0x4342), zp, dd, v[2 * t + 1], v[16 + 2 * t + 1]);
-          dq2(__byte_perm(highs, 0x64646464u, 0x4140), zp, dd, v[8 + 2 * t + 0], v[24 + 2 * t + 0]);
-          dq2(__byte_perm(highs, 0x64646464u, 0x4342), zp, dd, v[8 + 2 * t + 1], v[24 + 2 * t + 1]);
+          q[2 * t] = __hsub2(bits_h2(__byte_perm(lows, 0x64646464u, 0x4140)), zp), q[2 * t + 1] = __hsub2(bits_h2(__byte_perm(lows, 0x64646464u, 0x4342)), zp);
+          q[8 + 2 * t] = __hsub2(bits_h2(__byte_perm(highs, 0x64646464u, 0x4140)), zp), q[8 + 2 * t + 1] = __hsub2(bits_h2(__byte_perm(highs, 0x64646464u, 0x4342)), zp);
         }
+      }
+    };
+    // [0, 16): hi = f16(d * q), [16, 32): lo = d * q - hi, exact
+    auto scale_up = [&](const __half2 (&q)[16], uint32_t scale, uint32_t (&v)[32]) {
+      const __half2 dd = __half2half2(half ? __high2half(bits_h2(scale)) : __low2half(bits_h2(scale)));
+#pragma unroll
+      for (int c = 0; c < 16; c++) {
+        const __half2 h = __hmul2(dd, q[c]);
+        v[c] = h2_bits(h), v[16 + c] = h2_bits(__hfma2(dd, q[c], __hneg2(h)));
       }
     };
     for (uint32_t item = item_beg; item < n_items && ok; item += item_step) {
@@ -516,13 +511,16 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         uint32_t w[RAW_WORDS], w1[RAW_WORDS], scale, scale1, v[32];
         load(tile0 + stage * RAW_BYTES, mine, w, scale);
         load(tile0 + stage * RAW_BYTES, mine + 1, w1, scale1);
-        convert(w, scale, v);
-        // The first block is converted, and the second in registers, ahead of the wait: they are then off the cycle of
-        // MMAs -> done -> store -> MMAs.
+        __half2 q0[16], q1[16];
+        integers(w, q0);
+        scale_up(q0, scale, v);
+        integers(w1, q1);
+        // The first block is converted, and the second as far as its integers, ahead of the wait: that is then off the cycle of MMAs -> done -> store
+        // -> MMAs.  (All of the second would spill; its raw words only: 536 us for 528 on 256 tokens and 8 experts of 4096 x 14336.)
 #pragma unroll
         for (int i = 0; i < 32; i++) asm volatile("" : "+r"(v[i]));
 #pragma unroll
-        for (int i = 0; i < RAW_WORDS; i++) asm volatile("" : "+r"(w1[i]));
+        for (int i = 0; i < 16; i++) asm volatile("" : "+r"(*reinterpret_cast<uint32_t *>(&q1[i])));
         asm volatile("" : "+r"(scale1));
         __syncwarp();
         if (lane == 0) mbar_arrive(&raw_empty[stage]);
@@ -537,7 +535,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         tc_fence_after();
         const uint32_t a = a_tmem + grp % A_RING * GROUP * A_STAGE_COLS;
         tc_st32(a, v);
-        convert(w1, scale1, v);
+        scale_up(q1, scale1, v);
         tc_st32(a + A_STAGE_COLS, v);
         tc_wait_st();
         tc_fence_before();
