@@ -821,10 +821,10 @@ uint32_t gemm_pick_bn(const MoeDispatch &d, uint32_t min_mean_tokens, int sm_cou
   if (mean < min_mean_tokens || P > d.scratch_pairs) return 0;
   // Passes of up to 256 tokens instead of 128 save conversions of the weights (129 to 256 tokens of an expert: half of them) and leave the MMAs idle while
   // an item's epilogue drains both buffers, some 5000 cycles.  That pays where an item's K is long and where there are enough items to
-  // share out evenly.  Us a pass, 128 / 256: 4096 tokens on 256 experts of 7168 x 2048 9516 / 8827; 2048 on 128 of 2048 x 768 (24 blocks of K
-  // in the down phase) 658 / 705; 256 on 8 of 4096 x 14336 (two items a pair of CTAs in the down phase) 690 / 720.  Beside the line of K, mean of 163 to 256 tokens: 64 experts
-  // of 4096 x 1536 1477 / 1518, of 2048 x 1536 808 / 880, 128 of 3072 x 2048 3198 / 3256, of 2048 x 2048 1611 / 1580.  Below the line of items (five to seven a pair) it
-  // depends on how the experts' tokens fill passes: 32 of 4096 x 2048, 200 tokens each, 787 / 769, with Zipf(1) routing 830 / 866; 32 of 4096 x 8192, 162 each, 2859 / 2376.
+  // share out evenly.  Us a pass, 128 / 256: 4096 tokens on 256 experts of 7168 x 2048 8490 / 8340; 2 layers of 2048 on 128 of 2048 x 768 (24 blocks of K
+  // in the down phase) 1053 / 1226; 256 on 8 of 4096 x 14336 (two items a pair of CTAs in the down phase) 528 / 582.  Beside the line of K, 200 tokens each: 64 experts
+  // of 2048 x 1536 624 / 786, of 4096 x 1536 with Zipf routing 1224 / 1300.  Below the line of items (five to seven a pair) it depends on how
+  // the experts' tokens fill passes: 2 layers of 32 of 4096 x 2048, 200 each, 1540 / 1500; 32 of 4096 x 8192, 162 each, 2590 / 2520.
   const bool long_k = d.D / 32 >= 128 && d.F / 32 >= 64, many = (uint64_t)groups * (std::min(2 * d.F, d.D) / 256) >= 8 * (uint64_t)(sm_count / PAIR);
   return long_k && many ? PASS_TOKENS : BUF_TOKENS;
 }

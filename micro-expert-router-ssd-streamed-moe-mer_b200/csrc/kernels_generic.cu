@@ -776,7 +776,9 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
     if (tt < n_here) build_x_image(d, t0 + tt, threadIdx.x, ROUTER_THREADS, &s_part[0][0][0]);
     return;
   }
-  if ((D & 1023u) == 0) {
+  // Rows of whole groups of 32 values: a slice of D / 32 groups of four for each warp, whatever that is (a warp per expert row with single loads, one token after the
+  // other: 16 tokens on 64 experts of 2816 x 1536 106 us a layer instead of 98, 7 on 16 of 736 x 992 33 instead of 30).
+  if ((D & 31u) == 0) {
     const uint32_t slice4 = D / 4 / ROUTER_WARPS;  // float4 per warp slice
     float acc[ROWS][ROUTER_TT];
 #pragma unroll
@@ -1310,7 +1312,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
     // (one token, 128 experts of 2048: 13.4 us with a row per CTA, 16.6 us with eight).
     const uint32_t tiles = (d.n_tokens + ROUTER_TT - 1) / ROUTER_TT;
     uint32_t rows = 8;
-    while (rows > 1 && d.D % 1024 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
+    while (rows > 1 && d.D % 32 == 0 && (E + rows - 1) / rows * tiles < ROUTER_CTAS) rows >>= 1;
     const uint32_t logit_ctas = (E + rows - 1) / rows;
     const dim3 grid(logit_ctas + (d.x_rows ? ROUTER_TT : 0), tiles);
     auto kern = rows == 1 ? k_router<1, 0> : rows == 2 ? k_router<2, 0> : rows == 4 ? k_router<4, 0> : k_router<8, 0>;

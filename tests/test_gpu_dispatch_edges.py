@@ -171,3 +171,26 @@ def test_a_device_payload_may_start_on_any_byte(dtype, D, F):
         got = [b.expert_forward_f32(0, e, x) for e in range(4)]
     ref = np.stack([oracle.expert_forward(dtype, blob, r, D, F) for r in x])
     assert rel_rms_err(got[0], ref) <= FFN_TOL and all(np.array_equal(got[0], g) for g in got)
+
+
+@pytest.mark.parametrize("D,E,n", [(32, 16, 1), (96, 24, 5), (736, 16, 7), (1056, 40, 3), (1280, 130, 9), (5376, 160, 17)])
+def test_router_logits_of_widths_that_are_no_multiple_of_1024(D, E, n):
+    # a warp's slice of a row is D / 32 groups of four values: fewer than its lanes, a ragged last step, many steps
+    k = 4
+    rng = np.random.default_rng([7, D, E])
+    W, x = (rng.standard_normal((E, D)) * 0.02).astype(np.float32), rng.standard_normal((n, D)).astype(np.float32)
+    stride = (256 + mer_b200.expert_bytes(mer_b200.DTYPE_Q8_0, D, 32) + 4095) // 4096 * 4096
+    with mer_b200.Backend(mer_b200.DTYPE_Q8_0, D, 32, stride, E, max_tokens=n, max_top_k=k) as b:
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        ids, w = b.route(0, x)
+    logits = x.astype(np.float64) @ W.astype(np.float64).T
+    p = np.exp(logits - logits.max(1, keepdims=True))
+    # a lane adds D / 256 products (four at a time), the warp five sums, the CTA eight: so many roundings of at most the terms' magnitude
+    err = ((D / 256 + 14) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(W).T.astype(np.float64))).max(1)
+    for t in range(n):
+        best = np.argsort(-logits[t], kind="stable")
+        if np.diff(-logits[t][best[:k + 1]]).min() <= 2 * err[t]:
+            continue  # a tie within rounding has two right answers
+        assert ids[t].tolist() == best[:k].tolist()
+        want = p[t][best[:k]] / p[t][best[:k]].sum()
+        assert (np.abs(w[t] - want) <= want * (4 * err[t] + 2e-6)).all()
