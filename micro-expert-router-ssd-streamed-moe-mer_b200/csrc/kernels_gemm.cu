@@ -1,5 +1,5 @@
 // Grouped expert FFN for token groups of a dozen tokens and more (prefill, expert-parallel decode):
-// tcgen05 tensor-core GEMM per (expert, 256 weight rows, up to 128 tokens) on pairs of CTAs, accumulators in TMEM.
+// tcgen05 tensor-core GEMM per (expert, 256 weight rows, up to 128 or 256 tokens) on pairs of CTAs, accumulators in TMEM.
 //
 //   D[256 weight rows x N tokens] += A[256 x 32] * B[N x 32]^T      per 32-value block of K
 //
@@ -196,7 +196,7 @@ template <int DT>
 __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_ffn_gemm(const GemmParams p, const __grid_constant__ ActMaps maps) {
   extern __shared__ __align__(1024) uint8_t smem[];
   constexpr uint32_t BB = DT == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
-  constexpr uint32_t TILE_RAW = RAW_BLOCKS * 16 * BB;  // bytes of RAW_BLOCKS blocks of one packed tile (2304 / 4352)
+  constexpr uint32_t TILE_RAW = RAW_BLOCKS * 16 * BB;  // bytes of RAW_BLOCKS blocks of one packed tile (1152 / 2176)
   constexpr uint32_t RAW_BYTES = 8 * TILE_RAW;
   const MoeDispatch &d = p.d;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -257,10 +257,11 @@ bool use_stream_path(mer_backend *b, const MoeDispatch &d) {
   return stream_ffn_supported(d.dtype, d.D, d.F) && b->d_stream_scratch != nullptr;
 }
 
-// Mean tokens per expert from which the tcgen05 GEMM path takes over: one line between the formats' own.  Us a layer, streaming / GEMM,
-// at means of 8, 12, 16, 20: Q8_0, 128 experts of 2048 x 768: 242 / 256, 311 / 266, 375 / 264, 469 / 283, and 64 of 2048 x 1408: 213 / 227, 266 / 229,
-// 328 / 238, 397 / 242 (they cross at 9); Q4_0, 8 of 4096 x 14336: 307 / 522, 403 / 524, 471 / 526, 594 / 526, and 64 of 7168 x 2048: 582 / 946,
-// 750 / 948, 936 / 952, 1131 / 971 (they cross at 17).
+// Mean tokens per expert from which the tcgen05 GEMM path takes over.  Us a layer, streaming / GEMM, at means of 6, 8, 10, 12, 16: Q8_0, 128 experts
+// of 2048 x 768: 182 / 201, 221 / 203, 260 / 207, 291 / 211, 340 / 215, and 64 of 2048 x 1408: 166 / 180, 209 / 182, 234 / 184, 256 / 184, 303 / 188 (they cross
+// at 7); Q4_0, 8 of 4096 x 14336: 252 / 389, 315 / 389, 356 / 389, 379 / 389, 512 / 393, and 64 of 7168 x 2048: 457 / 688, 559 / 688, 664 / 694, 758 / 698,
+// 926 / 696 (they cross at 11 to 12).  It lies at 12 for both formats because the streaming kernels' results are the more precise (largest error 3e-6 of the
+// outputs' root mean square; the GEMM's 7e-5): Q8_0 calls of 7 to 11 tokens an expert do not give that up for speed.
 constexpr uint32_t GEMM_MIN_MEAN_TOKENS = 12;
 
 // Chooses the kernel family of a dispatch and binds its scratch (call before the grouping kernel, which
