@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "../../include/mer_b200.h"
+#include "act_rows.h"
 #include "decode.cuh"
 #include "kernels.h"
 #include "layout.cuh"
@@ -57,7 +58,7 @@ constexpr uint32_t RAW_STAGES = 4;
 // CTAs' copies) and for its A stages of both CTAs (a_full: the dequantiser warps of the pair that convert it), issues the group's
 // MMAs and commits done[] in both CTAs, which releases all of it.  The barriers are counted by groups, of which no more than n_b are in flight.
 constexpr uint32_t GROUP = 4, A_RING = A_STAGES / GROUP, DONE_RING = 16, FULL_RING = 8;
-constexpr uint32_t CHUNK_K = 64, CHUNKS = GROUP * 32 / CHUNK_K;  // a row's piece of a chunk is 128 bytes, the swizzle span
+constexpr uint32_t CHUNKS = GROUP * 32 / ACT_CHUNK_K;
 constexpr uint32_t PASS_TOKENS = 256;    // tokens of a pass at most: N of one MMA
 // A pass of up to BUF_TOKENS takes one of the two accumulator buffers and one activation stage a group; a wider one takes both buffers (its MMAs then
 // wait for the epilogue of the item before) and two stages: what it saves is a second conversion of the weights.
@@ -673,16 +674,16 @@ __device__ __forceinline__ void split_values(float4 v, float sc, uint2 &hi, uint
   lo = make_uint2(h2_bits(__floats2half2_rn(a - f0.x, b - f0.y)), h2_bits(__floats2half2_rn(c - f1.x, e - f1.y)));
 }
 
-// Rows of activations -> rows of their f16 hi parts and lo parts, [hi K | lo K], after an exact power-of-two scaling of the
+// Rows of activations -> their f16 hi parts and lo parts (act_rows.h: `rows` of them), after an exact power-of-two scaling of the
 // row, and its inverse.  Row i of the output belongs to the i-th pair in group order, so that a pass is a run of rows and
 // one copy fetches a chunk of all of them.  The source is row i of h, the row of pair i's token with `perm`, or with `pos` the tokens' rows: a row is then read and
 // converted once and written to the places of all of its `slots` pairs (rows picked by the GEMM's own copies instead, four per gather, took 80 cycles per four
 // rows and doubled the GEMM's time).  TPR threads per row.  What bounds it is writing the rows.  With a row of x read and converted by each of
-// its pairs: 4096 tokens of 7168 for nine experts each 299 us.
+// its pairs: 4096 tokens of 7168 for nine experts each 299 us.  Three blocks an SM: without that bound the places' addresses take 122 registers instead of 54.
 template <int TPR, bool TOKENS>
-__global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ act, uint32_t n_rows, uint32_t K, const uint32_t *__restrict__ pos,
-                                                    const uint32_t *__restrict__ perm, uint32_t slots, const uint32_t *__restrict__ n_grouped, uint16_t *__restrict__ out,
-                                                    float *__restrict__ unscale) {
+__global__ void __launch_bounds__(256, 3) k_split_rows(const float *__restrict__ act, uint32_t n_rows, uint32_t K, const uint32_t *__restrict__ pos,
+                                                    const uint32_t *__restrict__ perm, uint32_t slots, const uint32_t *__restrict__ n_grouped, uint2 *__restrict__ out,
+                                                    uint32_t rows, float *__restrict__ unscale) {
   const uint32_t i = blockIdx.x * (256 / TPR) + threadIdx.x / TPR, t = threadIdx.x % TPR;
   const bool have = TOKENS ? i < n_rows : i < *n_grouped;  // fewer than the pairs of the dispatch under expert parallelism
   if (TPR <= 32 && !have) return;
@@ -716,11 +717,14 @@ __global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ ac
   } else if (mx != mx || isinf(mx)) {
     sc = mx;  // non-finite activations poison the row, as they would in fp32
   }
+  const size_t lo_part = act_rows_lo(rows);
   if (!TOKENS) {
     if (t == 0) unscale[i] = 1.0f / sc;
-    uint2 *hi = reinterpret_cast<uint2 *>(out + (size_t)i * 2 * K), *lo = hi + K / 4;
 #pragma unroll 4
-    for (uint32_t k = t; k < K / 4; k += TPR) split_values(__ldg(src + k), sc, hi[k], lo[k]);
+    for (uint32_t k = t; k < K / 4; k += TPR) {
+      uint2 *dst = out + act_rows_hi(rows, i, k);
+      split_values(__ldg(src + k), sc, dst[0], dst[lo_part]);
+    }
     return;
   }
   constexpr uint32_t S = 9, U = 4;  // places a pass over the row writes to; steps of it in flight
@@ -743,23 +747,21 @@ __global__ void __launch_bounds__(256) k_split_rows(const float *__restrict__ ac
         if (k >= K / 4) break;
         uint2 hi, lo;
         split_values(v[u], sc, hi, lo);
+        uint2 *first = out + act_rows_hi(rows, 0, k), *first_lo = first + lo_part;
 #pragma unroll
-        for (uint32_t j = 0; j < S; j++) {
-          if (at[j] == MER_NONE) continue;
-          uint2 *dst = reinterpret_cast<uint2 *>(out + (size_t)at[j] * 2 * K);
-          dst[k] = hi, dst[K / 4 + k] = lo;
-        }
+        for (uint32_t j = 0; j < S; j++)
+          if (at[j] != MER_NONE) first[at[j] * ACT_ROW] = hi, first_lo[at[j] * ACT_ROW] = lo;
       }
     }
   }
 }
 
 void launch_split_rows(const float *act, uint32_t n_rows, uint32_t K, const uint32_t *pos, const uint32_t *perm, uint32_t slots, const uint32_t *n_grouped,
-                       uint16_t *out, float *unscale, cudaStream_t s) {
+                       uint2 *out, uint32_t rows, float *unscale, cudaStream_t s) {
   // a warp per row keeps short rows of large batches cheap; long rows, and few of them, want more loads in flight
   const bool warps = K <= 2048 && n_rows >= 2048;
   auto kern = pos ? (warps ? k_split_rows<32, true> : k_split_rows<256, true>) : (warps ? k_split_rows<32, false> : k_split_rows<256, false>);
-  kern<<<warps ? (n_rows + 7) / 8 : n_rows, 256, 0, s>>>(act, n_rows, K, pos, perm, slots, n_grouped, out, unscale);
+  kern<<<warps ? (n_rows + 7) / 8 : n_rows, 256, 0, s>>>(act, n_rows, K, pos, perm, slots, n_grouped, out, rows, unscale);
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
@@ -774,14 +776,14 @@ EncodeTiled encode_tiled() {
   }();
   return fn;
 }
-// Rows of [hi K | lo K] f16 as (value of a chunk, row, part, chunk).  Rows past the end read as zeros.
+// Rows past the end read as zeros.
 bool activation_maps(ActMaps *maps, void *base, uint32_t rows, uint32_t K) {
   const EncodeTiled fn = encode_tiled();
   bool ok = fn != nullptr;
   for (uint32_t i = 0; i < PASS_TOKENS / 16 && ok; i++) {
-    const cuuint64_t dims[4] = {CHUNK_K, rows, 2, K / CHUNK_K}, strides[3] = {4ull * K, 2ull * K, 2 * CHUNK_K};
-    const cuuint32_t box[4] = {CHUNK_K, 8 * (i + 1), 2, CHUNKS}, step[4] = {1, 1, 1, 1};
-    ok = fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, dims, strides, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const ActMapShape a(rows, K, 8 * (i + 1), CHUNKS);
+    const cuuint32_t step[4] = {1, 1, 1, 1};
+    ok = fn(&maps->m[i], CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, base, a.dims, a.strides, a.box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   }
   return ok;
@@ -841,7 +843,7 @@ cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes,
   const uint32_t P = d.n_tokens * d.slots;
   float *unscale = reinterpret_cast<float *>(scratch);
   const size_t off = unscale_bytes(d.scratch_pairs);
-  uint16_t *rows = reinterpret_cast<uint16_t *>(static_cast<uint8_t *>(scratch) + off);
+  uint2 *rows = reinterpret_cast<uint2 *>(static_cast<uint8_t *>(scratch) + off);
   if (P > d.scratch_pairs || off + (size_t)P * (d.D > d.F ? d.D : d.F) * 4 > scratch_bytes) return cudaErrorInvalidConfiguration;
   auto kern = d.dtype == MER_DTYPE_Q4_0 ? k_ffn_gemm<MER_DTYPE_Q4_0> : k_ffn_gemm<MER_DTYPE_Q8_0>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
@@ -853,7 +855,7 @@ cudaError_t launch_ffn_gemm(MoeDispatch &d, void *scratch, size_t scratch_bytes,
     // 4096 x 1536 here: 274 us a layer by token).
     const bool by_token = phase == 0 && d.expected_pairs == 0;
     launch_split_rows(phase == 0 ? d.x : d.h, by_token ? d.n_tokens : P, K, by_token ? d.pos : nullptr, phase == 0 ? d.perm : nullptr, d.slots, d.offsets + d.n_groups, rows,
-                      unscale, s);
+                      P, unscale, s);
     ActMaps maps;
     if (!activation_maps(&maps, rows, P, K)) return cudaErrorNotSupported;
     GemmParams p{};

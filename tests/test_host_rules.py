@@ -138,3 +138,41 @@ def test_barriers_between_the_ctas_of_a_pair_name_their_scope():
     for wait, barrier in waits:
         assert wait in ({"mbar_wait_tmem", "mbar_wait_cluster"} if barrier == "done" else
                         {"mbar_wait_" + crossing[barrier]} if barrier in crossing else {"mbar_wait"}), (wait, barrier)
+
+
+ACT_SOURCE = r"""
+#include <cuda_runtime.h>
+#include "act_rows.h"
+extern "C" void act_map(uint32_t rows, uint32_t K, uint32_t box_rows, uint64_t *dims, uint64_t *strides, uint32_t *box) {
+  const ActMapShape a(rows, K, box_rows, 2);
+  for (int i = 0; i < 4; i++) dims[i] = a.dims[i], box[i] = a.box[i];
+  for (int i = 0; i < 3; i++) strides[i] = a.strides[i];
+}
+extern "C" uint64_t act_byte(uint32_t rows, uint32_t row, uint32_t k, uint32_t part) {
+  return (act_rows_hi(rows, row, k / 4) + part * act_rows_lo(rows)) * 8 + k % 4 * 2;
+}
+extern "C" uint32_t act_row() { return ACT_ROW; }
+"""
+
+
+@pytest.mark.parametrize("rows,K", [(12, 128), (33, 384), (2048 * 8, 2048), (2048 * 8, 768), (37 * 9, 14336), (4096 * 9, 7168), (65536, 16384)])
+def test_the_activations_tensor_map_is_one_of_the_documented_kind(tmp_path, rows, K):
+    # the encoder's description builds a stride from the one before it: a map whose strides fall may be refused, and the layer with it
+    src, lib = tmp_path / "act.cpp", tmp_path / "libact.so"
+    src.write_text(ACT_SOURCE)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-I", CSRC, "-I", "/usr/local/cuda/include", str(src), "-o", str(lib)])
+    r = C.CDLL(str(lib))
+    r.act_byte.restype = C.c_uint64
+    dims, strides, box = (C.c_uint64 * 4)(), (C.c_uint64 * 3)(), (C.c_uint32 * 4)()
+    for box_rows in range(8, 129, 8):
+        r.act_map(rows, K, box_rows, dims, strides, box)
+        assert list(box) == [64, box_rows, 2, 2] and box[0] * 2 <= 128 and all(1 <= b <= 256 for b in box)
+        assert dims[0] * dims[1] * dims[2] * dims[3] == 2 * rows * K and dims[1] == rows and dims[3] % 2 == 0
+        assert strides[0] == dims[0] * 2 and all(strides[i] == strides[i - 1] * dims[i] >= dims[i] for i in (1, 2))
+        assert all(s % 16 == 0 and s < 2 ** 40 for s in strides)
+    # the kernel that writes the rows puts a value where the map looks for it
+    for row in {0, 1, 7, rows // 2, rows - 1}:
+        for k in {0, 3, 63, 64, 127, K // 2, K - 1}:
+            for part in (0, 1):
+                assert r.act_byte(rows, row, k, part) == k % 64 * 2 + row * strides[0] + part * strides[1] + k // 64 * strides[2] < 4 * rows * K
+    assert r.act_row() * 8 == strides[0]
