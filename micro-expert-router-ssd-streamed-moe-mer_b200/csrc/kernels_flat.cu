@@ -2,13 +2,13 @@
 // in ONE cooperative launch (the no-allocation entry point).  HBM-bound: an expert's bytes are read once.
 //
 //   * A CTA owns whole 16-row tiles (8 gate + the 8 matching up rows, then 16 down rows) and walks K in ranges of 128 (Q4_0) or
-//     64 (Q8_0) blocks; partial tiles stay in shared memory between the ranges, so K needs no split over CTAs and no scratch.
+//     64 (Q8_0, short rows) blocks; partial tiles stay in shared memory between the ranges, so K needs no split over CTAs and no scratch.
 //   * Two producer warps copy each tile's sixteen row pieces global -> shared with bulk async copies into rows padded so that
 //     the eight rows a fragment load touches start in different banks.  A row piece that does not start on a 16-byte
 //     boundary (rows that are no multiple of 256 values) is copied from the boundary below and read with a byte shift.
-//   * Sixteen consumer warps split the range's blocks: every warp multiplies its few blocks of all tiles, two tiles at a time, with activation
+//   * Sixteen consumer warps split the range's blocks: every warp multiplies its few blocks of all tiles, mostly two tiles at a time, with activation
 //     fragments of its own (mma B fragments, f16 hi + lo after an exact power-of-two scaling of the slice), so no warp waits
-//     for another one's fragments; the values of the next range are fetched while this one is multiplied.  Integer weights become A fragments as in kernels_stream.cu; two adjacent blocks (36 or 68
+//     for another one's fragments; there the values of the next range are fetched while this one is multiplied.  Integer weights become A fragments as in kernels_stream.cu; two adjacent blocks (36 or 68
 //     bytes) are loaded as aligned 32-bit words and shifted by the two bytes of the first scale.
 //   * An epilogue warp adds the sixteen partial tiles of a step, and at the last range applies SiLU(gate) * up or stores the output.
 //   * Every wait is bounded.  A CTA whose wait ran out latches MER_DEVSTAT_TIMEOUT and stores NaN for what it has not computed: the
@@ -31,11 +31,18 @@ constexpr int FC_WARPS = 16, F_PROD = 17, F_PRODS = 2,  // warp 16 is the epilog
 constexpr uint32_t F_MAX_STAGES = 8, F_MAX_TILES = 16;  // tiles a CTA may own per phase
 constexpr size_t F_SMEM = 226 * 1024;
 
-template <int DT, int NT>
+template <int DT, int NT, bool ALIGNED, uint32_t RANGE_>
 struct Flat {
   static constexpr uint32_t BB = DT == MER_DTYPE_Q4_0 ? MER_Q4_BLOCK_BYTES : MER_Q8_BLOCK_BYTES;
-  static constexpr uint32_t TILES = NT == 1 ? 2 : 1;  // that a warp multiplies at a time (two token tiles leave room for two stages only)
-  static constexpr uint32_t RANGE = DT == MER_DTYPE_Q4_0 ? 128 : 64, PER_WARP = RANGE / FC_WARPS;
+  // A warp multiplies two tiles at a time and has the values of its next range fetched ahead, with one token tile (two leave room for two stages only), but not on
+  // Q4_0 rows off a 16-byte boundary: their shifted loads take the registers (8 bytes were spilled).  Us a call of four tokens, fragments from memory / both / neither: 4128 x
+  // 14336 57.8 / 59.7 / 55.0, 1056 x 4128 16.7 / 18.7 / 16.7, 4000 x 14304 51.2 / 49.5 / 47.5.
+  static constexpr bool BOTH = NT == 1 && (ALIGNED || DT != MER_DTYPE_Q4_0);
+  static constexpr uint32_t TILES = BOTH ? 2 : 1;
+  // A warp without a block of a short range makes no fragments (4128 x 14336 above 55.7 with them), except where the branch costs the loops more: Q4_0 on whole
+  // 16-byte boundaries (4096 x 14336 39.3, 41.2 with the branch).
+  static constexpr bool SKIP = RANGE_ == 64 || (NT == 1 && !BOTH);
+  static constexpr uint32_t RANGE = RANGE_, PER_WARP = RANGE / FC_WARPS;
   static constexpr uint32_t ROW = RANGE * BB + (DT == MER_DTYPE_Q4_0 ? 16 : 32);  // = 4 or 8 words mod 32
   static constexpr uint32_t STAGE = 16 * ROW;
   static constexpr uint32_t SEED_ROW = RANGE + 4;
@@ -120,10 +127,10 @@ __device__ __forceinline__ uint32_t lds_u16x2(uint32_t addr) {
 }
 
 // ALIGNED: every row piece starts on a 16-byte boundary (d_model and d_ff multiples of 256).
-template <int DT, int NT, bool ALIGNED>
+template <int DT, int NT, bool ALIGNED, uint32_t RANGE>
 __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
-  using S = Flat<DT, NT>;
+  using S = Flat<DT, NT, ALIGNED, RANGE>;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t = lane & 3;
   uint64_t *full = reinterpret_cast<uint64_t *>(smem), *empty = full + F_MAX_STAGES;
   uint64_t *red_full = full + 2 * F_MAX_STAGES, *red_empty = red_full + 1, *phase_ready = red_full + 2;
@@ -227,7 +234,7 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
         for (uint32_t j = 0; j < S::PER_WARP; j++)
           v[j] = tok < p.n_tokens && j < mine ? *reinterpret_cast<const float4 *>(row + j * 32) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       };
-      if (NT == 1) fetch(0, 0);
+      if (S::BOTH) fetch(0, 0);
 #pragma unroll 1
       for (uint32_t kb0 = 0; kb0 < kbt && ok; kb0 += S::RANGE) {
         uint32_t b0;
@@ -235,10 +242,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
         float un[NT];
 #pragma unroll
         for (int n = 0; n < NT; n++) {
-          if (NT > 1) fetch(kb0, n);
-          un[n] = flat_fragments<DT>(v, s_frag + n * 512, NT * 512, s_seed + (n * 4 + (g8 >> 1)) * S::SEED_ROW);
+          if (!S::BOTH) fetch(kb0, n);
+          un[n] = 0.0f;
+          if (!S::SKIP || mine > 0) un[n] = flat_fragments<DT>(v, s_frag + n * 512, NT * 512, s_seed + (n * 4 + (g8 >> 1)) * S::SEED_ROW);
         }
-        if (NT == 1 && kb0 + S::RANGE < kbt) fetch(kb0 + S::RANGE, 0);  // the next range's values arrive while this one is multiplied
+        if (S::BOTH && kb0 + S::RANGE < kbt) fetch(kb0 + S::RANGE, 0);  // the next range's values arrive while this one is multiplied
 #pragma unroll 1
         for (uint32_t tile = t0; tile < t1; tile += S::TILES) {
           const uint32_t live = min(S::TILES, t1 - tile);
@@ -427,11 +435,11 @@ __global__ void __launch_bounds__(F_THREADS, 1) k_flat_expert(const FlatParams p
   }
 }
 
-template <int DT, int NT, bool ALIGNED>
+template <int DT, int NT, bool ALIGNED, uint32_t RANGE>
 cudaError_t launch_flat(FlatParams p, int sm_count, cudaStream_t s) {
-  using S = Flat<DT, NT>;
+  using S = Flat<DT, NT, ALIGNED, RANGE>;
   if ((p.F / 8 + sm_count - 1) / sm_count > F_MAX_TILES || (p.D / 16 + sm_count - 1) / sm_count > F_MAX_TILES) return cudaErrorNotSupported;
-  auto kern = k_flat_expert<DT, NT, ALIGNED>;
+  auto kern = k_flat_expert<DT, NT, ALIGNED, RANGE>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
   if (e != cudaSuccess) return e;
   void *args[] = {&p};
@@ -440,8 +448,12 @@ cudaError_t launch_flat(FlatParams p, int sm_count, cudaStream_t s) {
 template <int DT>
 cudaError_t launch_flat_dt(const FlatParams &p, int sm_count, cudaStream_t s) {
   const bool aligned = p.D % 256 == 0 && p.F % 256 == 0;
-  if (p.n_tokens > 4) return aligned ? launch_flat<DT, 2, true>(p, sm_count, s) : launch_flat<DT, 2, false>(p, sm_count, s);
-  return aligned ? launch_flat<DT, 1, true>(p, sm_count, s) : launch_flat<DT, 1, false>(p, sm_count, s);
+  constexpr uint32_t RANGE = DT == MER_DTYPE_Q4_0 ? 128 : 64;
+  if (p.n_tokens > 4) return aligned ? launch_flat<DT, 2, true, RANGE>(p, sm_count, s) : launch_flat<DT, 2, false, RANGE>(p, sm_count, s);
+  if (!aligned) return launch_flat<DT, 1, false, RANGE>(p, sm_count, s);
+  // One range of at most 64 blocks: half the values a warp holds for 128, and no more tiles than CTAs to speak of.  Us a call of one token, ranges of 128 / 64:
+  // 2048 x 768 12.6 / 10.6 (10.6 with fragments from memory), 1024 x 1024 11.6 / 10.6, 2048 x 1536 12.6 / 11.6, 2048 x 2048 12.6 both.
+  return std::max(p.D, p.F) <= 2048 ? launch_flat<DT, 1, true, 64>(p, sm_count, s) : launch_flat<DT, 1, true, RANGE>(p, sm_count, s);
 }
 
 }  // namespace

@@ -62,3 +62,12 @@ def test_a_wait_that_runs_out_is_reported_once_and_leaves_nan(dtype, D, F, n):
     mer_b200.expert_noalloc_check(stream)
     ref = np.stack([oracle.expert_forward(dtype, blob, r, D, F) for r in x])
     assert np.abs(d_out.cpu().numpy() - ref).max() <= 1e-3 * np.sqrt(np.mean(ref.astype(np.float64) ** 2))
+
+
+@pytest.mark.parametrize("n", [1, 4, 5, 8])
+@pytest.mark.parametrize("dtype,D,F", [(mer_b200.DTYPE_Q4_0, 4128, 1056), (mer_b200.DTYPE_Q4_0, 1056, 4128), (mer_b200.DTYPE_Q8_0, 2080, 2336), (mer_b200.DTYPE_Q8_0, 512, 2304),
+                                       (mer_b200.DTYPE_Q4_0, 256, 256), (mer_b200.DTYPE_Q4_0, 2048, 2048), (mer_b200.DTYPE_Q4_0, 2048, 2304), (mer_b200.DTYPE_Q4_0, 2304, 512)])
+def test_ranges_that_leave_warps_without_a_block(dtype, D, F, n):
+    # a last range of one block (129 of Q4_0, 65 of Q8_0), of a few, and first ones of 33 or 16: the other warps make no fragments and add zeros,
+    # whatever the range before left them; Q4_0 rows off a 16-byte boundary take one tile at a time, those of up to 2048 values ranges of 64 blocks
+    test_flat_expert_matches_the_oracle(dtype, D, F, n)
