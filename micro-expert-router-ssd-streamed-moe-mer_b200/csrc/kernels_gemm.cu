@@ -455,6 +455,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
     const uint32_t q = warp & 3, team = (warp - W_DQ0) >> 2 & 1, mine = (warp - W_DQ0) >> 3 << 1;  // quarter of the rows; first of the two blocks
     const uint32_t T = 2 * q + (lane >> 4), g = lane & 7, half = (lane >> 3) & 1;
     const __half2 zp = DT == MER_DTYPE_Q4_0 ? __floats2half2_rn(1032.0f, 1032.0f) : __floats2half2_rn(1152.0f, 1152.0f);
+    constexpr bool EARLY = DT == MER_DTYPE_Q4_0;  // the second block's integers ahead of the wait
     constexpr int RAW_WORDS = DT == MER_DTYPE_Q4_0 ? 4 : 8;
     uint32_t groups = 0;  // groups of blocks before this item
     bool ready = false;   // the weight stage has been seen full
@@ -515,13 +516,16 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         __half2 q0[16], q1[16];
         integers(w, q0);
         scale_up(q0, scale, v);
-        integers(w1, q1);
-        // The first block is converted, and the second as far as its integers, ahead of the wait: that is then off the cycle of MMAs -> done -> store
-        // -> MMAs.  (All of the second would spill; its raw words only: 536 us for 528 on 256 tokens and 8 experts of 4096 x 14336.)
+        if (EARLY) integers(w1, q1);
+        // The first block is converted, and the second as far as registers go, ahead of the wait: that is then off the cycle of MMAs -> done -> store
+        // -> MMAs.  Q4_0: its integers (its raw words only: 536 us for 528 on 256 tokens and 8 experts of 4096 x 14336).  Q8_0: its raw words (its integers
+        // spill 8 bytes: 256 tokens on 128 experts of 2048 x 768 209 us for 205, on 64 of 2048 x 1408 195 for 193).
 #pragma unroll
         for (int i = 0; i < 32; i++) asm volatile("" : "+r"(v[i]));
 #pragma unroll
-        for (int i = 0; i < 16; i++) asm volatile("" : "+r"(*reinterpret_cast<uint32_t *>(&q1[i])));
+        for (int i = 0; i < (EARLY ? 16 : 0); i++) asm volatile("" : "+r"(*reinterpret_cast<uint32_t *>(&q1[i])));
+#pragma unroll
+        for (int i = 0; i < (EARLY ? 0 : RAW_WORDS); i++) asm volatile("" : "+r"(w1[i]));
         asm volatile("" : "+r"(scale1));
         __syncwarp();
         if (lane == 0) mbar_arrive(&raw_empty[stage]);
@@ -536,6 +540,7 @@ __global__ void __cluster_dims__(PAIR, 1, 1) __launch_bounds__(G_THREADS, 1) k_f
         tc_fence_after();
         const uint32_t a = a_tmem + grp % A_RING * GROUP * A_STAGE_COLS;
         tc_st32(a, v);
+        if (!EARLY) integers(w1, q1);
         scale_up(q1, scale1, v);
         tc_st32(a + A_STAGE_COLS, v);
         tc_wait_st();
