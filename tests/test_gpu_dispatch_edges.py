@@ -194,3 +194,38 @@ def test_router_logits_of_widths_that_are_no_multiple_of_1024(D, E, n):
         assert ids[t].tolist() == best[:k].tolist()
         want = p[t][best[:k]] / p[t][best[:k]].sum()
         assert (np.abs(w[t] - want) <= want * (4 * err[t] + 2e-6)).all()
+
+
+@pytest.mark.parametrize("D,E,n", [
+    (1056, 128, 40), (736, 160, 24), (2848, 24, 300),                    # four expert rows a CTA, slices that end short of a warp, or of several
+    (1056, 128, 80), (736, 160, 100), (5376, 160, 100), (2848, 24, 400),  # eight
+])
+def test_router_logits_of_several_rows_a_cta(D, E, n):
+    k = 4
+    rng = np.random.default_rng([8, D, E, n])
+    W, x = (rng.standard_normal((E, D)) * 0.02).astype(np.float32), rng.standard_normal((n, D)).astype(np.float32)
+    bad = [1, 6, n // 2, n - 1]  # a NaN, infinities: their own rows only
+    x_bad = x.copy()
+    x_bad[bad[0], D - 1], x_bad[bad[1], 0], x_bad[bad[2], D // 2], x_bad[bad[3], 33] = np.nan, np.inf, -np.inf, np.nan
+    stride = (256 + mer_b200.expert_bytes(mer_b200.DTYPE_Q8_0, D, 32) + 4095) // 4096 * 4096
+    with mer_b200.Backend(mer_b200.DTYPE_Q8_0, D, 32, stride, 2 * E, max_tokens=n, max_top_k=k) as b:
+        mer_b200.LinearGate(W, E, D, k).bind(b, 0)
+        ids, w = b.route(0, x)
+        mer_b200.LinearGate.with_routing(W, E, D, k, 1, True, None, 1, 1, 1.0).bind(b, 1)  # sigmoid: the softmax of a NaN is an error
+        clean, mixed = b.route(1, x), b.route(1, x_bad)
+        alone = [b.route(1, x_bad[t:t + 1]) for t in bad]
+    good = np.setdiff1d(np.arange(n), bad)
+    assert (clean[0][good] == mixed[0][good]).all() and (clean[1][good] == mixed[1][good]).all()
+    for t, (i1, w1) in zip(bad, alone):
+        assert np.array_equal(np.sort(mixed[0][t]), np.sort(i1[0])) and np.allclose(np.sort(mixed[1][t]), np.sort(w1[0]), rtol=1e-5, equal_nan=True)
+    logits = x.astype(np.float64) @ W.astype(np.float64).T
+    p = np.exp(logits - logits.max(1, keepdims=True))
+    # the roundings of the test above
+    err = ((D / 256 + 14) * 2.0 ** -24 * (np.abs(x).astype(np.float64) @ np.abs(W).T.astype(np.float64))).max(1)
+    best = np.argsort(-logits, axis=1, kind="stable")
+    clear = np.diff(-np.take_along_axis(logits, best[:, :k + 1], 1), axis=1).min(1) > 2 * err
+    assert clear.mean() > 0.8  # of the others, ties within rounding, either answer is right
+    assert (ids[clear] == best[clear, :k]).all()
+    want = np.take_along_axis(p, best[:, :k], 1)
+    want /= want.sum(1, keepdims=True)
+    assert (np.abs(w - want) <= want * (4 * err[:, None] + 2e-6))[clear].all()
