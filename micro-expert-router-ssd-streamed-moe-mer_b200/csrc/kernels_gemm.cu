@@ -24,9 +24,9 @@
 // ones.  A group of four blocks takes 1050 cycles on a pass of 32 tokens (1750 before) and 1150 on one of 80; the MMAs of N columns N / 2 each,
 // 24 a group, so 380 and 960 (alone, with A in tensor memory, they run at that rate for every N, whatever else uses tensor or shared memory).  The
 // rest is the cycle MMAs -> done -> store -> arrival at the issuer of the other CTA, 2000 cycles of which two are in flight.
-// Us a pass, before and after uniform operands, one activation copy a group, two weight producers and two teams of dequantisers: 256 tokens on 8
-// experts of 4096 x 14336 594 / 524, 2 layers of 2048 on 128 of 2048 x 768 1097 / 1050, 4096 on 256 of 7168 x 2048 8680 / 8240.
-// Tried without gain: one MMA for hi * [hi | lo] of passes up to 32 tokens, the conversion of both blocks ahead of the wait (spills),
+// Us a pass, L2 flushed, without uniform operands, one activation copy a group, two weight producers and two teams of dequantisers / now, one box: 256 tokens on 8
+// experts of 4096 x 14336 689 / 624, 2 layers of 2048 on 128 of 2048 x 768 1284 / 1214; 4096 on 256 of 7168 x 2048, at the power limit, 8565 / 8524: even.
+// Tried without gain: one MMA for hi * [hi | lo] of passes up to 32 tokens, the conversion of both blocks ahead of the wait (spills: 531 / 522),
 // commits or groups of two blocks, fewer instructions in the conversion, a look at the issuer's next barrier ahead.
 // Every wait is bounded; on expiry the CTA latches MER_DEVSTAT_TIMEOUT, stops issuing work, waits
 // (bounded) for its copies and MMAs in flight, frees its TMEM and returns.
