@@ -10,6 +10,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cfloat>
 
 #include "../../include/mer_b200.h"
@@ -646,10 +647,10 @@ __device__ __noinline__ void count_picks(const RouterDev &r, const MoeDispatch &
 }
 
 // Selection for the TT tokens from t0 on, whose logits are there, one warp per token; the last of `n_tiles` CTAs that get here groups all pairs.
-// `direct`: the logits [TT][stride] in shared memory, or null: `sets` partial sums of them in d.logits ([sets][T][E], added in order).
+// `direct`: the logits [TT][stride] in shared memory, or null: in d.logits, with PARTS as `sets` partial sums ([sets][T][E], added in order).
 // EJ > 0: at most 32 EJ experts and 32 pairs of the streaming kernels, with no other code in the kernel: it runs once a layer, cold, and what a call of one
 // token waits for is its instructions (one token on 128 experts of 2048 x 768: 1 us a layer).
-template <int TT, int EJ>
+template <int TT, int EJ, bool PARTS>
 __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispatch &d, uint32_t t0, uint32_t n_tiles, const float *direct, uint32_t stride, uint32_t sets,
                                               bool recheck, uint8_t *smem_raw, uint32_t *status, uint32_t max_tokens, int group_here) {
   const uint32_t E = r.num_experts, D = d.D, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -663,28 +664,46 @@ __device__ __forceinline__ void finish_tokens(const RouterDev &r, const MoeDispa
     uint8_t *s_ok = smem_raw + (size_t)TT * 2 * E * 4 + (size_t)warp * E;          // [E] allowed & not yet taken
     const uint32_t token = t0 + warp;
     bool bad = false;
-    // the loads of a row are in flight together (one by one, a round trip to L2 per 32 experts: 3 us of 256)
-    constexpr int BATCH = EJ > 0 ? EJ : 8;
+    // The loads of a row are in flight together (one by one, a round trip to L2 per 32 experts: 3 us of 256).  Up to 32 experts have one value a lane: there
+    // AHEAD partial sums are (set by set, 4097 tokens on 8 experts of 512 x 512 94.3 us a layer instead of 88.5, 600 on 32 of 7168 173.5 instead of 171).
+    auto gather = [&](auto batch_tag, auto ahead_tag) {
+      constexpr int BATCH = decltype(batch_tag)::value;
 #pragma unroll 1
-    for (uint32_t i0 = lane; i0 < E; i0 += 32 * BATCH) {
-      float v[BATCH];
+      for (uint32_t i0 = lane; i0 < E; i0 += 32 * BATCH) {
+        float v[BATCH];
 #pragma unroll
-      for (int j = 0; j < BATCH; j++) {
-        const uint32_t i = i0 + 32 * j;
-        v[j] = i >= E ? 0.0f : direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
-      }
+        for (int j = 0; j < BATCH; j++) {
+          const uint32_t i = i0 + 32 * j;
+          v[j] = i >= E ? 0.0f : direct ? direct[warp * stride + i] : __ldcg(d.logits + (size_t)token * E + i);
+        }
+        if constexpr (PARTS) {
+          constexpr int AHEAD = decltype(ahead_tag)::value;
 #pragma unroll 1
-      for (uint32_t z = 1; z < sets; z++) {
+          for (uint32_t z0 = 1; z0 < sets; z0 += AHEAD) {
+            float part[AHEAD][BATCH];
 #pragma unroll
-        for (int j = 0; j < BATCH; j++)
-          if (i0 + 32 * j < E) v[j] += __ldcg(d.logits + ((size_t)z * d.n_tokens + token) * E + i0 + 32 * j);
-      }
+            for (int z = 0; z < AHEAD; z++)
 #pragma unroll
-      for (int j = 0; j < BATCH; j++) {
-        if (i0 + 32 * j < E) s_score[i0 + 32 * j] = v[j];
-        bad |= !(fabsf(v[j]) <= FLT_MAX);
+              for (int j = 0; j < BATCH; j++)
+                part[z][j] = z0 + z < sets && i0 + 32 * j < E ? __ldcg(d.logits + ((size_t)(z0 + z) * d.n_tokens + token) * E + i0 + 32 * j) : 0.0f;
+#pragma unroll
+            for (int z = 0; z < AHEAD; z++)
+#pragma unroll
+              for (int j = 0; j < BATCH; j++)
+                if (z0 + z < sets) v[j] += part[z][j];
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < BATCH; j++) {
+          if (i0 + 32 * j < E) s_score[i0 + 32 * j] = v[j];
+          bad |= !(fabsf(v[j]) <= FLT_MAX);
+        }
       }
-    }
+    };
+    if (PARTS && E <= 32)
+      gather(std::integral_constant<int, 1>{}, std::integral_constant<int, 4>{});
+    else
+      gather(std::integral_constant<int, EJ == 0 ? 8 : EJ>{}, std::integral_constant<int, 1>{});
     // Non-finite values do not survive the split into parts (kernels_logits.cu): such a token's logits are made again in fp32.
     if (recheck && __any_sync(0xffffffffu, bad))
 #pragma unroll 1
@@ -874,7 +893,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router(RouterDev r, MoeDispa
   }
 
   // ---- this CTA holds the last logits of the token tile
-  finish_tokens<ROUTER_TT, EJ>(r, d, t0, gridDim.y, single ? &s_logit[0][0] : nullptr, ROWS, 1, false, smem_raw, status, max_tokens, group_here);
+  finish_tokens<ROUTER_TT, EJ, false>(r, d, t0, gridDim.y, single ? &s_logit[0][0] : nullptr, ROWS, 1, false, smem_raw, status, max_tokens, group_here);
 }
 
 // The same behind the logits kernel of a large batch: every warp has a token.  (In the kernel above, whose registers leave room for two CTAs on an SM,
@@ -888,7 +907,7 @@ __global__ void __launch_bounds__(ROUTER_THREADS) k_router_select(const __grid_c
     return;
   }
   uint32_t *const status = group_here ? d.counters + max_tokens + 1 : d.status;
-  finish_tokens<TT, 0>(r, d, blockIdx.x * TT, select_ctas, nullptr, 0, sets, recheck != 0, smem_raw, status, max_tokens, group_here);
+  finish_tokens<TT, 0, true>(r, d, blockIdx.x * TT, select_ctas, nullptr, 0, sets, recheck != 0, smem_raw, status, max_tokens, group_here);
 }
 
 // Routing of a whole layer supplied by the caller (pair_expert already filled): group by expert.  The first CTA; the others make the activation images.
