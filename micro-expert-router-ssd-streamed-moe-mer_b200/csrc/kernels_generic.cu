@@ -1315,10 +1315,11 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   cudaError_t e;
   // From a few hundred tokens the logits are a GEMM of their own, unless the experts are so few that most of a tile would be
   // padding (8 experts, 256 tokens of 4096: 19 us of logits kernel).  Up to 16 experts, rows of whole 1024 values never go there.  Others did while the vector code
-  // took whole 1024 only; now those go that are more than VECTOR_CTAS of its CTAs.  Us of a route call, GEMM / vector, 8 experts and 256 tokens of 2816 31 / 17, 8 and
-  // 4096 (1024 CTAs) of 1280 38 / 29, 16 and 2048 (1024) of 1280 32 / 31, of 5376 45 / 42, 12 and 2730 (1366) of 1280 30 / 36, of 5376 64 / 49, 4 and 8192 (2048) of 1280
-  // 38 / 43, 16 and 4096 (2048) of 2816 45 / 49, of 5376 60 / 78.  The vector code's weights are the nearer to 64 bits (rms 0.7 to 2.1e-7 for 0.8 to 2.5e-7).
-  constexpr uint32_t VECTOR_CTAS = 1024;
+  // took whole 1024 only; now those go that are more than VECTOR_CTAS of its CTAs.  Us a layer, GEMM / vector, 8 experts and 256 tokens of 2816 63 / 52, of 7936 139 / 91,
+  // 8 and 2048 (512 CTAs) of 1280 97 / 87, of 6400 239 / 214, 16 and 1024 (512) of 1280 80 / 68, of 5376 143 / 141; beyond the line 8 and 2900 (725) of 1280 116 / 123, of
+  // 5376 280 / 285, 16 and 2048 (1024) of 1280 103 / 103, 8 and 4096 (1024) of 512 72 / 78.  The vector code's weights are the nearer to 64 bits (rms 0.7 to 2.1e-7 for
+  // 0.8 to 2.5e-7).
+  constexpr uint32_t VECTOR_CTAS = 512;
   const uint64_t vector_ctas = (uint64_t)((E + 7) / 8) * ((d.n_tokens + ROUTER_TT - 1) / ROUTER_TT);
   if (d.n_tokens >= 256 && d.D % 256 == 0 && (E > 16 || (d.D % 1024 != 0 && vector_ctas > VECTOR_CTAS))) {
     uint32_t sets = 1;
