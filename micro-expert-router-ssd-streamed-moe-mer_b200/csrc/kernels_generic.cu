@@ -1297,6 +1297,14 @@ __global__ void k_f32_to_f16(const float *__restrict__ src, uint16_t *__restrict
   if (i < n) dst[i] = __half_as_ushort(__float2half_rn(src[i]));
 }
 
+// A kernel's dynamic shared memory needs leave where it and the kernel's own tables are more than 48 KB together; the routing and grouping kernels have up to 18 KB of
+// tables.  (Asked for from 48 KB of dynamic memory on, calls of 438 to 682 experts and 256 tokens, or of 900 to 1365 and a few, failed to launch.)
+constexpr size_t TABLE_BYTES = 20 * 1024;
+template <class Kernel>
+cudaError_t allow_smem(Kernel kern, size_t smem) {
+  return smem + TABLE_BYTES > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+}
+
 }  // namespace
 
 
@@ -1309,7 +1317,7 @@ cudaError_t launch_router(const RouterDev &r, const MoeDispatch &d, uint32_t max
   const int group_here = group && d.route_here ? ROUTE_LATER : grid_grouping ? 2 : group ? 1 : 0;
   auto room = [&](auto kern, uint32_t tokens, size_t &smem) -> cudaError_t {
     smem = (std::max((size_t)tokens * E * 9, group_here == 1 ? smem_grp : (size_t)0) + 15) & ~(size_t)15;
-    return smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
+    return allow_smem(kern, smem);
   };
   size_t smem;
   cudaError_t e;
@@ -1372,10 +1380,8 @@ cudaError_t launch_groups_layer(const RouterDev &r, const MoeDispatch &d, cudaSt
   }
   size_t smem = (size_t)(G + 1 + (G <= STABLE_G ? ROUTER_WARPS * G : G) + (P <= SMALL_P ? P : 0)) * 4;
   smem = (smem + 15) & ~(size_t)15;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_groups_layer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  const cudaError_t e = allow_smem(k_groups_layer, smem);
+  if (e != cudaSuccess) return e;
   k_groups_layer<<<d.x_rows ? 1 + d.n_tokens : 1, ROUTER_THREADS, smem, s>>>(r, d);
   if (launches) (*launches)++;
   return cudaGetLastError();

@@ -201,6 +201,7 @@ def test_router_logits_of_widths_that_are_no_multiple_of_1024(D, E, n):
     (1056, 128, 80), (736, 160, 100), (5376, 160, 100), (2848, 24, 400),  # eight
     (1280, 8, 2048), (1280, 8, 2049), (1280, 12, 1030), (2816, 16, 1024), (2816, 16, 1025), (2816, 3, 256),  # few experts: 512 CTAs, and the GEMM behind
     (7168, 32, 600), (4096, 32, 300), (4096, 33, 300),  # partial sums of up to 32 experts, a value a lane, and of more
+    (256, 437, 256), (256, 512, 256), (256, 683, 256), (64, 1000, 9), (64, 1366, 8),  # shared memory with the kernels' tables on either side of 48 KB
 ])
 def test_router_logits_of_several_rows_a_cta(D, E, n):
     k = min(4, E // 2) if E > 3 else 2
