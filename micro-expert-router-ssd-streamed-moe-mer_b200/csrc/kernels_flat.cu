@@ -40,8 +40,8 @@ struct Flat {
   static constexpr bool BOTH = NT == 1 && (ALIGNED || DT != MER_DTYPE_Q4_0);
   static constexpr uint32_t TILES = BOTH ? 2 : 1;
   // A warp without a block of a short range makes no fragments (4128 x 14336 above 55.7 with them), except where the branch costs the loops more: Q4_0 on whole
-  // 16-byte boundaries (4096 x 14336 39.3, 41.2 with the branch).
-  static constexpr bool SKIP = RANGE_ == 64 || (NT == 1 && !BOTH);
+  // 16-byte boundaries (4096 x 14336 39.3, 41.2 with the branch), and two token tiles (Q8_0, six tokens and 1792 x 3072 17.9, 18.3 with it).
+  static constexpr bool SKIP = NT == 1 && (RANGE_ == 64 || !BOTH);
   static constexpr uint32_t RANGE = RANGE_, PER_WARP = RANGE / FC_WARPS;
   static constexpr uint32_t ROW = RANGE * BB + (DT == MER_DTYPE_Q4_0 ? 16 : 32);  // = 4 or 8 words mod 32
   static constexpr uint32_t STAGE = 16 * ROW;
